@@ -186,8 +186,8 @@ def _params(case):
     return SimulationParams(
         radius=case.get("radius", 0.1), delta_t=case.get("dt", 0.18 if app else 0.01), friction=0.51,
         repulsion=64.83, attraction=3.06, k=29.45, balance=0.79, canvas_width=case["extent"],
-        canvas_height=case["extent"], canvas_depth=case["extent"], num_particle_types=case["types"], ratio_with_lfo=case.get("ratio", 0.0), force_multiplier=2.33,
-        max_expected_neighbors=400)
+        canvas_height=case["extent"], canvas_depth=case["extent"], num_particle_types=case["types"],
+        ratio_with_lfo=case.get("ratio", 0.0), force_multiplier=2.33, max_expected_neighbors=400)
 
 
 class _DeviceArray:
