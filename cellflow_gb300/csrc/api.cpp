@@ -396,6 +396,8 @@ int sync_and_check(cf_world* w)
 // Pair tables for a step (ParticleSimulation.cu:108-110, 116): effective
 // radius per type pair in the reference's float expression, the exact
 // sqrt threshold, and the force table; uploaded when anything changed.
+float filter_bound(float thr_max, float max_extent);
+
 int update_pair_tables(cf_world* w, const cf_step_params* p, float* r_cut, int* uniform_r, float* eff_u,
                        float* thr_u, float* thr_max_out)
 {
@@ -410,7 +412,10 @@ int update_pair_tables(cf_world* w, const cf_step_params* p, float* r_cut, int* 
         std::fill(std::begin(h.eff), std::end(h.eff), 0.0f);
         std::fill(std::begin(h.threshold), std::end(h.threshold), 0.0f);
         std::fill(std::begin(h.threshold_lo), std::end(h.threshold_lo), 0.0f);
+        std::fill(std::begin(h.filter_row), std::end(h.filter_row), 0.0f);
+        double band = 0.0;
         for (int a = 0; a < T; a++) {
+            float row_max = 0.0f;
             for (int b = 0; b < T; b++) {
                 const float ra = p->radius * (1.0f + w->radio[a] * p->ratio_with_lfo);
                 const float rb = p->radius * (1.0f + w->radio[b] * p->ratio_with_lfo);
@@ -420,8 +425,17 @@ int update_pair_tables(cf_world* w, const cf_step_params* p, float* r_cut, int* 
                 h.eff[k] = eff;
                 h.threshold[k] = sqrt_threshold(eff);
                 h.threshold_lo[k] = certain_bound(h.threshold[k], max_ext);
+                h.force_compact[a * T + b] = h.force[k];
+                h.pair_compact[a * T + b] = make_float2(1.0f / eff, h.threshold_lo[k]);
+                row_max = std::max(row_max, h.threshold[k]);
+                if (!std::isinf(h.threshold[k]))
+                    band = std::max(band, (double)filter_bound(h.threshold[k], max_ext) - (double)h.threshold_lo[k]);
             }
+            h.filter_row[a] = filter_bound(row_max, max_ext);
         }
+        // rounded up past the rounding of threshold_lo + band in the kernel
+        const double most = (double)filter_bound(*std::max_element(std::begin(h.threshold), std::end(h.threshold)), max_ext);
+        w->band = nextafterf((float)(band + (std::isinf(most) ? 0.0 : 0x1p-22 * std::max(most, 0.0))), INFINITY);
         CF_CUDA(cudaMemcpyAsync(w->tables, &h, sizeof(PairTables), cudaMemcpyHostToDevice, w->stream));
         w->uploaded_version = w->table_version;
         w->uploaded_radius = p->radius;
@@ -512,19 +526,21 @@ int prepare_step(cf_world* w, const cf_step_params* p, StepConsts* c)
     for (int a = 0; a < 3; a++) c->half[a] = c->ext[a] * 0.5f;
     c->inv_eff_uniform = 1.0f / c->eff_uniform;
     c->thr_lo_uniform = w->host_tables.threshold_lo[0];
-    if (w->force_variant < kForceStages * 3) {
-        c->variant = w->force_variant % kForceStages;
-        c->split = 1 << (w->force_variant / kForceStages);
-    } else {
-        // the balanced drain (staging 4): variants 12, 13, 14 for 1, 2, 4 warps per item
-        c->variant = kForceStages;
-        c->split = 1 << (w->force_variant - kForceStages * 3);
-    }
+    c->band = w->band;
+    c->thr_hi_uniform = c->thr_lo_uniform + c->band;
+    c->neg_k_log2e = -p->k * 1.4426950408889634f;
+    c->c1_uniform = c->neg_k_log2e * c->inv_eff_uniform * c->inv_eff_uniform;
+    c->att_uniform = p->attraction * c->inv_eff_uniform;
+    c->integrate_apart = integrate_apart(w->n) ? 1 : 0;
     c->thr_filter = filter_bound(thr_max, std::max(c->ext[0], std::max(c->ext[1], c->ext[2])));
     c->grid = choose_step_grid(c->ext, r_cut, kMaxCells);
     apply_worlds(c->grid, w->worlds);
+    const int variant = w->force_variant >= 0 ? w->force_variant : default_force_variant(w->n, c->grid);
+    c->variant = variant % kForceOccupancies;
+    c->split = 1 << (variant / kForceOccupancies);
+    for (int a = 0; a < 3; a++) c->cell[a] = c->ext[a] / (float)c->grid.m[a];
     // force tables: one per world (a plain world uses the pair tables' own)
-    c->world_force = w->worlds > 1 ? w->world_tables : w->tables->force;
+    c->world_force = w->worlds > 1 ? w->world_tables : w->tables->force_compact;
     c->n = w->n;
     c->num_types = w->num_types;
     c->repulsion = p->repulsion;
@@ -565,7 +581,7 @@ int enqueue_cell_list(cf_world* w, const StepConsts& c, int* which)
 int enqueue_force(cf_world* w, const StepConsts& c, int which)
 {
     Scratch& s = w->s;
-    CF_CUDA(launch_step_force(c, w->tables, s.pos_sorted, s.keys[which], s.vals[which], s.cell_off, s.items,
+    CF_CUDA(launch_step_force(c, w->tables, s.pos_sorted, s.vals[which], s.cell_off, s.items,
                               s.n_items, max_step_items(w->n, c.grid), w->pos, w->vel, w->acc, w->counts,
                               w->stream));
     return CF_OK;
@@ -1509,7 +1525,15 @@ int cf_autotune_step(cf_world* w, const cf_step_params* p, int steps, int* chose
     cudaError_t e = cudaEventCreate(&e0);
     if (!e) e = cudaEventCreate(&e1);
     if (!e) e = save(true);
+    float split_ms = 1e30f;  // the fastest variant of the current split (warps per item)
     for (int k = 0; k < CF_FORCE_VARIANTS && !e && rc == CF_OK; k++) {
+        if (k % kForceOccupancies == 0) {
+            // twice the warps gained nothing: more will not either
+            if (k > 0 && split_ms > 1.25f * best_ms) break;
+            split_ms = 1e30f;
+        } else if (k >= 3 * kForceOccupancies) {
+            continue;  // one kernel for 8 warps per item, and one for 16
+        }
         w->force_variant = k;
         rc = cf_step(w, p, 1);  // capture and warm
         if (rc) break;
@@ -1519,6 +1543,7 @@ int cf_autotune_step(cf_world* w, const cf_step_params* p, int steps, int* chose
         if (!e && !rc) e = cudaEventSynchronize(e1);
         float ms = 0.0f;
         if (!e && !rc) e = cudaEventElapsedTime(&ms, e0, e1);
+        if (!e && !rc) split_ms = std::min(split_ms, ms);
         if (!e && !rc && ms < best_ms) {
             best_ms = ms;
             best = k;
@@ -2047,14 +2072,14 @@ int cf_batch_create(int worlds, const int* n_per_world, int num_types, float w_,
     w->worlds = worlds;
     w->world_off.assign(worlds + 1, 0);
     for (int k = 0; k < worlds; k++) w->world_off[k + 1] = w->world_off[k] + n_per_world[k];
-    cudaError_t e = dev_alloc(&w->world_tables, (size_t)worlds * kTableSize);
+    cudaError_t e = dev_alloc(&w->world_tables, (size_t)worlds * num_types * num_types);
     if (e != cudaSuccess) {
         cf_destroy(w);
         return cuda_fail(e, "cudaMalloc(world tables)");
     }
     // world k: particles spawned from seed + k, raw table from seed + k, the
     // default transform (ParticleSimulation.cu:513-519)
-    std::vector<float> tables((size_t)worlds * kTableSize, 0.0f);
+    std::vector<float> tables((size_t)worlds * num_types * num_types, 0.0f);
     float lo[3], span[3];
     for (int a = 0; a < 3; a++) {
         span[a] = std::min(2000.0f, w->ext[a]);
@@ -2069,7 +2094,7 @@ int cf_batch_create(int worlds, const int* n_per_world, int num_types, float w_,
             for (int b2 = 0; b2 < num_types; b2++) {
                 const float raw = uniform_pm1(s);
                 const float t = tanhf(raw * 1.0f) * 0.28f + -0.20f;
-                tables[(size_t)k * kTableSize + a * kTableStride + b2] = fmaxf(-1.0f, fminf(1.0f, t));
+                tables[((size_t)k * num_types + a) * num_types + b2] = fmaxf(-1.0f, fminf(1.0f, t));
             }
     }
     if (e == cudaSuccess)
@@ -2155,13 +2180,7 @@ int cf_batch_set_force_tables(cf_batch* b, const float* tables, int count)
     cf_world* w = b->w;
     const int T = w->num_types;
     if (!tables || count != w->worlds * T * T) return fail(CF_ERR_INVALID, "count must be worlds * T * T");
-    std::vector<float> padded((size_t)w->worlds * kTableSize, 0.0f);
-    for (int k = 0; k < w->worlds; k++)
-        for (int a = 0; a < T; a++)
-            for (int c = 0; c < T; c++)
-                padded[(size_t)k * kTableSize + a * kTableStride + c] = tables[((size_t)k * T + a) * T + c];
-    CF_CUDA(cudaMemcpyAsync(w->world_tables, padded.data(), sizeof(float) * padded.size(), cudaMemcpyHostToDevice,
-                            w->stream));
+    CF_CUDA(cudaMemcpyAsync(w->world_tables, tables, sizeof(float) * (size_t)count, cudaMemcpyHostToDevice, w->stream));
     CF_CUDA(cudaStreamSynchronize(w->stream));
     return CF_OK;
 }

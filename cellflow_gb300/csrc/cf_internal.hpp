@@ -97,6 +97,9 @@ struct PairTables {
     float eff[kTableSize];           // effective radius (ParticleSimulation.cu:108-110)
     float threshold[kTableSize];     // smallest float t with sqrtf(t) >= eff
     float threshold_lo[kTableSize];  // contracted d^2 below this interacts for certain
+    float filter_row[CF_MAX_TYPES];  // per home type: no pair of it interacts at or above this contracted d^2
+    float force_compact[kTableSize];   // F[self * T + other]
+    float2 pair_compact[kTableSize];   // 1 / eff and threshold_lo at self * T + other
 };
 
 // Grid of one cell list.  A batch of independent worlds shares one grid
@@ -128,12 +131,17 @@ struct StepConsts {
     float thr_uniform;
     float inv_eff_uniform;
     float thr_lo_uniform;  // contracted d^2 below this interacts for certain (uniform radius)
+    float thr_hi_uniform;  // and at or above this never does
+    float neg_k_log2e, c1_uniform, att_uniform;  // -k log2(e); that / eff^2 and attraction / eff (uniform radius)
     float thr_filter;  // squared-distance bound of the approximate pre-test (>= every exact pass)
-    int variant;       // force-kernel staging variant (batch size, occupancy): cf_set_force_variant % 4
-    int split;         // warps per item (1, 2, 4): 1 << (cf_set_force_variant / 4)
+    float band;        // a contracted d^2 at or above threshold_lo + band never interacts
+    int variant;       // force-kernel occupancy variant: cf_set_force_variant % 3
+    int split;         // warps per item (1, 2, 4, 8, 16): 1 << (cf_set_force_variant / 3)
+    int integrate_apart;  // 1: the force kernel leaves force sums and counts in acc for the integrator's own kernel
     float repulsion, attraction, neg_k, balance, force_multiplier, delta_t, friction;
     int max_expected_neighbors;
-    const float* world_force;  // per-world force tables, kTableSize floats each (32-stride)
+    float cell[3];     // cell sides
+    const float* world_force;  // per-world force tables, T * T floats each
 };
 
 // One force-kernel item: up to 32 consecutive sorted particles of one row of
@@ -188,9 +196,9 @@ struct Scratch {
 // Cells of one tile of the CSR build (whole rows; 16 KB of shared memory).
 constexpr int kTileCellsMax = 4096;
 
-// Force-kernel staging variants (batch size and occupancy); a variant index
-// of cf_set_force_variant is stage + kForceStages * log2(warps per item).
-constexpr int kForceStages = 4;
+// Force-kernel occupancy variants; a variant index of cf_set_force_variant is
+// occupancy + kForceOccupancies * log2(warps per item).
+constexpr int kForceOccupancies = 3;
 
 // Differentiable rollout: checkpoints, one segment of replayed states, the
 // adjoint buffers and the record of the last forward (cf_rollout_*).
@@ -284,7 +292,7 @@ struct cf_world {
     // [world_off[k], world_off[k + 1]) and force table world_tables[k]
     int worlds = 1;
     std::vector<int> world_off;
-    float* world_tables = nullptr;  // device, worlds * kTableSize floats (32-stride)
+    float* world_tables = nullptr;  // device, worlds * T * T floats
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     float4* pos = nullptr;
@@ -307,6 +315,7 @@ struct cf_world {
     float uploaded_ratio = 0.0f;
     int uploaded_types = -1;
     float uploaded_extent = -1.0f;
+    float band = 0.0f;  // StepConsts::band of the uploaded tables
     cf::PairTables host_tables;
     // phase profiling (cf_profile_enable): per profiled step a triple of events
     // (start, after the cell list, after the force kernel) from a ring; the
@@ -328,7 +337,7 @@ struct cf_world {
     const void* graph_bufs[2] = {nullptr, nullptr};
     bool use_graphs = true;
     bool broken = false;  // a particle reallocation failed: no buffers until one succeeds
-    int force_variant = 0;  // force-kernel variant, chosen by cf_autotune_step
+    int force_variant = -1;  // force-kernel variant (cf_set_force_variant, cf_autotune_step); -1: chosen by rule
     // a captured multi-step graph (cf_batch_capture) and the constants it was captured with
     cudaGraphExec_t batch_graph = nullptr;
     int batch_graph_steps = 0;
@@ -376,7 +385,7 @@ cudaError_t launch_radix_sort(Scratch& s, int n, int key_bits, int* which, cudaS
 cudaError_t launch_cell_bounds(const uint32_t* keys, const uint32_t* vals, int n, const float4* pos, uint32_t* start,
                                uint32_t* end, int cells, float4* pos_sorted, cudaStream_t st);
 cudaError_t launch_step_force(const StepConsts& c, const PairTables* tables, const float4* pos_sorted,
-                              const uint32_t* keys_sorted, const uint32_t* vals_sorted, const uint32_t* cell_off,
+                              const uint32_t* vals_sorted, const uint32_t* cell_off,
                               const Item* items, const int* n_items, int max_items, float4* pos, float4* vel,
                               float4* acc, int* counts, cudaStream_t st);
 // Row-aligned items of at most 32 sorted particles (one cell row each).
@@ -385,8 +394,10 @@ cudaError_t launch_force_work(const StepConsts& c, const uint32_t* keys_sorted, 
                               cudaStream_t st);
 cudaError_t launch_step_plan(const uint32_t* cell_off, int n, const Grid& g, Item* items, int* n_items,
                              cudaStream_t st);
+int default_force_variant(int n, const Grid& g);
 int max_step_items(int n, const Grid& g);
 int step_launches(int n);
+bool integrate_apart(int n);  // whether the integrator is a kernel of its own
 cudaError_t configure_step_force();
 cudaError_t launch_scan_exclusive(const uint32_t* in, uint32_t* out, int n, uint32_t* tmp, size_t tmp_cap,
                                   cudaStream_t st);

@@ -2,49 +2,47 @@
 //
 // Work decomposition.  Particles are in cell order (the sorted snapshot of
 // positions).  An item is up to 32 consecutive particles of one row of cells
-// (same y and z cell): one warp, one particle per lane.  The candidates of
-// an item are the particles of the union of its homes' 27-cell stencils:
-// 9 rows, each a run of consecutive cells, i.e. one contiguous range of the
-// sorted snapshot (two where the run wraps around the box in x).  The warp
-// copies those ranges into shared memory, 256, 384 or 512 at a time (chosen
-// by the autotuner), with their periodic shift already applied, and every
-// lane tests every staged candidate (broadcast reads).  For worlds too small
-// to fill the GPU, 2 or 4 warps share an item, each taking an equal share of
-// its candidates; the first adds the others' partial sums in a fixed order.
-// Items are 16-B records (first particle, count, the row's y/z, world)
-// written by the cell list, so no per-item integer division is needed.
+// (same y and z cell), one home particle per lane.  The candidates of an item
+// are the particles of the union of its homes' 27-cell stencils: 9 rows, each
+// a run of consecutive cells, i.e. one contiguous range of the sorted snapshot
+// (two where the run wraps around the box in x), read as one concatenated
+// list.  The list is cut into units of at most kUnit candidates.  A warp works
+// one unit at a time: it stages the unit into shared memory with its periodic
+// shift applied, filters it for all 32 homes and drains the hits.  An item has
+// 1, 2, 4, 8 or 16 warps (c.split), which take its units in turn.
+//
+// Every unit's partial sums start from zero and are added in unit order, so a
+// step's result depends on neither the split nor the occupancy variant, bit
+// for bit, and a world steps the same alone and in a batch.
 //
 // Coordinates are staged relative to an origin per pass (the centre of the
-// stencil box where that keeps c - o exact, else 0), periodic shift folded
-// in, with |c|^2 beside them; an unshifted displacement is then the
-// reference's fl(c - h) bit for bit.
+// stencil box where that keeps c - o exact, else 0), periodic shift folded in;
+// an unshifted displacement is then the reference's fl(c - h) bit for bit.
 //
-// Per batch of staged candidates, two phases per lane:
-//   Filter: |c - h|^2 - bound = |c|^2 + (|h|^2 - bound) - 2 h.c for two
-//     candidates per instruction chain (packed f32x2 add/fma of sm_100+: one
-//     add and three fma per pair of candidates), the sign bit of each result
-//     shifted into a 32-bit mask per 32 candidates.  The bound is >= the
-//     exact test for every pair plus the expansion's rounding, which the
-//     origin keeps at the scale of the stencil box.  ~85% of pairs stop here.
-//   Drain: for every set bit (two per trip, three with lane pairing; a
-//     warp-uniform trip count from the filter's per-lane hit counts), the
-//     contracted distance of the displacement; pairs below a second bound
-//     (<= the exact test for every pair) interact for certain, and only the
-//     rare pairs between the two bounds (a band ~1e-6 wide) take the
+// Per unit, two phases:
+//   Filter: |c - h|^2 - B = |c|^2 + (|h|^2 - B) - 2 h.c for 32 homes x 8
+//     candidates by two m16n8k8 tensor-core products of half-precision
+//     operands with 32-bit sums; the sign bits, gathered over the quad of
+//     lanes that holds a home's row, give 32-bit masks per home.  Positions
+//     are rounded to half precision first and the squares are taken of the
+//     rounded positions (as high + low halves), so the value is the rounded
+//     points' own squared distance and B only has to cover the rounding of the
+//     positions.  The scalar form (four packed FP32 instructions per pair of
+//     candidates) cost 4 issue slots a candidate; this costs about 1.7.
+//   Drain: each lane walks its home's set bits (two pairs per trip; a
+//     warp-uniform trip count, the largest hit count): the contracted distance
+//     of the 32-bit displacement; pairs below a second bound (<= the exact
+//     test for every pair) interact for certain, pairs above a third do not,
+//     and only the rare pairs between (a band ~1e-6 wide) take the
 //     reference's exact test on the unshifted coordinates, in the trips where
-//     a warp vote finds one (written inline, its instructions ran predicated
-//     for every pair).  Interacting pairs add their force term.  In
-//     the lane-paired variant the lanes are sorted by hit count and paired
-//     busiest with idlest; the idler lane of a pair, after its own hits,
-//     walks the top part of its partner's with its partner's home and hands
-//     the partial sums over, so the trip count falls towards the mean.
+//     a warp vote finds one.  Interacting pairs add their force term.
 //
 // Exactness (cuda-native/src/ParticleSimulation.cu:86-165):
 //   - the neighbour test is the reference's: d^2 = (dx*dx + dy*dy) + dz*dz and
 //     s = d^2 + 1e-4 rounded as the reference (compiled without contraction)
 //     rounds them, and sqrtf(s) < eff is replaced by the equivalent s < t,
 //     t the smallest float whose correctly rounded square root is >= eff.
-//     The two bounds bracket that test, so neighbour counts match bit for bit;
+//     The bounds bracket that test, so neighbour counts match bit for bit;
 //   - a displacement is wrapped like the reference (subtract the extent where
 //     its test fires).  With at least 5 cells per axis that is exactly the
 //     stencil cells across the box edge: the union of an item spans at most
@@ -52,21 +50,37 @@
 //     added after the subtraction (exact path) as the reference does.  With
 //     fewer cells both phases run the reference's tests per candidate;
 //   - force terms use rsqrt and exp approximations (a few ulp) and the
-//     contracted distance; the sum runs in cell order.
+//     contracted distance.
 //   The density factor, integrator and wrap are the reference's operations.
-#include <type_traits>
+//
+// What bounds it: instruction issue (55 to 70 % of the slots used) and, in the
+// drain, latency and shared-memory bank conflicts at scattered slots.  Counted
+// at 100k evenly spread particles (3,340 items of 18 groups and 28 trips): about
+// 820 instructions for an item's start and end, 97 to stage and 67 to filter a
+// group of 32 candidates, 90 per trip of two pairs.  What brought the step there,
+// against one 32-bit lane per home filtering and draining stretches of the list
+// (force kernel, 100k and 1M in blobs): units dealt out entry by entry instead
+// of in stretches (28 trips per item instead of 37), band pairs put off to the end
+// of the unit instead of an exact test in the trip (61 instructions per trip),
+// predicated bit walking, all of a unit's positions in flight at once, the
+// tensor-core filter: 62 to 39 us and 737 to 469 us.  An application world of
+// 10,000 particles with ~125 neighbours each (313 items): 276 to 32 us with
+// four warps per item.
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <type_traits>
 
 #include "cf_internal.hpp"
 
 namespace cf {
 namespace {
 
-constexpr int kWarps = 4;
-constexpr int kThreads = 32 * kWarps;
-constexpr float kFar = 1e30f;  // padding slots sit at +kFar, idle homes at -kFar
-constexpr int kTypeShift = 27; // staged meta: sorted index | type << 27
-constexpr uint32_t kIndexMask = (1u << kTypeShift) - 1u;
+constexpr int kUnit = 256;          // candidates staged per unit at most
+constexpr int kGroups = kUnit / 32; // of 32 candidates
+constexpr float kFar = 1e30f;       // the sentinel slot's position, and idle homes' on generic grids (-kFar)
+constexpr uint32_t kAll = 0xffffffffu;
 
 __device__ __forceinline__ float wrap_ref(float d, float ext, float half)
 {
@@ -91,6 +105,13 @@ __device__ __forceinline__ float staged_shift(float staged, float raw, float ext
 
 __device__ __forceinline__ int wrap_index(int v, int m) { return v < 0 ? v + m : (v >= m ? v - m : v); }
 
+// A home's x cell, as the cell list's hash computed it.
+__device__ __forceinline__ int x_cell(float x, float inv, int m)
+{
+    const int c = __float2int_rd(__fmul_rn(x, inv));
+    return min(max(c, 0), m - 1);
+}
+
 // fmodf(x, W) of the integrator's wrap (ParticleSimulation.cu:159-161), exact:
 // for x in [0, 2W) it is x or x - W, and x - W is exact there (Sterbenz).
 __device__ __forceinline__ float wrap_pos(float x, float W)
@@ -107,8 +128,9 @@ __device__ __forceinline__ float wrap_pos(float x, float W)
 // reference's fl(c - h).  Otherwise the origin is 0 (also exact).
 __device__ __forceinline__ void stencil_origin(int clo, int chi, float cs, float& o, float& r)
 {
-    const float lo = (float)clo * cs, hi = (float)(chi + 1) * cs, mg = 0.05f * cs;
-    const float ctr = 0.5f * (lo + hi), half = 0.5f * (hi - lo) + mg;
+    // (rounded one by one: contracted here and not there, homes and candidates would get two origins)
+    const float lo = __fmul_rn((float)clo, cs), hi = __fmul_rn((float)(chi + 1), cs), mg = 0.05f * cs;
+    const float ctr = __fmul_rn(0.5f, __fadd_rn(lo, hi)), half = 0.5f * (hi - lo) + mg;
     if (ctr >= 2.0f * half) {
         o = ctr;
         r = half;
@@ -118,47 +140,24 @@ __device__ __forceinline__ void stencil_origin(int clo, int chi, float cs, float
     }
 }
 
-// Lane pairing scratch of the drain (the variants that pair lanes):
-// each lane's home and filter operands for the pass, its group bitmap for the
-// batch, its partner, and its own partial sums while it works on its partner's hits.
-struct PairScratch {
-    float4 home_h[32];
-    float4 home_m2[32];
-    float4 saved[32];
-    uint32_t nzw[32];
-    uint32_t pairing[32];
-};
-struct NoScratch {};
-// Balanced drain: each lane's home and filter operands, group bitmap and hit
-// count for the batch, and the partial sums of the (lane, home) pieces of the
-// task line, at index lane + rank of the home among the homes with hits.
-struct BalScratch {
-    float4 home_h[32];
-    float4 home_m2[32];
-    uint32_t nzw[32];
-    int hits[32];
-    float4 part[64];
-};
+constexpr int kSegs = 18;  // contiguous ranges of an item's candidates: 9 rows, two where a row wraps
 
-// Per-warp staging area, kStage candidates (a multiple of 32) per batch.
-// Drain modes: 0 one lane per home, 1 lanes paired (busiest with idlest),
-// 2 balanced (the batch's hits split evenly over the lanes).
-template <int kMode>
-using DrainScratch = typename std::conditional<kMode == 1, PairScratch,
-                                               typename std::conditional<kMode == 2, BalScratch, NoScratch>::type>::type;
-
-template <int kStage, int kMode>
+// Per-warp staging area.
 struct WarpSmem {
-    float4 xy[kStage / 2];              // staged (x_a, x_b, y_a, y_b) of slots 2p, 2p+1
-    float4 zc[kStage / 2];              // staged (z_a, z_b, |c_a|^2, |c_b|^2)
-    uint32_t meta[kStage];              // sorted index | type << 27
-    uint32_t mask[(kStage / 32) * 32];  // [group][lane]
-    float origin[4];                    // the pass's staging origin (x, y, z)
-    DrainScratch<kMode> pr;
+    float4 c[1 + kUnit];  // the sentinel (at kFar), then the staged x, y, z and force-table offset (4 type)
+    // row 0: the sentinel's masks, then the list's description (below).  Row 1 + g of
+    // group g: the filter's half-precision words (x, y), (z, s hi), (s lo, 1), with s = |c|^2, in
+    // fragment order, and once the group is filtered, in the first 32 words, the lanes' masks.
+    uint32_t row[1 + kGroups][96];
+    float4 seg[kSegs];  // per segment: what is added to its positions, and its first sorted index less its list start
 };
+// Words of row 0: the staging origin; where the segments start in the list; and,
+// for each segment with entries in the unit, what gives the sorted index of slot
+// s as (first word) + s * units, and the segment.
+constexpr int kOriginAt = 32, kStartAt = 36, kPartAt = 56;
 
-// Named barrier of the warps sharing an item: id 1 + slot (slot < kWarps),
-// immediate ids so only five hardware barriers are reserved.
+// Named barrier of the warps sharing an item: id 1 + slot (at most 4 items per
+// block), immediate ids so only five hardware barriers are reserved.
 __device__ __forceinline__ void item_barrier(int slot, int threads)
 {
     switch (slot) {
@@ -169,807 +168,657 @@ __device__ __forceinline__ void item_barrier(int slot, int threads)
     }
 }
 
-struct Lane {
-    float4 h;     // home position (raw)
-    uint32_t tp;  // home type
-    float fx, fy, fz;
-    int count;
-};
-
-// The origin-relative home of a pass as the filter's packed operands:
-// (-2 h', -2 h') per axis and (|h'|^2 - bound) twice.  h' itself is
-// -0.5 * m2h exactly, so the drain's displacement fl(c' - h') is
-// fmaf(0.5, m2h, c').
-struct HomeOps {
-    float2 m2x, m2y, m2z, k;
-};
-
-// Per type pair of the item's world, T-stride: (R F, A F / eff).  With
-// s = d^2 + 1e-4, dist = sqrt(s) and rs = 1/dist, the reference's term
-//   (d / dist) F (R exp(-k r^2) - A r),  r = dist / eff   (ParticleSimulation.cu:113-124)
-// is  d * (R F * exp2(c1 s) * rs - A F / eff),  c1 = -k log2(e) / eff^2.
-struct Tables {
-    const float2* coef;  // (R F, A F / eff), T-stride
-    const float* c1;     // 32-stride (unused with a uniform radius)
-    const float* thr;
-    const float* thr_lo;
-    int T;
-};
-
-constexpr float kLog2e = 1.4426950408889634f;
-
-// Displacement from the home to a staged candidate.  Generic grids stage raw
-// coordinates and wrap per candidate; otherwise both ends are origin-relative
-// and the shift is already in the staged value.
-template <bool kGeneric>
-__device__ __forceinline__ void staged_delta(const StepConsts& c, float cx, float cy, float cz, const float4& h,
-                                             const HomeOps& H, float& dx, float& dy, float& dz)
+// Two m16n8k8 products: 32 homes (fragments a[0..1] rows g and g + 8, a[2..3]
+// rows g + 16 and g + 24) against the 8 candidates of one fragment word b.
+// d[q]: row g + 8 q against columns 2 t (low half) and 2 t + 1 (high half).
+__device__ __forceinline__ void mma_32x8(const uint32_t (&a)[4], uint32_t b, uint32_t (&d)[4])
 {
-    if (kGeneric) {
-        dx = wrap_ref(cx - h.x, c.ext[0], c.half[0]);
-        dy = wrap_ref(cy - h.y, c.ext[1], c.half[1]);
-        dz = wrap_ref(cz - h.z, c.ext[2], c.half[2]);
-    } else {
-        dx = fmaf(0.5f, H.m2x.x, cx);
-        dy = fmaf(0.5f, H.m2y.x, cy);
-        dz = fmaf(0.5f, H.m2z.x, cz);
+    asm("mma.sync.aligned.m16n8k8.row.col.f16.f16.f16.f16 {%0, %1}, {%2, %3}, {%4}, {%5, %5};"
+        : "=r"(d[0]), "=r"(d[1])
+        : "r"(a[0]), "r"(a[1]), "r"(b), "r"(0u));
+    asm("mma.sync.aligned.m16n8k8.row.col.f16.f16.f16.f16 {%0, %1}, {%2, %3}, {%4}, {%5, %5};"
+        : "=r"(d[2]), "=r"(d[3])
+        : "r"(a[2]), "r"(a[3]), "r"(b), "r"(0u));
+}
+
+// Quotient and remainder of x by units, x at most kUnit * units (so that the
+// rounded quotient is off by one at most).
+__device__ __forceinline__ void deal(int x, int units, float per_unit, int& q, int& r)
+{
+    q = (int)((float)x * per_unit);
+    r = x - q * units;
+    if (r < 0) {
+        q--;
+        r += units;
+    }
+    if (r >= units) {
+        q++;
+        r -= units;
     }
 }
 
-// One queued pair's interaction test: certain-interaction bound, exact
-// fallback.  Returns the staged displacement and its contracted d^2.
-// `origin` is the pass's staging origin (unused on generic grids).
-template <bool kGeneric, bool kUniformR>
-__device__ __forceinline__ bool pair_fast(const StepConsts& c, const Lane& L, const HomeOps& H, float cx, float cy,
-                                          float cz, uint32_t meta, const Tables& tb, float& dx, float& dy, float& dz,
-                                          float& d2)
+// a where the mask has a bit, b elsewhere.
+__device__ __forceinline__ uint32_t bit_select(uint32_t a, uint32_t b, uint32_t mask) { return (a & mask) | (b & ~mask); }
+
+// Two floats rounded to half precision, lo in the low half.
+__device__ __forceinline__ uint32_t half2_bits(float lo, float hi)
 {
-    staged_delta<kGeneric>(c, cx, cy, cz, L.h, H, dx, dy, dz);
-    d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-    const uint32_t other = meta >> kTypeShift;
-    const uint32_t pair = L.tp * kTableStride + other;
-    return d2 < (kUniformR ? c.thr_lo_uniform : tb.thr_lo[pair]);
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ float half_lo(uint32_t h) { return __low2float(*reinterpret_cast<const __half2*>(&h)); }
+__device__ __forceinline__ float half_hi(uint32_t h) { return __high2float(*reinterpret_cast<const __half2*>(&h)); }
+
+// Square root to about 2^-22 (the filter's bound has 2^-16 to spare).
+__device__ __forceinline__ float sqrt_approx(float x)
+{
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
-// The reference's exact test for a pair the certain-interaction bound left
-// open (within rounding of the threshold), on the unshifted coordinates.
-template <bool kGeneric, bool kUniformR>
-__device__ __forceinline__ bool pair_exact(const StepConsts& c, const Lane& L, const float* origin, float cx, float cy,
-                                           float cz, uint32_t meta, const float4* __restrict__ pos_sorted,
-                                           const Tables& tb)
+__device__ __forceinline__ int top_bit(uint32_t m)
 {
-    if (!CF_IN_BOUNDS(meta & kIndexMask, c.n)) return false;
-    const float4 o = pos_sorted[meta & kIndexMask];
-    float ex = __fsub_rn(o.x, L.h.x), ey = __fsub_rn(o.y, L.h.y), ez = __fsub_rn(o.z, L.h.z);
+    int r;
+    asm("bfind.u32 %0, %1;" : "=r"(r) : "r"(m));
+    return r;
+}
+
+// A value the compiler keeps in a register instead of computing it again from
+// the thread index at each use.
+__device__ __forceinline__ uint32_t pinned(uint32_t x)
+{
+    asm volatile("" : "+r"(x));
+    return x;
+}
+
+// Loads by shared-memory address.
+__device__ __forceinline__ float4 lds128(uint32_t at)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+    return v;
+}
+__device__ __forceinline__ float lds32(uint32_t at)
+{
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at));
+    return v;
+}
+
+// 16 bytes from global to shared memory, asynchronously, if `copy`.
+__device__ __forceinline__ void copy_async16(bool copy, uint32_t to, const float4* from)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.ne.u32 p, %2, 0;\n\t"
+                 "@p cp.async.ca.shared.global [%0], [%1], 16;\n\t}" ::"r"(to), "l"(from), "r"((uint32_t)copy)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_wait()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// The reference's exact test for a pair the two bounds left open (within
+// rounding of the threshold), on the unshifted coordinates h and o; p is the
+// staged candidate.
+template <bool kGeneric>
+__device__ __forceinline__ bool pair_exact(const StepConsts& c, const float4& h, const float* origin, const float4& p,
+                                           const float4& o, float thr)
+{
+    float ex = __fsub_rn(o.x, h.x), ey = __fsub_rn(o.y, h.y), ez = __fsub_rn(o.z, h.z);
     if (kGeneric) {
         ex = wrap_ref(ex, c.ext[0], c.half[0]);
         ey = wrap_ref(ey, c.ext[1], c.half[1]);
         ez = wrap_ref(ez, c.ext[2], c.half[2]);
     } else {
-        ex = __fadd_rn(ex, staged_shift(cx + origin[0], o.x, c.ext[0]));
-        ey = __fadd_rn(ey, staged_shift(cy + origin[1], o.y, c.ext[1]));
-        ez = __fadd_rn(ez, staged_shift(cz + origin[2], o.z, c.ext[2]));
+        ex = __fadd_rn(ex, staged_shift(p.x + origin[0], o.x, c.ext[0]));
+        ey = __fadd_rn(ey, staged_shift(p.y + origin[1], o.y, c.ext[1]));
+        ez = __fadd_rn(ez, staged_shift(p.z + origin[2], o.z, c.ext[2]));
     }
     const float e2 = __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez));
-    const uint32_t pair = L.tp * kTableStride + (meta >> kTypeShift);
-    return __fadd_rn(e2, 0.0001f) < (kUniformR ? c.thr_uniform : tb.thr[pair]);
+    return __fadd_rn(e2, 0.0001f) < thr;
 }
+
+// A home's displacement to a staged candidate p, its contracted square, the
+// bound below which it interacts for certain, and the weight of the displacement
+// in the force: with s = d^2 + 1e-4, dist = sqrt(s) and rs = 1/dist, the
+// reference's term (d / dist) F (R exp(-k r^2) - A r), r = dist / eff
+// (ParticleSimulation.cu:113-124) is d * F * (R exp2(c1 s) rs - A / eff),
+// c1 = -k log2(e) / eff^2.
+struct PairTerm {
+    float dx, dy, dz, d2, lo, weight;
+};
 
 template <bool kGeneric, bool kUniformR>
-__device__ __forceinline__ bool pair_test(const StepConsts& c, const Lane& L, const HomeOps& H,
-                                          const float* origin, float cx, float cy, float cz, uint32_t meta,
-                                          const float4* __restrict__ pos_sorted, const Tables& tb, float& dx,
-                                          float& dy, float& dz, float& d2)
+__device__ __forceinline__ PairTerm pair_term(const StepConsts& c, const float4& p, float hx, float hy, float hz,
+                                              uint32_t force_at, uint32_t pair_at)
 {
-    staged_delta<kGeneric>(c, cx, cy, cz, L.h, H, dx, dy, dz);
-    d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-    const uint32_t other = meta >> kTypeShift;
-    const uint32_t pair = L.tp * kTableStride + other;
-    bool inter = d2 < (kUniformR ? c.thr_lo_uniform : tb.thr_lo[pair]);
-    if (!inter) {
-        // within rounding of the threshold: the reference's exact test
-        if (!CF_IN_BOUNDS(meta & kIndexMask, c.n)) return false;
-        const float4 o = pos_sorted[meta & kIndexMask];
-        float ex = __fsub_rn(o.x, L.h.x), ey = __fsub_rn(o.y, L.h.y), ez = __fsub_rn(o.z, L.h.z);
-        if (kGeneric) {
-            ex = wrap_ref(ex, c.ext[0], c.half[0]);
-            ey = wrap_ref(ey, c.ext[1], c.half[1]);
-            ez = wrap_ref(ez, c.ext[2], c.half[2]);
-        } else {
-            ex = __fadd_rn(ex, staged_shift(cx + origin[0], o.x, c.ext[0]));
-            ey = __fadd_rn(ey, staged_shift(cy + origin[1], o.y, c.ext[1]));
-            ez = __fadd_rn(ez, staged_shift(cz + origin[2], o.z, c.ext[2]));
-        }
-        const float e2 = __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez));
-        inter = __fadd_rn(e2, 0.0001f) < (kUniformR ? c.thr_uniform : tb.thr[pair]);
-    }
-    return inter;
-}
-
-// The force weight of an interacting pair (multiplies the displacement).
-template <bool kUniformR>
-__device__ __forceinline__ float pair_weight(float d2, uint32_t meta, const Lane& L, const Tables& tb, float c1u)
-{
-    const uint32_t other = meta >> kTypeShift;
-    const float2 k = tb.coef[L.tp * tb.T + other];
-    const float s = d2 + 0.0001f;
-    const float rs = rsqrtf(s);
-    const float c1 = kUniformR ? c1u : tb.c1[L.tp * kTableStride + other];
-    float e;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(c1 * s));
-    return fmaf(k.x * e, rs, -k.y);
-}
-
-// The staged coordinates of a slot.
-__device__ __forceinline__ void staged_xyz(const float* xyf, const float* zcf, int slot, float& x, float& y, float& z)
-{
-    const int pb = (slot >> 1) * 4 + (slot & 1);
-    x = xyf[pb];
-    y = xyf[pb + 2];
-    z = zcf[pb];
-}
-
-template <int kStage, int kMinBlocks, int kMode, bool kGeneric, bool kUniformR>
-__global__ void __launch_bounds__(kThreads, kMinBlocks)
-    step_force_kernel(StepConsts c, const PairTables* __restrict__ tables, const float4* __restrict__ pos_sorted,
-                      const uint32_t* __restrict__ keys_sorted, const uint32_t* __restrict__ vals_sorted,
-                      const uint32_t* __restrict__ cell_off, const Item* __restrict__ items,
-                      const int* __restrict__ n_items, float4* __restrict__ pos, float4* __restrict__ vel,
-                      float4* __restrict__ acc, int* __restrict__ counts)
-{
-    __shared__ float s_inv_eff[kUniformR ? 1 : kTableSize];
-    __shared__ float s_c1[kUniformR ? 1 : kTableSize];
-    __shared__ float s_thr[kUniformR ? 1 : kTableSize];
-    __shared__ float s_thr_lo[kUniformR ? 1 : kTableSize];
-    __shared__ float4 s_part[kWarps][32];  // partial sums of the item's other warps (split > 1)
-    extern __shared__ __align__(16) unsigned char s_dyn[];
-    const int T = c.num_types;
-    // force coefficients, compact T-stride: one copy per block for a single
-    // world, one per warp (filled once its item's world is known) for a batch
-    const bool one_world = c.grid.worlds == 1;
-    float2* coef_base = reinterpret_cast<float2*>(s_dyn + sizeof(WarpSmem<kStage, kMode>) * kWarps);
+    PairTerm k;
+    const uint32_t type4 = __float_as_uint(p.w);
+    const float F = lds32(force_at + type4);
+    float a_eff = c.att_uniform, c1 = c.c1_uniform;
+    k.lo = c.thr_lo_uniform;
     if (!kUniformR) {
-        for (int e = threadIdx.x; e < T * T; e += kThreads) {
-            const int a = e / T, b = e - a * T;
-            const int k = a * kTableStride + b;
-            const float inv = 1.0f / tables->eff[k];
-            s_inv_eff[k] = inv;
-            s_c1[k] = c.neg_k * kLog2e * inv * inv;
-            s_thr[k] = tables->threshold[k];
-            s_thr_lo[k] = tables->threshold_lo[k];
-        }
+        const float4 v = lds128(pair_at + 4 * type4);
+        a_eff = v.x;
+        c1 = v.y;
+        k.lo = v.z;
     }
-    if (one_world) {
-        for (int e = threadIdx.x; e < T * T; e += kThreads) {
-            const int a = e / T, b = e - a * T;
-            const float F = c.world_force[a * kTableStride + b];
-            const float inv = kUniformR ? c.inv_eff_uniform : 1.0f / tables->eff[a * kTableStride + b];
-            coef_base[e] = make_float2(c.repulsion * F, c.attraction * F * inv);
-        }
+    k.dx = p.x - hx;
+    k.dy = p.y - hy;
+    k.dz = p.z - hz;
+    if (kGeneric) {
+        k.dx = wrap_ref(k.dx, c.ext[0], c.half[0]);
+        k.dy = wrap_ref(k.dy, c.ext[1], c.half[1]);
+        k.dz = wrap_ref(k.dz, c.ext[2], c.half[2]);
     }
-    __syncthreads();
-    const float c1u = c.neg_k * kLog2e * c.inv_eff_uniform * c.inv_eff_uniform;
-    // pairs per drain trip: two side by side where the register budget allows,
-    // three with lane pairing (more of the lanes stay busy, so more independent
-    // work per trip pays there; it does not without pairing)
-    constexpr int kPer = kMinBlocks >= 8 ? 1 : (kMode != 0 && !kGeneric ? 3 : 2);
-    // lane pairing or the balanced drain (regular grids)
-    constexpr bool kBalance = kMode == 1 && !kGeneric;
-    constexpr bool kBal = kMode == 2 && !kGeneric;
+    k.d2 = fmaf(k.dz, k.dz, fmaf(k.dy, k.dy, k.dx * k.dx));
+    const float s = k.d2 + 0.0001f;
+    float rs, e;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(s));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(c1 * s));
+    k.weight = F * fmaf(c.repulsion * e, rs, -a_eff);
+    return k;
+}
 
-    // c.split warps (1, 2 or 4) share an item, each taking an equal share of its
-    // candidates; part 0 adds the others' partial sums and integrates
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int split = c.split;
-    const int part = warp & (split - 1);
-    const int item = blockIdx.x * (kWarps / split) + warp / split;
-    if (item >= *n_items) return;  // the item's other warps leave too: no barrier is pending
-    using Smem = WarpSmem<kStage, kMode>;
-    Smem& w = reinterpret_cast<Smem*>(s_dyn)[warp];
-    float2* wcoef = coef_base + (one_world ? 0 : warp * T * T);
-    const float* xyf = reinterpret_cast<const float*>(w.xy);
-    const float* zcf = reinterpret_cast<const float*>(w.zc);
-    const Item it = items[item];
-    // (bounds-checked build) the item's particles lie in [0, n): else the item's warps skip it
-    if (!CF_IN_BOUNDS(it.count - 1, 32) || !CF_IN_BOUNDS(it.first, c.n) || !CF_IN_BOUNDS(it.first + it.count - 1, c.n))
-        return;
-    const bool active = lane < it.count;
-    const int t = it.first + (active ? lane : 0);
-    Lane L;
-    L.h = pos_sorted[t];
-    L.tp = __float_as_uint(L.h.w) & kTypeMask;
-    L.fx = L.fy = L.fz = 0.0f;
-    L.count = 0;
-
-    // cell coordinates inside the item's world (items never straddle worlds or rows)
-    const int mx = c.grid.m[0], my = c.grid.m[1], mz = c.grid.m[2];
-    const uint32_t world = (uint32_t)it.world;
-    const uint32_t world_base = world * (uint32_t)c.grid.cells_w;
-    const int yc = it.yz & 0xffff, zc = it.yz >> 16;
-    const uint32_t row_base = world_base + (uint32_t)((zc * my + yc) * mx);
-    const int x0 = (int)(keys_sorted[it.first] - row_base);
-    const int x1 = (int)(keys_sorted[it.first + it.count - 1] - row_base);
-    const int hx = (int)(keys_sorted[t] - row_base);
-    if (!one_world) {
-        for (int e = lane; e < T * T; e += 32) {
-            const int a = e / T, b = e - a * T;
-            const float F = c.world_force[(size_t)world * kTableSize + a * kTableStride + b];
-            const float inv = kUniformR ? c.inv_eff_uniform : s_inv_eff[a * kTableStride + b];
-            wcoef[e] = make_float2(c.repulsion * F, c.attraction * F * inv);
-        }
-        __syncwarp();
-    }
-    const Tables tb{wcoef, s_c1, s_thr, s_thr_lo, T};
-    // x sub-ranges whose union (range plus one cell each side) fits in the box
-    const int width = kGeneric ? mx : (mx - 2);
-    const int passes = kGeneric ? 1 : (x1 - x0 + width) / width;
-    const float thr_f = c.thr_filter;
-
-    for (int pass = 0; pass < passes; pass++) {
-        const int px0 = kGeneric ? x0 : x0 + pass * width;
-        const int px1 = kGeneric ? x1 : min(x1, px0 + width - 1);
-        const bool mine = active && (kGeneric || (hx >= px0 && hx <= px1));
-        // generic grids: an idle home sits at -kFar, 2e30 from every candidate and from the
-        // +kFar padding slots
-        const float hxf = mine ? L.h.x : -kFar, hyf = mine ? L.h.y : -kFar, hzf = mine ? L.h.z : -kFar;
-
-        const int xlo = mx > 1 ? px0 - 1 : 0;
-        const int xhi = mx > 1 ? min(px1 + 1, xlo + mx - 1) : 0;  // inclusive, at most mx cells
-
-        // Staging origin per axis (stencil_origin) for the stencil box (cells xlo..xhi,
-        // yc-1..yc+1, zc-1..zc+1 in shifted coordinates).  Every staged candidate and the
-        // homes lie within (rx, ry, rz) of it, so |c'|, |h'| <= R.  The expanded filter value
-        // |c'|^2 + (|h'|^2 - B) - 2 h'.c' carries at most 2^-24 (21 R^2 + 5 B) of rounding
-        // (three roundings in each square, one in the constant, four in the chain); the
-        // bound B = (thr_f (1 + 2^-18) + 2^-19 R^2)(1 + 2^-18) exceeds thr_f by more, so
-        // every pair whose staged d^2 is within thr_f stays negative.
-        HomeOps H;
-        float ox = 0.0f, oy = 0.0f, oz = 0.0f;
-        if (!kGeneric) {
-            float rx, ry, rz;
-            stencil_origin(xlo, xhi, c.ext[0] / (float)mx, ox, rx);
-            stencil_origin(yc - 1, yc + 1, c.ext[1] / (float)my, oy, ry);
-            stencil_origin(zc - 1, zc + 1, c.ext[2] / (float)mz, oz, rz);
-            const float r2 = fmaf(rz, rz, fmaf(ry, ry, rx * rx));
-            const float bnd = (thr_f * (1.0f + 0x1p-18f) + r2 * 0x1p-19f) * (1.0f + 0x1p-18f);
-            const float hpx = mine ? L.h.x - ox : 0.0f, hpy = mine ? L.h.y - oy : 0.0f,
-                        hpz = mine ? L.h.z - oz : 0.0f;
-            const float kk = mine ? fmaf(hpz, hpz, fmaf(hpy, hpy, hpx * hpx)) - bnd : kFar;
-            H.m2x = make_float2(-2.0f * hpx, -2.0f * hpx);
-            H.m2y = make_float2(-2.0f * hpy, -2.0f * hpy);
-            H.m2z = make_float2(-2.0f * hpz, -2.0f * hpz);
-            H.k = make_float2(kk, kk);
-            if (lane == 0) {
-                w.origin[0] = ox;
-                w.origin[1] = oy;
-                w.origin[2] = oz;
-            }
-            if constexpr (kBalance || kBal) {
-                w.pr.home_h[lane] = L.h;
-                w.pr.home_m2[lane] = make_float4(H.m2x.x, H.m2y.x, H.m2z.x, 0.0f);
-            }
-        } else {
-            H.m2x = H.m2y = H.m2z = H.k = make_float2(0.0f, 0.0f);
-        }
-        // segments: lane 2*row + half describes one contiguous range of the snapshot and
-        // its periodic shift less the origin (zero on generic grids)
-        int seg_beg = 0, seg_len = 0;
-        float seg_sx = 0.0f, seg_sy = 0.0f, seg_sz = 0.0f;
-        const int ny = my > 1 ? 3 : 1, nz = mz > 1 ? 3 : 1;
-        const int nseg = 2 * ny * nz;
-        {
-            const int row = lane >> 1, half = lane & 1;
-            const int dy_row = ny > 1 ? (row % ny) - 1 : 0, dz_row = nz > 1 ? (row / ny) - 1 : 0;
-            const int yy = wrap_index(yc + dy_row, my), zz = wrap_index(zc + dz_row, mz);
-            const uint32_t cy = (yc + dy_row < 0) ? 1u : (yc + dy_row >= my ? 2u : 0u);
-            const uint32_t cz = (zc + dz_row < 0) ? 1u : (zc + dz_row >= mz ? 2u : 0u);
-            // split [xlo, xhi] at the box edge: half 0 is the in-box part, half 1 the wrapped part
-            int a = xlo, b = xhi;
-            uint32_t cx = 0u;
-            if (xlo < 0) {
-                if (half == 0) a = 0;
-                else { a = xlo + mx; b = mx - 1; cx = 1u; }
-            } else if (xhi >= mx) {
-                if (half == 0) b = mx - 1;
-                else { a = 0; b = xhi - mx; cx = 2u; }
-            } else if (half == 1) {
-                b = a - 1;
-            }
-            if (row < ny * nz && b >= a && CF_IN_BOUNDS(world_base + (uint32_t)((zz * my + yy) * mx) + b + 1,
-                                                        c.grid.cells + 1)) {
-                const uint32_t base = world_base + (uint32_t)((zz * my + yy) * mx);
-                seg_beg = (int)cell_off[base + a];
-                seg_len = (int)cell_off[base + b + 1] - seg_beg;
-                if (!CF_IN_BOUNDS(seg_len, c.n + 1) || !CF_IN_BOUNDS(seg_beg + seg_len, c.n + 1)) seg_len = 0;
-                if (!kGeneric) {
-                    seg_sx = code_shift(cx, c.ext[0]) - ox;
-                    seg_sy = code_shift(cy, c.ext[1]) - oy;
-                    seg_sz = code_shift(cz, c.ext[2]) - oz;
-                }
-            }
-        }
-        int seg_pre = seg_len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, seg_pre, o);
-            if (lane >= o) seg_pre += v;
-        }
-        const int total = __shfl_sync(0xffffffffu, seg_pre, 31);
-        seg_pre -= seg_len;
-        // the home's place in the concatenation: its cell is in the centre row's in-box part
-        const int seg_c = 2 * ((nz > 1 ? ny : 0) + (ny > 1 ? 1 : 0));
-        const int beg_c = __shfl_sync(0xffffffffu, seg_beg, seg_c);
-        const int len_c = __shfl_sync(0xffffffffu, seg_len, seg_c);
-        const int pre_c = __shfl_sync(0xffffffffu, seg_pre, seg_c);
-        const int g_own = (t >= beg_c && t < beg_c + len_c) ? pre_c + (t - beg_c) : -1;
-
-        const int share_lo = (int)((long long)total * part / split);
-        const int share_hi = (int)((long long)total * (part + 1) / split);
-        for (int base = share_lo; base < share_hi; base += kStage) {
-            const int lim = min(kStage, share_hi - base);
-            const int ngroups = (lim + 31) >> 5;
-            // this lane's own slot in the batch (self exclusion), -1 when elsewhere
-            const int own = (g_own >= base && g_own < base + lim) ? g_own - base : -1;
-            // ---- stage [base, base + lim) of the concatenated segments: only the segments
-            // that overlap it (a warp-uniform ballot over the segment lanes)
-            uint32_t overlap = __ballot_sync(0xffffffffu, lane < nseg && seg_len > 0 && seg_pre < base + lim &&
-                                                              seg_pre + seg_len > base);
-            while (overlap) {
-                const int sg = __ffs(overlap) - 1;
-                overlap &= overlap - 1u;
-                const int pre = __shfl_sync(0xffffffffu, seg_pre, sg);
-                const int len = __shfl_sync(0xffffffffu, seg_len, sg);
-                const int beg = __shfl_sync(0xffffffffu, seg_beg, sg);
-                const float sx = __shfl_sync(0xffffffffu, seg_sx, sg);
-                const float sy = __shfl_sync(0xffffffffu, seg_sy, sg);
-                const float sz = __shfl_sync(0xffffffffu, seg_sz, sg);
-                const int lo = max(pre, base), hi = min(pre + len, base + lim);
-                for (int g = lo + lane; g < hi; g += 32) {
-                    const int slot = g - base;
-                    const int j = beg + (g - pre);
-                    const float4 p = CF_IN_BOUNDS(j, c.n) ? pos_sorted[j] : make_float4(kFar, kFar, kFar, 0.0f);
-                    float* xy = reinterpret_cast<float*>(&w.xy[slot >> 1]);
-                    float* zc = reinterpret_cast<float*>(&w.zc[slot >> 1]);
-                    const float x = p.x + sx, y = p.y + sy, z = p.z + sz;
-                    xy[slot & 1] = x;
-                    xy[2 + (slot & 1)] = y;
-                    zc[slot & 1] = z;
-                    zc[2 + (slot & 1)] = fmaf(z, z, fmaf(y, y, x * x));
-                    w.meta[slot] = (uint32_t)j | ((__float_as_uint(p.w) & (kTableStride - 1)) << kTypeShift);
-                }
-            }
-            // padding up to a whole group: never passes the filter (at +kFar on generic
-            // grids, |c|^2 = kFar otherwise)
-            for (int slot = lim + lane; slot < ngroups * 32; slot += 32) {
-                float* xy = reinterpret_cast<float*>(&w.xy[slot >> 1]);
-                float* zc = reinterpret_cast<float*>(&w.zc[slot >> 1]);
-                const float far = kGeneric ? kFar : 0.0f;
-                xy[slot & 1] = far;
-                xy[2 + (slot & 1)] = far;
-                zc[slot & 1] = far;
-                zc[2 + (slot & 1)] = kFar;
-            }
-            __syncwarp();
-            const int own_g = own >> 5;  // -1 when the home is not in this batch
-            const uint32_t own_keep = ~(1u << (own & 31));
-            int hits = 0;      // set bits of this lane in the batch
-            uint32_t nz = 0u;  // bit g: group g has a set bit
-
-            // ---- filter: one bit per candidate
-            if (kGeneric) {
-                const float4 hh = make_float4(hxf, hyf, hzf, 0.0f);
-                for (int gi = 0; gi < ngroups; gi++) {
-                    uint32_t m = 0;
-                    for (int q = 0; q < 32; q++) {
-                        const int slot = gi * 32 + q;
-                        if (slot >= lim) break;
-                        float dx, dy, dz;
-                        const int pb = (slot >> 1) * 4 + (slot & 1);
-                        staged_delta<true>(c, xyf[pb], xyf[pb + 2], zcf[pb], hh, H, dx, dy, dz);
-                        const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-                        if (d2 < thr_f) m |= 1u << q;
-                    }
-                    const uint32_t mm = gi == own_g ? (m & own_keep) : m;
-                    w.mask[gi * 32 + lane] = mm;
-                    hits += __popc(mm);
-                    nz |= (mm != 0u ? 1u : 0u) << gi;
-                }
-            } else {
-                for (int gi = 0; gi < ngroups; gi++) {
-                    // |c'|^2 + (|h'|^2 - bound) - 2 h'.c', two candidates per chain; the sign
-                    // bit of each result is shifted into the mask (last pair first, so pair p
-                    // lands on bits 2p, 2p + 1)
-                    uint32_t m = 0;
-#pragma unroll
-                    for (int p = 15; p >= 0; p--) {
-                        const float4 a = w.xy[gi * 16 + p];
-                        const float4 b = w.zc[gi * 16 + p];
-                        float2 q = __fadd2_rn(make_float2(b.z, b.w), H.k);
-                        q = __ffma2_rn(make_float2(a.x, a.y), H.m2x, q);
-                        q = __ffma2_rn(make_float2(a.z, a.w), H.m2y, q);
-                        q = __ffma2_rn(make_float2(b.x, b.y), H.m2z, q);
-                        m = __funnelshift_l(__float_as_uint(q.y), m, 1);
-                        m = __funnelshift_l(__float_as_uint(q.x), m, 1);
-                    }
-                    const uint32_t mm = gi == own_g ? (m & own_keep) : m;
-                    w.mask[gi * 32 + lane] = mm;
-                    hits += __popc(mm);
-                    nz |= (mm != 0u ? 1u : 0u) << gi;
-                }
-            }
-
-            // ---- drain: every set bit of this lane in slot order, kPer per trip.  The trip
-            // count is uniform over the warp (the largest hit count over kPer), and a lane
-            // whose current group mask runs out moves to the next non-empty group (the
-            // lowest remaining bit of nz) with one load: no nested loop, no vote per trip.
-            // A lane with fewer than kPer hits left repeats its first pair of the trip
-            // without accumulating it.
-            //
-            // Lane pairing (kBalance): the trip count is the busiest lane's, so lanes are
-            // paired heaviest with lightest (a bitonic sort of the hit counts) and the light
-            // lane of a pair, once its own hits are done (rounded up to a whole trip), takes
-            // the top part of its partner's hits with its partner's home, accumulating them
-            // apart; the partner adds that partial after the trips.  Each pair's work is then
-            // about half its total.
-            if constexpr (kBal) {
-                // ---- balanced drain: the batch's H hits, home by home in lane order, form a
-                // task line; lane l takes tasks [l H / 32, (l + 1) H / 32), walking each home's
-                // set bits with that home's position (a new home starts a new trip), and
-                // writes the partial sums of each (lane, home) piece to part[lane + rank of
-                // the home]; each home then adds its pieces in lane order (deterministic).
-                w.pr.nzw[lane] = nz;
-                w.pr.hits[lane] = hits;
-                int pre = hits;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, pre, o);
-                    if (lane >= o) pre += v;
-                }
-                const int H_all = __shfl_sync(0xffffffffu, pre, 31);
-                pre -= hits;  // exclusive prefix: where this lane's home starts on the task line
-                const uint32_t has = __ballot_sync(0xffffffffu, hits > 0);
-                const int t0 = (lane * H_all) >> 5, t1 = ((lane + 1) * H_all) >> 5;
-                int left = t1 - t0;
-                // the home of task t0: the last home whose start is <= t0 (a home with hits)
-                int hm = 0;
-#pragma unroll
-                for (int step = 16; step >= 1; step >>= 1) {
-                    const int cand = hm + step;
-                    if (__shfl_sync(0xffffffffu, pre, cand) <= t0) hm = cand;
-                }
-                const int rank0 = t0 - __shfl_sync(0xffffffffu, pre, hm);
-                __syncwarp();
-                uint32_t m = 0u;
-                int gi = 0, inh = 0;
-                if (left > 0) {
-                    // skip the first rank0 set bits of home hm
-                    int r = rank0;
-                    nz = w.pr.nzw[hm];
-                    for (;;) {
-                        gi = __ffs(nz) - 1;
-                        m = w.mask[gi * 32 + hm];
-                        const int cnt = __popc(m);
-                        if (r < cnt) break;
-                        r -= cnt;
-                        nz &= nz - 1u;
-                    }
-                    for (; r > 0; r--) m &= m - 1u;
-                    inh = min(left, w.pr.hits[hm] - rank0);
-                    const float4 ph = w.pr.home_h[hm];
-                    const float4 pm = w.pr.home_m2[hm];
-                    L.h = ph;
-                    L.tp = __float_as_uint(ph.w) & kTypeMask;
-                    H.m2x.x = pm.x;
-                    H.m2y.x = pm.y;
-                    H.m2z.x = pm.z;
-                }
-                const bool worked = left > 0;
-                // running sums of this lane's own home stay in (sx, sy, sz, sc); L accumulates pieces
-                const float sx = L.fx, sy = L.fy, sz = L.fz;
-                const int sc = L.count;
-                L.fx = L.fy = L.fz = 0.0f;
-                L.count = 0;
-                while (__any_sync(0xffffffffu, left > 0)) {
-                    if (left > 0 && inh == 0) {
-                        // this home's tasks are done: its piece goes to part[], the next home starts
-                        w.pr.part[lane + __popc(has & ((1u << hm) - 1u))] =
-                            make_float4(L.fx, L.fy, L.fz, __int_as_float(L.count));
-                        L.fx = L.fy = L.fz = 0.0f;
-                        L.count = 0;
-                        hm = __ffs(has & (0xfffffffeu << hm)) - 1;
-                        nz = w.pr.nzw[hm];
-                        gi = __ffs(nz) - 1;
-                        m = w.mask[gi * 32 + hm];
-                        inh = min(left, w.pr.hits[hm]);
-                        const float4 ph = w.pr.home_h[hm];
-                        const float4 pm = w.pr.home_m2[hm];
-                        L.h = ph;
-                        L.tp = __float_as_uint(ph.w) & kTypeMask;
-                        H.m2x.x = pm.x;
-                        H.m2y.x = pm.y;
-                        H.m2z.x = pm.z;
-                    }
-                    const int nq = min(kPer, inh);
-                    int slot[kPer];
-                    bool valid[kPer];
-#pragma unroll
-                    for (int q = 0; q < kPer; q++) {
-                        valid[q] = q < nq;
-                        if (valid[q] && m == 0u) {
-                            nz &= nz - 1u;
-                            gi = __ffs(nz) - 1;
-                            m = w.mask[gi * 32 + hm];
-                        }
-                        slot[q] = valid[q] ? gi * 32 + (__ffs(m) - 1) : 0;
-                        if (valid[q]) m &= m - 1u;
-                    }
-                    float dx[kPer], dy[kPer], dz[kPer], d2[kPer], wgt[kPer];
-                    uint32_t meta[kPer];
-                    bool inter[kPer];
-                    // (every lane runs this body in every pass of the loop, so the vote is warp-wide)
-                    float sx[kPer], sy[kPer], sz[kPer];
-                    bool band = false;
-#pragma unroll
-                    for (int q = 0; q < kPer; q++) {
-                        staged_xyz(xyf, zcf, slot[q], sx[q], sy[q], sz[q]);
-                        meta[q] = w.meta[slot[q]];
-                        const bool fast = pair_fast<kGeneric, kUniformR>(c, L, H, sx[q], sy[q], sz[q], meta[q], tb,
-                                                                        dx[q], dy[q], dz[q], d2[q]);
-                        inter[q] = fast && valid[q];
-                        band |= valid[q] && !fast;
-                    }
-                    if (__any_sync(0xffffffffu, band)) {
-#pragma unroll
-                        for (int q = 0; q < kPer; q++)
-                            if (valid[q] && !inter[q])
-                                inter[q] = pair_exact<kGeneric, kUniformR>(c, L, w.origin, sx[q], sy[q], sz[q],
-                                                                           meta[q], pos_sorted, tb);
-                    }
-#pragma unroll
-                    for (int q = 0; q < kPer; q++) wgt[q] = pair_weight<kUniformR>(d2[q], meta[q], L, tb, c1u);
-#pragma unroll
-                    for (int q = 0; q < kPer; q++) {
-                        if (inter[q]) {
-                            L.count++;
-                            L.fx = fmaf(dx[q], wgt[q], L.fx);
-                            L.fy = fmaf(dy[q], wgt[q], L.fy);
-                            L.fz = fmaf(dz[q], wgt[q], L.fz);
-                        }
-                    }
-                    inh -= nq;
-                    left -= nq;
-                }
-                if (worked)
-                    w.pr.part[lane + __popc(has & ((1u << hm) - 1u))] =
-                        make_float4(L.fx, L.fy, L.fz, __int_as_float(L.count));
-                __syncwarp();
-                // each home adds its pieces in lane order; back to the lane's own home
-                L.fx = sx;
-                L.fy = sy;
-                L.fz = sz;
-                L.count = sc;
-                if (hits > 0) {
-                    // lanes la..lb hold the home's tasks (those with an empty range, when the
-                    // batch has fewer hits than lanes, hold none)
-                    const int rk = __popc(has & ((1u << lane) - 1u));
-                    const int la = (32 * (pre + 1) - 1) / H_all;
-                    const int lb = (32 * (pre + hits) - 1) / H_all;
-                    for (int l2 = la; l2 <= lb; l2++) {
-                        if (((l2 + 1) * H_all) >> 5 == (l2 * H_all) >> 5) continue;
-                        const float4 v = w.pr.part[l2 + rk];
-                        L.fx += v.x;
-                        L.fy += v.y;
-                        L.fz += v.z;
-                        L.count += __float_as_int(v.w);
-                    }
-                }
-                const float4 oh = w.pr.home_h[lane];
-                const float4 om = w.pr.home_m2[lane];
-                L.h = oh;
-                L.tp = __float_as_uint(oh.w) & kTypeMask;
-                H.m2x.x = om.x;
-                H.m2y.x = om.y;
-                H.m2z.x = om.z;
-            } else {
-            int upto = hits;         // pair indices below upto are valid in the current phase
-            int work = hits;         // pairs this lane walks in the batch
-            int switch_trip = -1;    // trip at which a light lane turns to its partner's hits
-            int partner = lane, fw = 0, src = lane;
-            bool light = false;
-            int fgi = 0;             // where a light lane's share of its partner's hits starts
-            uint32_t fm = 0u, fnz = 0u;
-            if constexpr (kBalance) {
-                uint32_t key = ((uint32_t)hits << 5) | (uint32_t)lane;
-#pragma unroll
-                for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-                    for (int j = k >> 1; j > 0; j >>= 1) {
-                        const uint32_t o = __shfl_xor_sync(0xffffffffu, key, j);
-                        key = (((lane & j) == 0) == ((lane & k) == 0)) ? min(key, o) : max(key, o);
-                    }
-                }
-                // sorted position lane holds key; it pairs with position 31 - lane
-                const uint32_t mate = __shfl_sync(0xffffffffu, key, 31 - lane);
-                w.pr.pairing[key & 31u] = (mate & 31u) | (lane < 16 ? 0x100u : 0u);
-                w.pr.nzw[lane] = nz;
-                __syncwarp();
-                const uint32_t pr = w.pr.pairing[lane];
-                partner = (int)(pr & 31u);
-                light = (pr & 0x100u) != 0u;
-                const int hp = __shfl_sync(0xffffffffu, hits, partner);
-                if (light) {
-                    const int padded = (hits + kPer - 1) / kPer * kPer;
-                    fw = max(0, (hp - padded) >> 1);
-                    work = padded + fw;
-                    if (fw > 0) {
-                        switch_trip = padded / kPer;
-                        // skip the partner's own share, its first hp - fw set bits; the group
-                        // bitmap keeps the current group as its lowest bit, like nz
-                        int skip = hp - fw;
-                        fnz = w.pr.nzw[partner];
-                        while (fnz) {
-                            fgi = __ffs(fnz) - 1;
-                            fm = w.mask[fgi * 32 + partner];
-                            const int cnt = __popc(fm);
-                            if (skip < cnt) break;
-                            skip -= cnt;
-                            fnz &= fnz - 1u;
-                        }
-                        for (; skip > 0; skip--) fm &= fm - 1u;
-                    }
-                } else {
-                    fw = max(0, (hits - (hp + kPer - 1) / kPer * kPer) >> 1);
-                    upto = work = hits - fw;
-                }
-            }
-            const int trips = (__reduce_max_sync(0xffffffffu, work) + kPer - 1) / kPer;
-            int gi = nz ? __ffs(nz) - 1 : 0;
-            uint32_t m = w.mask[gi * 32 + lane];
-            for (int it = 0; it < trips; it++) {
-                if constexpr (kBalance) {
-                    if (it == switch_trip) {
-                        // own hits done: keep their sums, take the partner's home and its top fw hits
-                        w.pr.saved[lane] = make_float4(L.fx, L.fy, L.fz, __int_as_float(L.count));
-                        L.fx = L.fy = L.fz = 0.0f;
-                        L.count = 0;
-                        const float4 ph = w.pr.home_h[partner];
-                        const float4 pm = w.pr.home_m2[partner];
-                        L.h = ph;
-                        L.tp = __float_as_uint(ph.w) & kTypeMask;
-                        H.m2x.x = pm.x;
-                        H.m2y.x = pm.y;
-                        H.m2z.x = pm.z;
-                        src = partner;
-                        gi = fgi;
-                        m = fm;
-                        nz = fnz;
-                        upto = kPer * it + fw;
-                    }
-                }
-                // every lane runs the trip (a lane whose pairs are done has none valid), so the
-                // warp-wide vote below is reached by all 32 lanes in every trip
-                {
-                    int slot[kPer];
-                    bool valid[kPer];
-#pragma unroll
-                    for (int q = 0; q < kPer; q++) {
-                        valid[q] = kPer * it + q < upto;
-                        if (valid[q] && m == 0u) {
-                            nz &= nz - 1u;
-                            gi = __ffs(nz) - 1;  // a later group holds a hit
-                            m = w.mask[gi * 32 + src];
-                        }
-                        slot[q] = valid[q] ? gi * 32 + (__ffs(m) - 1) : (q == 0 ? 0 : slot[0]);
-                        if (valid[q]) m &= m - 1u;
-                    }
-                    float dx[kPer], dy[kPer], dz[kPer], d2[kPer], wgt[kPer];
-                    uint32_t meta[kPer];
-                    bool inter[kPer];
-                    float sx[kPer], sy[kPer], sz[kPer];
-                    bool band = false;
-#pragma unroll
-                    for (int q = 0; q < kPer; q++) {
-                        staged_xyz(xyf, zcf, slot[q], sx[q], sy[q], sz[q]);
-                        meta[q] = w.meta[slot[q]];
-                        const bool fast = pair_fast<kGeneric, kUniformR>(c, L, H, sx[q], sy[q], sz[q], meta[q], tb,
-                                                                        dx[q], dy[q], dz[q], d2[q]);
-                        inter[q] = fast && valid[q];
-                        band |= valid[q] && !fast;
-                    }
-                    // pairs within rounding of the threshold are rare: the exact test runs only in
-                    // the trips where some lane of the warp holds one
-                    if (__any_sync(0xffffffffu, band)) {
-#pragma unroll
-                        for (int q = 0; q < kPer; q++)
-                            if (valid[q] && !inter[q])
-                                inter[q] = pair_exact<kGeneric, kUniformR>(c, L, w.origin, sx[q], sy[q], sz[q],
-                                                                           meta[q], pos_sorted, tb);
-                    }
-#pragma unroll
-                    for (int q = 0; q < kPer; q++) wgt[q] = pair_weight<kUniformR>(d2[q], meta[q], L, tb, c1u);
-#pragma unroll
-                    for (int q = 0; q < kPer; q++) {
-                        if (inter[q]) {
-                            L.count++;
-                            L.fx = fmaf(dx[q], wgt[q], L.fx);
-                            L.fy = fmaf(dy[q], wgt[q], L.fy);
-                            L.fz = fmaf(dz[q], wgt[q], L.fz);
-                        }
-                    }
-                }
-            }
-            if constexpr (kBalance) {
-                // a light lane that switched holds its partner's partial: hand it over and
-                // take back its own sums and home
-                const float px = __shfl_sync(0xffffffffu, L.fx, partner);
-                const float py = __shfl_sync(0xffffffffu, L.fy, partner);
-                const float pz = __shfl_sync(0xffffffffu, L.fz, partner);
-                const int pc = __shfl_sync(0xffffffffu, L.count, partner);
-                if (switch_trip >= 0) {
-                    const float4 sv = w.pr.saved[lane];
-                    L.fx = sv.x;
-                    L.fy = sv.y;
-                    L.fz = sv.z;
-                    L.count = __float_as_int(sv.w);
-                    const float4 oh = w.pr.home_h[lane];
-                    const float4 om = w.pr.home_m2[lane];
-                    L.h = oh;
-                    L.tp = __float_as_uint(oh.w) & kTypeMask;
-                    H.m2x.x = om.x;
-                    H.m2y.x = om.y;
-                    H.m2z.x = om.z;
-                } else if (!light && fw > 0) {
-                    L.fx += px;
-                    L.fy += py;
-                    L.fz += pz;
-                    L.count += pc;
-                }
-            }
-            }
-            __syncwarp();
-        }
-    }
-    if (split > 1) {
-        // the item's warps meet at a named barrier (id 1 + item slot, 32 * split threads);
-        // part 0 adds the partial sums in part order, so the result is deterministic
-        if (part != 0) s_part[warp][lane] = make_float4(L.fx, L.fy, L.fz, __int_as_float(L.count));
-        item_barrier(warp / split, 32 * split);
-        if (part != 0) return;
-        for (int q = 1; q < split; q++) {
-            const float4 v = s_part[warp + q][lane];
-            L.fx += v.x;
-            L.fy += v.y;
-            L.fz += v.z;
-            L.count += __float_as_int(v.w);
-        }
-    }
-    if (!active) return;
-
-    // density-adaptive scale and integrator (ParticleSimulation.cu:136-161)
-    const uint32_t i = vals_sorted[t];
-    if (!CF_IN_BOUNDS(i, c.n)) return;
-    const int prev = counts[i];
-    const float avg = __fmul_rn((float)(L.count + prev), 0.5f);
+// Density-adaptive scale, integrator and wrap of particle i at h with force sum
+// f and n neighbours (ParticleSimulation.cu:136-165).
+__device__ __forceinline__ void integrate(const StepConsts& c, const float4& h, const float4& f, int n, uint32_t i,
+                                          float4* __restrict__ pos, float4* __restrict__ vel,
+                                          float4* __restrict__ acc, int* __restrict__ counts)
+{
+    const float avg = __fmul_rn((float)(n + counts[i]), 0.5f);
     const float density = fminf(__fdiv_rn(avg, (float)c.max_expected_neighbors), 1.0f);
     const float adapt = __fsub_rn(1.0f, __fmul_rn(__fsub_rn(1.0f, c.balance), density));
-    const float scale = __fmul_rn(c.force_multiplier, adapt);
-    const float fx = __fmul_rn(L.fx, scale);
-    const float fy = __fmul_rn(L.fy, scale);
-    const float fz = __fmul_rn(L.fz, scale);
+    const float strength = __fmul_rn(c.force_multiplier, adapt);
+    const float fx = __fmul_rn(f.x, strength);
+    const float fy = __fmul_rn(f.y, strength);
+    const float fz = __fmul_rn(f.z, strength);
     const float4 v = vel[i];
     const float vx = __fadd_rn(__fmul_rn(v.x, c.friction), __fmul_rn(fx, c.delta_t));
     const float vy = __fadd_rn(__fmul_rn(v.y, c.friction), __fmul_rn(fy, c.delta_t));
     const float vz = __fadd_rn(__fmul_rn(v.z, c.friction), __fmul_rn(fz, c.delta_t));
-    float px = __fadd_rn(L.h.x, __fmul_rn(vx, c.delta_t));
-    float py = __fadd_rn(L.h.y, __fmul_rn(vy, c.delta_t));
-    float pz = __fadd_rn(L.h.z, __fmul_rn(vz, c.delta_t));
+    float px = __fadd_rn(h.x, __fmul_rn(vx, c.delta_t));
+    float py = __fadd_rn(h.y, __fmul_rn(vy, c.delta_t));
+    float pz = __fadd_rn(h.z, __fmul_rn(vz, c.delta_t));
     px = wrap_pos(__fadd_rn(px, c.ext[0]), c.ext[0]);
     py = wrap_pos(__fadd_rn(py, c.ext[1]), c.ext[1]);
     pz = wrap_pos(__fadd_rn(pz, c.ext[2]), c.ext[2]);
-    pos[i] = make_float4(px, py, pz, L.h.w);
+    pos[i] = make_float4(px, py, pz, h.w);
     vel[i] = make_float4(vx, vy, vz, 0.0f);
     acc[i] = make_float4(fx, fy, fz, 0.0f);
-    counts[i] = L.count;
+    counts[i] = n;
+}
+
+// kBlockWarps warps per block, kMinBlocks resident blocks the register budget
+// is sized for.  Shared memory: the warps' staging, the force tables (one for a
+// plain world, one per item of the block in a batch) and, without a uniform
+// radius, (A / eff, c1, certain-interaction bound) per type pair.
+template <int kBlockWarps, int kMinBlocks, bool kGeneric, bool kUniformR>
+__global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
+    step_force_kernel(StepConsts c, const PairTables* __restrict__ tables, const float4* __restrict__ pos_sorted,
+                      const uint32_t* __restrict__ vals_sorted, const uint32_t* __restrict__ cell_off,
+                      const Item* __restrict__ items, const int* __restrict__ n_items, int max_items,
+                      float4* __restrict__ pos, float4* __restrict__ vel, float4* __restrict__ acc,
+                      int* __restrict__ counts)
+{
+    // pairs per drain trip: three where the registers allow (more independent work in each)
+    constexpr int kPer = kBlockWarps * kMinBlocks > 20 ? 2 : 3;
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    const int T = c.num_types, TT = T * T;
+    const bool one_world = c.grid.worlds == 1;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    WarpSmem& w = reinterpret_cast<WarpSmem*>(s_dyn)[warp];
+    float4* s_pair = reinterpret_cast<float4*>(s_dyn + sizeof(WarpSmem) * kBlockWarps);
+    float* s_force = reinterpret_cast<float*>(s_pair + (kUniformR ? 0 : TT));
+
+    // the item and its count are read together (the array holds max_items entries)
+    const int split = c.split;
+    const int part = warp & (split - 1);
+    const int slot_of_item = warp / split;
+    const int item = blockIdx.x * (kBlockWarps / split) + slot_of_item;
+    Item it{0, 0, 0, 0};
+    if (item < max_items) it = items[item];
+    if (item >= *n_items) it.count = 0;
+    if (!kUniformR) {
+        for (int e = threadIdx.x; e < TT; e += 32 * kBlockWarps) {
+            const float2 v = tables->pair_compact[e];  // 1 / eff, certain-interaction bound
+            s_pair[e] = make_float4(c.attraction * v.x, c.neg_k_log2e * v.x * v.x, v.y, 0.0f);
+        }
+    }
+    if (one_world) {
+        for (int e = threadIdx.x; e < TT; e += 32 * kBlockWarps) s_force[e] = c.world_force[e];
+    }
+    if (one_world || !kUniformR) __syncthreads();
+    if (it.count == 0) return;  // the item's other warps leave too: no barrier is pending
+    // (bounds-checked build) the item's particles lie in [0, n): else the item's warps skip it
+    if (!CF_IN_BOUNDS(it.count - 1, 32) || !CF_IN_BOUNDS(it.first, c.n) || !CF_IN_BOUNDS(it.first + it.count - 1, c.n))
+        return;
+    if (!one_world) {
+        // each of the item's warps writes all of the item's table (the same values)
+        s_force += slot_of_item * TT;
+        const float* f = c.world_force + (size_t)it.world * TT;
+        for (int e = lane; e < TT; e += 32) s_force[e] = f[e];
+    }
+    // lane 4 g + t holds home g + 8 t: the row whose mask the filter's quad of lanes leaves in it
+    const int home = (lane >> 2) + 8 * (lane & 3);
+    const bool active = home < it.count;
+    const int t = it.first + (active ? home : 0);
+    const float4 h = pos_sorted[t];
+    const uint32_t i = vals_sorted[t];
+    // a type outside [0, T) is reported by the cell list's hash; it stays inside the tables here
+    const uint32_t type = min(__float_as_uint(h.w) & kTypeMask, (uint32_t)(T - 1));
+    const int mx = c.grid.m[0], my = c.grid.m[1], mz = c.grid.m[2];
+    const int yc = it.yz & 0xffff, zc = it.yz >> 16;
+    const int hx = x_cell(h.x, c.grid.inv[0], mx);
+    const int last = it.count - 1;
+    const int x0 = __shfl_sync(kAll, hx, 0);
+    const int x1 = __shfl_sync(kAll, hx, ((last & 7) << 2) | (last >> 3));
+    if (lane == 0) w.c[0] = make_float4(kFar, kFar, kFar, 0.0f);
+    w.row[0][lane] = 0x80000000u;
+    // no pair of this home's type interacts at or above thr_f (a contracted squared distance)
+    const float thr_f = kUniformR ? c.thr_filter : tables->filter_row[type];
+    const uint32_t force_at = pinned((uint32_t)__cvta_generic_to_shared(s_force + type * T));
+    const uint32_t pair_at = pinned((uint32_t)__cvta_generic_to_shared(s_pair + type * T));
+    // slot b of row r: + (32 r + b) 16
+    const uint32_t slots_at = pinned((uint32_t)__cvta_generic_to_shared(&w.c[0]) - 31 * 16);
+    const uint32_t masks_at = pinned((uint32_t)__cvta_generic_to_shared(&w.row[0][lane]));
+
+    // the item's sums so far, in part 0 (units are added in order)
+    float sum_x = 0.0f, sum_y = 0.0f, sum_z = 0.0f;
+    int sum_n = 0;
+    bool first_round = true;
+
+    // x sub-ranges whose union (range plus one cell each side) fits in the box
+    const int width = kGeneric ? mx : (mx - 2);
+    const int passes = kGeneric || x1 - x0 < width ? 1 : (x1 - x0 + width) / width;
+    for (int pass = 0; pass < passes; pass++) {
+        const int px0 = kGeneric ? x0 : x0 + pass * width;
+        const int px1 = kGeneric ? x1 : min(x1, px0 + width - 1);
+        const bool mine = active && (kGeneric || (hx >= px0 && hx <= px1));
+        const int xlo = mx > 1 ? px0 - 1 : 0;
+        const int xhi = mx > 1 ? min(px1 + 1, xlo + mx - 1) : 0;  // inclusive, at most mx cells
+
+        // segments: lane 2*row + half describes one contiguous range of the snapshot and
+        // its periodic shift less the origin (zero on generic grids)
+        const int ny = !kGeneric || my > 1 ? 3 : 1, nz = !kGeneric || mz > 1 ? 3 : 1;
+        int seg_beg = 0, seg_len = 0;
+        uint32_t shift = 0u;
+        {
+            const int row = lane >> 1, half = lane & 1;
+            const int dz = ny == 3 ? (row * 11) >> 5 : row;  // row / ny (row < 16)
+            const int yy = yc + (row - dz * ny) - (ny > 1 ? 1 : 0), zz = zc + dz - (nz > 1 ? 1 : 0);
+            const uint32_t cy = yy < 0 ? 1u : (yy >= my ? 2u : 0u);
+            const uint32_t cz = zz < 0 ? 1u : (zz >= mz ? 2u : 0u);
+            // split [xlo, xhi] at the box edge: half 0 is the in-box part, half 1 the wrapped part
+            int xa = xlo, xb = xhi;
+            uint32_t cx = 0u;
+            if (xlo < 0) {
+                if (half == 0) xa = 0;
+                else { xa = xlo + mx; xb = mx - 1; cx = 1u; }
+            } else if (xhi >= mx) {
+                if (half == 0) xb = mx - 1;
+                else { xa = 0; xb = xhi - mx; cx = 2u; }
+            } else if (half == 1) {
+                xb = xa - 1;
+            }
+            const uint32_t base = (uint32_t)it.world * (uint32_t)c.grid.cells_w +
+                                  (uint32_t)((wrap_index(zz, mz) * my + wrap_index(yy, my)) * mx);
+            if (row < ny * nz && xb >= xa && CF_IN_BOUNDS(base + xb + 1, c.grid.cells + 1)) {
+                seg_beg = (int)cell_off[base + xa];
+                seg_len = (int)cell_off[base + xb + 1] - seg_beg;
+                if (!CF_IN_BOUNDS(seg_len, c.n + 1) || !CF_IN_BOUNDS(seg_beg + seg_len, c.n + 1)) seg_len = 0;
+            }
+            shift = cx | cy << 2 | cz << 4;
+        }
+
+        // Staging origin per axis (stencil_origin) for the stencil box (cells xlo..xhi,
+        // yc-1..yc+1, zc-1..zc+1 in shifted coordinates): every staged candidate and the homes
+        // lie within (rx, ry, rz) of it.  The filter works on them scaled by a power of two
+        // that puts the box's radius in [64, 128) (squares stay below 65504) and rounded to
+        // half precision: at most 2^-11 of the coordinate each, or 2^-25 where it is tiny, and
+        // 2^-23 of the box for the contracted scaling, so two points' distance moves by at
+        // most the norm of (2^-10 r + 2^-22 box) over the axes.
+        // The sums (products exact in 32 bits; |c|^2 and |h|^2 - B as two halves, 2^-22 each;
+        // eight terms of at most 4 R^2 together) are off by less than 2^-16 R^2.
+        float ox = 0.0f, oy = 0.0f, oz = 0.0f, scale = 1.0f;
+        uint32_t a[4];
+        if (!kGeneric) {
+            float rx, ry, rz;
+            stencil_origin(xlo, xhi, c.cell[0], ox, rx);
+            stencil_origin(yc - 1, yc + 1, c.cell[1], oy, ry);
+            stencil_origin(zc - 1, zc + 1, c.cell[2], oz, rz);
+            const int e = (int)(__float_as_uint(fmaxf(rx, fmaxf(ry, rz))) >> 23);
+            scale = __uint_as_float((uint32_t)min(max(260 - e, 1), 254) << 23);
+            rx *= scale;
+            ry *= scale;
+            rz *= scale;
+            const float r2 = fmaf(rz, rz, fmaf(ry, ry, rx * rx));
+            const float ex = fmaf(rx, 0x1p-10f, c.ext[0] * scale * 0x1p-22f),
+                        ey = fmaf(ry, 0x1p-10f, c.ext[1] * scale * 0x1p-22f),
+                        ez = fmaf(rz, 0x1p-10f, c.ext[2] * scale * 0x1p-22f);
+            const float reach = sqrt_approx(fmaxf(thr_f, 0.0f)) * scale + sqrt_approx(fmaf(ez, ez, fmaf(ey, ey, ex * ex)));
+            const float bnd = fmaf(reach * reach, 1.0f + 0x1p-16f, r2 * 0x1p-16f);
+            const uint32_t xy = half2_bits((h.x - ox) * scale, (h.y - oy) * scale);
+            const float qx = half_lo(xy), qy = half_hi(xy), qz = half_lo(half2_bits((h.z - oz) * scale, 0.0f));
+            const float k = fmaf(qz, qz, fmaf(qy, qy, qx * qx)) - bnd;
+            const float khi = half_lo(half2_bits(k, 0.0f));
+            // the home's row of the A operand, k = 0..7: -2 h (3), 1, 1, k hi, 0, k lo (a home that
+            // tests nothing in this pass: 60000 beside any |c|^2); fragment word t of the four
+            // rows that this lane's quad holds, exchanged through shared memory
+            __syncwarp();
+            *reinterpret_cast<uint4*>(&w.row[1][0] + lane * 4) =
+                mine && thr_f > 0.0f ? make_uint4(half2_bits(-2.0f * qx, -2.0f * qy), half2_bits(-2.0f * qz, 1.0f),
+                                                  half2_bits(1.0f, khi), half2_bits(0.0f, k - khi))
+                                     : make_uint4(0u, 0x3c000000u, half2_bits(1.0f, 60000.0f), 0u);
+            __syncwarp();
+            const uint32_t* quad = &w.row[1][0] + (lane & ~3) * 4 + (lane & 3);
+#pragma unroll
+            for (int q = 0; q < 4; q++) a[q] = quad[4 * q];
+        }
+        int seg_pre = seg_len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kAll, seg_pre, o);
+            if (lane >= o) seg_pre += v;
+        }
+        const int total = __shfl_sync(kAll, seg_pre, 31);
+        seg_pre -= seg_len;
+        // the home's place in the list: its cell is in the centre row's in-box part
+        const int seg_c = 2 * ((nz > 1 ? ny : 0) + (ny > 1 ? 1 : 0));
+        const int own = t - __shfl_sync(kAll, seg_beg - seg_pre, seg_c);
+        // the list's segments without the empty ones
+        const uint32_t full = __ballot_sync(kAll, seg_len > 0);
+        const bool shifted = __any_sync(kAll, seg_len > 0 && shift != 0u);
+        int* starts = reinterpret_cast<int*>(&w.row[0][kStartAt]);
+        if (seg_len > 0) {
+            const int k = __popc(full & ((1u << lane) - 1u));
+            starts[k] = seg_pre;
+            if (lane == top_bit(full)) starts[k + 1] = 0x7fffffff;
+            w.seg[k] = make_float4(code_shift(shift & 3u, c.ext[0]) - ox, code_shift((shift >> 2) & 3u, c.ext[1]) - oy,
+                                   code_shift(shift >> 4, c.ext[2]) - oz, __int_as_float(seg_beg - seg_pre));
+        }
+        if (lane == 0) {
+            w.row[0][kOriginAt] = __float_as_uint(shifted ? ox : 0.0f);
+            w.row[0][kOriginAt + 1] = __float_as_uint(shifted ? oy : 0.0f);
+            w.row[0][kOriginAt + 2] = __float_as_uint(shifted ? oz : 0.0f);
+        }
+        __syncwarp();
+        // the drain's coordinates: relative to the origin where some segment is shifted, raw elsewhere
+        const float hpx = shifted ? h.x - ox : h.x, hpy = shifted ? h.y - oy : h.y, hpz = shifted ? h.z - oz : h.z;
+
+        // units: the list's entries dealt out in turn (entry g to unit g mod units), so that every
+        // unit holds an even share of every home's neighbours and its busiest lane stands out
+        // less than it does over a stretch of the list
+        const int units = (total + kUnit - 1) / kUnit;
+        const float per_unit = __fdividef(1.0f, (float)units);
+        int own_slot, own_unit, q0, r0, q1, r1;  // (this lane's segment: its start is entry q0 of unit r0, its end q1 of r1)
+        int total_q, total_r;
+        deal(total, units, per_unit, total_q, total_r);
+        deal(own, units, per_unit, own_slot, own_unit);
+        deal(seg_pre, units, per_unit, q0, r0);
+        deal(seg_pre + seg_len, units, per_unit, q1, r1);
+        for (int u0 = 0; u0 < units; u0 += split, first_round = false) {
+            // (before any warp stages over partial sums that part 0 may still be reading)
+            if (split > 1 && !first_round) item_barrier(slot_of_item, 32 * split);
+            const int unit = u0 + part;
+            float fx = 0.0f, fy = 0.0f, fz = 0.0f;
+            int count = 0;
+            if (unit < units) {
+                // ---- stage the unit's groups
+                const int entries = total_q + (unit < total_r ? 1 : 0);
+                const int ngroups = (entries + 31) >> 5;
+                // the slot's column and fragment, so that its sign arrives at its bit of the mask: bit
+                // 4 k + 3 - t is column 2 t + j of fragment n, k = 0..7: (n, j) = (2, 0), (0, 0),
+                // (2, 1), (0, 1), (3, 0), (1, 0), (3, 1), (1, 1)
+                uint32_t* frag = w.row[1] + (2 * (3 - (lane & 3)) + ((lane >> 3) & 1)) * 4 + (lane & 4 ? 0 : 2) + (lane >> 4);
+                // the unit's part of each segment: slots [slot0, slot1), list entry slot * units + unit
+                const int slot0 = q0 + (unit < r0 ? 1 : 0), slot1 = q1 + (unit < r1 ? 1 : 0);
+                const bool has = slot1 > slot0;
+                const uint32_t parts = __ballot_sync(kAll, has);
+                int2* part_rec = reinterpret_cast<int2*>(&w.row[0][kPartAt]);
+                if (has)
+                    part_rec[__popc(parts & ((1u << lane) - 1u))] =
+                        make_int2(seg_beg - seg_pre + unit, __popc(full & ((1u << lane) - 1u)));
+                __syncwarp();
+                // every position in flight at once (asynchronous copies: one round trip to L2 per
+                // unit); a slot's segment is the count of segments that start at or before it
+                const uint32_t start_bit = has ? 1u << (slot0 & 31) : 0u;
+                const int start_group = slot0 >> 5;
+                int before = -1;
+                for (int gi = 0; gi < ngroups; gi++) {
+                    const uint32_t begins = __reduce_or_sync(kAll, start_group == gi ? start_bit : 0u);
+                    const int2 rec = part_rec[before + __popc(begins & (0xffffffffu >> (31 - lane)))];
+                    before += __popc(begins);
+                    const int slot = gi * 32 + lane, j = rec.x + slot * units;
+                    copy_async16(slot < entries && CF_IN_BOUNDS(j, c.n), slots_at + 512 + 16 * slot, pos_sorted + j);
+                    if (shifted) w.row[1 + gi][lane] = (uint32_t)rec.y;
+                }
+                copy_async_wait();
+                __syncwarp();
+#pragma unroll 2
+                for (int gi = 0; gi < ngroups; gi++) {
+                    float4& slot = w.c[1 + gi * 32 + lane];
+                    float4 p = slot;
+                    const uint32_t other = min(__float_as_uint(p.w) & kTypeMask, (uint32_t)(T - 1));
+                    p.w = __uint_as_float(4u * other);
+                    if (!kGeneric) {
+                        float fx, fy, fz;
+                        if (shifted) {
+                            const float4 add = w.seg[w.row[1 + gi][lane]];
+                            p.x += add.x;
+                            p.y += add.y;
+                            p.z += add.z;
+                            fx = p.x * scale;
+                            fy = p.y * scale;
+                            fz = p.z * scale;
+                            __syncwarp();  // every lane has read the group's segments
+                        } else {
+                            fx = fmaf(p.x, scale, -ox * scale);
+                            fy = fmaf(p.y, scale, -oy * scale);
+                            fz = fmaf(p.z, scale, -oz * scale);
+                        }
+                        const uint32_t xy = half2_bits(fx, fy);
+                        const uint32_t z0 = half2_bits(fz, 0.0f);
+                        const float qx = half_lo(xy), qy = half_hi(xy), qz = half_lo(z0);
+                        const float sq = fmaf(qz, qz, fmaf(qy, qy, qx * qx));
+                        const uint32_t s_hi = half2_bits(0.0f, sq);
+                        frag[96 * gi] = xy;
+                        frag[96 * gi + 32] = z0 | s_hi;
+                        frag[96 * gi + 64] = half2_bits(sq - half_hi(s_hi), 1.0f);
+                    }
+                    slot = p;
+                }
+                __syncwarp();
+                if (!kGeneric && (entries & 31) != 0 && lane >= (entries & 31)) {
+                    // padding up to a whole group: at the origin, with a square (60000 + 60000) that no
+                    // home passes
+                    frag[96 * ngroups - 96] = 0u;
+                    frag[96 * ngroups - 64] = 0x7b530000u;
+                    frag[96 * ngroups - 32] = 0x3c007b53u;
+                }
+                __syncwarp();
+                int hits = 0;      // set bits of this lane in the unit
+                uint32_t nz = 1u;  // bit 0: the sentinel's row; bit 1 + g: group g has a set bit
+
+                // ---- filter: one bit per candidate
+                for (int gi = 0; gi < ngroups; gi++) {
+                    uint32_t m;
+                    if (kGeneric) {
+                        // an idle home sits at -kFar, far from every candidate
+                        const float gx = mine ? h.x : -kFar, gy = mine ? h.y : -kFar, gz = mine ? h.z : -kFar;
+                        const int lim = entries - gi * 32;
+                        m = 0u;
+                        for (int q = 0; q < 32 && q < lim; q++) {
+                            const float4 p = w.c[1 + gi * 32 + q];
+                            const float dx = wrap_ref(p.x - gx, c.ext[0], c.half[0]);
+                            const float dy = wrap_ref(p.y - gy, c.ext[1], c.half[1]);
+                            const float dz = wrap_ref(p.z - gz, c.ext[2], c.half[2]);
+                            if (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) < thr_f) m |= 1u << q;
+                        }
+                    } else {
+                        const uint4 b = *reinterpret_cast<const uint4*>(
+                            w.row[1 + gi] + min(lane & 3, 2) * 32 + (lane >> 2) * 4);
+                        const uint32_t bn[4] = {b.x, b.y, b.z, b.w};
+                        uint32_t d[4][4];
+#pragma unroll
+                        for (int n = 0; n < 4; n++) mma_32x8(a, bn[n], d[n]);
+                        // row q's eight sign bits: the top bytes of its four words' halves side by side in
+                        // two words, the second shifted by four, so bit 3 of every nibble is a sign
+                        uint32_t r[4];
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const uint32_t lo = __byte_perm(d[0][q], d[1][q], 0x7531),
+                                           hi = __byte_perm(d[2][q], d[3][q], 0x7531);
+                            r[q] = bit_select(lo, hi >> 4, 0x80808080u);
+                        }
+                        // the four rows' signs into one word, row q at bit 3 - q of every nibble; then a
+                        // 4 x 4 transposition of the nibbles' bits over the quad leaves in lane 4 g + t the
+                        // whole row g + 8 t, the signs of lane 4 g + t' at bit 3 - t' of every nibble
+                        m = bit_select(bit_select(r[0], r[1] >> 1, 0x88888888u),
+                                       bit_select(r[2], r[3] >> 1, 0x88888888u) >> 2, 0xccccccccu);
+                        uint32_t o = __shfl_xor_sync(kAll, m, 2);
+                        m = bit_select(m, __funnelshift_l(o, o, lane & 2 ? 2 : 30), lane & 2 ? 0x33333333u : 0xccccccccu);
+                        o = __shfl_xor_sync(kAll, m, 1);
+                        m = bit_select(m, __funnelshift_l(o, o, lane & 1 ? 1 : 31), lane & 1 ? 0x55555555u : 0xaaaaaaaau);
+                    }
+                    if (unit == own_unit && gi == own_slot >> 5) m &= ~(1u << (own_slot & 31));
+                    __syncwarp();  // every lane has read the group's words
+                    w.row[1 + gi][lane] = m;
+                    hits += __popc(m);
+                    nz |= m != 0u ? 2u << gi : 0u;
+                }
+
+                // ---- drain: every set bit of this lane, highest first, kPer per trip.  The trip
+                // count is uniform over the warp; a lane whose mask runs out moves to its next
+                // non-empty row with one load, and one with no hit left stays at row 0, whose one
+                // bit is the sentinel.
+                __syncwarp();
+                const int trips = (__reduce_max_sync(kAll, hits) + kPer - 1) / kPer;
+                int r = top_bit(nz);
+                uint32_t m = r ? w.row[r][lane] : 0x80000000u;
+                uint32_t row_at = slots_at + 512 * r;
+                // pairs within rounding of the threshold wait: the last one's slot and how many
+                uint32_t open_at = 0u;
+                int open = 0;
+                for (int trip = 0; trip < trips; trip++) {
+                    uint32_t at[kPer];
+                    float4 p[kPer];
+#pragma unroll
+                    for (int q = 0; q < kPer; q++) {
+                        // the slot of the mask's top bit; the bit cleared; if it was the row's last,
+                        // the next row with a bit (predicated: no divergence in the trip)
+                        asm volatile("{\n\t.reg .pred z;\n\t.reg .u32 b, o;\n\t"
+                                     "bfind.u32 b, %1;\n\t"
+                                     "mad.lo.u32 %0, b, 16, %2;\n\t"
+                                     "shl.b32 o, 1, b;\n\t"
+                                     "xor.b32 %1, %1, o;\n\t"
+                                     "setp.eq.u32 z, %1, 0;\n\t"
+                                     "@z shl.b32 o, 1, %4;\n\t"
+                                     "@z lop3.b32 %3, %3, o, 1, 0xba;\n\t"  // (nz & ~o) | 1
+                                     "@z bfind.u32 %4, %3;\n\t"
+                                     "@z mad.lo.u32 %2, %4, 512, %5;\n\t"
+                                     "@z mad.lo.u32 o, %4, 384, %6;\n\t"
+                                     "@z ld.shared.u32 %1, [o];\n\t}"
+                                     : "=r"(at[q]), "+r"(m), "+r"(row_at), "+r"(nz), "+r"(r)
+                                     : "r"(slots_at), "r"(masks_at));
+                        p[q] = lds128(at[q]);
+                    }
+                    PairTerm k[kPer];
+#pragma unroll
+                    for (int q = 0; q < kPer; q++)
+                        k[q] = pair_term<kGeneric, kUniformR>(c, p[q], hpx, hpy, hpz, force_at, pair_at);
+#pragma unroll
+                    for (int q = 0; q < kPer; q++)
+                        asm("{\n\t.reg .pred p, b;\n\t"
+                            "setp.lt.f32 p, %6, %7;\n\t"
+                            "setp.lt.and.f32 b, %6, %8, !p;\n\t"
+                            "@p fma.rn.f32 %0, %9, %12, %0;\n\t"
+                            "@p fma.rn.f32 %1, %10, %12, %1;\n\t"
+                            "@p fma.rn.f32 %2, %11, %12, %2;\n\t"
+                            "@p add.s32 %3, %3, 1;\n\t"
+                            "@b mov.u32 %4, %13;\n\t"
+                            "@b add.s32 %5, %5, 1;\n\t}"
+                            : "+f"(fx), "+f"(fy), "+f"(fz), "+r"(count), "+r"(open_at), "+r"(open)
+                            : "f"(k[q].d2), "f"(k[q].lo), "f"(kUniformR ? c.thr_hi_uniform : k[q].lo + c.band), "f"(k[q].dx),
+                              "f"(k[q].dy), "f"(k[q].dz), "f"(k[q].weight), "r"(at[q]));
+                }
+                // the pairs left open take the exact test, after the unit's others: the one of a lane
+                // that has one; a lane with more walks its masks again for them
+                if (__any_sync(kAll, open > 0)) {
+                    int row = open > 1 ? ngroups : 0;
+                    m = row ? w.row[row][lane] : 0u;
+                    while (open > 0) {
+                        if (row) {
+                            while (m == 0u) m = w.row[--row][lane];
+                            const int bit = top_bit(m);
+                            m ^= 1u << bit;
+                            open_at = slots_at + 512 * row + 16 * bit;
+                        }
+                        const float4 p = lds128(open_at);
+                        const PairTerm k = pair_term<kGeneric, kUniformR>(c, p, hpx, hpy, hpz, force_at, pair_at);
+                        if (!(k.d2 < k.lo) && k.d2 < k.lo + c.band) {
+                            open--;
+                            // the candidate's sorted index, from its place in the list
+                            const int g = ((int)(open_at - slots_at) / 16 - 32) * units + unit;
+                            int s = 0;
+                            while (starts[s + 1] <= g) s++;
+                            const int j = __float_as_int(w.seg[s].w) + g;
+                            const float* origin = reinterpret_cast<const float*>(&w.row[0][kOriginAt]);
+                            const float thr = kUniformR ? c.thr_uniform
+                                                        : tables->threshold[type * kTableStride +
+                                                                            (__float_as_uint(p.w) >> 2)];
+                            if (g < total && CF_IN_BOUNDS(j, c.n) && pair_exact<kGeneric>(c, h, origin, p, pos_sorted[j], thr)) {
+                                count++;
+                                fx = fmaf(k.dx, k.weight, fx);
+                                fy = fmaf(k.dy, k.weight, fy);
+                                fz = fmaf(k.dz, k.weight, fz);
+                            }
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            if (split > 1) {
+                // the round's units in order: the other warps leave their partial sums in their own
+                // staging area, the item's warps meet at a named barrier (id 1 + item slot,
+                // 32 * split threads) and part 0 adds them
+                if (part != 0) w.c[1 + lane] = make_float4(fx, fy, fz, __int_as_float(count));
+                item_barrier(slot_of_item, 32 * split);
+            }
+            sum_x += fx;
+            sum_y += fy;
+            sum_z += fz;
+            sum_n += count;
+            if (split > 1 && part == 0) {
+                const int more = min(split, units - u0);
+                for (int q = 1; q < more; q++) {
+                    const float4 v = (&w)[q].c[1 + lane];
+                    sum_x += v.x;
+                    sum_y += v.y;
+                    sum_z += v.z;
+                    sum_n += __float_as_int(v.w);
+                }
+            }
+        }
+        __syncwarp();
+    }
+    if (part != 0 || !active || !CF_IN_BOUNDS(i, c.n)) return;
+    if (c.integrate_apart)
+        acc[i] = make_float4(sum_x, sum_y, sum_z, __int_as_float(sum_n));  // for integrate_kernel
+    else
+        integrate(c, h, make_float4(sum_x, sum_y, sum_z, 0.0f), sum_n, i, pos, vel, acc, counts);
+}
+
+__global__ void __launch_bounds__(256)
+    integrate_kernel(StepConsts c, float4* __restrict__ pos, float4* __restrict__ vel, float4* __restrict__ acc,
+                     int* __restrict__ counts)
+{
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= c.n) return;
+    const float4 f = acc[i];
+    integrate(c, pos[i], f, __float_as_int(f.w), (uint32_t)i, pos, vel, acc, counts);
 }
 
 // The filter's work of one step, from the cell list alone: per item and pass
@@ -1074,37 +923,42 @@ __global__ void __launch_bounds__(1024)
     if (tid == 1023) *n_items = (int)s_chunk[1023];
 }
 
-template <int S, int B, int P, bool G, bool U>
-cudaError_t configure_one()
+// Shared memory of a block: staging per warp, the pair table without a uniform
+// radius, and the force table of one world or, in a batch, of each item of the block.
+size_t force_smem(int warps, int T, bool uniform, int force_tables)
 {
-    return cudaFuncSetAttribute(step_force_kernel<S, B, P, G, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)((sizeof(WarpSmem<S, P>) + sizeof(float2) * kTableSize) * kWarps));
+    return sizeof(WarpSmem) * warps + (size_t)T * T * ((uniform ? 0 : sizeof(float4)) + sizeof(float) * force_tables);
 }
 
-template <int S, int B, int P>
+template <int W, int B, bool G, bool U>
+cudaError_t configure_one()
+{
+    return cudaFuncSetAttribute(step_force_kernel<W, B, G, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)force_smem(W, CF_MAX_TYPES, U, W <= 4 ? W : 1));
+}
+
+template <int W, int B>
 cudaError_t configure_variant()
 {
-    cudaError_t e = configure_one<S, B, P, false, false>();
-    if (e == cudaSuccess) e = configure_one<S, B, P, false, true>();
-    if (e == cudaSuccess) e = configure_one<S, B, P, true, false>();
-    if (e == cudaSuccess) e = configure_one<S, B, P, true, true>();
+    cudaError_t e = configure_one<W, B, false, false>();
+    if (e == cudaSuccess) e = configure_one<W, B, false, true>();
+    if (e == cudaSuccess) e = configure_one<W, B, true, false>();
+    if (e == cudaSuccess) e = configure_one<W, B, true, true>();
     return e;
 }
 
-// Variant S = staged candidates per batch, B = resident blocks per SM the
-// register budget is sized for, P = lanes paired in the drain.
-template <int S, int B, int P>
+// W = warps per block, B = resident blocks per SM the register budget is sized for.
+template <int W, int B>
 cudaError_t launch_variant(const StepConsts& c, const PairTables* tables, const float4* pos_sorted,
-                           const uint32_t* keys_sorted, const uint32_t* vals_sorted, const uint32_t* cell_off,
-                           const Item* items, const int* n_items, int blocks, float4* pos, float4* vel, float4* acc,
-                           int* counts, cudaStream_t st)
+                           const uint32_t* vals_sorted, const uint32_t* cell_off, const Item* items,
+                           const int* n_items, int max_items, float4* pos, float4* vel, float4* acc, int* counts,
+                           cudaStream_t st)
 {
-    // staging per warp; force coefficients per block (one world) or per warp (a batch)
-    const size_t smem = sizeof(WarpSmem<S, P>) * kWarps +
-                        sizeof(float2) * c.num_types * c.num_types * (c.grid.worlds == 1 ? 1 : kWarps);
-#define CF_FORCE_LAUNCH(G, U)                                                                                        \
-    step_force_kernel<S, B, P, G, U><<<blocks, kThreads, smem, st>>>(c, tables, pos_sorted, keys_sorted, vals_sorted,   \
-                                                                  cell_off, items, n_items, pos, vel, acc, counts)
+    const size_t smem = force_smem(W, c.num_types, c.uniform_r != 0, c.grid.worlds == 1 ? 1 : W / c.split);
+    const int blocks = (int)(((long long)max_items * c.split + W - 1) / W);
+#define CF_FORCE_LAUNCH(G, U)                                                                                      \
+    step_force_kernel<W, B, G, U><<<blocks, 32 * W, smem, st>>>(c, tables, pos_sorted, vals_sorted, cell_off, items, \
+                                                               n_items, max_items, pos, vel, acc, counts)
     if (c.grid.generic) {
         if (c.uniform_r)
             CF_FORCE_LAUNCH(true, true);
@@ -1136,9 +990,44 @@ cudaError_t launch_force_work(const StepConsts& c, const uint32_t* keys_sorted, 
     return cudaGetLastError();
 }
 
+namespace {
+// From this many particles the integrator is a kernel of its own, in particle order: the
+// force kernel's scattered access to a particle's state (six sectors) shrinks to one store.
+// 1.17M particles in 64 worlds: 304 against 321 us; 300k: equal; 100k: 45.9 against 44.3 (the
+// launch).
+constexpr int kIntegrateApart = 500000;
+constexpr int kSms = 152;
+}
+
 int max_step_items(int n, const Grid& g) { return (n + 31) / 32 + g.worlds * g.m[1] * g.m[2]; }
 
-int step_launches(int n) { return n > 0 ? 1 : 0; }  // the force kernel (the plan is part of the cell list)
+// The force kernel, and the integrator where it is a kernel of its own (the plan is part of the cell list).
+int step_launches(int n) { return n > 0 ? 1 + (integrate_apart(n) ? 1 : 0) : 0; }
+
+bool integrate_apart(int n) { return n >= kIntegrateApart; }
+
+// The variant of a world that chose none.  Warps per item: the power of two that
+// fills the GPU, at most two per unit that an item of evenly spread particles
+// has (one below half a unit, where further warps only add their start: 10.9
+// against 13.6 us at 2,048 particles).  Occupancy: the most registers that hold
+// all warps at once, else (several waves) five blocks per SM, whose three
+// pairs per trip beat six blocks' two (469 against 494 us at 1M).
+int default_force_variant(int n, const Grid& g)
+{
+    const double cells = (double)g.cells, pop = (double)n / cells;
+    const double homes = std::min(32.0, std::max(pop * g.m[0], 1.0));
+    const double candidates = 9.0 * pop * std::min((double)g.m[0], homes / pop + 3.0);
+    const double items = n / 32.0 + 0.5 * std::min(cells / g.m[0], (double)n);
+    const double slots = 24.0 * kSms;
+    int split = 1;
+    if (candidates >= 0.5 * kUnit)
+        while (split < 8 && 2 * split * (n / 32.0) <= slots && split < 2.0 * std::ceil(candidates / kUnit)) split *= 2;
+    const double warps = items * split;
+    const int occupancy = warps <= 16.0 * kSms ? 2 : warps <= 20.0 * kSms ? 1 : warps <= slots ? 0 : 1;
+    int log2 = 0;
+    while ((1 << log2) < split) log2++;
+    return occupancy + kForceOccupancies * log2;
+}
 
 cudaError_t launch_step_plan(const uint32_t* cell_off, int n, const Grid& g, Item* items, int* n_items,
                              cudaStream_t st)
@@ -1153,39 +1042,36 @@ cudaError_t launch_step_plan(const uint32_t* cell_off, int n, const Grid& g, Ite
 // stream capture).
 cudaError_t configure_step_force()
 {
-    cudaError_t e = configure_variant<256, 8, 0>();
-    if (e == cudaSuccess) e = configure_variant<256, 6, 0>();
-    if (e == cudaSuccess) e = configure_variant<256, 6, 1>();
-    if (e == cudaSuccess) e = configure_variant<384, 6, 0>();
-    if (e == cudaSuccess) e = configure_variant<256, 6, 2>();
+    cudaError_t e = configure_variant<4, 6>();
+    if (e == cudaSuccess) e = configure_variant<4, 5>();
+    if (e == cudaSuccess) e = configure_variant<4, 4>();
+    if (e == cudaSuccess) e = configure_variant<2, 10>();
+    if (e == cudaSuccess) e = configure_variant<8, 2>();
+    if (e == cudaSuccess) e = configure_variant<16, 1>();
     return e;
 }
 
 cudaError_t launch_step_force(const StepConsts& c, const PairTables* tables, const float4* pos_sorted,
-                              const uint32_t* keys_sorted, const uint32_t* vals_sorted, const uint32_t* cell_off,
-                              const Item* items, const int* n_items, int max_items, float4* pos, float4* vel,
-                              float4* acc, int* counts, cudaStream_t st)
+                              const uint32_t* vals_sorted, const uint32_t* cell_off, const Item* items,
+                              const int* n_items, int max_items, float4* pos, float4* vel, float4* acc, int* counts,
+                              cudaStream_t st)
 {
     if (c.n <= 0 || max_items <= 0) return cudaSuccess;
-    if (c.split != 1 && c.split != 2 && c.split != 4) return cudaErrorInvalidValue;
-    const int blocks = (int)(((long long)max_items * c.split + kWarps - 1) / kWarps);
-    switch (c.variant) {
-    case 1:
-        return launch_variant<256, 6, 0>(c, tables, pos_sorted, keys_sorted, vals_sorted, cell_off, items, n_items,
-                                      blocks, pos, vel, acc, counts, st);
-    case 2:
-        return launch_variant<256, 6, 1>(c, tables, pos_sorted, keys_sorted, vals_sorted, cell_off, items, n_items,
-                                      blocks, pos, vel, acc, counts, st);
-    case 4:
-        return launch_variant<256, 6, 2>(c, tables, pos_sorted, keys_sorted, vals_sorted, cell_off, items, n_items,
-                                         blocks, pos, vel, acc, counts, st);
-    case 3:
-        return launch_variant<384, 6, 0>(c, tables, pos_sorted, keys_sorted, vals_sorted, cell_off, items, n_items,
-                                      blocks, pos, vel, acc, counts, st);
-    default:
-        return launch_variant<256, 8, 0>(c, tables, pos_sorted, keys_sorted, vals_sorted, cell_off, items, n_items,
-                                      blocks, pos, vel, acc, counts, st);
-    }
+    if (c.split < 1 || c.split > 16 || (c.split & (c.split - 1)) != 0) return cudaErrorInvalidValue;
+    cudaError_t e;
+#define CF_FORCE_VARIANT(W, B) \
+    launch_variant<W, B>(c, tables, pos_sorted, vals_sorted, cell_off, items, n_items, max_items, pos, vel, acc, counts, st)
+    if (c.split <= 2)
+        e = c.variant == 0 ? CF_FORCE_VARIANT(4, 6) : c.variant == 1 ? CF_FORCE_VARIANT(2, 10) : CF_FORCE_VARIANT(4, 4);
+    else if (c.split == 4)
+        e = c.variant == 0 ? CF_FORCE_VARIANT(4, 6) : c.variant == 1 ? CF_FORCE_VARIANT(4, 5) : CF_FORCE_VARIANT(4, 4);
+    else
+        e = c.split == 8 ? CF_FORCE_VARIANT(8, 2) : CF_FORCE_VARIANT(16, 1);
+#undef CF_FORCE_VARIANT
+    if (e != cudaSuccess || !c.integrate_apart) return e;
+    integrate_kernel<<<(c.n + 255) / 256, 256, 0, st>>>(c, pos, vel, acc, counts);
+    note_launches(st);
+    return cudaGetLastError();
 }
 
 }  // namespace cf

@@ -236,20 +236,15 @@ int cf_step(cf_world* w, const cf_step_params* p, int nsteps);
  * state stays on the device and only getParticleData copies it back). */
 int cf_step_host(cf_world* w, const cf_step_params* p, const cf_particle* in, cf_particle* out, int n);
 
-/* Force-kernel variants: v % 4 picks the staging: 0 = 256 candidates staged
- * per warp batch, register budget for 8 blocks per SM; 1 = 256 staged, 6
- * blocks per SM; 2 = as 1 with lanes paired in the drain (the lane with the
- * fewest hits of a batch takes part of the busiest lane's, and so on down the
- * sorted hit counts); 3 = 384 staged, 6 blocks per SM.  v / 4 picks the warps
- * per 32-particle item: 1, 2 or 4 (each warp takes an equal share of the
- * item's candidates; more warps for worlds too small to fill the GPU).
- * Variants 12, 13 and 14 use the balanced drain (256 staged, 6 blocks per
- * SM) with 1, 2 or 4 warps per item: a batch's hits, home by home, are split
- * into 32 equal ranges, one per lane, and each home adds the partial sums of
- * its pieces in lane order.
- * Results are bit-identical across stagings 0, 1 and 3; with lane pairing,
- * the balanced drain, and 2 or 4 warps, partial sums are added in a fixed
- * order, which differs from the single-lane order by rounding only. */
+/* Force-kernel variants: v % 3 picks the registers and resident warps the
+ * kernel is built for (0: 24 warps per SM, two pairs of a home at a time;
+ * 1: 20 warps and 2: 16 warps, three pairs), v / 3 picks the warps per
+ * 32-particle item: 1, 2, 4, 8 or 16, which take the item's units of 256
+ * candidates in turn (more warps for worlds too small to fill the GPU, or with
+ * many neighbours; with 8 and 16 warps v % 3 makes no difference).  A world
+ * that selected none uses the one a rule gives for its particle count and
+ * grid.  Partial sums are added unit by unit in a fixed order, so all variants
+ * give the same results bit for bit. */
 #define CF_FORCE_VARIANTS 15
 /* Autotuner of the step (no counterpart in the reference): runs `steps`
  * trial steps with each force-kernel variant, restores the particle state,
