@@ -158,6 +158,8 @@ _SIGNATURES = {
     "cf_create": (C.c_int, [C.c_int, C.c_int, C.c_float, C.c_float, C.c_float, C.c_uint64, _P(_W)]),
     "cf_destroy": (C.c_int, [_W]),
     "cf_set_stream": (C.c_int, [_W, C.c_void_p]),
+    "cf_stream_wait": (C.c_int, [_W, C.c_void_p]),
+    "cf_stream_signal": (C.c_int, [_W, C.c_void_p]),
     "cf_sync": (C.c_int, [_W]),
     "cf_particle_count": (C.c_int, [_W, _P(C.c_int)]),
     "cf_num_particle_types": (C.c_int, [_W, _P(C.c_int)]),
@@ -231,6 +233,12 @@ _SIGNATURES = {
                                      C.c_void_p]),
     "cf_rollout_backward": (C.c_int, [_W, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int,
                                       C.c_void_p]),
+    "cf_rollout_forward_xyz": (C.c_int, [_W, _P(StepParams), C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p,
+                                         C.c_void_p]),
+    "cf_rollout_backward_xyz": (C.c_int, [_W, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                          C.c_void_p]),
+    "cf_rdf_xyz": (C.c_int, [_W, C.c_void_p, C.c_int, C.c_float, C.c_void_p]),
+    "cf_rdf_backward_xyz": (C.c_int, [_W, C.c_void_p, C.c_int, C.c_float, C.c_void_p, C.c_void_p]),
     "cf_rdf": (C.c_int, [_W, C.c_void_p, C.c_int, C.c_float, C.c_void_p]),
     "cf_rdf_backward": (C.c_int, [_W, C.c_void_p, C.c_int, C.c_float, C.c_void_p, C.c_void_p]),
     "cf_preset_parse": (C.c_int, [C.c_char_p, C.c_size_t, _P(Preset)]),

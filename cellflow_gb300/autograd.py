@@ -12,54 +12,35 @@ No counterpart in the reference.
 
 from __future__ import annotations
 
-import dataclasses
+import ctypes as C
 
-import numpy as np
 import torch
 
-from ._lib import GRAD_PARAMS
+from ._lib import GRAD_PARAMS, check, load
 from .world import ParticleSimulation, SimulationParams
 
 
-class _LibraryStream:
-    """Runs a block on a torch stream that the world also uses, ordered after the
-    caller's current stream on entry and before it on exit.  (The caller's stream
-    may be the legacy default stream, which the world's own non-blocking stream
-    would not wait for.)  Tensors made inside and used after are recorded on the
-    caller's stream."""
+class _Ordered:
+    """Runs a block's library calls between the caller's current torch stream's earlier and
+    later work: the world's stream waits for the caller's on entry and the caller's for the
+    world's on exit, so tensors of the caller's stream can be handed over in both directions."""
 
     def __init__(self, sim: ParticleSimulation):
         self.sim = sim
+        # (the raw handle; torch.cuda.current_stream() builds a Stream object in about 15 us)
+        self.stream = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
     def __enter__(self):
-        s = getattr(self.sim, "_torch_stream", None)
-        if s is None:
-            s = torch.cuda.Stream()
-            self.sim._torch_stream = s
-            self.sim.set_stream(s.cuda_stream)
-        self.caller = torch.cuda.current_stream()
-        s.wait_stream(self.caller)
-        self.ctx = torch.cuda.stream(s)
-        self.ctx.__enter__()
-        return self
-
-    def keep(self, *tensors):
-        for t in tensors:
-            t.record_stream(self.caller)
-        return tensors
+        check(load().cf_stream_wait(self.sim.handle, self.stream), "cf_stream_wait")
 
     def __exit__(self, *exc):
-        s = torch.cuda.current_stream()
-        self.ctx.__exit__(*exc)
-        self.caller.wait_stream(s)
+        check(load().cf_stream_signal(self.sim.handle, self.stream), "cf_stream_signal")
         return False
 
 
-def _as4(x: torch.Tensor | None, n: int) -> torch.Tensor:
-    out = torch.zeros((n, 4), dtype=torch.float32, device="cuda")
-    if x is not None:
-        out[:, :3] = x
-    return out
+def _rows(x: torch.Tensor, n: int, copy: bool = False) -> torch.Tensor:
+    """x as contiguous (n, 3) float32 on the GPU (its own memory with copy)."""
+    return x.detach().to("cuda", torch.float32, copy=copy).expand(n, 3).contiguous()
 
 
 class Rollout(torch.autograd.Function):
@@ -69,15 +50,15 @@ class Rollout(torch.autograd.Function):
     def forward(ctx, pos, vel, table, phys, sim: ParticleSimulation, params: SimulationParams, steps: int,
                 checkpoint_every: int = 16):
         n = sim.getParticleCount()
-        values = {name: float(v) for name, v in zip(GRAD_PARAMS, phys.detach().cpu().tolist())}
-        p = dataclasses.replace(params, **values)
+        p = params.to_c()
+        for name, v in zip(GRAD_PARAMS, phys.detach().cpu().tolist()):
+            setattr(p, name, v)
         sim.setForceTable(table.detach().to("cpu", torch.float32).numpy())
-        with _LibraryStream(sim) as ls:
-            pos4, vel4 = _as4(pos.detach(), n), _as4(vel.detach(), n)
-            out_p, out_v = torch.empty_like(pos4), torch.empty_like(vel4)
-            sim.rollout_forward(p, steps, checkpoint_every, pos4.data_ptr(), vel4.data_ptr(), out_p.data_ptr(),
-                                out_v.data_ptr())
-            xk, vk = ls.keep(out_p[:, :3].contiguous(), out_v[:, :3].contiguous())
+        x0, v0 = _rows(pos, n), _rows(vel, n)
+        xk, vk = torch.empty_like(x0), torch.empty_like(v0)
+        with _Ordered(sim):
+            check(load().cf_rollout_forward_xyz(sim.handle, C.byref(p), x0.data_ptr(), v0.data_ptr(), steps,
+                                                checkpoint_every, xk.data_ptr(), vk.data_ptr()), "cf_rollout_forward")
         ctx.sim = sim
         ctx.table_meta = (table.dtype, table.device)
         ctx.phys_meta = (phys.dtype, phys.device)
@@ -86,21 +67,19 @@ class Rollout(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gpos, gvel):
         sim = ctx.sim
-        n = sim.getParticleCount()
-        with _LibraryStream(sim) as ls:
-            g4 = _as4(gpos, n) if gpos is not None else None
-            gv4 = _as4(gvel, n) if gvel is not None else None
-            out_g, out_v = torch.empty((n, 4), dtype=torch.float32, device="cuda"), torch.empty(
-                (n, 4), dtype=torch.float32, device="cuda")
-            gF, gp = sim.rollout_backward(g4.data_ptr() if g4 is not None else None,
-                                          gv4.data_ptr() if gv4 is not None else None, out_g.data_ptr(),
-                                          out_v.data_ptr())
-            gx0, gv0 = ls.keep(out_g[:, :3].contiguous(), out_v[:, :3].contiguous())
+        n, T = sim.getParticleCount(), sim.getNumParticleTypes()
+        gxk = _rows(gpos, n) if gpos is not None else None
+        gvk = _rows(gvel, n) if gvel is not None else None
+        gx0, gv0 = (torch.empty((n, 3), dtype=torch.float32, device="cuda") for _ in range(2))
+        gF = torch.empty((T, T), dtype=torch.float32, device="cuda")
+        gp = torch.empty(len(GRAD_PARAMS), dtype=torch.float32, device="cuda")
+        with _Ordered(sim):
+            check(load().cf_rollout_backward_xyz(sim.handle, gxk.data_ptr() if gxk is not None else None,
+                                                 gvk.data_ptr() if gvk is not None else None, gx0.data_ptr(),
+                                                 gv0.data_ptr(), gF.data_ptr(), gp.data_ptr()), "cf_rollout_backward")
         tdt, tdev = ctx.table_meta
         pdt, pdev = ctx.phys_meta
-        return (gx0, gv0,
-                torch.from_numpy(np.ascontiguousarray(gF)).to(device=tdev, dtype=tdt),
-                torch.from_numpy(gp.astype(np.float64)).to(device=pdev, dtype=pdt), None, None, None, None)
+        return gx0, gv0, gF.to(device=tdev, dtype=tdt), gp.to(device=pdev, dtype=pdt), None, None, None, None
 
 
 class RadialDistribution(torch.autograd.Function):
@@ -109,24 +88,22 @@ class RadialDistribution(torch.autograd.Function):
     @staticmethod
     def forward(ctx, pos, sim: ParticleSimulation, bins: int, r_max: float):
         n, T = sim.getParticleCount(), sim.getNumParticleTypes()
-        with _LibraryStream(sim) as ls:
-            pos4 = _as4(pos.detach(), n)
-            hist = torch.empty((T, T, bins), dtype=torch.float32, device="cuda")
-            sim.rdf(bins, r_max, hist.data_ptr(), pos4.data_ptr())
-            ls.keep(hist, pos4)
+        x = _rows(pos, n, copy=True)  # (kept for the backward, whatever becomes of pos)
+        hist = torch.empty((T, T, bins), dtype=torch.float32, device="cuda")
+        with _Ordered(sim):
+            check(load().cf_rdf_xyz(sim.handle, x.data_ptr(), bins, r_max, hist.data_ptr()), "cf_rdf")
         ctx.sim, ctx.bins, ctx.r_max = sim, bins, r_max
-        ctx.save_for_backward(pos4)
+        ctx.save_for_backward(x)
         return hist
 
     @staticmethod
     def backward(ctx, ghist):
-        (pos4,) = ctx.saved_tensors
-        sim = ctx.sim
-        with _LibraryStream(sim) as ls:
-            gh = ghist.to(torch.float32).contiguous()
-            g4 = torch.empty_like(pos4)
-            sim.rdf_backward(ctx.bins, ctx.r_max, gh.data_ptr(), g4.data_ptr(), pos4.data_ptr())
-            (gx,) = ls.keep(g4[:, :3].contiguous())
+        (x,) = ctx.saved_tensors
+        gh = ghist.to(torch.float32).contiguous()
+        gx = torch.empty_like(x)
+        with _Ordered(ctx.sim):
+            check(load().cf_rdf_backward_xyz(ctx.sim.handle, x.data_ptr(), ctx.bins, ctx.r_max, gh.data_ptr(),
+                                             gx.data_ptr()), "cf_rdf_backward")
         return gx, None, None, None
 
 

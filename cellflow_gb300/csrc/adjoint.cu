@@ -425,7 +425,7 @@ __global__ void rdf_finish_kernel(RdfConsts c, const double* __restrict__ acc,
 __global__ void rdf_grad_kernel(RdfConsts c, const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ keys,
                                 const uint32_t* __restrict__ vals, const uint32_t* __restrict__ cell_off,
                                 const float* __restrict__ ghist, const unsigned long long* __restrict__ type_count,
-                                float4* __restrict__ gpos)
+                                float* __restrict__ gpos, int gpos_stride)
 {
     extern __shared__ float s_g[];  // ghist / den
     __shared__ uint32_t s_list[kAdjThreads / 32][kListCap];
@@ -462,17 +462,62 @@ __global__ void rdf_grad_kernel(RdfConsts c, const float4* __restrict__ pos_sort
         ax = warp_sum(ax);
         ay = warp_sum(ay);
         az = warp_sum(az);
-        if (lane == 0) gpos[vals[k]] = make_float4(ax, ay, az, 0.0f);
+        if (lane == 0) {
+            float* g = gpos + (size_t)vals[k] * gpos_stride;
+            if (gpos_stride == 4) {
+                *reinterpret_cast<float4*>(g) = make_float4(ax, ay, az, 0.0f);
+            } else {
+                g[0] = ax;
+                g[1] = ay;
+                g[2] = az;
+            }
+        }
     }
 }
 
-// dst.xyz = src.xyz, dst.w = typesrc.w (the particle's type bits).
-__global__ void pack_pos_kernel(const float4* __restrict__ src, const float4* typesrc, float4* dst, int n)
+__global__ void pack_pos_kernel(const float* __restrict__ rows, int stride, const float4* typesrc, float4* dst, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float4 s = src[i];
-    dst[i] = make_float4(s.x, s.y, s.z, typesrc[i].w);
+    const float* s = rows + (size_t)i * stride;
+    dst[i] = make_float4(s[0], s[1], s[2], typesrc[i].w);
+}
+
+__global__ void rows_in_kernel(const float* __restrict__ a_rows, const float* __restrict__ b_rows,
+                               float4* __restrict__ a, float4* __restrict__ b, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const size_t k = 3 * (size_t)i;
+    if (a) a[i] = a_rows ? make_float4(a_rows[k], a_rows[k + 1], a_rows[k + 2], 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (b) b[i] = b_rows ? make_float4(b_rows[k], b_rows[k + 1], b_rows[k + 2], 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+}
+
+__global__ void rows_out_kernel(const float4* __restrict__ a, const float4* __restrict__ b, float* __restrict__ a_rows,
+                                float* __restrict__ b_rows, int n, const double* __restrict__ gacc, int T,
+                                float* __restrict__ grad_force, float* __restrict__ grad_params)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0 && gacc) {
+        if (grad_force)
+            for (int e = threadIdx.x; e < T * T; e += blockDim.x)
+                grad_force[e] = (float)gacc[e / T * kTableStride + e % T];
+        if (grad_params && threadIdx.x < CF_GRAD_PARAMS) grad_params[threadIdx.x] = (float)gacc[kTableSize + threadIdx.x];
+    }
+    if (i >= n) return;
+    const size_t k = 3 * (size_t)i;
+    if (a_rows) {
+        const float4 v = a[i];
+        a_rows[k] = v.x;
+        a_rows[k + 1] = v.y;
+        a_rows[k + 2] = v.z;
+    }
+    if (b_rows) {
+        const float4 v = b[i];
+        b_rows[k] = v.x;
+        b_rows[k + 1] = v.y;
+        b_rows[k + 2] = v.z;
+    }
 }
 
 RdfConsts rdf_consts(const float* ext, const Grid& g, int n, int T, int bins, float r_max)
@@ -523,10 +568,27 @@ cudaError_t launch_adjoint_step(const StepConsts& c, const PairTables* tables, c
     return cudaGetLastError();
 }
 
-cudaError_t launch_pack_pos(const float4* src, const float4* typesrc, float4* dst, int n, cudaStream_t st)
+cudaError_t launch_pack_pos(const float* rows, int stride, const float4* typesrc, float4* dst, int n, cudaStream_t st)
 {
     if (n == 0) return cudaSuccess;
-    pack_pos_kernel<<<(n + 255) / 256, 256, 0, st>>>(src, typesrc, dst, n);
+    pack_pos_kernel<<<(n + 255) / 256, 256, 0, st>>>(rows, stride, typesrc, dst, n);
+    note_launches(st);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_rows_in(const float* a_rows, const float* b_rows, float4* a, float4* b, int n, cudaStream_t st)
+{
+    if (n == 0) return cudaSuccess;
+    rows_in_kernel<<<(n + 255) / 256, 256, 0, st>>>(a_rows, b_rows, a, b, n);
+    note_launches(st);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_rows_out(const float4* a, const float4* b, float* a_rows, float* b_rows, int n, const double* gacc,
+                            int T, float* grad_force, float* grad_params, cudaStream_t st)
+{
+    rows_out_kernel<<<std::max(1, (n + 255) / 256), 256, 0, st>>>(a, b, a_rows, b_rows, n, gacc, T, grad_force,
+                                                                  grad_params);
     note_launches(st);
     return cudaGetLastError();
 }
@@ -557,7 +619,7 @@ cudaError_t launch_rdf(const float* ext, const Grid& g, int n, int T, int bins, 
 cudaError_t launch_rdf_grad(const float* ext, const Grid& g, int n, int T, int bins, float r_max,
                             const float4* pos, const float4* pos_sorted, const uint32_t* keys_sorted,
                             const uint32_t* vals_sorted, const uint32_t* cell_off, const float* ghist,
-                            unsigned long long* type_count, float4* gpos, cudaStream_t st)
+                            unsigned long long* type_count, float* gpos, int gpos_stride, cudaStream_t st)
 {
     const RdfConsts c = rdf_consts(ext, g, n, T, bins, r_max);
     cudaError_t e = cudaMemsetAsync(type_count, 0, sizeof(unsigned long long) * CF_MAX_TYPES, st);
@@ -567,7 +629,7 @@ cudaError_t launch_rdf_grad(const float* ext, const Grid& g, int n, int T, int b
     const int warps_per_block = kAdjThreads / 32;
     rdf_grad_kernel<<<std::min((n + warps_per_block - 1) / warps_per_block, 8 * num_sms()), kAdjThreads,
                       rdf_smem_bytes(T, bins), st>>>(c, pos_sorted, keys_sorted, vals_sorted, cell_off, ghist,
-                                                     type_count, gpos);
+                                                     type_count, gpos, gpos_stride);
     note_launches(st);
     return cudaGetLastError();
 }

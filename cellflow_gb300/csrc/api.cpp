@@ -992,6 +992,7 @@ int cf_destroy(cf_world* w)
     if (w->host_words) cudaFreeHost(w->host_words);
     dev_free(w->tables);
     dev_free(w->world_tables);
+    if (w->order_event) cudaEventDestroy(w->order_event);
     if (w->own_stream) cudaStreamDestroy(w->own_stream);
     delete w;
     return CF_OK;
@@ -1003,6 +1004,35 @@ int cf_set_stream(cf_world* w, void* stream)
     if (rc) return rc;
     CF_CUDA(cudaStreamSynchronize(w->stream));
     w->stream = stream ? (cudaStream_t)stream : w->own_stream;
+    return CF_OK;
+}
+
+namespace {
+int order_event(cf_world* w)
+{
+    if (w->order_event) return CF_OK;
+    CF_CUDA(cudaEventCreateWithFlags(&w->order_event, cudaEventDisableTiming));
+    return CF_OK;
+}
+}  // namespace
+
+int cf_stream_wait(cf_world* w, void* cuda_stream)
+{
+    int rc = check_world(w);
+    if (!rc) rc = order_event(w);
+    if (rc) return rc;
+    CF_CUDA(cudaEventRecord(w->order_event, (cudaStream_t)cuda_stream));
+    CF_CUDA(cudaStreamWaitEvent(w->stream, w->order_event, 0));
+    return CF_OK;
+}
+
+int cf_stream_signal(cf_world* w, void* cuda_stream)
+{
+    int rc = check_world(w);
+    if (!rc) rc = order_event(w);
+    if (rc) return rc;
+    CF_CUDA(cudaEventRecord(w->order_event, w->stream));
+    CF_CUDA(cudaStreamWaitEvent((cudaStream_t)cuda_stream, w->order_event, 0));
     return CF_OK;
 }
 
@@ -2527,10 +2557,11 @@ int enqueue_rollout_backward(cf_world* w, const StepConsts& c, bool overlap)
 }  // namespace
 }  // namespace cf
 
-extern "C" {
+namespace {
 
-int cf_rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos4_in, const float* d_vel4_in,
-                       int nsteps, int checkpoint_every, float* d_pos4_out, float* d_vel4_out)
+// stride: floats per row of the caller's arrays, 4 or 3
+int rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos_in, const float* d_vel_in, int stride,
+                    int nsteps, int checkpoint_every, float* d_pos_out, float* d_vel_out)
 {
     int rc = check_world(w);
     if (rc) return rc;
@@ -2549,9 +2580,11 @@ int cf_rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos4
     Rollout& r = w->ro;
     r.steps = 0;
     const size_t n = (size_t)w->n;
-    if (d_pos4_in) CF_CUDA(launch_pack_pos(reinterpret_cast<const float4*>(d_pos4_in), w->pos, w->pos, w->n, w->stream));
-    if (d_vel4_in)
-        CF_CUDA(cudaMemcpyAsync(w->vel, d_vel4_in, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
+    if (d_pos_in) CF_CUDA(launch_pack_pos(d_pos_in, stride, w->pos, w->pos, w->n, w->stream));
+    if (d_vel_in && stride == 3)
+        CF_CUDA(launch_rows_in(d_vel_in, nullptr, w->vel, nullptr, w->n, w->stream));
+    else if (d_vel_in)
+        CF_CUDA(cudaMemcpyAsync(w->vel, d_vel_in, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
     // the step loop with its checkpoint copies
     auto loop = [&]() -> int {
         for (int s = 0; s < nsteps; s++) {
@@ -2597,10 +2630,14 @@ int cf_rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos4
     } else if ((rc = loop())) {
         return rc;
     }
-    if (d_pos4_out)
-        CF_CUDA(cudaMemcpyAsync(d_pos4_out, w->pos, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
-    if (d_vel4_out)
-        CF_CUDA(cudaMemcpyAsync(d_vel4_out, w->vel, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
+    if (stride == 3 && n > 0 && (d_pos_out || d_vel_out)) {
+        CF_CUDA(launch_rows_out(w->pos, w->vel, d_pos_out, d_vel_out, w->n, nullptr, 0, nullptr, nullptr, w->stream));
+    } else if (stride == 4) {
+        if (d_pos_out)
+            CF_CUDA(cudaMemcpyAsync(d_pos_out, w->pos, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
+        if (d_vel_out)
+            CF_CUDA(cudaMemcpyAsync(d_vel_out, w->vel, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
+    }
     r.steps = nsteps;
     r.every = checkpoint_every;
     r.n = w->n;
@@ -2610,17 +2647,11 @@ int cf_rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos4
     return CF_OK;
 }
 
-int cf_rollout_backward(cf_world* w, const float* d_gpos4, const float* d_gvel4, float* d_gpos4_out,
-                        float* d_gvel4_out, float* grad_force, int grad_force_count, float* grad_params)
+// The backward up to dL/dx_0 and dL/dv_0 in ro.gx and ro.gv and the gradient sums in ro.gacc.
+int rollout_backward(cf_world* w, const float* d_gpos, const float* d_gvel, int stride)
 {
-    int rc = check_world(w);
-    if (rc) return rc;
     Rollout& r = w->ro;
-    if (r.steps < 1) return fail(CF_ERR_INVALID, "no rollout to differentiate (cf_rollout_forward)");
-    if (r.n != w->n || r.table_version != w->table_version || std::memcmp(r.radio, w->radio, sizeof(r.radio)) != 0)
-        return fail(CF_ERR_INVALID, "the particle count, force table or radii changed since cf_rollout_forward");
-    const int T = w->num_types;
-    if (grad_force && grad_force_count != T * T) return fail(CF_ERR_INVALID, "grad_force_count must be T * T");
+    int rc = CF_OK;
     StepConsts c;
     rc = prepare_step(w, &r.params, &c);
     if (!rc) rc = ensure_cells(w, c.grid.cells);
@@ -2629,14 +2660,18 @@ int cf_rollout_backward(cf_world* w, const float* d_gpos4, const float* d_gvel4,
     if (!rc) rc = ensure_rollout_lists(w, std::min(r.every, r.steps), c.grid.cells);
     if (rc) return rc;
     const size_t n = (size_t)w->n;
-    if (d_gpos4)
-        CF_CUDA(cudaMemcpyAsync(r.gx, d_gpos4, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
-    else
-        CF_CUDA(cudaMemsetAsync(r.gx, 0, sizeof(float4) * n, w->stream));
-    if (d_gvel4)
-        CF_CUDA(cudaMemcpyAsync(r.gv, d_gvel4, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
-    else
-        CF_CUDA(cudaMemsetAsync(r.gv, 0, sizeof(float4) * n, w->stream));
+    if (stride == 3) {
+        CF_CUDA(launch_rows_in(d_gpos, d_gvel, r.gx, r.gv, w->n, w->stream));
+    } else {
+        if (d_gpos)
+            CF_CUDA(cudaMemcpyAsync(r.gx, d_gpos, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
+        else
+            CF_CUDA(cudaMemsetAsync(r.gx, 0, sizeof(float4) * n, w->stream));
+        if (d_gvel)
+            CF_CUDA(cudaMemcpyAsync(r.gv, d_gvel, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
+        else
+            CF_CUDA(cudaMemsetAsync(r.gv, 0, sizeof(float4) * n, w->stream));
+    }
     if (w->use_graphs && w->stream != nullptr && !w->profiling) {
         const void* bufs = w->s.cell_start;
         const bool same = r.bwd_graph && r.bwd_steps == r.steps && r.bwd_every == r.every && r.bwd_bufs == bufs &&
@@ -2674,6 +2709,60 @@ int cf_rollout_backward(cf_world* w, const float* d_gpos4, const float* d_gvel4,
         rc = enqueue_rollout_backward(w, c, false);
         if (rc) return rc;
     }
+    return CF_OK;
+}
+
+// The last forward's record fits the world (else an error).
+int check_rollout(cf_world* w)
+{
+    int rc = check_world(w);
+    if (rc) return rc;
+    const Rollout& r = w->ro;
+    if (r.steps < 1) return fail(CF_ERR_INVALID, "no rollout to differentiate (cf_rollout_forward)");
+    if (r.n != w->n || r.table_version != w->table_version || std::memcmp(r.radio, w->radio, sizeof(r.radio)) != 0)
+        return fail(CF_ERR_INVALID, "the particle count, force table or radii changed since cf_rollout_forward");
+    return CF_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int cf_rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos4_in, const float* d_vel4_in,
+                       int nsteps, int checkpoint_every, float* d_pos4_out, float* d_vel4_out)
+{
+    return rollout_forward(w, p, d_pos4_in, d_vel4_in, 4, nsteps, checkpoint_every, d_pos4_out, d_vel4_out);
+}
+
+int cf_rollout_forward_xyz(cf_world* w, const cf_step_params* p, const float* d_pos_in, const float* d_vel_in,
+                           int nsteps, int checkpoint_every, float* d_pos_out, float* d_vel_out)
+{
+    return rollout_forward(w, p, d_pos_in, d_vel_in, 3, nsteps, checkpoint_every, d_pos_out, d_vel_out);
+}
+
+int cf_rollout_backward_xyz(cf_world* w, const float* d_gpos, const float* d_gvel, float* d_gpos_out,
+                            float* d_gvel_out, float* d_grad_force, float* d_grad_params)
+{
+    int rc = check_rollout(w);
+    if (!rc) rc = rollout_backward(w, d_gpos, d_gvel, 3);
+    if (rc) return rc;
+    Rollout& r = w->ro;
+    CF_CUDA(launch_rows_out(r.gx, r.gv, d_gpos_out, d_gvel_out, w->n, r.gacc, w->num_types, d_grad_force, d_grad_params,
+                            w->stream));
+    return sync_and_check(w);
+}
+
+int cf_rollout_backward(cf_world* w, const float* d_gpos4, const float* d_gvel4, float* d_gpos4_out,
+                        float* d_gvel4_out, float* grad_force, int grad_force_count, float* grad_params)
+{
+    int rc = check_rollout(w);
+    if (rc) return rc;
+    Rollout& r = w->ro;
+    const size_t n = (size_t)w->n;
+    const int T = w->num_types;
+    if (grad_force && grad_force_count != T * T) return fail(CF_ERR_INVALID, "grad_force_count must be T * T");
+    rc = rollout_backward(w, d_gpos4, d_gvel4, 4);
+    if (rc) return rc;
     if (d_gpos4_out)
         CF_CUDA(cudaMemcpyAsync(d_gpos4_out, r.gx, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
     if (d_gvel4_out)
@@ -2694,7 +2783,37 @@ int cf_rollout_backward(cf_world* w, const float* d_gpos4, const float* d_gvel4,
     return CF_OK;
 }
 
-int cf_rdf(cf_world* w, const float* d_pos4, int bins, float r_max, float* d_hist)
+}  // extern "C"
+
+namespace {
+
+// Checks, scratch and the cell list of the radial distribution of d_pos (rows of `stride`
+// floats; NULL: the world's positions): *pos the positions used, *g the grid, *which the list.
+int rdf_list(cf_world* w, const float* d_pos, int stride, int bins, float r_max, const float4** pos, Grid* g, int* which)
+{
+    const int T = w->num_types;
+    if (!(r_max > 0.0f) || !std::isfinite(r_max)) return fail(CF_ERR_INVALID, "r_max must be finite and positive");
+    int rc = ensure_rdf(w);
+    if (rc) return rc;
+    *g = choose_step_grid(w->ext, rdf_cutoff(bins, r_max), kMaxCells);
+    apply_worlds(*g, 1);
+    rc = ensure_cells(w, g->cells);
+    if (!rc) rc = ensure_offsets(w, g->cells);
+    if (rc) return rc;
+    CF_CUDA(configure_adjoint());
+    Rollout& r = w->ro;
+    *pos = w->pos;
+    if (d_pos) {
+        CF_CUDA(launch_pack_pos(d_pos, stride, w->pos, r.rdf_pos, w->n, w->stream));
+        *pos = r.rdf_pos;
+    }
+    Scratch& s = w->s;
+    *which = 0;
+    CF_CUDA(launch_cell_list_csr(*pos, w->n, *g, w->ext, T, s, s.cell_off, nullptr, nullptr, w->err, which, w->stream));
+    return CF_OK;
+}
+
+int rdf_forward(cf_world* w, const float* d_pos, int stride, int bins, float r_max, float* d_hist)
 {
     int rc = check_world(w);
     if (rc) return rc;
@@ -2702,58 +2821,60 @@ int cf_rdf(cf_world* w, const float* d_pos4, int bins, float r_max, float* d_his
     const int T = w->num_types;
     if (bins < 1 || !d_hist || (long long)T * T * bins > kRdfMaxEntries)
         return fail(CF_ERR_INVALID, "bins must be >= 1 with T * T * bins <= 49152, d_hist not NULL");
-    if (!(r_max > 0.0f) || !std::isfinite(r_max)) return fail(CF_ERR_INVALID, "r_max must be finite and positive");
-    rc = ensure_rdf(w);
-    if (rc) return rc;
-    Grid g = choose_step_grid(w->ext, rdf_cutoff(bins, r_max), kMaxCells);
-    apply_worlds(g, 1);
-    rc = ensure_cells(w, g.cells);
-    if (!rc) rc = ensure_offsets(w, g.cells);
-    if (rc) return rc;
-    CF_CUDA(configure_adjoint());
-    Rollout& r = w->ro;
-    const float4* pos = w->pos;
-    if (d_pos4) {
-        CF_CUDA(launch_pack_pos(reinterpret_cast<const float4*>(d_pos4), w->pos, r.rdf_pos, w->n, w->stream));
-        pos = r.rdf_pos;
-    }
-    Scratch& s = w->s;
+    const float4* pos = nullptr;
+    Grid g;
     int which = 0;
-    CF_CUDA(launch_cell_list_csr(pos, w->n, g, w->ext, T, s, s.cell_off, nullptr, nullptr, w->err, &which, w->stream));
-    CF_CUDA(launch_rdf(w->ext, g, w->n, T, bins, r_max, s.pos_sorted, s.keys[which], s.cell_off, r.rdf_acc,
-                       r.type_count, d_hist, w->stream));
+    rc = rdf_list(w, d_pos, stride, bins, r_max, &pos, &g, &which);
+    if (rc) return rc;
+    Scratch& s = w->s;
+    CF_CUDA(launch_rdf(w->ext, g, w->n, T, bins, r_max, s.pos_sorted, s.keys[which], s.cell_off, w->ro.rdf_acc,
+                       w->ro.type_count, d_hist, w->stream));
     return CF_OK;
 }
 
-int cf_rdf_backward(cf_world* w, const float* d_pos4, int bins, float r_max, const float* d_ghist, float* d_gpos4)
+int rdf_gradient(cf_world* w, const float* d_pos, int stride, int bins, float r_max, const float* d_ghist, float* d_gpos)
 {
     int rc = check_world(w);
     if (rc) return rc;
     if (w->worlds > 1) return fail(CF_ERR_INVALID, "the radial distribution covers a single world");
     const int T = w->num_types;
-    if (bins < 1 || !d_ghist || !d_gpos4 || (long long)T * T * bins > kRdfMaxEntries)
+    if (bins < 1 || !d_ghist || !d_gpos || (long long)T * T * bins > kRdfMaxEntries)
         return fail(CF_ERR_INVALID, "bins must be >= 1 with T * T * bins <= 49152, buffers not NULL");
-    if (!(r_max > 0.0f) || !std::isfinite(r_max)) return fail(CF_ERR_INVALID, "r_max must be finite and positive");
-    rc = ensure_rdf(w);
-    if (rc) return rc;
-    Grid g = choose_step_grid(w->ext, rdf_cutoff(bins, r_max), kMaxCells);
-    apply_worlds(g, 1);
-    rc = ensure_cells(w, g.cells);
-    if (!rc) rc = ensure_offsets(w, g.cells);
-    if (rc) return rc;
-    CF_CUDA(configure_adjoint());
-    Rollout& r = w->ro;
-    const float4* pos = w->pos;
-    if (d_pos4) {
-        CF_CUDA(launch_pack_pos(reinterpret_cast<const float4*>(d_pos4), w->pos, r.rdf_pos, w->n, w->stream));
-        pos = r.rdf_pos;
-    }
-    Scratch& s = w->s;
+    const float4* pos = nullptr;
+    Grid g;
     int which = 0;
-    CF_CUDA(launch_cell_list_csr(pos, w->n, g, w->ext, T, s, s.cell_off, nullptr, nullptr, w->err, &which, w->stream));
-    CF_CUDA(launch_rdf_grad(w->ext, g, w->n, T, bins, r_max, pos, s.pos_sorted, s.keys[which], s.vals[which],
-                            s.cell_off, d_ghist, r.type_count, reinterpret_cast<float4*>(d_gpos4), w->stream));
+    rc = rdf_list(w, d_pos, stride, bins, r_max, &pos, &g, &which);
+    if (rc) return rc;
+    Scratch& s = w->s;
+    CF_CUDA(launch_rdf_grad(w->ext, g, w->n, T, bins, r_max, pos, s.pos_sorted, s.keys[which], s.vals[which], s.cell_off,
+                            d_ghist, w->ro.type_count, d_gpos, stride, w->stream));
     return CF_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int cf_rdf(cf_world* w, const float* d_pos4, int bins, float r_max, float* d_hist)
+{
+    return rdf_forward(w, d_pos4, 4, bins, r_max, d_hist);
+}
+
+int cf_rdf_xyz(cf_world* w, const float* d_pos, int bins, float r_max, float* d_hist)
+{
+    if (!d_pos) return fail(CF_ERR_INVALID, "null positions");
+    return rdf_forward(w, d_pos, 3, bins, r_max, d_hist);
+}
+
+int cf_rdf_backward(cf_world* w, const float* d_pos4, int bins, float r_max, const float* d_ghist, float* d_gpos4)
+{
+    return rdf_gradient(w, d_pos4, 4, bins, r_max, d_ghist, d_gpos4);
+}
+
+int cf_rdf_backward_xyz(cf_world* w, const float* d_pos, int bins, float r_max, const float* d_ghist, float* d_gpos)
+{
+    if (!d_pos) return fail(CF_ERR_INVALID, "null positions");
+    return rdf_gradient(w, d_pos, 3, bins, r_max, d_ghist, d_gpos);
 }
 
 }  // extern "C"

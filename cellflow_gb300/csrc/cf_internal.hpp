@@ -294,6 +294,7 @@ struct cf_world {
     std::vector<int> world_off;
     float* world_tables = nullptr;  // device, worlds * T * T floats
     cudaStream_t own_stream = nullptr;
+    cudaEvent_t order_event = nullptr;  // cf_stream_wait / cf_stream_signal
     cudaStream_t stream = nullptr;
     float4* pos = nullptr;
     float4* vel = nullptr;
@@ -466,14 +467,20 @@ cudaError_t launch_adjoint_step(const StepConsts& c, const PairTables* tables, c
                                 const uint32_t* keys_sorted, const uint32_t* vals_sorted, const uint32_t* cell_off,
                                 const float4* vel, const int* cnt_prev, const int* cnt_new, float4* gx, float4* gv,
                                 float4* gf_sorted, float4* ga_sorted, double* gacc, cudaStream_t st);
-cudaError_t launch_pack_pos(const float4* src, const float4* typesrc, float4* dst, int n, cudaStream_t st);
+// dst.xyz = rows of `stride` floats (3 or 4), dst.w = typesrc.w (the particle's type bits).
+cudaError_t launch_pack_pos(const float* rows, int stride, const float4* typesrc, float4* dst, int n, cudaStream_t st);
+// a.xyz, b.xyz = rows of three floats (NULL: zeros), w = 0.
+cudaError_t launch_rows_in(const float* a_rows, const float* b_rows, float4* a, float4* b, int n, cudaStream_t st);
+// Rows of three floats = a.xyz, b.xyz (NULL rows: none); and, with gacc, the table and parameter gradients as floats.
+cudaError_t launch_rows_out(const float4* a, const float4* b, float* a_rows, float* b_rows, int n, const double* gacc,
+                            int T, float* grad_force, float* grad_params, cudaStream_t st);
 cudaError_t launch_rdf(const float* ext, const Grid& g, int n, int T, int bins, float r_max, const float4* pos_sorted,
                        const uint32_t* keys_sorted, const uint32_t* cell_off, double* acc,
                        unsigned long long* type_count, float* hist, cudaStream_t st);
 cudaError_t launch_rdf_grad(const float* ext, const Grid& g, int n, int T, int bins, float r_max,
                             const float4* pos, const float4* pos_sorted, const uint32_t* keys_sorted,
                             const uint32_t* vals_sorted, const uint32_t* cell_off, const float* ghist,
-                            unsigned long long* type_count, float4* gpos, cudaStream_t st);
+                            unsigned long long* type_count, float* gpos, int gpos_stride, cudaStream_t st);
 
 // Host helpers (api.cpp).
 Grid choose_step_grid(const float* ext, float r_cut, int max_cells);

@@ -9,6 +9,7 @@ call goes through libcellflow.so.  Arrays are numpy; a failing call raises
 from __future__ import annotations
 
 import ctypes as C
+import operator
 from dataclasses import dataclass, fields
 
 import numpy as np
@@ -42,10 +43,11 @@ class SimulationParams:
     max_expected_neighbors: int = 400
 
     def to_c(self) -> StepParams:
-        p = StepParams()
-        for f in fields(self):
-            setattr(p, f.name, getattr(self, f.name))
-        return p
+        # (positional: the fields in the structure's own order)
+        return StepParams(*_PARAM_VALUES(self))
+
+
+_PARAM_VALUES = operator.attrgetter(*(name for name, _ in StepParams._fields_))
 
 
 def _ptr(a: np.ndarray) -> C.c_void_p:

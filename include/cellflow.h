@@ -143,6 +143,12 @@ int cf_destroy(cf_world* w);
 /* Run the world's work on a caller-owned cudaStream_t (NULL restores the
  * world's own stream).  The caller keeps the stream alive. */
 int cf_set_stream(cf_world* w, void* cuda_stream);
+/* Ordering with a caller's stream without running on it: the world's later work
+ * waits for what `cuda_stream` holds now (cf_stream_wait); later work on
+ * `cuda_stream` waits for the world's work so far (cf_stream_signal).  NULL is
+ * the legacy default stream.  Neither waits on the host. */
+int cf_stream_wait(cf_world* w, void* cuda_stream);
+int cf_stream_signal(cf_world* w, void* cuda_stream);
 int cf_sync(cf_world* w);
 int cf_particle_count(const cf_world* w, int* n);
 int cf_num_particle_types(const cf_world* w, int* t);
@@ -424,6 +430,14 @@ int cf_rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos4
  * The world's state is left as the forward left it. */
 int cf_rollout_backward(cf_world* w, const float* d_gpos4, const float* d_gvel4, float* d_gpos4_out,
                         float* d_gvel4_out, float* grad_force, int grad_force_count, float* grad_params);
+/* The two calls above with rows of three floats (x, y, z) instead of float4,
+ * and the gradients left on the device: d_grad_force (T*T floats) and
+ * d_grad_params (CF_GRAD_PARAMS floats), either may be NULL.  The backward
+ * waits for its work and reports device errors, as cf_rollout_backward. */
+int cf_rollout_forward_xyz(cf_world* w, const cf_step_params* p, const float* d_pos_in, const float* d_vel_in,
+                           int nsteps, int checkpoint_every, float* d_pos_out, float* d_vel_out);
+int cf_rollout_backward_xyz(cf_world* w, const float* d_gpos, const float* d_gvel, float* d_gpos_out,
+                            float* d_gvel_out, float* d_grad_force, float* d_grad_params);
 /* Soft type-resolved radial distribution of the positions d_pos4 (NULL: the
  * world's current ones): bins of width D = r_max / bins, cubic B-spline
  * weights of support 2 bins each side of the centre (k + 1/2) D, each entry
@@ -432,6 +446,9 @@ int cf_rollout_backward(cf_world* w, const float* d_gpos4, const float* d_gvel4,
 int cf_rdf(cf_world* w, const float* d_pos4, int bins, float r_max, float* d_hist);
 /* dL/dpos (device, n float4) of L(hist) given d_ghist = dL/dhist (device). */
 int cf_rdf_backward(cf_world* w, const float* d_pos4, int bins, float r_max, const float* d_ghist, float* d_gpos4);
+/* Both with rows of three floats instead of float4 (d_pos not NULL). */
+int cf_rdf_xyz(cf_world* w, const float* d_pos, int bins, float r_max, float* d_hist);
+int cf_rdf_backward_xyz(cf_world* w, const float* d_pos, int bins, float r_max, const float* d_ghist, float* d_gpos);
 
 /* ---- presets ----------------------------------------------------------------
  *
