@@ -312,81 +312,166 @@ struct RdfConsts {
     int n, T, bins;
     float inv_bin;  // 1 / D
     float r_cut;    // r_max + 1.5 D
+    float r_cut2;   // its square
 };
 
-__device__ __forceinline__ float bspline3(float t)
+// Both radial-distribution kernels: one warp per home (grid-stride), lanes striding over the
+// home's stencil run by run.  Few candidates are within range (one in eight when evenly
+// spread), so those that are go to a queue in shared memory (by ballot) and are worked off 32 at a
+// time with every lane busy, instead of by the few lanes of each 32 that hold one.  The
+// queue is what the time went on before: 16,384 particles, 607 candidates and 78 in range
+// each, 75 us for the histogram and 132 for its gradient.
+constexpr int kRdfWarps = 8;
+constexpr int kRdfQueue = 64;  // entries per warp: fewer than 32 kept, at most 32 more per push
+
+// The stencil's runs of cell `cell` as one run per lane: sorted range [beg, beg + len) and the
+// periodic shift of its positions as a code per axis (1 subtract the extent, 2 add it).
+__device__ __forceinline__ void stencil_run(const RdfConsts& c, uint32_t cell, const uint32_t* __restrict__ cell_off,
+                                            int lane, uint32_t& beg, int& len, uint32_t& shift)
 {
-    const float a = fabsf(t);
-    if (a < 1.0f) return 2.0f / 3.0f - a * a + 0.5f * a * a * a;
-    if (a < 2.0f) {
-        const float u = 2.0f - a;
-        return u * u * u * (1.0f / 6.0f);
+    const int m0 = c.m[0], m1 = c.m[1], m2 = c.m[2];
+    const int cx = (int)(cell % (uint32_t)m0), cy = (int)((cell / (uint32_t)m0) % (uint32_t)m1),
+              cz = (int)(cell / ((uint32_t)m0 * (uint32_t)m1));
+    int ylo, yhi, zlo, zhi, a0, b0, a1, b1;
+    axis_range(m1, ylo, yhi);
+    axis_range(m2, zlo, zhi);
+    x_runs(cx, m0, a0, b0, a1, b1);
+    const int ny = yhi - ylo + 1, nrows = ny * (zhi - zlo + 1);
+    beg = 0u;
+    len = 0;
+    shift = 0u;
+    if (lane < 2 * nrows) {
+        const int r = lane >> 1, run = lane & 1;
+        const int y = cy + ylo + r % ny, z = cz + zlo + r / ny;
+        const int ra = run ? a1 : a0, rb = run ? b1 : b0;
+        if (rb >= ra) {
+            const int row = (wrap_cell(z, m2) * m1 + wrap_cell(y, m1)) * m0;
+            beg = cell_off[row + ra];
+            len = (int)(cell_off[row + rb + 1] - beg);
+            const uint32_t sx = ra > cx + 1 ? 1u : (rb < cx - 1 ? 2u : 0u);
+            shift = sx | (y < 0 ? 1u : (y >= m1 ? 2u : 0u)) << 2 | (z < 0 ? 1u : (z >= m2 ? 2u : 0u)) << 4;
+        }
     }
-    return 0.0f;
 }
 
-__device__ __forceinline__ float bspline3_d(float t)
+__device__ __forceinline__ float run_shift(uint32_t code, float ext) { return code == 1u ? -ext : (code == 2u ? ext : 0.0f); }
+
+// Calls push(hit, o, dx, dy, dz, d2) for the candidates of one home, 32 at a time, the whole
+// warp together; hit: the lane's candidate o is another particle within r_cut of the home.
+// kAfter: only candidates behind the home in the sorted order.  kWrap: fewer than five cells on
+// some axis, the reference's wrap per candidate; else a run's shift is the wrap.
+template <bool kWrap, bool kAfter, typename Push>
+__device__ __forceinline__ void rdf_candidates(const RdfConsts& c, const float4* __restrict__ pos_sorted, uint32_t cell,
+                                               const uint32_t* __restrict__ cell_off, int k, const float4& h, int lane,
+                                               Push push)
 {
-    const float a = fabsf(t);
-    float g = 0.0f;
-    if (a < 1.0f)
-        g = -2.0f * a + 1.5f * a * a;
-    else if (a < 2.0f) {
-        const float u = 2.0f - a;
-        g = -0.5f * u * u;
+    uint32_t beg, shift;
+    int len;
+    stencil_run(c, cell, cell_off, lane, beg, len, shift);
+    if (kAfter) {
+        const int skip = min(len, max(0, k + 1 - (int)beg));
+        beg += (uint32_t)skip;
+        len -= skip;
     }
-    return t < 0.0f ? -g : g;
+    uint32_t runs = __ballot_sync(0xffffffffu, len > 0);
+    while (runs) {
+        const int src = __ffs(runs) - 1;
+        runs &= runs - 1u;
+        const uint32_t b = __shfl_sync(0xffffffffu, beg, src), code = __shfl_sync(0xffffffffu, shift, src);
+        const int l = __shfl_sync(0xffffffffu, len, src);
+        const float sx = run_shift(code & 3u, c.ext[0]), sy = run_shift((code >> 2) & 3u, c.ext[1]),
+                    sz = run_shift(code >> 4, c.ext[2]);
+        for (int e0 = 0; e0 < l; e0 += 32) {
+            const int q = (int)b + min(e0 + lane, l - 1);
+            const float4 o = pos_sorted[q];
+            float dx = o.x - h.x, dy = o.y - h.y, dz = o.z - h.z;
+            if (kWrap) {
+                dx = wrap_ref(dx, c.ext[0], c.half[0]);
+                dy = wrap_ref(dy, c.ext[1], c.half[1]);
+                dz = wrap_ref(dz, c.ext[2], c.half[2]);
+            } else {
+                dx += sx;
+                dy += sy;
+                dz += sz;
+            }
+            const float d2 = dx * dx + dy * dy + dz * dz;
+            push(d2 < c.r_cut2 && e0 + lane < l && (kAfter || q != k), o, dx, dy, dz, d2);
+        }
+    }
 }
 
-// Calls fn(q, o, dx, dy, dz, r) for every other particle q (position o) within r_cut of
-// home k, spread over the lanes of the calling warp (for_stencil).
-template <typename Fn>
-__device__ __forceinline__ void rdf_neighbours_warp(const RdfConsts& c, const float4* __restrict__ pos_sorted,
-                                                    const uint32_t* __restrict__ keys,
-                                                    const uint32_t* __restrict__ cell_off, uint32_t* list, int k,
-                                                    const float4& h, int lane, Fn fn)
+// The first of the four bins that a pair at distance r touches and where r lies past it: bin
+// first + j has the cubic B-spline weight of t0 - (first + j), t0 = r / D - 1/2.
+__device__ __forceinline__ int rdf_first_bin(const RdfConsts& c, float r, float& u)
 {
-    for_stencil(c.m[0], c.m[1], c.m[2], keys[k], cell_off, list, lane, [&](uint32_t q) {
-        if ((int)q == k) return;
-        const float4 o = pos_sorted[q];
-        const float dx = wrap_ref(o.x - h.x, c.ext[0], c.half[0]);
-        const float dy = wrap_ref(o.y - h.y, c.ext[1], c.half[1]);
-        const float dz = wrap_ref(o.z - h.z, c.ext[2], c.half[2]);
-        const float r = sqrtf(dx * dx + dy * dy + dz * dz);
-        if (r < c.r_cut) fn(q, o, dx, dy, dz, r);
-    });
+    const float t0 = r * c.inv_bin - 0.5f;
+    const float f = floorf(t0);
+    u = t0 - f;
+    return (int)f - 1;
 }
 
-// One warp per home (grid-stride), the histogram in shared memory per block.
-__global__ void rdf_kernel(RdfConsts c, const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ keys,
-                           const uint32_t* __restrict__ cell_off, double* __restrict__ acc,
-                           unsigned long long* __restrict__ type_count)
+// One warp per home and each pair once (from its first particle in the sorted order): the
+// histogram of type pairs a <= b in shared memory per block, doubled or mirrored by
+// rdf_finish_kernel.
+template <bool kWrap>
+__global__ void __launch_bounds__(32 * kRdfWarps)
+    rdf_kernel(RdfConsts c, const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ keys,
+               const uint32_t* __restrict__ cell_off, double* __restrict__ acc,
+               unsigned long long* __restrict__ type_count)
 {
     extern __shared__ float s_hist[];
     __shared__ unsigned int s_count[CF_MAX_TYPES];
-    __shared__ uint32_t s_list[kAdjThreads / 32][kListCap];
+    __shared__ float2 s_queue[kRdfWarps][kRdfQueue];  // squared distance, first bin of the type pair (as bits)
     const int H = c.T * c.T * c.bins;
     for (int q = threadIdx.x; q < H; q += blockDim.x) s_hist[q] = 0.0f;
     if (threadIdx.x < CF_MAX_TYPES) s_count[threadIdx.x] = 0u;
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int warps = (int)(gridDim.x * (blockDim.x >> 5));
-    for (int k = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); k < c.n; k += warps) {
+    float2* queue = s_queue[threadIdx.x >> 5];
+    int held = 0;  // entries in the queue
+    const auto work_off = [&](int entries) {
+        __syncwarp();
+        if (lane < entries) {
+            const float2 e = queue[lane];
+            float u;
+            const int first = rdf_first_bin(c, sqrtf(e.x), u);
+            float* row = s_hist + __float_as_int(e.y);
+            const float v = 1.0f - u, u2 = u * u, v2 = v * v;
+            const float w[4] = {v2 * v * (1.0f / 6.0f), 2.0f / 3.0f - u2 + 0.5f * u2 * u, 2.0f / 3.0f - v2 + 0.5f * v2 * v,
+                                u2 * u * (1.0f / 6.0f)};
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (first + j >= 0 && first + j < c.bins) atomicAdd(&row[first + j], w[j]);
+        }
+        __syncwarp();
+        // what is left moves to the front
+        const float2 rest = queue[32 + lane];
+        __syncwarp();
+        queue[lane] = rest;
+        held = max(0, held - 32);
+    };
+    const int warps = (int)gridDim.x * kRdfWarps;
+    for (int k = (int)blockIdx.x * kRdfWarps + (int)(threadIdx.x >> 5); k < c.n; k += warps) {
         const float4 h = pos_sorted[k];
         const uint32_t ti = type_of(h);
         // a type outside [0, T) is reported by the cell list's hash; skip it here
         if (ti >= (uint32_t)c.T) continue;
         if (lane == 0) atomicAdd(&s_count[ti], 1u);
-        rdf_neighbours_warp(c, pos_sorted, keys, cell_off, s_list[threadIdx.x >> 5], k, h, lane,
-                            [&](uint32_t, const float4& o, float, float, float, float r) {
-                                if (type_of(o) >= (uint32_t)c.T) return;
-                                const float t0 = r * c.inv_bin - 0.5f;
-                                const int k0 = max(0, (int)ceilf(t0 - 2.0f));
-                                const int k1 = min(c.bins - 1, (int)floorf(t0 + 2.0f));
-                                float* row = s_hist + ((int)ti * c.T + (int)type_of(o)) * c.bins;
-                                for (int b = k0; b <= k1; b++) atomicAdd(&row[b], bspline3(t0 - (float)b));
-                            });
+        rdf_candidates<kWrap, true>(c, pos_sorted, keys[k], cell_off, k, h, lane,
+                                    [&](bool hit, const float4& o, float, float, float, float d2) {
+                                        const uint32_t tj = type_of(o);
+                                        hit = hit && tj < (uint32_t)c.T;
+                                        const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+                                        if (hit) {
+                                            const int row = (int)(min(ti, tj) * c.T + max(ti, tj)) * c.bins;
+                                            queue[held + __popc(hits & ((1u << lane) - 1u))] =
+                                                make_float2(d2, __int_as_float(row));
+                                        }
+                                        held += __popc(hits);
+                                        if (held >= 32) work_off(32);
+                                    });
     }
+    work_off(held);
     __syncthreads();
     for (int q = threadIdx.x; q < H; q += blockDim.x)
         if (s_hist[q] != 0.0f) atomicAdd(&acc[q], (double)s_hist[q]);
@@ -419,46 +504,85 @@ __global__ void rdf_finish_kernel(RdfConsts c, const double* __restrict__ acc,
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= c.T * c.T * c.bins) return;
     const double den = rdf_den(c, type_count, q);
-    hist[q] = den > 0.0 ? (float)(acc[q] / den) : 0.0f;
+    // acc holds each pair once, under its smaller type first
+    const int k = q % c.bins, ab = q / c.bins, a = ab / c.T, b = ab % c.T;
+    const double sum = a == b ? 2.0 * acc[q] : acc[(min(a, b) * c.T + max(a, b)) * c.bins + k];
+    hist[q] = den > 0.0 ? (float)(sum / den) : 0.0f;
 }
 
-__global__ void rdf_grad_kernel(RdfConsts c, const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ keys,
-                                const uint32_t* __restrict__ vals, const uint32_t* __restrict__ cell_off,
-                                const float* __restrict__ ghist, const unsigned long long* __restrict__ type_count,
-                                float* __restrict__ gpos, int gpos_stride)
+// The gradient's weights of bin (a, b, k): ghist / normalisation of (a, b) and (b, a) together (a
+// pair moves both).  Once per call: its double divisions, done by every block of the gradient
+// kernel, took 70 of that kernel's 98 us.
+__global__ void rdf_weight_kernel(RdfConsts c, const float* __restrict__ ghist,
+                                  const unsigned long long* __restrict__ type_count, float* __restrict__ weight)
 {
-    extern __shared__ float s_g[];  // ghist / den
-    __shared__ uint32_t s_list[kAdjThreads / 32][kListCap];
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= c.T * c.T * c.bins) return;
+    const int k = q % c.bins, ab = q / c.bins, a = ab / c.T, b = ab % c.T;
+    const double den = rdf_den(c, type_count, q);
+    weight[q] = den > 0.0 ? (float)(((double)ghist[q] + (double)ghist[(b * c.T + a) * c.bins + k]) / den) : 0.0f;
+}
+
+template <bool kWrap>
+__global__ void __launch_bounds__(32 * kRdfWarps)
+    rdf_grad_kernel(RdfConsts c, const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ keys,
+                    const uint32_t* __restrict__ vals, const uint32_t* __restrict__ cell_off,
+                    const float* __restrict__ weight, float* __restrict__ gpos, int gpos_stride)
+{
+    extern __shared__ float s_g[];                     // weight
+    __shared__ float4 s_queue[kRdfWarps][kRdfQueue];  // displacement, type
     const int H = c.T * c.T * c.bins;
-    for (int q = threadIdx.x; q < H; q += blockDim.x) {
-        const double den = rdf_den(c, type_count, q);
-        s_g[q] = den > 0.0 ? (float)((double)ghist[q] / den) : 0.0f;
-    }
+    for (int q = threadIdx.x; q < H; q += blockDim.x) s_g[q] = weight[q];
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    const int warps = (int)(gridDim.x * (blockDim.x >> 5));
-    for (int k = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); k < c.n; k += warps) {
+    float4* queue = s_queue[threadIdx.x >> 5];
+    const int warps = (int)gridDim.x * kRdfWarps;
+    for (int k = (int)blockIdx.x * kRdfWarps + (int)(threadIdx.x >> 5); k < c.n; k += warps) {
         const float4 h = pos_sorted[k];
         const uint32_t ti = type_of(h);
         float ax = 0.0f, ay = 0.0f, az = 0.0f;
+        int held = 0;
+        const auto work_off = [&](int entries) {
+            __syncwarp();
+            if (lane < entries) {
+                const float4 e = queue[lane];
+                const uint32_t tj = __float_as_uint(e.w);
+                const float r = sqrtf(e.x * e.x + e.y * e.y + e.z * e.z);
+                float u;
+                const int first = rdf_first_bin(c, r, u);
+                const float* g = s_g + ((int)ti * c.T + (int)tj) * c.bins;
+                // derivatives of the four B-spline weights (work_off of rdf_kernel) by t0
+                const float v = 1.0f - u;
+                const float w[4] = {-0.5f * v * v, u * (1.5f * u - 2.0f), v * (2.0f - 1.5f * v), 0.5f * u * u};
+                float G = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (first + j >= 0 && first + j < c.bins) G += g[first + j] * w[j];
+                const float s = r > 0.0f ? G * c.inv_bin / r : 0.0f;
+                ax -= s * e.x;
+                ay -= s * e.y;
+                az -= s * e.z;
+            }
+            __syncwarp();
+            const float4 rest = queue[32 + lane];
+            __syncwarp();
+            queue[lane] = rest;
+            held = max(0, held - 32);
+        };
         // a type outside [0, T) is reported by the cell list's hash; it contributes nothing here
         if (ti < (uint32_t)c.T)
-            rdf_neighbours_warp(c, pos_sorted, keys, cell_off, s_list[threadIdx.x >> 5], k, h, lane,
-                                [&](uint32_t, const float4& o, float dx, float dy, float dz, float r) {
-                                    const uint32_t tj = type_of(o);
-                                    if (!(r > 0.0f) || tj >= (uint32_t)c.T) return;
-                                    const float t0 = r * c.inv_bin - 0.5f;
-                                    const int k0 = max(0, (int)ceilf(t0 - 2.0f));
-                                    const int k1 = min(c.bins - 1, (int)floorf(t0 + 2.0f));
-                                    const float* gij = s_g + ((int)ti * c.T + (int)tj) * c.bins;
-                                    const float* gji = s_g + ((int)tj * c.T + (int)ti) * c.bins;
-                                    float G = 0.0f;
-                                    for (int b = k0; b <= k1; b++) G += (gij[b] + gji[b]) * bspline3_d(t0 - (float)b);
-                                    const float s = G * c.inv_bin / r;
-                                    ax -= s * dx;
-                                    ay -= s * dy;
-                                    az -= s * dz;
-                                });
+            rdf_candidates<kWrap, false>(c, pos_sorted, keys[k], cell_off, k, h, lane,
+                                         [&](bool hit, const float4& o, float dx, float dy, float dz, float) {
+                                             const uint32_t tj = type_of(o);
+                                             hit = hit && tj < (uint32_t)c.T;
+                                             const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+                                             if (hit)
+                                                 queue[held + __popc(hits & ((1u << lane) - 1u))] =
+                                                     make_float4(dx, dy, dz, __uint_as_float(tj));
+                                             held += __popc(hits);
+                                             if (held >= 32) work_off(32);
+                                         });
+        if (held > 0) work_off(held);
         ax = warp_sum(ax);
         ay = warp_sum(ay);
         az = warp_sum(az);
@@ -533,6 +657,7 @@ RdfConsts rdf_consts(const float* ext, const Grid& g, int n, int T, int bins, fl
     c.bins = bins;
     c.inv_bin = (float)bins / r_max;
     c.r_cut = rdf_cutoff(bins, r_max);
+    c.r_cut2 = c.r_cut * c.r_cut;
     return c;
 }
 
@@ -544,9 +669,10 @@ size_t rdf_smem_bytes(int T, int bins) { return sizeof(float) * (size_t)T * T * 
 
 cudaError_t configure_adjoint()
 {
-    cudaError_t e = cudaFuncSetAttribute(rdf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRdfMaxSmem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(rdf_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRdfMaxSmem);
+    cudaError_t e = cudaSuccess;
+    for (const void* f : {(const void*)rdf_kernel<false>, (const void*)rdf_kernel<true>,
+                          (const void*)rdf_grad_kernel<false>, (const void*)rdf_grad_kernel<true>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kRdfMaxSmem);
     return e;
 }
 
@@ -593,22 +719,30 @@ cudaError_t launch_rows_out(const float4* a, const float4* b, float* a_rows, flo
     return cudaGetLastError();
 }
 
+cudaError_t launch_rdf_clear(int n, int T, int bins, const float4* pos, double* acc, unsigned long long* type_count,
+                             cudaStream_t st)
+{
+    cudaError_t e = cudaMemsetAsync(type_count, 0, sizeof(unsigned long long) * CF_MAX_TYPES, st);
+    if (e == cudaSuccess && acc) e = cudaMemsetAsync(acc, 0, sizeof(double) * T * T * bins, st);
+    if (e != cudaSuccess || acc || n == 0) return e;
+    type_count_kernel<<<(n + 255) / 256, 256, 0, st>>>(pos, n, type_count);
+    note_launches(st);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_rdf(const float* ext, const Grid& g, int n, int T, int bins, float r_max, const float4* pos_sorted,
                        const uint32_t* keys_sorted, const uint32_t* cell_off, double* acc,
                        unsigned long long* type_count, float* hist, cudaStream_t st)
 {
     const RdfConsts c = rdf_consts(ext, g, n, T, bins, r_max);
     const int H = T * T * bins;
-    cudaError_t e = cudaMemsetAsync(acc, 0, sizeof(double) * H, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(type_count, 0, sizeof(unsigned long long) * CF_MAX_TYPES, st);
-    if (e != cudaSuccess) return e;
-    // one warp per home, grid-stride; up to eight blocks per SM while their histograms
-    // stay within 48 KB of shared memory (every block flushes its histogram once)
-    const int warps_per_block = kAdjThreads / 32;
-    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(8, (48u << 10) / rdf_smem_bytes(T, bins)));
+    // grid-stride; up to six blocks per SM while their histograms stay within 64 KB of shared
+    // memory (every block flushes its histogram once)
+    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(6, (64u << 10) / rdf_smem_bytes(T, bins)));
     if (n > 0) {
-        rdf_kernel<<<std::min((n + warps_per_block - 1) / warps_per_block, per_sm * num_sms()), kAdjThreads,
-                     rdf_smem_bytes(T, bins), st>>>(c, pos_sorted, keys_sorted, cell_off, acc, type_count);
+        (g.generic ? rdf_kernel<true> : rdf_kernel<false>)<<<std::min((n + kRdfWarps - 1) / kRdfWarps, per_sm * num_sms()),
+                                                             32 * kRdfWarps, rdf_smem_bytes(T, bins), st>>>(
+            c, pos_sorted, keys_sorted, cell_off, acc, type_count);
         note_launches(st);
     }
     rdf_finish_kernel<<<(H + 255) / 256, 256, 0, st>>>(c, acc, type_count, hist);
@@ -617,19 +751,18 @@ cudaError_t launch_rdf(const float* ext, const Grid& g, int n, int T, int bins, 
 }
 
 cudaError_t launch_rdf_grad(const float* ext, const Grid& g, int n, int T, int bins, float r_max,
-                            const float4* pos, const float4* pos_sorted, const uint32_t* keys_sorted,
-                            const uint32_t* vals_sorted, const uint32_t* cell_off, const float* ghist,
-                            unsigned long long* type_count, float* gpos, int gpos_stride, cudaStream_t st)
+                            const float4* pos_sorted, const uint32_t* keys_sorted, const uint32_t* vals_sorted,
+                            const uint32_t* cell_off, const float* ghist, unsigned long long* type_count,
+                            float* weight, float* gpos, int gpos_stride, cudaStream_t st)
 {
+    if (n == 0) return cudaSuccess;
     const RdfConsts c = rdf_consts(ext, g, n, T, bins, r_max);
-    cudaError_t e = cudaMemsetAsync(type_count, 0, sizeof(unsigned long long) * CF_MAX_TYPES, st);
-    if (e != cudaSuccess || n == 0) return e;
-    type_count_kernel<<<(n + 255) / 256, 256, 0, st>>>(pos, n, type_count);
+    const int H = T * T * bins;
+    rdf_weight_kernel<<<(H + 127) / 128, 128, 0, st>>>(c, ghist, type_count, weight);
     note_launches(st);
-    const int warps_per_block = kAdjThreads / 32;
-    rdf_grad_kernel<<<std::min((n + warps_per_block - 1) / warps_per_block, 8 * num_sms()), kAdjThreads,
-                      rdf_smem_bytes(T, bins), st>>>(c, pos_sorted, keys_sorted, vals_sorted, cell_off, ghist,
-                                                     type_count, gpos, gpos_stride);
+    (g.generic ? rdf_grad_kernel<true> : rdf_grad_kernel<false>)<<<std::min((n + kRdfWarps - 1) / kRdfWarps, 6 * num_sms()),
+                                                                   32 * kRdfWarps, rdf_smem_bytes(T, bins), st>>>(
+        c, pos_sorted, keys_sorted, vals_sorted, cell_off, weight, gpos, gpos_stride);
     note_launches(st);
     return cudaGetLastError();
 }

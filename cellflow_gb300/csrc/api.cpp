@@ -185,6 +185,11 @@ void free_rollout(cf_world* w)
     Rollout& r = w->ro;
     if (r.bwd_graph) cudaGraphExecDestroy(r.bwd_graph);
     if (r.fwd_graph) cudaGraphExecDestroy(r.fwd_graph);
+    // (the radial distribution's list graphs hold its scratch by address)
+    for (int k = 3; k < 5; k++) {
+        if (w->sel_graph[k].exec) cudaGraphExecDestroy(w->sel_graph[k].exec);
+        w->sel_graph[k] = SelGraph();
+    }
     if (r.ev_fork) cudaEventDestroy(r.ev_fork);
     if (r.ev_join) cudaEventDestroy(r.ev_join);
     if (r.side) cudaStreamDestroy(r.side);
@@ -2373,6 +2378,7 @@ int ensure_rdf(cf_world* w)
 {
     Rollout& r = w->ro;
     if (r.rdf_pos) return CF_OK;
+    CF_CUDA(configure_adjoint());
     if (!r.rdf_acc) {
         const int rc = alloc_pair(&r.rdf_acc, (size_t)kRdfMaxEntries, &r.type_count, (size_t)CF_MAX_TYPES);
         if (rc) return rc;
@@ -2788,8 +2794,9 @@ int cf_rollout_backward(cf_world* w, const float* d_gpos4, const float* d_gvel4,
 namespace {
 
 // Checks, scratch and the cell list of the radial distribution of d_pos (rows of `stride`
-// floats; NULL: the world's positions): *pos the positions used, *g the grid, *which the list.
-int rdf_list(cf_world* w, const float* d_pos, int stride, int bins, float r_max, const float4** pos, Grid* g, int* which)
+// floats; NULL: the world's positions): *g the grid, *which the list.  The list's kernels, with
+// the type counts (`count`) or, without, the cleared histogram, run as one cached graph.
+int rdf_list(cf_world* w, const float* d_pos, int stride, int bins, float r_max, bool count, Grid* g, int* which)
 {
     const int T = w->num_types;
     if (!(r_max > 0.0f) || !std::isfinite(r_max)) return fail(CF_ERR_INVALID, "r_max must be finite and positive");
@@ -2800,17 +2807,24 @@ int rdf_list(cf_world* w, const float* d_pos, int stride, int bins, float r_max,
     rc = ensure_cells(w, g->cells);
     if (!rc) rc = ensure_offsets(w, g->cells);
     if (rc) return rc;
-    CF_CUDA(configure_adjoint());
     Rollout& r = w->ro;
-    *pos = w->pos;
+    const float4* pos = w->pos;
     if (d_pos) {
         CF_CUDA(launch_pack_pos(d_pos, stride, w->pos, r.rdf_pos, w->n, w->stream));
-        *pos = r.rdf_pos;
+        pos = r.rdf_pos;
     }
     Scratch& s = w->s;
-    *which = 0;
-    CF_CUDA(launch_cell_list_csr(*pos, w->n, *g, w->ext, T, s, s.cell_off, nullptr, nullptr, w->err, which, w->stream));
-    return CF_OK;
+    *which = cell_list_csr_buffer(w->n, *g);
+    return run_selection(
+        w, count ? 4 : 3, *g, 0.0f, bins,
+        [&]() -> int {
+            int buf = 0;
+            CF_CUDA(launch_cell_list_csr(pos, w->n, *g, w->ext, T, s, s.cell_off, nullptr, nullptr, w->err, &buf,
+                                         w->stream));
+            CF_CUDA(launch_rdf_clear(w->n, T, bins, pos, count ? nullptr : r.rdf_acc, r.type_count, w->stream));
+            return CF_OK;
+        },
+        pos);
 }
 
 int rdf_forward(cf_world* w, const float* d_pos, int stride, int bins, float r_max, float* d_hist)
@@ -2821,10 +2835,9 @@ int rdf_forward(cf_world* w, const float* d_pos, int stride, int bins, float r_m
     const int T = w->num_types;
     if (bins < 1 || !d_hist || (long long)T * T * bins > kRdfMaxEntries)
         return fail(CF_ERR_INVALID, "bins must be >= 1 with T * T * bins <= 49152, d_hist not NULL");
-    const float4* pos = nullptr;
     Grid g;
     int which = 0;
-    rc = rdf_list(w, d_pos, stride, bins, r_max, &pos, &g, &which);
+    rc = rdf_list(w, d_pos, stride, bins, r_max, false, &g, &which);
     if (rc) return rc;
     Scratch& s = w->s;
     CF_CUDA(launch_rdf(w->ext, g, w->n, T, bins, r_max, s.pos_sorted, s.keys[which], s.cell_off, w->ro.rdf_acc,
@@ -2840,14 +2853,14 @@ int rdf_gradient(cf_world* w, const float* d_pos, int stride, int bins, float r_
     const int T = w->num_types;
     if (bins < 1 || !d_ghist || !d_gpos || (long long)T * T * bins > kRdfMaxEntries)
         return fail(CF_ERR_INVALID, "bins must be >= 1 with T * T * bins <= 49152, buffers not NULL");
-    const float4* pos = nullptr;
     Grid g;
     int which = 0;
-    rc = rdf_list(w, d_pos, stride, bins, r_max, &pos, &g, &which);
+    rc = rdf_list(w, d_pos, stride, bins, r_max, true, &g, &which);
     if (rc) return rc;
     Scratch& s = w->s;
-    CF_CUDA(launch_rdf_grad(w->ext, g, w->n, T, bins, r_max, pos, s.pos_sorted, s.keys[which], s.vals[which], s.cell_off,
-                            d_ghist, w->ro.type_count, d_gpos, stride, w->stream));
+    CF_CUDA(launch_rdf_grad(w->ext, g, w->n, T, bins, r_max, s.pos_sorted, s.keys[which], s.vals[which], s.cell_off,
+                            d_ghist, w->ro.type_count, reinterpret_cast<float*>(w->ro.rdf_acc), d_gpos, stride,
+                            w->stream));
     return CF_OK;
 }
 

@@ -352,7 +352,9 @@ struct cf_world {
     const void* host_in = nullptr;
     void* host_out = nullptr;
     const void* host_bufs = nullptr;
-    cf::SelGraph sel_graph[3];  // proximity (counts + scan), triangle mesh, proximity vertices
+    // proximity (counts + scan), triangle mesh, proximity vertices, the radial distribution's cell list
+    // (histogram, gradient)
+    cf::SelGraph sel_graph[5];
 };
 
 namespace cf {
@@ -474,13 +476,16 @@ cudaError_t launch_rows_in(const float* a_rows, const float* b_rows, float4* a, 
 // Rows of three floats = a.xyz, b.xyz (NULL rows: none); and, with gacc, the table and parameter gradients as floats.
 cudaError_t launch_rows_out(const float4* a, const float4* b, float* a_rows, float* b_rows, int n, const double* gacc,
                             int T, float* grad_force, float* grad_params, cudaStream_t st);
+// The histogram sums (acc) and type counts cleared; without acc the type counts taken from pos.
+cudaError_t launch_rdf_clear(int n, int T, int bins, const float4* pos, double* acc, unsigned long long* type_count,
+                             cudaStream_t st);
 cudaError_t launch_rdf(const float* ext, const Grid& g, int n, int T, int bins, float r_max, const float4* pos_sorted,
                        const uint32_t* keys_sorted, const uint32_t* cell_off, double* acc,
                        unsigned long long* type_count, float* hist, cudaStream_t st);
 cudaError_t launch_rdf_grad(const float* ext, const Grid& g, int n, int T, int bins, float r_max,
-                            const float4* pos, const float4* pos_sorted, const uint32_t* keys_sorted,
-                            const uint32_t* vals_sorted, const uint32_t* cell_off, const float* ghist,
-                            unsigned long long* type_count, float* gpos, int gpos_stride, cudaStream_t st);
+                            const float4* pos_sorted, const uint32_t* keys_sorted, const uint32_t* vals_sorted,
+                            const uint32_t* cell_off, const float* ghist, unsigned long long* type_count,
+                            float* weight, float* gpos, int gpos_stride, cudaStream_t st);
 
 // Host helpers (api.cpp).
 Grid choose_step_grid(const float* ext, float r_cut, int max_cells);
