@@ -846,6 +846,21 @@ Grid choose_prox_grid(const float* ext, float distance, int max_cells)
     return g;
 }
 
+// The grid of the proximity selections, which pair particles of one type only: every type has cells
+// of its own (type * cells_w + cell), at most eight per particle in all, coarser where the distance would
+// give more (the cells are cleared and scanned in every call).
+Grid choose_type_grid(const float* ext, float distance, int types, int n)
+{
+    const long long limit = std::max(1ll, std::min<long long>(kMaxCells, std::max(8ll * n, 32768ll)) / types);
+    Grid g = choose_prox_grid(ext, distance, (int)limit);
+    g.by_type = 1;
+    g.worlds = types;
+    g.cells = types * g.cells_w;
+    g.key_bits = 0;
+    while ((1ll << g.key_bits) < (long long)g.cells) g.key_bits++;
+    return g;
+}
+
 // The work model's grid: floor(L / r_max) cells per axis of side L / cells.
 Grid canonical_grid(const float* ext, float r_max)
 {
@@ -1872,21 +1887,21 @@ int proximity_enqueue(cf_world* w, float distance, int max_conn)
         return fail(CF_ERR_INVALID, "max_conn must be in [0, 16] (the reference overflowed its buffer above 16)");
     int rc = ensure_prox(w);
     if (rc) return rc;
-    Grid g = choose_prox_grid(w->ext, distance, kMaxCells);
+    Grid g = choose_type_grid(w->ext, distance, w->num_types, w->n);
     rc = ensure_offsets(w, g.cells);
     if (rc) return rc;
     Scratch& s = w->s;
     const float dsq = distance * distance;  // ParticleSimulation.cu:660
     return run_selection(w, 0, g, dsq, max_conn, [&]() -> int {
-        // the tiled cell list on the proximity grid, unordered within a cell (the selection
+        // the tiled cell list on the grid by type, unordered within a cell (the selection
         // keeps the smallest qualifying indices whatever the order): cell c holds
         // cell_off[c] .. cell_off[c + 1]
         int which = 0;
         CF_CUDA(launch_cell_list_csr(w->pos, w->n, g, w->ext, w->num_types, s, s.cell_off, nullptr, nullptr, w->err,
                                      &which, w->stream, false));
         CF_CUDA(cudaMemsetAsync(s.prox_count + w->n, 0, sizeof(uint32_t), w->stream));
-        CF_CUDA(launch_proximity_select(s.pos_sorted, s.keys[which], s.vals[which], s.cell_off, s.cell_off + 1, true, g,
-                                        w->n, dsq, max_conn, s.prox_slots, s.prox_count, w->stream));
+        CF_CUDA(launch_proximity_select(s.pos_sorted, s.vals[which], s.cell_off, g, w->n, dsq, max_conn, s.prox_slots,
+                                        s.prox_count, w->stream));
         CF_CUDA(launch_scan_exclusive(s.prox_count, s.prox_count, w->n + 1, s.scan_tmp, s.scan_tmp_cap, w->stream));
         CF_CUDA(cudaMemcpyAsync(&w->host_words[1], s.prox_count + w->n, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                 w->stream));
@@ -1908,7 +1923,7 @@ int mesh_enqueue(cf_world* w, float distance, int max_conn)
     // ParticleSimulation.cu:723-724: 20 % hysteresis on the distance
     const float hysteresis = 1.2f;
     const float dsq = distance * distance * (hysteresis * hysteresis);
-    Grid g = choose_prox_grid(w->ext, nextafterf(std::sqrt(dsq), INFINITY), kMaxCells);
+    Grid g = choose_type_grid(w->ext, nextafterf(std::sqrt(dsq), INFINITY), w->num_types, w->n);
     rc = ensure_offsets(w, g.cells);
     if (rc) return rc;
     Scratch& s = w->s;
@@ -1917,8 +1932,8 @@ int mesh_enqueue(cf_world* w, float distance, int max_conn)
         CF_CUDA(launch_cell_list_csr(w->pos, w->n, g, w->ext, w->num_types, s, s.cell_off, nullptr, nullptr, w->err,
                                      &which, w->stream, false));
         CF_CUDA(cudaMemsetAsync(s.mesh_count + w->n, 0, sizeof(uint32_t), w->stream));
-        CF_CUDA(launch_mesh_select(s.pos_sorted, s.keys[which], s.vals[which], s.cell_off, s.cell_off + 1, g, w->n,
-                                   dsq, std::min(max_conn, CF_MESH_MAX_CONN), s.mesh_slots, s.mesh_count, w->stream));
+        CF_CUDA(launch_mesh_select(s.pos_sorted, s.vals[which], s.cell_off, g, w->n, dsq,
+                                   std::min(max_conn, CF_MESH_MAX_CONN), s.mesh_slots, s.mesh_count, w->stream));
         CF_CUDA(launch_scan_exclusive(s.mesh_count, s.mesh_count, w->n + 1, s.scan_tmp, s.scan_tmp_cap, w->stream));
         CF_CUDA(cudaMemcpyAsync(&w->host_words[1], s.mesh_count + w->n, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                 w->stream));
@@ -2029,7 +2044,7 @@ int cf_proximity_vertices_device(cf_world* w, float distance, int max_conn, cons
         return fail(CF_ERR_INVALID, "max_conn must be in [0, 16] (the reference overflowed its buffer above 16)");
     rc = ensure_prox(w);
     if (rc) return rc;
-    Grid g = choose_prox_grid(w->ext, distance, kMaxCells);
+    Grid g = choose_type_grid(w->ext, distance, w->num_types, w->n);
     rc = ensure_offsets(w, g.cells);
     if (rc) return rc;
     Scratch& s = w->s;
@@ -2047,8 +2062,8 @@ int cf_proximity_vertices_device(cf_world* w, float distance, int max_conn, cons
             CF_CUDA(launch_cell_list_csr(w->pos, w->n, g, w->ext, w->num_types, s, s.cell_off, nullptr, nullptr,
                                          w->err, &which, w->stream, false));
             CF_CUDA(cudaMemsetAsync(total, 0, sizeof(uint32_t), w->stream));
-            CF_CUDA(launch_proximity_select_vertices(s.pos_sorted, s.keys[which], s.vals[which], s.cell_off, g, w->n,
-                                                     dsq, max_conn, w->pos, ct, w->num_types, vertices, cap_vertices,
+            CF_CUDA(launch_proximity_select_vertices(s.pos_sorted, s.vals[which], s.cell_off, g, w->n, dsq,
+                                                     max_conn, w->pos, ct, w->num_types, vertices, cap_vertices,
                                                      total, w->stream));
             CF_CUDA(cudaMemcpyAsync(&w->host_words[1], total, sizeof(uint32_t), cudaMemcpyDeviceToHost, w->stream));
             return CF_OK;

@@ -44,8 +44,8 @@ __global__ void __launch_bounds__(kThreads)
     keys[i] = (uint32_t)((cz * g.m[1] + cy) * g.m[0] + cx);
 }
 
-// Cell id of every particle (world * cells_w + cell) and the population of
-// every cell (counts must be zero on entry); flags positions outside the box,
+// Cell id of every particle (world * cells_w + cell; on a grid by type, type * cells_w + cell) and
+// the population of every cell (counts must be zero on entry); flags positions outside the box,
 // types outside [0, T) and world indices outside the batch.  With slot, the
 // particle's arrival slot in its cell (unordered: it only places the
 // particle for the stable ranking that follows).
@@ -60,8 +60,9 @@ __global__ void __launch_bounds__(kThreads)
     bool inside = (p.x >= 0.0f && p.x < ex) && (p.y >= 0.0f && p.y < ey) && (p.z >= 0.0f && p.z < ez);
     if (!inside) atomicOr(err, kDevErrDomain);
     const uint32_t bits = __float_as_uint(p.w);
-    uint32_t world = bits >> kWorldShift;
-    if ((bits & kTypeMask) >= (uint32_t)num_types || world >= (uint32_t)g.worlds) atomicOr(err, kDevErrType);
+    const uint32_t type = bits & kTypeMask, own = bits >> kWorldShift;
+    if (type >= (uint32_t)num_types || own >= (g.by_type ? 1u : (uint32_t)g.worlds)) atomicOr(err, kDevErrType);
+    uint32_t world = g.by_type ? type : own;
     if (world >= (uint32_t)g.worlds) world = 0;
     int cx = cell_coord(p.x, g.inv[0], g.m[0]);
     int cy = cell_coord(p.y, g.inv[1], g.m[1]);
@@ -217,9 +218,19 @@ __global__ void __launch_bounds__(kThreads) scan_single_block(uint32_t* data, in
     }
 }
 
+// sums: exclusive prefix sums of the tiles; with raw_sums the tiles' own sums, of which each block adds
+// up those before it (few tiles: one launch fewer).
 __global__ void __launch_bounds__(kThreads)
-    scan_apply(const uint32_t* in, uint32_t* out, int n, const uint32_t* __restrict__ sums)
+    scan_apply(const uint32_t* in, uint32_t* out, int n, const uint32_t* __restrict__ sums, bool raw_sums)
 {
+    uint32_t before = 0;
+    if (raw_sums) {
+        uint32_t s = 0;
+        for (int q = threadIdx.x; q < (int)blockIdx.x; q += kThreads) s += sums[q];
+        block_exclusive_scan(s, &before);
+    } else {
+        before = sums[blockIdx.x];
+    }
     int idx = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
     uint32_t s = 0;
@@ -229,7 +240,7 @@ __global__ void __launch_bounds__(kThreads)
         s += v[k];
     }
     uint32_t total;
-    uint32_t run = sums[blockIdx.x] + block_exclusive_scan(s, &total);
+    uint32_t run = before + block_exclusive_scan(s, &total);
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
         if (idx + k < n) out[idx + k] = run;
@@ -587,6 +598,16 @@ __global__ void __launch_bounds__(kThreads)
 
 inline int blocks_for(int n, int per_block) { return (n + per_block - 1) / per_block; }
 
+// Up to this many tiles a scan's blocks add up the tile sums before theirs (four reads per thread).
+constexpr int kScanRawTiles = 4 * kThreads;
+
+// Kernel launches of launch_scan_exclusive.
+inline int scan_launches(int n)
+{
+    const int tiles = blocks_for(n, kScanTile);
+    return tiles == 1 ? 1 : (tiles <= kScanRawTiles ? 2 : 3);
+}
+
 constexpr int kSortItemsSmall = 4;
 constexpr int kSortItemsLarge = 16;
 
@@ -613,8 +634,7 @@ int cell_list_launches(int n, int key_bits)
     int passes = (key_bits + 7) / 8;
     if (passes < 1) passes = 1;
     int entries = (int)radix_hist_entries(n);
-    int scan = blocks_for(entries, kScanTile) == 1 ? 1 : 3;
-    return 1 + passes * (2 + scan) + 1;
+    return 1 + passes * (2 + scan_launches(entries)) + 1;
 }
 
 cudaError_t launch_cell_hash(const float4* pos, int n, const Grid& g, const float* ext, int num_types,
@@ -644,9 +664,12 @@ cudaError_t launch_scan_exclusive(const uint32_t* in, uint32_t* out, int n, uint
     }
     scan_tile_sums<<<tiles, kThreads, 0, st>>>(in, n, tmp);
     note_launches(st);
-    scan_single_block<<<1, kThreads, 0, st>>>(tmp, tiles);
-    note_launches(st);
-    scan_apply<<<tiles, kThreads, 0, st>>>(in, out, n, tmp);
+    const bool raw = tiles <= kScanRawTiles;
+    if (!raw) {
+        scan_single_block<<<1, kThreads, 0, st>>>(tmp, tiles);
+        note_launches(st);
+    }
+    scan_apply<<<tiles, kThreads, 0, st>>>(in, out, n, tmp, raw);
     note_launches(st);
     return cudaGetLastError();
 }
@@ -791,9 +814,7 @@ int cell_list_csr_launches(int n, const Grid& g, bool with_plan)
         int passes = (g.key_bits + 7) / 8;
         if (passes < 1) passes = 1;
         int entries = (int)radix_hist_entries(n);
-        int scan = blocks_for(entries, kScanTile) == 1 ? 1 : 3;
-        int cscan = blocks_for(g.cells + 1, kScanTile) == 1 ? 1 : 3;
-        return 1 + passes * (2 + scan) + cscan + 1 + (with_plan ? 1 : 0);
+        return 1 + passes * (2 + scan_launches(entries)) + scan_launches(g.cells + 1) + 1 + (with_plan ? 1 : 0);
     }
     return 2 + (n > 0 ? 3 : 0);  // tile reduce and apply; hash, place, rank
 }

@@ -111,7 +111,8 @@ struct Grid {
     int key_bits;     // bits of a cell id
     int generic;      // 1: full reference wrap per candidate (some axis < 5 cells)
     int periodic;     // 1: periodic stencil (step), 0: clipped (proximity)
-    int worlds;       // independent worlds sharing the grid (1 for a plain world)
+    int worlds;       // independent worlds sharing the grid (1 for a plain world; the types with by_type)
+    int by_type;      // 1: the particles' types take the place of the worlds (one world's proximity selections)
     int cells_w;      // cells per world: m0 * m1 * m2
 };
 
@@ -421,16 +422,17 @@ cudaError_t launch_cell_list_csr(const float4* pos, int n, const Grid& g, const 
 int cell_list_csr_buffer(int n, const Grid& g);
 int cell_list_csr_launches(int n, const Grid& g, bool with_plan);
 int cell_list_tiles(const Grid& g);  // 0 when the rows are longer than a tile
-// csr: cell_start = CSR offsets and cell_end = offsets + 1 (rows read as
-// ranges); else per-cell start/end arrays.
-cudaError_t launch_proximity_select(const float4* pos_sorted, const uint32_t* keys_sorted,
-                                    const uint32_t* vals_sorted, const uint32_t* cell_start,
-                                    const uint32_t* cell_end, bool csr, const Grid& g, int n, float dsq,
-                                    int max_conn, int32_t* slots, uint32_t* count, cudaStream_t st);
-// cell_start = CSR offsets, cell_end = offsets + 1.
-cudaError_t launch_mesh_select(const float4* pos_sorted, const uint32_t* keys_sorted, const uint32_t* vals_sorted,
-                               const uint32_t* cell_start, const uint32_t* cell_end, const Grid& g, int n, float dsq,
-                               int max_conn, int32_t* slots, uint32_t* count, cudaStream_t st);
+// On per-cell start/end arrays.
+cudaError_t launch_proximity_select_cells(const float4* pos_sorted, const uint32_t* vals_sorted,
+                                          const uint32_t* cell_start, const uint32_t* cell_end, const Grid& g, int n,
+                                          float dsq, int max_conn, int32_t* slots, uint32_t* count, cudaStream_t st);
+// On the CSR list of a grid by type.
+cudaError_t launch_proximity_select(const float4* pos_sorted, const uint32_t* vals_sorted, const uint32_t* cell_off,
+                                    const Grid& g, int n, float dsq, int max_conn, int32_t* slots, uint32_t* count,
+                                    cudaStream_t st);
+cudaError_t launch_mesh_select(const float4* pos_sorted, const uint32_t* vals_sorted, const uint32_t* cell_off,
+                               const Grid& g, int n, float dsq, int max_conn, int32_t* slots, uint32_t* count,
+                               cudaStream_t st);
 cudaError_t launch_mesh_emit(const int32_t* slots, const uint32_t* offsets, int n, const float4* pos,
                              const ColorTable& colors, int n_colors, int32_t* tris, float* vertices, long long cap_tris,
                              cudaStream_t st);
@@ -439,11 +441,10 @@ cudaError_t launch_proximity_emit_edges(const int32_t* slots, const uint32_t* of
 // The CSR selection that writes each particle's line vertices itself, at an
 // offset reserved by one atomic per particle (vertex order is arbitrary, as the
 // reference's atomicAdd append); *total = edges found (zero on entry).
-cudaError_t launch_proximity_select_vertices(const float4* pos_sorted, const uint32_t* keys_sorted,
-                                             const uint32_t* vals_sorted, const uint32_t* cell_off, const Grid& g,
-                                             int n, float dsq, int max_conn, const float4* pos,
-                                             const ColorTable& colors, int n_colors, float* vertices,
-                                             int cap_vertices, uint32_t* total, cudaStream_t st);
+cudaError_t launch_proximity_select_vertices(const float4* pos_sorted, const uint32_t* vals_sorted,
+                                             const uint32_t* cell_off, const Grid& g, int n, float dsq, int max_conn,
+                                             const float4* pos, const ColorTable& colors, int n_colors,
+                                             float* vertices, int cap_vertices, uint32_t* total, cudaStream_t st);
 cudaError_t launch_init_particles(float4* pos, float4* vel, float4* acc, int* counts, int n, int num_types,
                                   const float* lo, const float* span, uint64_t seed, cudaStream_t st,
                                   uint32_t world = 0);
@@ -490,6 +491,7 @@ cudaError_t launch_rdf_grad(const float* ext, const Grid& g, int n, int T, int b
 // Host helpers (api.cpp).
 Grid choose_step_grid(const float* ext, float r_cut, int max_cells);
 Grid choose_prox_grid(const float* ext, float distance, int max_cells);
+Grid choose_type_grid(const float* ext, float distance, int types, int n);
 Grid canonical_grid(const float* ext, float r_max);
 float sqrt_threshold(float eff);
 float cutoff_distance(float threshold);

@@ -33,46 +33,28 @@ __device__ __forceinline__ int axis_cell(float x, float inv, int m)
 }
 
 // Calls fn(u) for every sorted slot u in the cells within one cell of (cx, cy,
-// cz), clipped at the box (the proximity grid is not periodic), in cell order.
-// kCsr: cell_start = CSR offsets, cell_end = offsets + 1, so each of the
-// (at most) nine rows of the stencil is one contiguous range, read up front;
-// otherwise per-cell start/end arrays (zeros for empty cells).
-template <bool kCsr, typename Fn>
+// cz), clipped at the box (the proximity grid is not periodic), in cell order:
+// per-cell start/end arrays (zeros for empty cells).
+template <typename Fn>
 __device__ __forceinline__ void for_each_candidate(const uint32_t* __restrict__ cell_start,
                                                    const uint32_t* __restrict__ cell_end, const Grid& g, int cx,
                                                    int cy, int cz, Fn fn)
 {
     const int mx = g.m[0], my = g.m[1], mz = g.m[2];
-    const int xlo = max(cx - 1, 0), xhi = min(cx + 1, mx - 1);
-    if (kCsr) {
-        uint32_t rb[9], re[9];
-        int nr = 0;
-        for (int z = max(cz - 1, 0); z <= min(cz + 1, mz - 1); z++)
-            for (int y = max(cy - 1, 0); y <= min(cy + 1, my - 1); y++) {
-                const uint32_t row = (uint32_t)((z * my + y) * mx);
-                rb[nr] = cell_start[row + xlo];
-                re[nr] = cell_end[row + xhi];
-                nr++;
+    for (int z = max(cz - 1, 0); z <= min(cz + 1, mz - 1); z++)
+        for (int y = max(cy - 1, 0); y <= min(cy + 1, my - 1); y++)
+            for (int x = max(cx - 1, 0); x <= min(cx + 1, mx - 1); x++) {
+                const uint32_t cell = (uint32_t)((z * my + y) * mx + x);
+                const uint32_t u_end = cell_end[cell];
+                for (uint32_t u = cell_start[cell]; u < u_end; u++) fn(u);
             }
-        for (int r = 0; r < nr; r++)
-            for (uint32_t u = rb[r]; u < re[r]; u++) fn(u);
-    } else {
-        for (int z = max(cz - 1, 0); z <= min(cz + 1, mz - 1); z++)
-            for (int y = max(cy - 1, 0); y <= min(cy + 1, my - 1); y++)
-                for (int x = xlo; x <= xhi; x++) {
-                    const uint32_t cell = (uint32_t)((z * my + y) * mx + x);
-                    const uint32_t u_end = cell_end[cell];
-                    for (uint32_t u = cell_start[cell]; u < u_end; u++) fn(u);
-                }
-    }
 }
 
-template <bool kCsr>
+// The selection on per-cell start/end arrays (the allocation-free call), one thread per particle.
 __global__ void __launch_bounds__(kThreads)
-    proximity_select_kernel(const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ keys_sorted,
-                            const uint32_t* __restrict__ vals_sorted, const uint32_t* __restrict__ cell_start,
-                            const uint32_t* __restrict__ cell_end, Grid g, int n, float dsq, int max_conn,
-                            int32_t* __restrict__ slots, uint32_t* __restrict__ count)
+    proximity_select_kernel(const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ vals_sorted,
+                            const uint32_t* __restrict__ cell_start, const uint32_t* __restrict__ cell_end, Grid g,
+                            int n, float dsq, int max_conn, int32_t* __restrict__ slots, uint32_t* __restrict__ count)
 {
     const int t = blockIdx.x * kThreads + threadIdx.x;
     if (t >= n) return;
@@ -91,7 +73,7 @@ __global__ void __launch_bounds__(kThreads)
     int held = 0;
     int hj[kMaxHeld];
     float hd[kMaxHeld];
-    for_each_candidate<kCsr>(cell_start, cell_end, g, cx, cy, cz, [&](uint32_t u) {
+    for_each_candidate(cell_start, cell_end, g, cx, cy, cz, [&](uint32_t u) {
         const float4 q = pos_sorted[u];
         if (__float_as_uint(q.w) != __float_as_uint(h.w)) return;
         const int j = (int)vals_sorted[u];
@@ -131,151 +113,261 @@ __global__ void __launch_bounds__(kThreads)
     count[i] = (uint32_t)emit;
 }
 
-// The CSR cell list's selection with one warp per particle (grid-stride): the
-// warp stages the particle's clipped stencil (at most nine rows, one contiguous
-// range each, one lane per row, concatenated by a prefix sum) as a list of
-// sorted slots and its lanes test 32 candidates at a time.  Qualifying
-// candidates join the held set one at a time in ballot order; the set lives in
-// lanes 0 .. held-1, ordered by index, and keeps the 2*maxConn smallest indices,
-// as the per-thread kernel does.  The final order is the stable sort by squared
-// distance of that index-ordered set, i.e. by (distance, index): each held lane
-// counts the entries before it.
+// The selections on the CSR cell list: half a warp per particle.  The list is sorted by type first
+// (Grid::by_type), so the particle's clipped stencil, at most nine rows of one contiguous range each,
+// holds particles of its own type only: with 8 types an eighth of the candidates.  The
+// ranges (one lane per row, concatenated by a prefix sum) are staged as a list of sorted
+// slots and the lanes test 16 candidates at a time.  A particle with more than 16 in range, or more
+// than the limit, is done again by the whole warp.  Bound by the dependent reads of one particle's work
+// (position, row offsets, candidates).  100,000 particles, half of them in clumps (proximity
+// / mesh): 49 / 99 us with all types in one list (the mesh one thread per particle), 29 / 34 by
+// type with a warp per particle.
 constexpr int kSelWarps = kThreads / 32;
-constexpr int kSelListCap = 256;
+constexpr int kSelListCap = 256;  // candidates staged per warp at a time, 128 per half
 
+struct SelRange {
+    uint32_t beg;  // this lane's row: first sorted slot
+    int len, pre;  // entries, and those of the rows before
+    int total;
+};
+
+// Rows of the stencil of a particle at h, for the 16 lanes of half a warp (lane: 0 .. 15; whole = the
+// same in both halves).
+__device__ __forceinline__ SelRange stencil_rows(const float4& h, const uint32_t* __restrict__ cell_off, const Grid& g,
+                                                 int n, int lane)
+{
+    const int mx = g.m[0], my = g.m[1], mz = g.m[2];
+    const int cx = axis_cell(h.x, g.inv[0], mx);
+    const int cy = axis_cell(h.y, g.inv[1], my);
+    const int cz = axis_cell(h.z, g.inv[2], mz);
+    const int xlo = max(cx - 1, 0), xhi = min(cx + 1, mx - 1);
+    const int ylo = max(cy - 1, 0), yhi = min(cy + 1, my - 1);
+    const int zlo = max(cz - 1, 0), zhi = min(cz + 1, mz - 1);
+    const int ny = yhi - ylo + 1, nrows = ny * (zhi - zlo + 1);
+    // (a type outside [0, T) is reported by the hash, which counts it as type 0)
+    const uint32_t type = __float_as_uint(h.w) & kTypeMask;
+    const uint32_t base = (type < (uint32_t)g.worlds ? type : 0u) * (uint32_t)g.cells_w;
+    SelRange r;
+    r.beg = 0u;
+    r.len = 0;
+    if (lane < nrows) {
+        // lane / ny for lane < 9 and ny in {1, 2, 3} without a division: (lane * 11) >> 5 = lane / 3
+        const int zq = ny == 3 ? (lane * 11) >> 5 : (ny == 2 ? lane >> 1 : lane);
+        const int y = ylo + (lane - zq * ny), z = zlo + zq;
+        const uint32_t row = base + (uint32_t)((z * my + y) * mx);
+        r.beg = cell_off[row + xlo];
+        r.len = (int)(cell_off[row + xhi + 1] - r.beg);
+        if (!CF_IN_BOUNDS(r.len, n + 1) || !CF_IN_BOUNDS(r.beg + r.len, n + 1)) r.len = 0;
+    }
+    int incl = r.len;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o, 16);
+        if (lane >= o) incl += v;
+    }
+    r.total = __shfl_sync(0xffffffffu, incl, 8, 16);
+    r.pre = incl - r.len;
+    return r;
+}
+
+// Calls fn(ok, j, d2) for the stencil's candidates, kLanes (16: each half its own particle's; 32)
+// at a time, the whole warp together: j is the candidate's particle index, ok: it is another
+// particle (with kAbove: of a larger index) within the distance.  list: the particle's staging
+// area, 8 kLanes entries; lane: 0 .. kLanes - 1.
+template <int kLanes, bool kAbove, typename Fn>
+__device__ __forceinline__ void sel_candidates(const SelRange& r, const float4* __restrict__ pos_sorted,
+                                               const uint32_t* __restrict__ vals_sorted, const float4& h, uint32_t i,
+                                               int n, float dsq, uint32_t* list, int lane, Fn fn)
+{
+    constexpr int kCap = 8 * kLanes;
+    const int most = kLanes == 32 ? r.total : max(r.total, __shfl_xor_sync(0xffffffffu, r.total, 16));
+    for (int base = 0; base < most; base += kCap) {
+        if (lane < 9) {
+            const int j0 = max(0, base - r.pre), j1 = min(r.len, base + kCap - r.pre);
+            for (int j = j0; j < j1; j++) list[r.pre + j - base] = r.beg + (uint32_t)j;
+        }
+        __syncwarp();
+        const int lim = min(kCap, r.total - base), most_here = min(kCap, most - base);
+        for (int g0 = 0; g0 < most_here; g0 += kLanes) {
+            const int gg = g0 + lane;
+            bool ok = false;
+            int j = 0;
+            float d2 = 0.0f;
+            if (gg < lim && CF_IN_BOUNDS(list[gg], n)) {
+                const uint32_t u = list[gg];
+                const float4 q = pos_sorted[u];
+                j = (int)vals_sorted[u];
+                const float dx = __fsub_rn(q.x, h.x);
+                const float dy = __fsub_rn(q.y, h.y);
+                const float dz = __fsub_rn(q.z, h.z);
+                d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                ok = d2 < dsq && (kAbove ? j > (int)i : j != (int)i) && __float_as_uint(q.w) == __float_as_uint(h.w);
+            }
+            fn(ok, j, d2);
+        }
+        __syncwarp();
+    }
+}
+
+// How many candidates of each half's particle qualify; the first 16, in any order, in `found`.
+template <bool kAbove>
+__device__ __forceinline__ int sel_found(const SelRange& r, const float4* __restrict__ pos_sorted,
+                                         const uint32_t* __restrict__ vals_sorted, const float4& h, uint32_t i, int n,
+                                         float dsq, uint32_t* list, float2* found, int half, int lane)
+{
+    int held = 0;
+    sel_candidates<16, kAbove>(r, pos_sorted, vals_sorted, h, i, n, dsq, list, lane, [&](bool ok, int j, float d2) {
+        const uint32_t qm = (__ballot_sync(0xffffffffu, ok) >> (16 * half)) & 0xffffu;
+        const int at = held + __popc(qm & ((1u << lane) - 1u));
+        if (ok && at < 16) found[at] = make_float2(__int_as_float(j), d2);
+        held += __popc(qm);
+    });
+    __syncwarp();
+    return held;
+}
+
+// The `cap` (at most 32) smallest qualifying indices of one particle as (j, d2) in lanes 0 ..
+// held-1, in index order: one at a time in ballot order, past the end of a full set dropped.
+template <bool kAbove>
+__device__ __forceinline__ int sel_smallest(const SelRange& r, const float4* __restrict__ pos_sorted,
+                                            const uint32_t* __restrict__ vals_sorted, const float4& h, uint32_t i, int n,
+                                            float dsq, int cap, uint32_t* list, int lane, int& hj, float& hd)
+{
+    int held = 0;
+    hj = 0;
+    hd = 0.0f;
+    sel_candidates<32, kAbove>(r, pos_sorted, vals_sorted, h, i, n, dsq, list, lane, [&](bool ok, int cj, float cd) {
+        uint32_t qm = __ballot_sync(0xffffffffu, ok);
+        while (qm) {
+            const int src = __ffs(qm) - 1;
+            qm &= qm - 1u;
+            const int j = __shfl_sync(0xffffffffu, cj, src);
+            const float d2 = __shfl_sync(0xffffffffu, cd, src);
+            const int pos = __popc(__ballot_sync(0xffffffffu, lane < held && hj < j));
+            if (pos >= cap) continue;
+            const int uj = __shfl_up_sync(0xffffffffu, hj, 1);
+            const float ud = __shfl_up_sync(0xffffffffu, hd, 1);
+            if (lane > pos && lane < cap) {
+                hj = uj;
+                hd = ud;
+            }
+            if (lane == pos) {
+                hj = j;
+                hd = d2;
+            }
+            held = min(held + 1, cap);
+        }
+    });
+    return held;
+}
+
+__device__ __forceinline__ float4 shfl4(const float4& v, int src)
+{
+    return make_float4(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
+                       __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
+}
+
+// Calls fn(lane, i, h, held, hj, hd, rank, begin, whole) for the two particles of a warp's halves: with
+// whole = false once for both, lane 0 .. 15 of each half, its particle's held entries (all that
+// qualify) in lanes 0 .. held-1 with their rank (kByDistance: by (distance, index), else by index)
+// and held < 0 where the particle is left to the second form; with whole = true for one such
+// particle at a time, lane 0 .. 31, its `cap` smallest indices.
+template <bool kAbove, bool kByDistance, typename Fn>
+__device__ __forceinline__ void select_pair(const float4* __restrict__ pos_sorted,
+                                            const uint32_t* __restrict__ vals_sorted,
+                                            const uint32_t* __restrict__ cell_off, const Grid& g, int n, float dsq, int cap,
+                                            Fn fn)
+{
+    __shared__ uint32_t s_list[kSelWarps][kSelListCap];
+    __shared__ float2 s_found[kSelWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, l16 = lane & 15;
+    const int t = ((int)blockIdx.x * kSelWarps + warp) * 2 + half;
+    if (__all_sync(0xffffffffu, t >= n)) return;
+    const bool mine = t < n;
+    const float4 h = pos_sorted[mine ? t : n - 1];
+    const uint32_t i = vals_sorted[mine ? t : n - 1];
+    SelRange r = stencil_rows(h, cell_off, g, n, l16);
+    if (!mine || !CF_IN_BOUNDS(i, n)) r.len = r.total = 0;  // (bounds-checked build)
+    int held = sel_found<kAbove>(r, pos_sorted, vals_sorted, h, i, n, dsq, s_list[warp] + half * (kSelListCap / 2),
+                                 s_found[warp] + half * 16, half, l16);
+    const bool over = held > min(cap, 16);
+    const uint32_t again = __ballot_sync(0xffffffffu, over);
+    int hj = 0, rank = 0;
+    float hd = 0.0f;
+    if (over || !mine) held = -1;
+    if (l16 < held) {
+        hj = __float_as_int(s_found[warp][half * 16 + l16].x);
+        hd = s_found[warp][half * 16 + l16].y;
+    }
+    const int most = max(held, __shfl_xor_sync(0xffffffffu, held, 16));
+    for (int k = 0; k < most; k++) {
+        const float od = __shfl_sync(0xffffffffu, hd, k, 16);
+        const int oj = __shfl_sync(0xffffffffu, hj, k, 16);
+        if (k < held) rank += kByDistance ? (od < hd || (od == hd && oj < hj)) : oj < hj;
+    }
+    fn(l16, i, h, held, hj, rank, false);
+    for (int q = 0; q < 2; q++) {
+        if (!((again >> (16 * q)) & 1u)) continue;
+        const float4 hq = shfl4(h, 16 * q);
+        const uint32_t iq = __shfl_sync(0xffffffffu, i, 16 * q);
+        SelRange rq;
+        rq.beg = __shfl_sync(0xffffffffu, r.beg, 16 * q + l16);
+        rq.len = __shfl_sync(0xffffffffu, r.len, 16 * q + l16);
+        rq.pre = __shfl_sync(0xffffffffu, r.pre, 16 * q + l16);
+        rq.total = __shfl_sync(0xffffffffu, r.total, 16 * q);
+        const int all = sel_smallest<kAbove>(rq, pos_sorted, vals_sorted, hq, iq, n, dsq, cap, s_list[warp], lane, hj, hd);
+        rank = lane;
+        if (kByDistance) {
+            rank = 0;
+            for (int k = 0; k < all; k++) {
+                const float od = __shfl_sync(0xffffffffu, hd, k);
+                const int oj = __shfl_sync(0xffffffffu, hj, k);
+                rank += (od < hd || (od == hd && oj < hj)) ? 1 : 0;
+            }
+        }
+        fn(lane, iq, hq, all, hj, rank, true);
+    }
+}
+
+// The proximity graph's selection: of the 2 * maxConn smallest qualifying indices above i the maxConn
+// nearest, in the stable sort's order (ParticleSimulation.cu:235-243), i.e. by (distance, index):
+// each held lane counts the entries before it.
 // kEmit: instead of the per-particle slots and counts, each particle's warp
 // reserves its edges' places with one atomic on *count (the running total) and
 // writes their line vertices itself (ParticleSimulation.cu:253-275: per edge the
 // vertex of i then of j, each x, y, z, r, g, b with the colour of i's type).
 template <bool kEmit>
 __global__ void __launch_bounds__(kThreads)
-    proximity_select_warp_kernel(const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ keys_sorted,
-                                 const uint32_t* __restrict__ vals_sorted, const uint32_t* __restrict__ cell_off,
-                                 Grid g, int n, float dsq, int max_conn, int32_t* __restrict__ slots,
-                                 uint32_t* __restrict__ count, const float4* __restrict__ pos, ColorTable colors,
-                                 int n_colors, float* __restrict__ vertices, int cap_vertices)
+    proximity_select_warp_kernel(const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ vals_sorted,
+                                 const uint32_t* __restrict__ cell_off, Grid g, int n, float dsq, int max_conn,
+                                 int32_t* __restrict__ slots, uint32_t* __restrict__ count,
+                                 const float4* __restrict__ pos, ColorTable colors, int n_colors,
+                                 float* __restrict__ vertices, int cap_vertices)
 {
-    __shared__ uint32_t s_list[kSelWarps][kSelListCap];
-    const int lane = threadIdx.x & 31;
-    uint32_t* list = s_list[threadIdx.x >> 5];
-    const int warps = (int)gridDim.x * kSelWarps;
-    const int mx = g.m[0], my = g.m[1], mz = g.m[2];
-    const int cap = 2 * max_conn;
-    for (int t = (int)blockIdx.x * kSelWarps + (threadIdx.x >> 5); t < n; t += warps) {
-        const float4 h = pos_sorted[t];
-        const uint32_t i = vals_sorted[t];
-        const uint32_t key = keys_sorted[t];
-        if (!CF_IN_BOUNDS(i, n) || !CF_IN_BOUNDS(key, g.cells)) continue;  // (bounds-checked build)
-        if (cap <= 0) {
-            if (!kEmit && lane == 0) count[i] = 0;
-            continue;
-        }
-        const int cx = axis_cell(h.x, g.inv[0], mx);
-        const int cy = axis_cell(h.y, g.inv[1], my);
-        const int cz = axis_cell(h.z, g.inv[2], mz);
-        const int xlo = max(cx - 1, 0), xhi = min(cx + 1, mx - 1);
-        const int ylo = max(cy - 1, 0), yhi = min(cy + 1, my - 1);
-        const int zlo = max(cz - 1, 0), zhi = min(cz + 1, mz - 1);
-        const int ny = yhi - ylo + 1, nrows = ny * (zhi - zlo + 1);
-        uint32_t beg = 0u;
-        int len = 0;
-        if (lane < nrows) {
-            // lane / ny for lane < 9 and ny in {1, 2, 3} without a division: (lane * 11) >> 5 = lane / 3
-            const int zq = ny == 3 ? (lane * 11) >> 5 : (ny == 2 ? lane >> 1 : lane);
-            const int y = ylo + (lane - zq * ny), z = zlo + zq;
-            const uint32_t row = (uint32_t)((z * my + y) * mx);
-            beg = cell_off[row + xlo];
-            len = (int)(cell_off[row + xhi + 1] - beg);
-            if (!CF_IN_BOUNDS(len, n + 1) || !CF_IN_BOUNDS(beg + len, n + 1)) len = 0;
-        }
-        int incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        const int pre = incl - len;
-        int held = 0;
-        int hj = 0;
-        float hd = 0.0f;
-        for (int base = 0; base < total; base += kSelListCap) {
-            const int j0 = max(0, base - pre), j1 = min(len, base + kSelListCap - pre);
-            for (int j = j0; j < j1; j++) list[pre + j - base] = beg + (uint32_t)j;
-            __syncwarp();
-            const int lim = min(kSelListCap, total - base);
-            for (int g0 = 0; g0 < lim; g0 += 32) {
-                const int gg = g0 + lane;
-                bool ok = false;
-                int cj = 0;
-                float cd = 0.0f;
-                if (gg < lim && CF_IN_BOUNDS(list[gg], n)) {
-                    const uint32_t u = list[gg];
-                    const float4 q = pos_sorted[u];
-                    if (__float_as_uint(q.w) == __float_as_uint(h.w)) {
-                        cj = (int)vals_sorted[u];
-                        if (cj > (int)i) {
-                            const float dx = __fsub_rn(q.x, h.x);
-                            const float dy = __fsub_rn(q.y, h.y);
-                            const float dz = __fsub_rn(q.z, h.z);
-                            cd = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-                            ok = cd < dsq;
-                        }
-                    }
-                }
-                uint32_t qm = __ballot_sync(0xffffffffu, ok);
-                while (qm) {
-                    const int src = __ffs(qm) - 1;
-                    qm &= qm - 1u;
-                    const int j = __shfl_sync(0xffffffffu, cj, src);
-                    const float d2 = __shfl_sync(0xffffffffu, cd, src);
-                    // its place in the index-ordered set; past the end of a full set it is dropped
-                    const int pos = __popc(__ballot_sync(0xffffffffu, lane < held && hj < j));
-                    if (pos >= cap) continue;
-                    const int uj = __shfl_up_sync(0xffffffffu, hj, 1);
-                    const float ud = __shfl_up_sync(0xffffffffu, hd, 1);
-                    if (lane > pos && lane < cap) {
-                        hj = uj;
-                        hd = ud;
-                    }
-                    if (lane == pos) {
-                        hj = j;
-                        hd = d2;
-                    }
-                    held = min(held + 1, cap);
-                }
-            }
-            __syncwarp();
-        }
-        // stable sort by squared distance (ParticleSimulation.cu:235-243): rank by (distance, index)
-        int rank = 0;
-        for (int r = 0; r < held; r++) {
-            const float od = __shfl_sync(0xffffffffu, hd, r);
-            const int oj = __shfl_sync(0xffffffffu, hj, r);
-            rank += (od < hd || (od == hd && oj < hj)) ? 1 : 0;
-        }
+    select_pair<true, true>(pos_sorted, vals_sorted, cell_off, g, n, dsq, 2 * max_conn,
+                            [&](int lane, uint32_t i, const float4& h, int held, int hj, int rank, bool whole) {
         const int emit = min(held, max_conn);
         if constexpr (kEmit) {
             uint32_t base = 0u;
             if (lane == 0 && emit > 0) base = atomicAdd(count, (uint32_t)emit);
-            base = __shfl_sync(0xffffffffu, base, 0);
+            base = __shfl_sync(0xffffffffu, base, 0, whole ? 32 : 16);
             if (lane < held && rank < emit && CF_IN_BOUNDS(hj, n)) {
                 const size_t k = (size_t)base + (size_t)rank;
                 if (2 * k + 1 < (size_t)cap_vertices) {
                     // ParticleSimulation.cu:253-275: i then j, each x, y, z, r, g, b with i's colour
                     const float4 q = pos[hj];
                     const uint32_t c = (__float_as_uint(h.w) & kTypeMask) % (uint32_t)n_colors;
-                    const float r = colors.c[3 * c], gg = colors.c[3 * c + 1], b = colors.c[3 * c + 2];
+                    const float cr = colors.c[3 * c], cg = colors.c[3 * c + 1], cb = colors.c[3 * c + 2];
                     float* v = vertices + k * 12;
-                    v[0] = h.x; v[1] = h.y; v[2] = h.z; v[3] = r; v[4] = gg; v[5] = b;
-                    v[6] = q.x; v[7] = q.y; v[8] = q.z; v[9] = r; v[10] = gg; v[11] = b;
+                    v[0] = h.x; v[1] = h.y; v[2] = h.z; v[3] = cr; v[4] = cg; v[5] = cb;
+                    v[6] = q.x; v[7] = q.y; v[8] = q.z; v[9] = cr; v[10] = cg; v[11] = cb;
                 }
             }
         } else {
             if (lane < held && rank < emit) slots[(size_t)i * CF_MAX_PROX_CONN + rank] = hj;
-            if (lane == 0) count[i] = (uint32_t)emit;
+            if (lane == 0 && held >= 0 && CF_IN_BOUNDS(i, n)) count[i] = (uint32_t)emit;
         }
-    }
+    });
 }
 
 __global__ void __launch_bounds__(256)
@@ -308,134 +400,120 @@ __global__ void __launch_bounds__(256)
 constexpr int kMeshHeld = CF_MESH_MAX_CONN;
 constexpr int kMeshMaxTriangles = 64;
 
+// slots: the particle's list entries above it, in index order; in the last slot, where fewer than
+// all slots are taken, their number, negated.
 __global__ void __launch_bounds__(kThreads)
-    mesh_select_kernel(const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ keys_sorted,
-                       const uint32_t* __restrict__ vals_sorted, const uint32_t* __restrict__ cell_start,
-                       const uint32_t* __restrict__ cell_end, Grid g, int n, float dsq, int max_conn,
+    mesh_select_kernel(const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ vals_sorted,
+                       const uint32_t* __restrict__ cell_off, Grid g, int n, float dsq, int max_conn,
                        int32_t* __restrict__ slots, uint32_t* __restrict__ count)
 {
-    const int t = blockIdx.x * kThreads + threadIdx.x;
-    if (t >= n) return;
-    const float4 h = pos_sorted[t];
-    const uint32_t i = vals_sorted[t];
-    const int mx = g.m[0], my = g.m[1], mz = g.m[2];
-    const int cx = axis_cell(h.x, g.inv[0], mx);
-    const int cy = axis_cell(h.y, g.inv[1], my);
-    const int cz = axis_cell(h.z, g.inv[2], mz);
-    const int cap = min(max_conn, kMeshHeld);
-    int held = 0;
-    int hj[kMeshHeld];
-    if (cap > 0) {
-        for_each_candidate<true>(cell_start, cell_end, g, cx, cy, cz, [&](uint32_t u) {
-            const float4 q = pos_sorted[u];
-            if (__float_as_uint(q.w) != __float_as_uint(h.w)) return;
-            const int j = (int)vals_sorted[u];
-            if (j == (int)i) return;
-            if (held == cap && j >= hj[cap - 1]) return;
-            // ParticleSimulation.cu:314-317, rounded on its own in source order
-            const float dx = __fsub_rn(q.x, h.x);
-            const float dy = __fsub_rn(q.y, h.y);
-            const float dz = __fsub_rn(q.z, h.z);
-            const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-            if (!(d2 < dsq)) return;
-            int p = held < cap ? held : cap - 1;
-            while (p > 0 && hj[p - 1] > j) {
-                hj[p] = hj[p - 1];
-                p--;
-            }
-            hj[p] = j;
-            if (held < cap) held++;
-        });
-    }
-    // the held list is in index order: the ones above i form its tail
-    int above = 0;
-    for (int e = 0; e < held; e++) {
-        slots[(size_t)i * kMeshHeld + e] = hj[e];
-        above += hj[e] > (int)i ? 1 : 0;
-    }
-    if (held < kMeshHeld) slots[(size_t)i * kMeshHeld + held] = -1;
-    count[i] = (uint32_t)min(above * (above - 1) / 2, kMeshMaxTriangles);
+    // (distances as ParticleSimulation.cu:314-317, each operation rounded on its own in source order)
+    select_pair<false, false>(pos_sorted, vals_sorted, cell_off, g, n, dsq, min(max_conn, kMeshHeld),
+                              [&](int lane, uint32_t i, const float4&, int held, int hj, int rank, bool whole) {
+        const bool up = lane < held && hj > (int)i;
+        uint32_t ups = __ballot_sync(0xffffffffu, up);
+        if (!whole) ups = (ups >> (threadIdx.x & 16)) & 0xffffu;
+        const int above = __popc(ups), at = rank - (held - above);  // the entries above form the list's tail
+        if (up) slots[(size_t)i * kMeshHeld + at] = hj;
+        if (lane == 0 && held >= 0 && CF_IN_BOUNDS(i, n)) {
+            if (above < kMeshHeld) slots[(size_t)i * kMeshHeld + kMeshHeld - 1] = -above;
+            count[i] = (uint32_t)min(above * (above - 1) / 2, kMeshMaxTriangles);
+        }
+    });
 }
 
-// Triangles of particle i in the reference's pair order, placed at offsets[i];
-// index triples and / or vertices of 9 floats (position, flat normal, colour).
-__global__ void __launch_bounds__(256)
+// Triangles in particle order, each particle's in the reference's pair order, at offsets[i]; index
+// triples and / or vertices of 9 floats (position, flat normal, colour).  One warp
+// per 32 particles, whose triangles are consecutive: one triangle per lane, its
+// vertices through shared memory so that the warp writes one contiguous stretch (27 floats
+// a triangle).  Bound by that write: 100,000 particles with 195,000 triangles took 40 us
+// with a thread per particle writing its own, 30 with a warp per particle.
+constexpr int kEmitWarps = 4;
+
+__global__ void __launch_bounds__(32 * kEmitWarps)
     mesh_emit_kernel(const int32_t* __restrict__ slots, const uint32_t* __restrict__ offsets, int n,
                      const float4* __restrict__ pos, ColorTable colors, int n_colors,
                      int32_t* __restrict__ tris, float* __restrict__ vertices, long long cap_tris)
 {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t o = offsets[i], total = offsets[i + 1] - o;
-    if (total == 0) return;
-    int list[kMeshHeld];
-    int m = 0;
-    for (int e = 0; e < kMeshHeld; e++) {
-        const int j = slots[(size_t)i * kMeshHeld + e];
-        if (j < 0) break;
-        if (j > i) list[m++] = j;
-    }
-    const float4 v1 = pos[i];
-    float cr = 0.0f, cg = 0.0f, cb = 0.0f;
-    if (vertices) {  // colours are given only with a vertex buffer
-        const uint32_t c = (__float_as_uint(v1.w) & kTypeMask) % (uint32_t)n_colors;
-        cr = colors.c[3 * c];
-        cg = colors.c[3 * c + 1];
-        cb = colors.c[3 * c + 2];
-    }
-    uint32_t made = 0;
-    for (int a = 0; a < m && made < total; a++)
-        for (int b = a + 1; b < m && made < total; b++, made++) {
-            const long long k = (long long)o + made;
-            if (k >= cap_tris) return;
-            if (tris) {
-                tris[3 * k] = i;
-                tris[3 * k + 1] = list[a];
-                tris[3 * k + 2] = list[b];
-            }
-            if (!vertices) continue;
-            const float4 v2 = pos[list[a]], v3 = pos[list[b]];
-            // ParticleSimulation.cu:365-382, each operation rounded on its own
-            const float e1x = __fsub_rn(v2.x, v1.x), e1y = __fsub_rn(v2.y, v1.y), e1z = __fsub_rn(v2.z, v1.z);
-            const float e2x = __fsub_rn(v3.x, v1.x), e2y = __fsub_rn(v3.y, v1.y), e2z = __fsub_rn(v3.z, v1.z);
-            float nx = __fsub_rn(__fmul_rn(e1y, e2z), __fmul_rn(e1z, e2y));
-            float ny = __fsub_rn(__fmul_rn(e1z, e2x), __fmul_rn(e1x, e2z));
-            float nz = __fsub_rn(__fmul_rn(e1x, e2y), __fmul_rn(e1y, e2x));
-            const float len =
-                __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(nx, nx), __fmul_rn(ny, ny)), __fmul_rn(nz, nz)));
-            if (len > 0.0001f) {
-                nx = __fdiv_rn(nx, len);
-                ny = __fdiv_rn(ny, len);
-                nz = __fdiv_rn(nz, len);
-            }
-            float* v = vertices + k * 27;
-            const float4* vs[3] = {&v1, &v2, &v3};
-            for (int q = 0; q < 3; q++) {
-                v[9 * q + 0] = vs[q]->x;
-                v[9 * q + 1] = vs[q]->y;
-                v[9 * q + 2] = vs[q]->z;
-                v[9 * q + 3] = nx;
-                v[9 * q + 4] = ny;
-                v[9 * q + 5] = nz;
-                v[9 * q + 6] = cr;
-                v[9 * q + 7] = cg;
-                v[9 * q + 8] = cb;
-            }
+    __shared__ float s_vertices[kEmitWarps][32 * 27];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i0 = ((int)blockIdx.x * kEmitWarps + warp) * 32;
+    if (i0 >= n) return;
+    const uint32_t off = offsets[min(i0 + lane, n)];
+    const uint32_t begin = __shfl_sync(0xffffffffu, off, 0), end = offsets[min(i0 + 32, n)];
+    float* out = s_vertices[warp];
+    for (uint32_t t0 = begin; t0 < end; t0 += 32u) {
+        const uint32_t t = min(t0 + (uint32_t)lane, end - 1u);
+        // the last particle whose triangles start at or before t
+        int p = 0;
+#pragma unroll
+        for (int step = 16; step >= 1; step >>= 1)
+            if (__shfl_sync(0xffffffffu, off, p + step) <= t) p += step;
+        // (i0 + p < n: offsets[n] = end > t)
+        const int i = i0 + p;
+        int rest = (int)(t - __shfl_sync(0xffffffffu, off, p));
+        const int32_t* list = slots + (size_t)i * kMeshHeld;
+        // pair `rest` of (a, b), a < b < m, in order of a then b
+        const int last = list[kMeshHeld - 1], m = last < 0 ? -last : kMeshHeld;
+        int a = 0;
+        while (rest >= m - 1 - a) rest -= m - 1 - a++;
+        const int ja = list[a], jb = list[a + 1 + rest];
+        const long long room = cap_tris - (long long)t0;
+        const int here = (int)min((long long)min(32u, end - t0), max(room, 0ll));  // triangles written
+        if (tris && lane < here) {
+            int32_t* o = tris + 3 * (long long)t;
+            o[0] = i;
+            o[1] = ja;
+            o[2] = jb;
         }
+        if (!vertices) continue;
+        const float4 v1 = pos[i], v2 = pos[ja], v3 = pos[jb];
+        // ParticleSimulation.cu:365-382, each operation rounded on its own
+        const float e1x = __fsub_rn(v2.x, v1.x), e1y = __fsub_rn(v2.y, v1.y), e1z = __fsub_rn(v2.z, v1.z);
+        const float e2x = __fsub_rn(v3.x, v1.x), e2y = __fsub_rn(v3.y, v1.y), e2z = __fsub_rn(v3.z, v1.z);
+        float nx = __fsub_rn(__fmul_rn(e1y, e2z), __fmul_rn(e1z, e2y));
+        float ny = __fsub_rn(__fmul_rn(e1z, e2x), __fmul_rn(e1x, e2z));
+        float nz = __fsub_rn(__fmul_rn(e1x, e2y), __fmul_rn(e1y, e2x));
+        const float len = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(nx, nx), __fmul_rn(ny, ny)), __fmul_rn(nz, nz)));
+        if (len > 0.0001f) {
+            nx = __fdiv_rn(nx, len);
+            ny = __fdiv_rn(ny, len);
+            nz = __fdiv_rn(nz, len);
+        }
+        const uint32_t c = (__float_as_uint(v1.w) & kTypeMask) % (uint32_t)n_colors;
+        const float cr = colors.c[3 * c], cg = colors.c[3 * c + 1], cb = colors.c[3 * c + 2];
+        float* v = out + 27 * lane;  // (27 is odd: no two lanes on one bank)
+        const float4* vs[3] = {&v1, &v2, &v3};
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            v[9 * q + 0] = vs[q]->x;
+            v[9 * q + 1] = vs[q]->y;
+            v[9 * q + 2] = vs[q]->z;
+            v[9 * q + 3] = nx;
+            v[9 * q + 4] = ny;
+            v[9 * q + 5] = nz;
+            v[9 * q + 6] = cr;
+            v[9 * q + 7] = cg;
+            v[9 * q + 8] = cb;
+        }
+        __syncwarp();
+        float* to = vertices + 27 * (long long)t0;
+        for (int e = lane; e < 27 * here; e += 32) to[e] = out[e];
+        __syncwarp();
+    }
 }
 
 }  // namespace
 
 CF_BOUNDS_READER(proximity)
 
-cudaError_t launch_mesh_select(const float4* pos_sorted, const uint32_t* keys_sorted, const uint32_t* vals_sorted,
-                               const uint32_t* cell_start, const uint32_t* cell_end, const Grid& g, int n, float dsq,
-                               int max_conn, int32_t* slots, uint32_t* count, cudaStream_t st)
+cudaError_t launch_mesh_select(const float4* pos_sorted, const uint32_t* vals_sorted, const uint32_t* cell_off,
+                               const Grid& g, int n, float dsq, int max_conn, int32_t* slots, uint32_t* count,
+                               cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    mesh_select_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(pos_sorted, keys_sorted, vals_sorted,
-                                                                          cell_start, cell_end, g, n, dsq, max_conn,
-                                                                          slots, count);
+    mesh_select_kernel<<<(n + 2 * kSelWarps - 1) / (2 * kSelWarps), kThreads, 0, st>>>(pos_sorted, vals_sorted, cell_off, g, n, dsq,
+                                                                            max_conn, slots, count);
     note_launches(st);
     return cudaGetLastError();
 }
@@ -445,48 +523,43 @@ cudaError_t launch_mesh_emit(const int32_t* slots, const uint32_t* offsets, int 
                              cudaStream_t st)
 {
     if (n <= 0 || cap_tris <= 0) return cudaSuccess;
-    mesh_emit_kernel<<<(n + 255) / 256, 256, 0, st>>>(slots, offsets, n, pos, colors, n_colors, tris, vertices,
-                                                      cap_tris);
+    mesh_emit_kernel<<<(n + 32 * kEmitWarps - 1) / (32 * kEmitWarps), 32 * kEmitWarps, 0, st>>>(slots, offsets, n, pos, colors,
+                                                                                   n_colors, tris, vertices, cap_tris);
     note_launches(st);
     return cudaGetLastError();
 }
 
-cudaError_t launch_proximity_select(const float4* pos_sorted, const uint32_t* keys_sorted,
-                                    const uint32_t* vals_sorted, const uint32_t* cell_start,
-                                    const uint32_t* cell_end, bool csr, const Grid& g, int n, float dsq,
-                                    int max_conn, int32_t* slots, uint32_t* count, cudaStream_t st)
+cudaError_t launch_proximity_select_cells(const float4* pos_sorted, const uint32_t* vals_sorted,
+                                          const uint32_t* cell_start, const uint32_t* cell_end, const Grid& g, int n,
+                                          float dsq, int max_conn, int32_t* slots, uint32_t* count, cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    const int blocks = (n + kThreads - 1) / kThreads;
-    if (csr) {
-        // a warp per particle: on clustered states (hundreds of candidates) it is up to 1.6x
-        // faster than a thread per particle, which wins only on near-uniform ones (0.081 against
-        // 0.093 ms per call at 100k)
-        const int warp_blocks = (n + kSelWarps - 1) / kSelWarps;
-        proximity_select_warp_kernel<false><<<warp_blocks, kThreads, 0, st>>>(
-            pos_sorted, keys_sorted, vals_sorted, cell_start, g, n, dsq, max_conn, slots, count, nullptr,
-            ColorTable{}, 1, nullptr, 0);
-        note_launches(st);
-    } else {
-        proximity_select_kernel<false><<<blocks, kThreads, 0, st>>>(pos_sorted, keys_sorted, vals_sorted, cell_start,
-                                                                   cell_end, g, n, dsq, max_conn, slots, count);
-        note_launches(st);
-    }
+    proximity_select_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(pos_sorted, vals_sorted, cell_start,
+                                                                               cell_end, g, n, dsq, max_conn, slots, count);
+    note_launches(st);
     return cudaGetLastError();
 }
 
-cudaError_t launch_proximity_select_vertices(const float4* pos_sorted, const uint32_t* keys_sorted,
-                                             const uint32_t* vals_sorted, const uint32_t* cell_off, const Grid& g,
-                                             int n, float dsq, int max_conn, const float4* pos,
-                                             const ColorTable& colors, int n_colors, float* vertices,
-                                             int cap_vertices, uint32_t* total, cudaStream_t st)
+cudaError_t launch_proximity_select(const float4* pos_sorted, const uint32_t* vals_sorted, const uint32_t* cell_off,
+                                    const Grid& g, int n, float dsq, int max_conn, int32_t* slots, uint32_t* count,
+                                    cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    const int warp_blocks = (n + kSelWarps - 1) / kSelWarps;
-    proximity_select_warp_kernel<true><<<warp_blocks, kThreads, 0, st>>>(pos_sorted, keys_sorted, vals_sorted,
-                                                                         cell_off, g, n, dsq, max_conn, nullptr,
-                                                                         total, pos, colors, n_colors, vertices,
-                                                                         cap_vertices);
+    proximity_select_warp_kernel<false><<<(n + 2 * kSelWarps - 1) / (2 * kSelWarps), kThreads, 0, st>>>(
+        pos_sorted, vals_sorted, cell_off, g, n, dsq, max_conn, slots, count, nullptr, ColorTable{}, 1, nullptr, 0);
+    note_launches(st);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_proximity_select_vertices(const float4* pos_sorted, const uint32_t* vals_sorted,
+                                             const uint32_t* cell_off, const Grid& g, int n, float dsq, int max_conn,
+                                             const float4* pos, const ColorTable& colors, int n_colors,
+                                             float* vertices, int cap_vertices, uint32_t* total, cudaStream_t st)
+{
+    if (n <= 0) return cudaSuccess;
+    proximity_select_warp_kernel<true><<<(n + 2 * kSelWarps - 1) / (2 * kSelWarps), kThreads, 0, st>>>(
+        pos_sorted, vals_sorted, cell_off, g, n, dsq, max_conn, nullptr, total, pos, colors, n_colors, vertices,
+        cap_vertices);
     note_launches(st);
     return cudaGetLastError();
 }
