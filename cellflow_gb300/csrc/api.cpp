@@ -26,6 +26,8 @@ namespace {
 thread_local std::string g_error;
 
 constexpr int kMaxCells = 1 << 22;        // cap of the step and proximity grids
+constexpr int kBinTarget = 1 << 18;       // offset entries that a sparse grid's bins come down to
+constexpr long long kBinCellsPerParticle = 24;  // cells per particle from which on a grid is sparse
 constexpr int kProfRing = 1024;           // event triples of profiled steps in flight
 constexpr int kMaxCanonicalCells = 1 << 24;  // cap of the work-model grid
 
@@ -517,7 +519,7 @@ float filter_bound(float thr_max, float max_extent)
     return nextafterf((float)(bound * (1.0 + 0x1p-19)), INFINITY);
 }
 
-int prepare_step(cf_world* w, const cf_step_params* p, StepConsts* c)
+int prepare_step(cf_world* w, const cf_step_params* p, StepConsts* c, bool bins)
 {
     int rc = check_params(w, p);
     if (rc) return rc;
@@ -540,6 +542,7 @@ int prepare_step(cf_world* w, const cf_step_params* p, StepConsts* c)
     c->thr_filter = filter_bound(thr_max, std::max(c->ext[0], std::max(c->ext[1], c->ext[2])));
     c->grid = choose_step_grid(c->ext, r_cut, kMaxCells);
     apply_worlds(c->grid, w->worlds);
+    c->grid.bin_shift = bins ? choose_bin_shift(c->grid, w->n) : 0;
     const int variant = w->force_variant >= 0 ? w->force_variant : default_force_variant(w->n, c->grid);
     c->variant = variant % kForceOccupancies;
     c->split = 1 << (variant / kForceOccupancies);
@@ -832,6 +835,23 @@ Grid choose_step_grid(const float* ext, float r_cut, int max_cells)
     for (int a = 0; a < 3; a++) g.m[a] = cells_for_cutoff(ext[a], r_cut);
     finish_grid(g, ext, max_cells);
     return g;
+}
+
+// The step's offsets are kept per bin of 2^shift cells of a row where the grid has far more cells
+// than particles: clearing and scanning the cells is then most of the step.  The order of the
+// particles and the force kernel's segments are the same with and without: it looks for a
+// segment's ends among the bins' few particles.  A step per cell / with bins, particles
+// spread evenly: 10,000 on 1 and 4 million cells 37 / 32 and 51 / 35 us; on 4 million
+// cells 120,000 (34 cells each) 80 / 74 and 250,000 (16 each) 92 / 90; on 1 million
+// 60,000 (17 each) 51 / 51, 120,000 (8 each) 57 / 60.  In clumps of 200 the same, except
+// 250,000 on 4 million 125 / 128: hence the line at 24 cells per particle.
+int choose_bin_shift(const Grid& g, int n)
+{
+    int shift = 0;
+    if (g.generic || g.m[0] > kTileCellsMax || (long long)g.cells < kBinCellsPerParticle * n) return 0;
+    const long long rows = g.cells / g.m[0];
+    while (shift < kBinShiftMax && rows * ((g.m[0] + (1 << shift) - 1) >> shift) > kBinTarget) shift++;
+    return shift;
 }
 
 Grid choose_prox_grid(const float* ext, float distance, int max_cells)
@@ -1357,7 +1377,7 @@ int cf_step(cf_world* w, const cf_step_params* p, int nsteps)
     if (rc) return rc;
     if (nsteps < 0) return fail(CF_ERR_INVALID, "nsteps must be >= 0");
     StepConsts c;
-    rc = prepare_step(w, p, &c);
+    rc = prepare_step(w, p, &c, true);
     if (rc) return rc;
     rc = ensure_cells(w, c.grid.cells);
     if (rc) return rc;
@@ -1485,7 +1505,7 @@ int cf_step_host(cf_world* w, const cf_step_params* p, const cf_particle* in, cf
         return rc;
     }
     StepConsts c;
-    rc = prepare_step(w, p, &c);
+    rc = prepare_step(w, p, &c, true);
     if (!rc) rc = ensure_cells(w, c.grid.cells);
     if (!rc) rc = ensure_plan(w, c.grid);
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
@@ -1666,7 +1686,7 @@ int cf_get_grid(cf_world* w, const cf_step_params* p, cf_grid_info* out)
     if (rc) return rc;
     if (!out) return fail(CF_ERR_INVALID, "null output");
     StepConsts c;
-    rc = prepare_step(w, p, &c);
+    rc = prepare_step(w, p, &c, false);
     if (rc) return rc;
     for (int a = 0; a < 3; a++) {
         out->cells[a] = c.grid.m[a];
@@ -1687,7 +1707,7 @@ int cf_debug_cell_list(cf_world* w, const cf_step_params* p, uint32_t* cell_of, 
     int rc = check_world(w);
     if (rc) return rc;
     StepConsts c;
-    rc = prepare_step(w, p, &c);
+    rc = prepare_step(w, p, &c, false);
     if (rc) return rc;
     if (cells_cap < c.grid.cells) return fail(CF_ERR_CAPACITY, "cell arrays smaller than the grid");
     rc = ensure_cells(w, c.grid.cells);
@@ -1724,7 +1744,7 @@ int cf_force_work(cf_world* w, const cf_step_params* p, uint64_t* staged, uint64
     int rc = check_world(w);
     if (rc) return rc;
     StepConsts c;
-    rc = prepare_step(w, p, &c);
+    rc = prepare_step(w, p, &c, false);
     if (!rc) rc = ensure_cells(w, c.grid.cells);
     if (!rc) rc = ensure_plan(w, c.grid);
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
@@ -1783,7 +1803,7 @@ int cf_debug_force_bad_item(cf_world* w, const cf_step_params* p, int first)
     int rc = check_world(w);
     if (rc) return rc;
     StepConsts c;
-    rc = prepare_step(w, p, &c);
+    rc = prepare_step(w, p, &c, true);
     if (!rc) rc = ensure_cells(w, c.grid.cells);
     if (!rc) rc = ensure_plan(w, c.grid);
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
@@ -1805,7 +1825,7 @@ int cf_work_counters(cf_world* w, const cf_step_params* p, uint64_t* c27, uint64
     int rc = check_world(w);
     if (rc) return rc;
     StepConsts c;
-    rc = prepare_step(w, p, &c);
+    rc = prepare_step(w, p, &c, false);
     if (rc) return rc;
     float r_max = 0.0f;
     for (int a = 0; a < w->num_types; a++)
@@ -2250,7 +2270,7 @@ int cf_batch_capture(cf_batch* b, const cf_step_params* p, int nsteps)
     if (nsteps < 1) return fail(CF_ERR_INVALID, "nsteps must be >= 1");
     if (!w->stream) return fail(CF_ERR_INVALID, "capture needs a non-default stream");
     StepConsts c;
-    rc = prepare_step(w, p, &c);
+    rc = prepare_step(w, p, &c, true);
     if (rc) return rc;
     rc = ensure_cells(w, c.grid.cells);
     if (!rc) rc = ensure_plan(w, c.grid);
@@ -2590,7 +2610,7 @@ int rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos_in,
     if (nsteps < 1) return fail(CF_ERR_INVALID, "nsteps must be >= 1");
     if (checkpoint_every < 1) return fail(CF_ERR_INVALID, "checkpoint_every must be >= 1");
     StepConsts c;
-    rc = prepare_step(w, p, &c);
+    rc = prepare_step(w, p, &c, false);
     if (!rc) rc = ensure_cells(w, c.grid.cells);
     if (!rc) rc = ensure_plan(w, c.grid);
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
@@ -2674,7 +2694,7 @@ int rollout_backward(cf_world* w, const float* d_gpos, const float* d_gvel, int 
     Rollout& r = w->ro;
     int rc = CF_OK;
     StepConsts c;
-    rc = prepare_step(w, &r.params, &c);
+    rc = prepare_step(w, &r.params, &c, false);
     if (!rc) rc = ensure_cells(w, c.grid.cells);
     if (!rc) rc = ensure_plan(w, c.grid);
     if (!rc) rc = ensure_offsets(w, c.grid.cells);

@@ -48,7 +48,8 @@ __global__ void __launch_bounds__(kThreads)
 // the population of every cell (counts must be zero on entry); flags positions outside the box,
 // types outside [0, T) and world indices outside the batch.  With slot, the
 // particle's arrival slot in its cell (unordered: it only places the
-// particle for the stable ranking that follows).
+// particle for the stable ranking that follows).  With bins, populations and
+// slots are those of the cell's bin.
 __global__ void __launch_bounds__(kThreads)
     cell_hash_count_kernel(const float4* __restrict__ pos, int n, Grid g, float ex, float ey, float ez, int num_types,
                            uint32_t* __restrict__ keys, uint32_t* __restrict__ counts, uint32_t* __restrict__ slot,
@@ -70,7 +71,11 @@ __global__ void __launch_bounds__(kThreads)
     const uint32_t key = world * (uint32_t)g.cells_w + (uint32_t)((cz * g.m[1] + cy) * g.m[0] + cx);
     keys[i] = key;
     if (!CF_IN_BOUNDS(key, g.cells)) return;
-    const uint32_t s = atomicAdd(&counts[key], 1u);
+    uint32_t bin = key;
+    if (g.bin_shift)
+        bin = (world * (uint32_t)(g.m[1] * g.m[2]) + (uint32_t)(cz * g.m[1] + cy)) * (uint32_t)row_bins(g) +
+              ((uint32_t)cx >> g.bin_shift);
+    const uint32_t s = atomicAdd(&counts[bin], 1u);
     if (slot) slot[i] = s;
 }
 
@@ -422,16 +427,31 @@ __global__ void __launch_bounds__(kTileThreads)
     if (last && threadIdx.x == 0) *n_items = (int)(prefix_i + L.items);
 }
 
+// A cell's entry of the offset table; with bins, `sub` = the cell's place in its bin.
+template <bool kBins>
+__device__ __forceinline__ uint32_t offset_entry(uint32_t key, const Grid& g, uint32_t* sub)
+{
+    *sub = 0u;
+    if (!kBins) return key;
+    const uint32_t row = key / (uint32_t)g.m[0], x = key - row * (uint32_t)g.m[0];
+    *sub = x & ((1u << g.bin_shift) - 1u);
+    return row * (uint32_t)row_bins(g) + (x >> g.bin_shift);
+}
+
+// With bins a bin's entries are (place in the bin, index) pairs, so that their order is that of
+// (cell, index).
+template <bool kBins>
 __global__ void __launch_bounds__(kThreads)
     place_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ slot,
-                 const uint32_t* __restrict__ cell_off, int n, int cells, uint32_t* __restrict__ unsorted)
+                 const uint32_t* __restrict__ cell_off, int n, Grid g, uint32_t* __restrict__ unsorted)
 {
     const int i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= n) return;
     const uint32_t key = keys[i];
-    if (!CF_IN_BOUNDS(key, cells)) return;
-    const uint32_t dst = cell_off[key] + slot[i];
-    if (CF_IN_BOUNDS(dst, n)) unsorted[dst] = (uint32_t)i;
+    if (!CF_IN_BOUNDS(key, g.cells)) return;
+    uint32_t sub;
+    const uint32_t dst = cell_off[offset_entry<kBins>(key, g, &sub)] + slot[i];
+    if (CF_IN_BOUNDS(dst, n)) unsorted[dst] = sub << kBinIndexBits | (uint32_t)i;
 }
 
 // Unordered cell list: particle i straight to offset[cell] + arrival slot,
@@ -458,9 +478,10 @@ __global__ void __launch_bounds__(kThreads)
 // below when a warp's 32 positions all lie in one of them.
 constexpr uint32_t kRankWarpMin = 64;
 
+template <bool kBins>
 __global__ void __launch_bounds__(kThreads)
     rank_gather_kernel(const uint32_t* __restrict__ unsorted, const uint32_t* __restrict__ keys,
-                       const uint32_t* __restrict__ cell_off, const float4* __restrict__ pos, int n, int cells,
+                       const uint32_t* __restrict__ cell_off, const float4* __restrict__ pos, int n, Grid g,
                        uint32_t* __restrict__ vals_sorted, uint32_t* __restrict__ keys_sorted,
                        float4* __restrict__ pos_sorted)
 {
@@ -468,21 +489,23 @@ __global__ void __launch_bounds__(kThreads)
     const int p = blockIdx.x * kThreads + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     bool valid = p < n;
-    uint32_t i = valid ? unsorted[p] : 0u;
+    const uint32_t entry = valid ? unsorted[p] : 0u;
+    uint32_t i = kBins ? entry & kBinIndexMask : entry;
     valid = valid && CF_IN_BOUNDS(i, n);
-    uint32_t key = valid ? keys[i] : 0xffffffffu;
-    valid = valid && CF_IN_BOUNDS(key, cells);
-    uint32_t b = valid ? cell_off[key] : 0u, e = valid ? cell_off[key + 1] : 0u;
+    const uint32_t key = valid ? keys[i] : 0xffffffffu;
+    valid = valid && CF_IN_BOUNDS(key, g.cells);
+    uint32_t sub, bin = valid ? offset_entry<kBins>(key, g, &sub) : 0xffffffffu;
+    uint32_t b = valid ? cell_off[bin] : 0u, e = valid ? cell_off[bin + 1] : 0u;
     valid = valid && CF_IN_BOUNDS(e, n + 1) && b <= e;
-    if (!valid) key = 0xffffffffu;
-    const uint32_t key0 = __shfl_sync(0xffffffffu, key, 0);
-    if (__all_sync(0xffffffffu, valid && key == key0) && e - b > kRankWarpMin) {
+    if (!valid) bin = 0xffffffffu;
+    const uint32_t bin0 = __shfl_sync(0xffffffffu, bin, 0);
+    if (__all_sync(0xffffffffu, valid && bin == bin0) && e - b > kRankWarpMin) {
         // The warp's 32 positions lie in one large cell [b, e).  Sort the warp's own
         // particle indices (bitonic over shuffles: lane j then holds the j-th smallest,
         // s_j).  For every entry x of the cell, c(x) = #{j : s_j <= x} by a binary
         // search over the lanes; x < s_j exactly when c(x) <= j, so the rank of s_j in
         // the cell is the number of entries with c(x) <= j: a histogram of c, summed.
-        uint32_t v = i;
+        uint32_t v = entry;
 #pragma unroll
         for (int k = 2; k <= 32; k <<= 1) {
 #pragma unroll
@@ -511,17 +534,17 @@ __global__ void __launch_bounds__(kThreads)
             const uint32_t y = __shfl_up_sync(0xffffffffu, rank, o);
             if (lane >= o) rank += y;
         }
-        i = v;
+        i = kBins ? v & kBinIndexMask : v;
         const uint32_t dst = b + rank;
         if (!CF_IN_BOUNDS(i, n) || !CF_IN_BOUNDS(dst, n)) return;
         vals_sorted[dst] = i;
-        keys_sorted[dst] = key;
+        keys_sorted[dst] = kBins ? keys[i] : key;
         pos_sorted[dst] = pos[i];
         return;
     }
     if (!valid) return;
     uint32_t rank = 0;
-    for (uint32_t q = b; q < e; q++) rank += unsorted[q] < i ? 1u : 0u;
+    for (uint32_t q = b; q < e; q++) rank += unsorted[q] < entry ? 1u : 0u;
     const uint32_t dst = b + rank;
     if (!CF_IN_BOUNDS(dst, n)) return;
     vals_sorted[dst] = i;
@@ -735,14 +758,14 @@ cudaError_t launch_cell_bounds(const uint32_t* keys, const uint32_t* vals, int n
 int tile_rows(const Grid& g)
 {
     const int rows = g.cells / g.m[0];
-    const int fit = kTileCellsMax / g.m[0];
+    const int fit = kTileCellsMax / row_bins(g);
     const int spread = (rows + kTileTarget - 1) / kTileTarget;
     return std::max(1, std::min(fit, spread));
 }
 
 int cell_list_tiles(const Grid& g)
 {
-    if (g.m[0] > kTileCellsMax) return 0;
+    if (row_bins(g) > kTileCellsMax) return 0;
     const int rows = g.cells / g.m[0];
     const int per = tile_rows(g);
     return (rows + per - 1) / per;
@@ -752,7 +775,7 @@ cudaError_t launch_cell_list_csr(const float4* pos, int n, const Grid& g, const 
                                  Scratch& s, uint32_t* cell_off, Item* items, int* n_items, int* err, int* which,
                                  cudaStream_t st, bool stable)
 {
-    cudaError_t e = cudaMemsetAsync(cell_off, 0, sizeof(uint32_t) * ((size_t)g.cells + 1), st);
+    cudaError_t e = cudaMemsetAsync(cell_off, 0, sizeof(uint32_t) * ((size_t)grid_bins(g) + 1), st);
     if (e != cudaSuccess) return e;
     const int tiles = cell_list_tiles(g);
     if (n > 0) {
@@ -772,7 +795,7 @@ cudaError_t launch_cell_list_csr(const float4* pos, int n, const Grid& g, const 
         return e == cudaSuccess ? cudaGetLastError() : e;
     }
     TileGeom tg;
-    tg.m0 = g.m[0];
+    tg.m0 = row_bins(g);
     tg.m1 = g.m[1];
     tg.m2 = g.m[2];
     tg.rows = g.cells / g.m[0];
@@ -788,10 +811,11 @@ cudaError_t launch_cell_list_csr(const float4* pos, int n, const Grid& g, const 
                                                                           s.vals[1], s.keys[1], s.pos_sorted);
         note_launches(st);
     } else if (n > 0) {
-        place_kernel<<<blocks_for(n, kThreads), kThreads, 0, st>>>(s.keys[0], s.aux, cell_off, n, g.cells, s.vals[0]);
+        (g.bin_shift ? place_kernel<true> : place_kernel<false>)<<<blocks_for(n, kThreads), kThreads, 0, st>>>(
+            s.keys[0], s.aux, cell_off, n, g, s.vals[0]);
         note_launches(st);
-        rank_gather_kernel<<<blocks_for(n, kThreads), kThreads, 0, st>>>(s.vals[0], s.keys[0], cell_off, pos, n,
-                                                                         g.cells, s.vals[1], s.keys[1], s.pos_sorted);
+        (g.bin_shift ? rank_gather_kernel<true> : rank_gather_kernel<false>)<<<blocks_for(n, kThreads), kThreads, 0, st>>>(
+            s.vals[0], s.keys[0], cell_off, pos, n, g, s.vals[1], s.keys[1], s.pos_sorted);
         note_launches(st);
     }
     return cudaGetLastError();

@@ -114,7 +114,20 @@ struct Grid {
     int worlds;       // independent worlds sharing the grid (1 for a plain world; the types with by_type)
     int by_type;      // 1: the particles' types take the place of the worlds (one world's proximity selections)
     int cells_w;      // cells per world: m0 * m1 * m2
+    int bin_shift;    // offsets are kept per 2^bin_shift cells of a row (0: per cell; bin_rows)
 };
+
+// Bits of a particle index in a bin's entry (place_kernel); the bits above hold the cell's place in
+// its bin.
+constexpr int kBinIndexBits = 27;
+constexpr uint32_t kBinIndexMask = (1u << kBinIndexBits) - 1u;
+constexpr int kBinShiftMax = 32 - kBinIndexBits;
+
+// Offset entries of one row of cells.
+__host__ __device__ inline int row_bins(const Grid& g) { return (g.m[0] + (1 << g.bin_shift) - 1) >> g.bin_shift; }
+
+// Entries of the offset table but the last: rows, each of row_bins(g).
+inline int grid_bins(const Grid& g) { return g.bin_shift ? g.cells / g.m[0] * row_bins(g) : g.cells; }
 
 // pos4.w of a particle: type in the low 5 bits, world index above.
 constexpr int kWorldShift = 5;
@@ -490,6 +503,7 @@ cudaError_t launch_rdf_grad(const float* ext, const Grid& g, int n, int T, int b
 
 // Host helpers (api.cpp).
 Grid choose_step_grid(const float* ext, float r_cut, int max_cells);
+int choose_bin_shift(const Grid& g, int n);
 Grid choose_prox_grid(const float* ext, float distance, int max_cells);
 Grid choose_type_grid(const float* ext, float distance, int types, int n);
 Grid canonical_grid(const float* ext, float r_max);

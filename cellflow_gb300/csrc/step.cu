@@ -112,6 +112,19 @@ __device__ __forceinline__ int x_cell(float x, float inv, int m)
     return min(max(c, 0), m - 1);
 }
 
+// The first of the sorted slots [b, e) of a row of cells whose x cell is at least x (e: none).
+__device__ __forceinline__ int first_at_cell(const float4* __restrict__ pos_sorted, int b, int e, int x, float inv, int m)
+{
+    while (b < e) {
+        const int mid = (b + e) >> 1;
+        if (x_cell(pos_sorted[mid].x, inv, m) < x)
+            b = mid + 1;
+        else
+            e = mid;
+    }
+    return b;
+}
+
 // fmodf(x, W) of the integrator's wrap (ParticleSimulation.cu:159-161), exact:
 // for x in [0, 2W) it is x or x - W, and x - W is exact there (Sterbenz).
 __device__ __forceinline__ float wrap_pos(float x, float W)
@@ -354,8 +367,10 @@ __device__ __forceinline__ void integrate(const StepConsts& c, const float4& h, 
 // kBlockWarps warps per block, kMinBlocks resident blocks the register budget
 // is sized for.  Shared memory: the warps' staging, the force tables (one for a
 // plain world, one per item of the block in a batch) and, without a uniform
-// radius, (A / eff, c1, certain-interaction bound) per type pair.
-template <int kBlockWarps, int kMinBlocks, bool kGeneric, bool kUniformR>
+// radius, (A / eff, c1, certain-interaction bound) per type pair.  kBins: the offsets are per bin of cells
+// (a form of its own: the search for a segment's ends in the same one cost the others 3 % at
+// 64 worlds of 20,000).
+template <int kBlockWarps, int kMinBlocks, bool kGeneric, bool kUniformR, bool kBins>
 __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
     step_force_kernel(StepConsts c, const PairTables* __restrict__ tables, const float4* __restrict__ pos_sorted,
                       const uint32_t* __restrict__ vals_sorted, const uint32_t* __restrict__ cell_off,
@@ -466,8 +481,19 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
             const uint32_t base = (uint32_t)it.world * (uint32_t)c.grid.cells_w +
                                   (uint32_t)((wrap_index(zz, mz) * my + wrap_index(yy, my)) * mx);
             if (row < ny * nz && xb >= xa && CF_IN_BOUNDS(base + xb + 1, c.grid.cells + 1)) {
-                seg_beg = (int)cell_off[base + xa];
-                seg_len = (int)cell_off[base + xb + 1] - seg_beg;
+                if (kBins) {
+                    // the bins of cells xa..xb, less the particles of their other cells
+                    const uint32_t bins = base / (uint32_t)mx * (uint32_t)row_bins(c.grid);
+                    const int first = (int)cell_off[bins + (xa >> c.grid.bin_shift)],
+                              last = (int)cell_off[bins + (xb >> c.grid.bin_shift) + 1];
+                    if (CF_IN_BOUNDS(first, c.n + 1) && CF_IN_BOUNDS(last, c.n + 1)) {
+                        seg_beg = first_at_cell(pos_sorted, first, last, xa, c.grid.inv[0], mx);
+                        seg_len = first_at_cell(pos_sorted, seg_beg, last, xb + 1, c.grid.inv[0], mx) - seg_beg;
+                    }
+                } else {
+                    seg_beg = (int)cell_off[base + xa];
+                    seg_len = (int)cell_off[base + xb + 1] - seg_beg;
+                }
                 if (!CF_IN_BOUNDS(seg_len, c.n + 1) || !CF_IN_BOUNDS(seg_beg + seg_len, c.n + 1)) seg_len = 0;
             }
             shift = cx | cy << 2 | cz << 4;
@@ -930,20 +956,22 @@ size_t force_smem(int warps, int T, bool uniform, int force_tables)
     return sizeof(WarpSmem) * warps + (size_t)T * T * ((uniform ? 0 : sizeof(float4)) + sizeof(float) * force_tables);
 }
 
-template <int W, int B, bool G, bool U>
+template <int W, int B, bool G, bool U, bool N>
 cudaError_t configure_one()
 {
-    return cudaFuncSetAttribute(step_force_kernel<W, B, G, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(step_force_kernel<W, B, G, U, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)force_smem(W, CF_MAX_TYPES, U, W <= 4 ? W : 1));
 }
 
 template <int W, int B>
 cudaError_t configure_variant()
 {
-    cudaError_t e = configure_one<W, B, false, false>();
-    if (e == cudaSuccess) e = configure_one<W, B, false, true>();
-    if (e == cudaSuccess) e = configure_one<W, B, true, false>();
-    if (e == cudaSuccess) e = configure_one<W, B, true, true>();
+    cudaError_t e = configure_one<W, B, false, false, false>();
+    if (e == cudaSuccess) e = configure_one<W, B, false, true, false>();
+    if (e == cudaSuccess) e = configure_one<W, B, true, false, false>();
+    if (e == cudaSuccess) e = configure_one<W, B, true, true, false>();
+    if (e == cudaSuccess) e = configure_one<W, B, false, false, true>();
+    if (e == cudaSuccess) e = configure_one<W, B, false, true, true>();
     return e;
 }
 
@@ -956,19 +984,24 @@ cudaError_t launch_variant(const StepConsts& c, const PairTables* tables, const 
 {
     const size_t smem = force_smem(W, c.num_types, c.uniform_r != 0, c.grid.worlds == 1 ? 1 : W / c.split);
     const int blocks = (int)(((long long)max_items * c.split + W - 1) / W);
-#define CF_FORCE_LAUNCH(G, U)                                                                                      \
-    step_force_kernel<W, B, G, U><<<blocks, 32 * W, smem, st>>>(c, tables, pos_sorted, vals_sorted, cell_off, items, \
-                                                               n_items, max_items, pos, vel, acc, counts)
+#define CF_FORCE_LAUNCH(G, U, N)                                                                                   \
+    step_force_kernel<W, B, G, U, N><<<blocks, 32 * W, smem, st>>>(c, tables, pos_sorted, vals_sorted, cell_off,    \
+                                                                  items, n_items, max_items, pos, vel, acc, counts)
     if (c.grid.generic) {
         if (c.uniform_r)
-            CF_FORCE_LAUNCH(true, true);
+            CF_FORCE_LAUNCH(true, true, false);
         else
-            CF_FORCE_LAUNCH(true, false);
+            CF_FORCE_LAUNCH(true, false, false);
+    } else if (c.grid.bin_shift) {
+        if (c.uniform_r)
+            CF_FORCE_LAUNCH(false, true, true);
+        else
+            CF_FORCE_LAUNCH(false, false, true);
     } else {
         if (c.uniform_r)
-            CF_FORCE_LAUNCH(false, true);
+            CF_FORCE_LAUNCH(false, true, false);
         else
-            CF_FORCE_LAUNCH(false, false);
+            CF_FORCE_LAUNCH(false, false, false);
     }
 #undef CF_FORCE_LAUNCH
     note_launches(st);
