@@ -196,7 +196,7 @@ void free_rollout(cf_world* w)
     if (r.ev_join) cudaEventDestroy(r.ev_join);
     if (r.side) cudaStreamDestroy(r.side);
     for (void* p : {(void*)r.ckpt_pos, (void*)r.ckpt_vel, (void*)r.ckpt_cnt, (void*)r.seg_pos, (void*)r.seg_vel,
-                    (void*)r.seg_cnt, (void*)r.fin_pos, (void*)r.fin_vel, (void*)r.fin_cnt, (void*)r.gx,
+                    (void*)r.seg_cnt, (void*)r.fin_cnt, (void*)r.acc_sink, (void*)r.gx,
                     (void*)r.gv, (void*)r.gf_sorted, (void*)r.ga_sorted, (void*)r.gacc, (void*)r.rdf_pos,
                     (void*)r.rdf_acc, (void*)r.type_count, (void*)r.seg_sorted, (void*)r.seg_keys,
                     (void*)r.seg_vals, (void*)r.seg_off})
@@ -578,31 +578,34 @@ void apply_worlds(Grid& g, int worlds)
 // The step's two phases.  The cell list leaves the sorted keys and values in
 // buffer `which` of the scratch pair, a function of the grid alone
 // (cell_list_csr_buffer), which the force kernel reads.
-int enqueue_cell_list(cf_world* w, const StepConsts& c, int* which)
+int enqueue_cell_list(cf_world* w, const StepConsts& c, const float4* pos, int* which)
 {
     Scratch& s = w->s;
-    CF_CUDA(launch_cell_list_csr(w->pos, w->n, c.grid, c.ext, w->num_types, s, s.cell_off, s.items, s.n_items, w->err,
+    CF_CUDA(launch_cell_list_csr(pos, w->n, c.grid, c.ext, w->num_types, s, s.cell_off, s.items, s.n_items, w->err,
                                  which, w->stream));
     return CF_OK;
 }
 
-int enqueue_force(cf_world* w, const StepConsts& c, int which)
+int enqueue_force(cf_world* w, const StepConsts& c, int which, const StepState& state)
 {
     Scratch& s = w->s;
-    CF_CUDA(launch_step_force(c, w->tables, s.pos_sorted, s.vals[which], s.cell_off, s.items,
-                              s.n_items, max_step_items(w->n, c.grid), w->pos, w->vel, w->acc, w->counts,
-                              w->stream));
+    CF_CUDA(launch_step_force(c, w->tables, s.pos_sorted, s.vals[which], s.cell_off, s.items, s.n_items,
+                              max_step_items(w->n, c.grid), state, w->stream));
     return CF_OK;
 }
 
-int enqueue_step(cf_world* w, const StepConsts& c, int prof)
+// The world's own state, stepped in place.
+StepState in_place(cf_world* w) { return {w->pos, w->vel, w->counts, w->pos, w->vel, w->counts, w->acc}; }
+
+int enqueue_step(cf_world* w, const StepConsts& c, const StepState& state)
 {
-    (void)prof;
     int which = 0;
-    int rc = enqueue_cell_list(w, c, &which);
+    int rc = enqueue_cell_list(w, c, state.pos, &which);
     if (rc) return rc;
-    return enqueue_force(w, c, which);
+    return enqueue_force(w, c, which, state);
 }
+
+int enqueue_step(cf_world* w, const StepConsts& c) { return enqueue_step(w, c, in_place(w)); }
 
 // The one-step graph for these constants (prof = 1: the cell list alone),
 // captured on first use and again whenever the constants or the scratch
@@ -621,7 +624,7 @@ int step_graph(cf_world* w, const StepConsts& c, int prof, cudaGraphExec_t* out)
     cudaGraph_t graph = nullptr;
     CF_CUDA(cudaStreamBeginCapture(w->stream, cudaStreamCaptureModeThreadLocal));
     int which = 0;
-    int rc = prof ? enqueue_cell_list(w, c, &which) : enqueue_step(w, c, 0);
+    int rc = prof ? enqueue_cell_list(w, c, w->pos, &which) : enqueue_step(w, c);
     cudaError_t e = cudaStreamEndCapture(w->stream, &graph);
     if (rc) {
         if (graph) cudaGraphDestroy(graph);
@@ -1398,7 +1401,7 @@ int cf_step(cf_world* w, const cf_step_params* p, int nsteps)
                 CF_CUDA(cudaGraphLaunch(exec, w->stream));
                 note_launches(w->stream, w->graph_kernels[0]);
             } else {
-                rc = enqueue_step(w, c, 0);
+                rc = enqueue_step(w, c);
                 if (rc) return rc;
             }
             continue;
@@ -1419,11 +1422,11 @@ int cf_step(cf_world* w, const cf_step_params* p, int nsteps)
             note_launches(w->stream, w->graph_kernels[1]);
             which = cell_list_csr_buffer(w->n, c.grid);
         } else {
-            rc = enqueue_cell_list(w, c, &which);
+            rc = enqueue_cell_list(w, c, w->pos, &which);
             if (rc) return rc;
         }
         CF_CUDA(cudaEventRecord(ev[1], w->stream));
-        rc = enqueue_force(w, c, which);
+        rc = enqueue_force(w, c, which, in_place(w));
         if (rc) return rc;
         CF_CUDA(cudaEventRecord(ev[2], w->stream));
         w->prof_launches += launches;
@@ -1475,7 +1478,7 @@ int enqueue_host_step(cf_world* w, const StepConsts& c, const cf_particle* in, c
         CF_CUDA(cudaMemcpyAsync(w->aos, in, bytes, cudaMemcpyHostToDevice, w->stream));
         CF_CUDA(launch_aos_to_soa(w->aos, w->pos, w->vel, w->acc, w->n, w->stream));
     }
-    int rc = enqueue_step(w, c, 0);
+    int rc = enqueue_step(w, c);
     if (rc) return rc;
     if (void* dout = device_view(out)) {
         CF_CUDA(launch_soa_to_aos_mapped(w->pos, w->vel, w->acc, static_cast<cf_particle*>(dout), w->n, w->stream));
@@ -1750,7 +1753,7 @@ int cf_force_work(cf_world* w, const cf_step_params* p, uint64_t* staged, uint64
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
     if (rc) return rc;
     int which = 0;
-    rc = enqueue_cell_list(w, c, &which);
+    rc = enqueue_cell_list(w, c, w->pos, &which);
     if (rc) return rc;
     Scratch& s = w->s;
     CF_CUDA(launch_force_work(c, s.keys[which], s.cell_off, s.items, s.n_items, max_step_items(w->n, c.grid),
@@ -1809,12 +1812,12 @@ int cf_debug_force_bad_item(cf_world* w, const cf_step_params* p, int first)
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
     if (rc) return rc;
     int which = 0;
-    rc = enqueue_cell_list(w, c, &which);
+    rc = enqueue_cell_list(w, c, w->pos, &which);
     if (rc) return rc;
     // the first item's first particle (Item::first, its first field) overwritten
     CF_CUDA(cudaMemcpyAsync(w->s.items, &first, sizeof(int), cudaMemcpyHostToDevice, w->stream));
     CF_CUDA(cudaStreamSynchronize(w->stream));
-    rc = enqueue_force(w, c, which);
+    rc = enqueue_force(w, c, which, in_place(w));
     if (rc) return rc;
     return sync_and_check(w);
 #endif
@@ -2282,7 +2285,7 @@ int cf_batch_capture(cf_batch* b, const cf_step_params* p, int nsteps)
     w->batch_graph_steps = 0;
     cudaGraph_t graph = nullptr;
     CF_CUDA(cudaStreamBeginCapture(w->stream, cudaStreamCaptureModeThreadLocal));
-    for (int s = 0; s < nsteps && rc == CF_OK; s++) rc = enqueue_step(w, c, 0);
+    for (int s = 0; s < nsteps && rc == CF_OK; s++) rc = enqueue_step(w, c);
     cudaError_t e = cudaStreamEndCapture(w->stream, &graph);
     if (rc) {
         if (graph) cudaGraphDestroy(graph);
@@ -2368,9 +2371,8 @@ int ensure_rollout(cf_world* w, int ckpts, int seg_states)
     CF_CUDA(dev_alloc(&r.seg_pos, nn * sg * 2));
     CF_CUDA(dev_alloc(&r.seg_vel, nn * sg * 2));
     CF_CUDA(dev_alloc(&r.seg_cnt, nn * sg * 2));
-    CF_CUDA(dev_alloc(&r.fin_pos, nn));
-    CF_CUDA(dev_alloc(&r.fin_vel, nn));
     CF_CUDA(dev_alloc(&r.fin_cnt, nn));
+    CF_CUDA(dev_alloc(&r.acc_sink, nn));
     CF_CUDA(dev_alloc(&r.gx, nn));
     CF_CUDA(dev_alloc(&r.gv, nn));
     CF_CUDA(dev_alloc(&r.gf_sorted, nn));
@@ -2392,6 +2394,7 @@ int ensure_rollout_lists(cf_world* w, int steps, int cells)
     // the backward's graph reads these lists by address: drop it with them
     if (r.bwd_graph) cudaGraphExecDestroy(r.bwd_graph);
     r.bwd_graph = nullptr;
+    r.kept = false;
     for (void* p : {(void*)r.seg_sorted, (void*)r.seg_keys, (void*)r.seg_vals, (void*)r.seg_off}) dev_free(p);
     r.seg_sorted = nullptr;
     r.seg_keys = r.seg_vals = r.seg_off = nullptr;
@@ -2422,21 +2425,6 @@ int ensure_rdf(cf_world* w)
     return CF_OK;
 }
 
-// Copy a state (positions, velocities, counts) between device buffers.
-int copy_state(cf_world* w, float4* dp, float4* dv, int* dc, const float4* sp, const float4* sv, const int* sc)
-{
-    const size_t n = (size_t)w->n;
-    CF_CUDA(cudaMemcpyAsync(dp, sp, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
-    CF_CUDA(cudaMemcpyAsync(dv, sv, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
-    CF_CUDA(cudaMemcpyAsync(dc, sc, sizeof(int) * n, cudaMemcpyDeviceToDevice, w->stream));
-    return CF_OK;
-}
-
-// The whole backward on the world's stream: save the final state, then per
-// segment (last first) replay the forward from its checkpoint keeping every
-// state, and run the adjoint steps of the segment in reverse; restore the
-// final state.  gx / gv hold dL/dx_K and dL/dv_K on entry, dL/dx_0 and
-// dL/dv_0 on exit; gacc collects the parameter gradients.
 // Segment buffer `buf` (0 or 1) of the replayed states and cell lists.
 struct SegBuf {
     float4 *pos, *vel, *sorted;
@@ -2459,53 +2447,89 @@ SegBuf seg_buf(const Rollout& r, size_t n, int buf)
     return b;
 }
 
-// Replay of segment `seg` from its checkpoint on the world's stream, keeping
-// every state in buffer `buf` and, with lists, every step's cell list.
+// A state of the rollout: before step t of segment `seg` (t = 0: its checkpoint, else in `b`).
+struct RollState {
+    float4 *pos, *vel;
+    int* cnt;
+};
+
+RollState roll_state(const Rollout& r, size_t n, int seg, int t, const SegBuf& b)
+{
+    if (t == 0) return {r.ckpt_pos + n * seg, r.ckpt_vel + n * seg, r.ckpt_cnt + n * seg};
+    const size_t k = n * (size_t)(t - 1);
+    return {b.pos + k, b.vel + k, b.cnt + k};
+}
+
+// The cell-list arrays that the next list is built in, for its life: step t's of a segment buffer in
+// place of the scratch ones (the tiled build leaves the sorted order in keys[1] / vals[1]).
+struct ListInto {
+    Scratch& s;
+    float4* sorted;
+    uint32_t *keys, *vals, *off;
+    ListInto(cf_world* w, const SegBuf& b, int t) : s(w->s), sorted(s.pos_sorted), keys(s.keys[1]), vals(s.vals[1]), off(s.cell_off)
+    {
+        const size_t k = (size_t)w->n * (size_t)t;
+        s.pos_sorted = b.sorted + k;
+        s.keys[1] = b.keys + k;
+        s.vals[1] = b.vals + k;
+        s.cell_off = b.off + w->ro.lists_cells * (size_t)t;
+    }
+    ~ListInto()
+    {
+        s.pos_sorted = sorted;
+        s.keys[1] = keys;
+        s.vals[1] = vals;
+        s.cell_off = off;
+    }
+};
+
+// Steps of segment `seg`.
+int segment_steps(const Rollout& r, int seg) { return std::min(r.every, r.steps - seg * r.every); }
+
+// Replay of segment `seg` from its checkpoint on the world's stream into buffer `b`: the states
+// after its first, by steps from one state to the next, and, with lists, every step's cell list.
+// The last step's end is known (the next checkpoint, or the forward's), so of that step only the
+// list is built.
 int replay_segment(cf_world* w, const StepConsts& c, int seg, const SegBuf& b, bool lists)
 {
     Rollout& r = w->ro;
     const size_t n = (size_t)w->n;
-    const int len = std::min(r.every, r.steps - seg * r.every);
-    Scratch& s = w->s;
-    int rc = copy_state(w, w->pos, w->vel, w->counts, r.ckpt_pos + n * seg, r.ckpt_vel + n * seg,
-                        r.ckpt_cnt + n * seg);
-    if (rc) return rc;
+    const int len = segment_steps(r, seg);
     for (int t = 0; t < len; t++) {
-        rc = copy_state(w, b.pos + n * t, b.vel + n * t, b.cnt + n * t, w->pos, w->vel, w->counts);
-        if (rc) return rc;
-        if (lists) {
-            // the replayed step builds its cell list straight into step t's arrays
-            // (the tiled build leaves it in keys[1] / vals[1]), kept for the adjoint step
-            float4* const ps = s.pos_sorted;
-            uint32_t* const k1 = s.keys[1];
-            uint32_t* const v1 = s.vals[1];
-            uint32_t* const off = s.cell_off;
-            s.pos_sorted = b.sorted + n * t;
-            s.keys[1] = b.keys + n * t;
-            s.vals[1] = b.vals + n * t;
-            s.cell_off = b.off + r.lists_cells * t;
-            rc = enqueue_step(w, c, 0);
-            s.pos_sorted = ps;
-            s.keys[1] = k1;
-            s.vals[1] = v1;
-            s.cell_off = off;
-        } else {
-            rc = enqueue_step(w, c, 0);
+        const RollState from = roll_state(r, n, seg, t, b);
+        int rc = CF_OK;
+        if (t + 1 < len) {
+            const RollState to = roll_state(r, n, seg, t + 1, b);
+            const StepState state{from.pos, from.vel, from.cnt, to.pos, to.vel, to.cnt, r.acc_sink};
+            if (lists) {
+                const ListInto into(w, b, t);
+                rc = enqueue_step(w, c, state);
+            } else {
+                rc = enqueue_step(w, c, state);
+            }
+        } else if (lists) {
+            const ListInto into(w, b, t);
+            int which = 0;
+            CF_CUDA(launch_cell_list_csr(from.pos, w->n, c.grid, c.ext, w->num_types, w->s, w->s.cell_off, nullptr, nullptr,
+                                         w->err, &which, w->stream));
         }
         if (rc) return rc;
     }
-    CF_CUDA(cudaMemcpyAsync(b.cnt + n * len, w->counts, sizeof(int) * n, cudaMemcpyDeviceToDevice, w->stream));
     return CF_OK;
 }
 
-// The adjoint steps of segment `seg` in reverse, from buffer `buf`.
+// The adjoint steps of segment `seg` in reverse, from buffer `b`.
 int adjoint_segment(cf_world* w, const StepConsts& c, int seg, const SegBuf& b, bool lists)
 {
     Rollout& r = w->ro;
     const size_t n = (size_t)w->n;
-    const int len = std::min(r.every, r.steps - seg * r.every);
+    const int len = segment_steps(r, seg);
+    const bool last = seg * r.every + len == r.steps;
     Scratch& s = w->s;
     for (int t = len - 1; t >= 0; t--) {
+        const RollState at = roll_state(r, n, seg, t, b);
+        const int* after = t + 1 < len ? roll_state(r, n, seg, t + 1, b).cnt
+                                       : (last ? r.fin_cnt : r.ckpt_cnt + n * (seg + 1));
         const float4* ps = s.pos_sorted;
         const uint32_t *ks = nullptr, *vs = nullptr, *off = s.cell_off;
         if (lists) {
@@ -2515,7 +2539,7 @@ int adjoint_segment(cf_world* w, const StepConsts& c, int seg, const SegBuf& b, 
             off = b.off + r.lists_cells * t;
         } else {
             int which = 0;
-            CF_CUDA(launch_cell_list_csr(b.pos + n * t, w->n, c.grid, c.ext, w->num_types, s, s.cell_off, nullptr,
+            CF_CUDA(launch_cell_list_csr(at.pos, w->n, c.grid, c.ext, w->num_types, s, s.cell_off, nullptr,
                                          nullptr, w->err, &which, w->stream));
             ks = s.keys[which];
             vs = s.vals[which];
@@ -2533,8 +2557,7 @@ int adjoint_segment(cf_world* w, const StepConsts& c, int seg, const SegBuf& b, 
             w->prof_pending++;
             CF_CUDA(cudaEventRecord((*ev)[0], w->stream));
         }
-        CF_CUDA(launch_adjoint_step(c, w->tables, ps, ks, vs, off, b.vel + n * t, b.cnt + n * t, b.cnt + n * (t + 1),
-                                    r.gx, r.gv, r.gf_sorted, r.ga_sorted, r.gacc, w->stream));
+        CF_CUDA(launch_adjoint_step(c, w->tables, ps, ks, vs, off, at.vel, at.cnt, after, r.gx, r.gv, r.gf_sorted, r.ga_sorted, r.gacc, w->stream));
         if (ev) {
             CF_CUDA(cudaEventRecord((*ev)[1], w->stream));
             CF_CUDA(cudaEventRecord((*ev)[2], w->stream));
@@ -2543,13 +2566,21 @@ int adjoint_segment(cf_world* w, const StepConsts& c, int seg, const SegBuf& b, 
     return CF_OK;
 }
 
-// The whole backward: save the final state, then per segment (last first)
-// replay the forward from its checkpoint keeping every state, and run the
-// adjoint steps of the segment in reverse; restore the final state.  gx / gv
-// hold dL/dx_K and dL/dv_K on entry, dL/dx_0 and dL/dv_0 on exit.  With
+// The lists of a segment's steps are kept where the tiled build is used (it always leaves the
+// sorted keys and indices in buffer 1) and the lists are allocated for this grid.
+bool rollout_lists(const Rollout& r, const StepConsts& c, int every, int steps)
+{
+    return cell_list_tiles(c.grid) > 0 && r.seg_off && r.lists_steps >= std::min(every, steps) &&
+           r.lists_cells >= (size_t)c.grid.cells + 1;
+}
+
+// The whole backward: per segment (last first) replay the forward from its
+// checkpoint keeping every state (the last segment's where the forward did not), and run the
+// adjoint steps of the segment in reverse.  gx / gv
+// hold dL/dx_K and dL/dv_K on entry, dL/dx_0 and dL/dv_0 on exit.  Segment s uses buffer s & 1.  With
 // `overlap` (while capturing the backward's graph, per-step cell lists kept),
 // the replay of segment s - 1 runs on the side stream while the adjoint steps
-// of segment s run on the world's stream: the replay touches the world state,
+// of segment s run on the world's stream: the replay touches
 // the cell-list scratch and segment buffer (s - 1) & 1 only, the adjoint steps
 // buffer s & 1 and the gradients only; the replay forks after the adjoint
 // steps of segment s + 1 (which read the same buffer) and joins before those
@@ -2557,29 +2588,16 @@ int adjoint_segment(cf_world* w, const StepConsts& c, int seg, const SegBuf& b, 
 int enqueue_rollout_backward(cf_world* w, const StepConsts& c, bool overlap)
 {
     Rollout& r = w->ro;
-    int rc = copy_state(w, r.fin_pos, r.fin_vel, r.fin_cnt, w->pos, w->vel, w->counts);
-    if (rc) return rc;
     CF_CUDA(cudaMemsetAsync(r.gacc, 0, sizeof(double) * kGradAccEntries, w->stream));
     const int segs = (r.steps + r.every - 1) / r.every;
-    // keep the replay's cell lists when the tiled build is used (it always leaves the
-    // sorted keys and indices in buffer 1) and the lists are allocated for this grid
-    const bool lists = cell_list_tiles(c.grid) > 0 && r.seg_off && r.lists_steps >= std::min(r.every, r.steps) &&
-                       r.lists_cells >= (size_t)c.grid.cells + 1;
+    const bool lists = rollout_lists(r, c, r.every, r.steps);
     const size_t n = (size_t)w->n;
-    if (!(overlap && lists && segs > 1 && r.side)) {
-        const SegBuf b = seg_buf(r, n, 0);
-        for (int seg = segs - 1; seg >= 0; seg--) {
-            rc = replay_segment(w, c, seg, b, lists);
-            if (!rc) rc = adjoint_segment(w, c, seg, b, lists);
-            if (rc) return rc;
-        }
-        return copy_state(w, w->pos, w->vel, w->counts, r.fin_pos, r.fin_vel, r.fin_cnt);
-    }
+    const bool fork = overlap && lists && r.side;
     const cudaStream_t own = w->stream;
-    rc = replay_segment(w, c, segs - 1, seg_buf(r, n, (segs - 1) & 1), lists);
-    if (rc) return rc;
-    for (int seg = segs - 1; seg >= 0; seg--) {
-        if (seg > 0) {
+    int rc = CF_OK;
+    if (!r.kept) rc = replay_segment(w, c, segs - 1, seg_buf(r, n, (segs - 1) & 1), lists);
+    for (int seg = segs - 1; seg >= 0 && !rc; seg--) {
+        if (seg > 0 && fork) {
             CF_CUDA(cudaEventRecord(r.ev_fork, own));
             CF_CUDA(cudaStreamWaitEvent(r.side, r.ev_fork, 0));
             w->stream = r.side;
@@ -2590,9 +2608,12 @@ int enqueue_rollout_backward(cf_world* w, const StepConsts& c, bool overlap)
         }
         rc = adjoint_segment(w, c, seg, seg_buf(r, n, seg & 1), lists);
         if (rc) return rc;
-        if (seg > 0) CF_CUDA(cudaStreamWaitEvent(own, r.ev_join, 0));
+        if (seg > 0 && fork)
+            CF_CUDA(cudaStreamWaitEvent(own, r.ev_join, 0));
+        else if (seg > 0)
+            rc = replay_segment(w, c, seg - 1, seg_buf(r, n, (seg - 1) & 1), lists);
     }
-    return copy_state(w, w->pos, w->vel, w->counts, r.fin_pos, r.fin_vel, r.fin_cnt);
+    return rc;
 }
 
 }  // namespace
@@ -2616,35 +2637,56 @@ int rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos_in,
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
     if (rc) return rc;
     const int ckpts = (nsteps + checkpoint_every - 1) / checkpoint_every;
-    rc = ensure_rollout(w, ckpts, std::min(checkpoint_every, nsteps) + 1);
+    rc = ensure_rollout(w, ckpts, std::max(1, std::min(checkpoint_every, nsteps) - 1));
     if (rc) return rc;
     Rollout& r = w->ro;
     r.steps = 0;
+    r.kept = false;
+    // once a backward has allocated the lists, the last segment's states and cell lists are kept for
+    // the next, which then need not replay it
+    const bool keep = rollout_lists(r, c, checkpoint_every, nsteps);
     const size_t n = (size_t)w->n;
-    if (d_pos_in) CF_CUDA(launch_pack_pos(d_pos_in, stride, w->pos, w->pos, w->n, w->stream));
+    // the state to start from into the first checkpoint
+    if (d_pos_in)
+        CF_CUDA(launch_pack_pos(d_pos_in, stride, w->pos, r.ckpt_pos, w->n, w->stream));
+    else
+        CF_CUDA(cudaMemcpyAsync(r.ckpt_pos, w->pos, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
     if (d_vel_in && stride == 3)
-        CF_CUDA(launch_rows_in(d_vel_in, nullptr, w->vel, nullptr, w->n, w->stream));
-    else if (d_vel_in)
-        CF_CUDA(cudaMemcpyAsync(w->vel, d_vel_in, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
-    // the step loop with its checkpoint copies
+        CF_CUDA(launch_rows_in(d_vel_in, nullptr, r.ckpt_vel, nullptr, w->n, w->stream));
+    else
+        CF_CUDA(cudaMemcpyAsync(r.ckpt_vel, d_vel_in ? reinterpret_cast<const float4*>(d_vel_in) : w->vel,
+                                sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
+    CF_CUDA(cudaMemcpyAsync(r.ckpt_cnt, w->counts, sizeof(int) * n, cudaMemcpyDeviceToDevice, w->stream));
+    // the steps, each from one state to the next: a checkpoint, a kept state of the last segment,
+    // else the world's own (where the last step ends)
     auto loop = [&]() -> int {
+        const int last_seg = ckpts - 1;
+        const SegBuf b = seg_buf(r, n, last_seg & 1);
+        const RollState own{w->pos, w->vel, w->counts};
+        RollState from = roll_state(r, n, 0, 0, b);
         for (int s = 0; s < nsteps; s++) {
-            if (s % checkpoint_every == 0) {
-                const int k = s / checkpoint_every;
-                const int e = copy_state(w, r.ckpt_pos + n * k, r.ckpt_vel + n * k, r.ckpt_cnt + n * k, w->pos,
-                                         w->vel, w->counts);
-                if (e) return e;
+            const int seg = s / checkpoint_every, next = (s + 1) / checkpoint_every, t = (s + 1) % checkpoint_every;
+            const bool kept = t == 0 || (keep && next == last_seg);
+            const RollState to = s + 1 < nsteps && kept ? roll_state(r, n, next, t, b) : own;
+            const StepState state{from.pos, from.vel, from.cnt, to.pos, to.vel, to.cnt, w->acc};
+            int e;
+            if (keep && seg == last_seg) {
+                const ListInto into(w, b, s - seg * checkpoint_every);
+                e = enqueue_step(w, c, state);
+            } else {
+                e = enqueue_step(w, c, state);
             }
-            const int e = enqueue_step(w, c, 0);
             if (e) return e;
+            from = to;
         }
+        CF_CUDA(cudaMemcpyAsync(r.fin_cnt, w->counts, sizeof(int) * n, cudaMemcpyDeviceToDevice, w->stream));
         return CF_OK;
     };
     if (w->use_graphs && w->stream != nullptr) {
         // one graph for the whole loop, re-captured when its shape or buffers change
         const void* bufs = w->s.cell_start;
         if (!(r.fwd_graph && r.fwd_steps == nsteps && r.fwd_every == checkpoint_every && r.fwd_bufs == bufs &&
-              r.fwd_ckpt == r.ckpt_pos && std::memcmp(&r.fwd_key, &c, sizeof(c)) == 0)) {
+              r.fwd_ckpt == r.ckpt_pos && r.fwd_lists == (keep ? r.seg_off : nullptr) && std::memcmp(&r.fwd_key, &c, sizeof(c)) == 0)) {
             if (r.fwd_graph) cudaGraphExecDestroy(r.fwd_graph);
             r.fwd_graph = nullptr;
             cudaGraph_t graph = nullptr;
@@ -2665,6 +2707,7 @@ int rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos_in,
             r.fwd_every = checkpoint_every;
             r.fwd_bufs = bufs;
             r.fwd_ckpt = r.ckpt_pos;
+            r.fwd_lists = keep ? r.seg_off : nullptr;
         }
         CF_CUDA(cudaGraphLaunch(r.fwd_graph, w->stream));
         note_launches(w->stream, r.fwd_kernels);
@@ -2680,6 +2723,7 @@ int rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos_in,
             CF_CUDA(cudaMemcpyAsync(d_vel_out, w->vel, sizeof(float4) * n, cudaMemcpyDeviceToDevice, w->stream));
     }
     r.steps = nsteps;
+    r.kept = keep;
     r.every = checkpoint_every;
     r.n = w->n;
     r.params = *p;
@@ -2716,7 +2760,7 @@ int rollout_backward(cf_world* w, const float* d_gpos, const float* d_gvel, int 
     if (w->use_graphs && w->stream != nullptr && !w->profiling) {
         const void* bufs = w->s.cell_start;
         const bool same = r.bwd_graph && r.bwd_steps == r.steps && r.bwd_every == r.every && r.bwd_bufs == bufs &&
-                          r.bwd_lists == r.seg_off && std::memcmp(&r.bwd_key, &c, sizeof(c)) == 0;
+                          r.bwd_lists == r.seg_off && r.bwd_kept == r.kept && std::memcmp(&r.bwd_key, &c, sizeof(c)) == 0;
         if (!same) {
             if (r.bwd_graph) cudaGraphExecDestroy(r.bwd_graph);
             r.bwd_graph = nullptr;
@@ -2743,6 +2787,7 @@ int rollout_backward(cf_world* w, const float* d_gpos, const float* d_gvel, int 
             r.bwd_every = r.every;
             r.bwd_bufs = bufs;
             r.bwd_lists = r.seg_off;
+            r.bwd_kept = r.kept;
         }
         CF_CUDA(cudaGraphLaunch(r.bwd_graph, w->stream));
         note_launches(w->stream, r.bwd_kernels);
@@ -2750,6 +2795,8 @@ int rollout_backward(cf_world* w, const float* d_gpos, const float* d_gvel, int 
         rc = enqueue_rollout_backward(w, c, false);
         if (rc) return rc;
     }
+    // (three segments or more: the buffer of the last one holds another by now)
+    if (r.steps > 2 * r.every) r.kept = false;
     return CF_OK;
 }
 

@@ -133,6 +133,18 @@ inline int grid_bins(const Grid& g) { return g.bin_shift ? g.cells / g.m[0] * ro
 constexpr int kWorldShift = 5;
 constexpr uint32_t kTypeMask = (1u << kWorldShift) - 1u;
 
+// A step's state before and after it: positions (types in w), velocities, neighbour counts.  The same
+// arrays for a step in place.  acc: out only.
+struct StepState {
+    const float4* pos;
+    const float4* vel;
+    const int* counts;
+    float4* pos_out;
+    float4* vel_out;
+    int* counts_out;
+    float4* acc;
+};
+
 // Everything the step kernels read besides the buffers.
 struct StepConsts {
     float ext[3];      // W, H, D
@@ -219,18 +231,17 @@ constexpr int kForceOccupancies = 3;
 struct Rollout {
     int n_cap = 0;     // particles the buffers hold
     int ckpt_cap = 0;  // checkpoint states allocated
-    int seg_cap = 0;   // segment states per segment buffer (checkpoint_every + 1); two buffers
+    int seg_cap = 0;   // segment states per segment buffer (those after the checkpoint); two buffers
     float4* ckpt_pos = nullptr;
     float4* ckpt_vel = nullptr;
     int* ckpt_cnt = nullptr;
     float4* seg_pos = nullptr;
     float4* seg_vel = nullptr;
     int* seg_cnt = nullptr;
-    float4* fin_pos = nullptr;  // the state after the forward, restored after the backward
-    float4* fin_vel = nullptr;
-    int* fin_cnt = nullptr;
-    // the cell list of every replayed step of a segment (sorted snapshot, sorted
-    // keys and indices, CSR offsets), written by the replay, read by the adjoint step
+    int* fin_cnt = nullptr;        // the neighbour counts after the forward
+    float4* acc_sink = nullptr;    // the replay's accelerations
+    // the cell list of every step of a segment (sorted snapshot, sorted keys and indices,
+    // CSR offsets), written by the replay or the forward, read by the adjoint step
     float4* seg_sorted = nullptr;
     uint32_t* seg_keys = nullptr;
     uint32_t* seg_vals = nullptr;
@@ -242,7 +253,8 @@ struct Rollout {
     float4* gf_sorted = nullptr;  // dL/df per particle, cell order
     float4* ga_sorted = nullptr;  // (dL/da, density), cell order
     double* gacc = nullptr;       // kTableSize table gradients (32-stride), then CF_GRAD_PARAMS
-    // the last forward
+    // the last forward; kept: its last segment's states and cell lists are in their buffer
+    bool kept = false;
     int steps = 0;
     int every = 0;
     int n = 0;
@@ -262,6 +274,7 @@ struct Rollout {
     int fwd_steps = 0, fwd_every = 0;
     const void* fwd_bufs = nullptr;
     const void* fwd_ckpt = nullptr;
+    const void* fwd_lists = nullptr;  // the lists that the forward fills (null: none)
     // the backward as one CUDA graph, re-captured when its key changes
     cudaGraphExec_t bwd_graph = nullptr;
     long long bwd_kernels = 0;  // kernel nodes of bwd_graph
@@ -269,6 +282,7 @@ struct Rollout {
     int bwd_steps = 0, bwd_every = 0;
     const void* bwd_bufs = nullptr;
     const void* bwd_lists = nullptr;
+    bool bwd_kept = false;
     // radial distribution scratch
     float4* rdf_pos = nullptr;
     double* rdf_acc = nullptr;
@@ -403,8 +417,8 @@ cudaError_t launch_cell_bounds(const uint32_t* keys, const uint32_t* vals, int n
                                uint32_t* end, int cells, float4* pos_sorted, cudaStream_t st);
 cudaError_t launch_step_force(const StepConsts& c, const PairTables* tables, const float4* pos_sorted,
                               const uint32_t* vals_sorted, const uint32_t* cell_off,
-                              const Item* items, const int* n_items, int max_items, float4* pos, float4* vel,
-                              float4* acc, int* counts, cudaStream_t st);
+                              const Item* items, const int* n_items, int max_items, const StepState& state,
+                              cudaStream_t st);
 // Row-aligned items of at most 32 sorted particles (one cell row each).
 cudaError_t launch_force_work(const StepConsts& c, const uint32_t* keys_sorted, const uint32_t* cell_off,
                               const Item* items, const int* n_items, int max_items, unsigned long long* out,

@@ -336,19 +336,20 @@ __device__ __forceinline__ PairTerm pair_term(const StepConsts& c, const float4&
 }
 
 // Density-adaptive scale, integrator and wrap of particle i at h with force sum
-// f and n neighbours (ParticleSimulation.cu:136-165).
+// f and n neighbours (ParticleSimulation.cu:136-165); vel_in and counts_in: the state before the step,
+// in place vel and counts.
 __device__ __forceinline__ void integrate(const StepConsts& c, const float4& h, const float4& f, int n, uint32_t i,
-                                          float4* __restrict__ pos, float4* __restrict__ vel,
-                                          float4* __restrict__ acc, int* __restrict__ counts)
+                                          const float4* vel_in, const int* counts_in, float4* __restrict__ pos,
+                                          float4* __restrict__ vel, float4* __restrict__ acc, int* __restrict__ counts)
 {
-    const float avg = __fmul_rn((float)(n + counts[i]), 0.5f);
+    const float avg = __fmul_rn((float)(n + counts_in[i]), 0.5f);
     const float density = fminf(__fdiv_rn(avg, (float)c.max_expected_neighbors), 1.0f);
     const float adapt = __fsub_rn(1.0f, __fmul_rn(__fsub_rn(1.0f, c.balance), density));
     const float strength = __fmul_rn(c.force_multiplier, adapt);
     const float fx = __fmul_rn(f.x, strength);
     const float fy = __fmul_rn(f.y, strength);
     const float fz = __fmul_rn(f.z, strength);
-    const float4 v = vel[i];
+    const float4 v = vel_in[i];
     const float vx = __fadd_rn(__fmul_rn(v.x, c.friction), __fmul_rn(fx, c.delta_t));
     const float vy = __fadd_rn(__fmul_rn(v.y, c.friction), __fmul_rn(fy, c.delta_t));
     const float vz = __fadd_rn(__fmul_rn(v.z, c.friction), __fmul_rn(fz, c.delta_t));
@@ -367,16 +368,19 @@ __device__ __forceinline__ void integrate(const StepConsts& c, const float4& h, 
 // kBlockWarps warps per block, kMinBlocks resident blocks the register budget
 // is sized for.  Shared memory: the warps' staging, the force tables (one for a
 // plain world, one per item of the block in a batch) and, without a uniform
-// radius, (A / eff, c1, certain-interaction bound) per type pair.  kBins: the offsets are per bin of cells
-// (a form of its own: the search for a segment's ends in the same one cost the others 3 % at
-// 64 worlds of 20,000).
-template <int kBlockWarps, int kMinBlocks, bool kGeneric, bool kUniformR, bool kBins>
+// radius, (A / eff, c1, certain-interaction bound) per type pair.  Forms of their own are kBins, with the
+// offsets per bin of cells (the search for a segment's ends in the same form cost the others 3 % at
+// 64 worlds of 20,000), and kApart, from one state to another (state arrays that may
+// be the same cost the step in place 1.4 % at 100,000 particles).
+enum StepForm { kInPlace, kBins, kApart };
+
+template <int kBlockWarps, int kMinBlocks, bool kGeneric, bool kUniformR, StepForm kForm>
 __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
     step_force_kernel(StepConsts c, const PairTables* __restrict__ tables, const float4* __restrict__ pos_sorted,
                       const uint32_t* __restrict__ vals_sorted, const uint32_t* __restrict__ cell_off,
                       const Item* __restrict__ items, const int* __restrict__ n_items, int max_items,
                       float4* __restrict__ pos, float4* __restrict__ vel, float4* __restrict__ acc,
-                      int* __restrict__ counts)
+                      int* __restrict__ counts, const float4* __restrict__ vel_in, const int* __restrict__ counts_in)
 {
     // pairs per drain trip: three where the registers allow (more independent work in each)
     constexpr int kPer = kBlockWarps * kMinBlocks > 20 ? 2 : 3;
@@ -481,7 +485,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
             const uint32_t base = (uint32_t)it.world * (uint32_t)c.grid.cells_w +
                                   (uint32_t)((wrap_index(zz, mz) * my + wrap_index(yy, my)) * mx);
             if (row < ny * nz && xb >= xa && CF_IN_BOUNDS(base + xb + 1, c.grid.cells + 1)) {
-                if (kBins) {
+                if (kForm == kBins) {
                     // the bins of cells xa..xb, less the particles of their other cells
                     const uint32_t bins = base / (uint32_t)mx * (uint32_t)row_bins(c.grid);
                     const int first = (int)cell_off[bins + (xa >> c.grid.bin_shift)],
@@ -834,17 +838,18 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
     if (c.integrate_apart)
         acc[i] = make_float4(sum_x, sum_y, sum_z, __int_as_float(sum_n));  // for integrate_kernel
     else
-        integrate(c, h, make_float4(sum_x, sum_y, sum_z, 0.0f), sum_n, i, pos, vel, acc, counts);
+        integrate(c, h, make_float4(sum_x, sum_y, sum_z, 0.0f), sum_n, i, kForm == kApart ? vel_in : vel,
+                  kForm == kApart ? counts_in : counts, pos, vel, acc, counts);
 }
 
 __global__ void __launch_bounds__(256)
-    integrate_kernel(StepConsts c, float4* __restrict__ pos, float4* __restrict__ vel, float4* __restrict__ acc,
-                     int* __restrict__ counts)
+    integrate_kernel(StepConsts c, StepState state)
 {
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= c.n) return;
-    const float4 f = acc[i];
-    integrate(c, pos[i], f, __float_as_int(f.w), (uint32_t)i, pos, vel, acc, counts);
+    const float4 f = state.acc[i];
+    integrate(c, state.pos[i], f, __float_as_int(f.w), (uint32_t)i, state.vel, state.counts, state.pos_out, state.vel_out,
+              state.acc, state.counts_out);
 }
 
 // The filter's work of one step, from the cell list alone: per item and pass
@@ -956,22 +961,27 @@ size_t force_smem(int warps, int T, bool uniform, int force_tables)
     return sizeof(WarpSmem) * warps + (size_t)T * T * ((uniform ? 0 : sizeof(float4)) + sizeof(float) * force_tables);
 }
 
-template <int W, int B, bool G, bool U, bool N>
+template <int W, int B, bool G, bool U, StepForm F>
 cudaError_t configure_one()
 {
-    return cudaFuncSetAttribute(step_force_kernel<W, B, G, U, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(step_force_kernel<W, B, G, U, F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)force_smem(W, CF_MAX_TYPES, U, W <= 4 ? W : 1));
 }
 
 template <int W, int B>
 cudaError_t configure_variant()
 {
-    cudaError_t e = configure_one<W, B, false, false, false>();
-    if (e == cudaSuccess) e = configure_one<W, B, false, true, false>();
-    if (e == cudaSuccess) e = configure_one<W, B, true, false, false>();
-    if (e == cudaSuccess) e = configure_one<W, B, true, true, false>();
-    if (e == cudaSuccess) e = configure_one<W, B, false, false, true>();
-    if (e == cudaSuccess) e = configure_one<W, B, false, true, true>();
+    cudaError_t e = cudaSuccess;
+    const auto forms = [&e](auto generic, auto uniform) {
+        constexpr bool G = decltype(generic)::value, U = decltype(uniform)::value;
+        if (e == cudaSuccess) e = configure_one<W, B, G, U, kInPlace>();
+        if (e == cudaSuccess) e = configure_one<W, B, G, U, kApart>();
+        if (e == cudaSuccess && !G) e = configure_one<W, B, false, U, kBins>();
+    };
+    forms(std::false_type(), std::false_type());
+    forms(std::false_type(), std::true_type());
+    forms(std::true_type(), std::false_type());
+    forms(std::true_type(), std::true_type());
     return e;
 }
 
@@ -979,31 +989,33 @@ cudaError_t configure_variant()
 template <int W, int B>
 cudaError_t launch_variant(const StepConsts& c, const PairTables* tables, const float4* pos_sorted,
                            const uint32_t* vals_sorted, const uint32_t* cell_off, const Item* items,
-                           const int* n_items, int max_items, float4* pos, float4* vel, float4* acc, int* counts,
-                           cudaStream_t st)
+                           const int* n_items, int max_items, const StepState& state, cudaStream_t st)
 {
     const size_t smem = force_smem(W, c.num_types, c.uniform_r != 0, c.grid.worlds == 1 ? 1 : W / c.split);
     const int blocks = (int)(((long long)max_items * c.split + W - 1) / W);
-#define CF_FORCE_LAUNCH(G, U, N)                                                                                   \
-    step_force_kernel<W, B, G, U, N><<<blocks, 32 * W, smem, st>>>(c, tables, pos_sorted, vals_sorted, cell_off,    \
-                                                                  items, n_items, max_items, pos, vel, acc, counts)
+    const bool apart = state.pos_out != state.pos;
+    const auto launch = [&](auto kernel) {
+        kernel<<<blocks, 32 * W, smem, st>>>(c, tables, pos_sorted, vals_sorted, cell_off, items, n_items, max_items,
+                                             state.pos_out, state.vel_out, state.acc, state.counts_out, state.vel,
+                                             state.counts);
+    };
+#define CF_FORCE_FORMS(G, U)                                                                       \
+    launch(apart ? step_force_kernel<W, B, G, U, kApart> : step_force_kernel<W, B, G, U, kInPlace>)
     if (c.grid.generic) {
         if (c.uniform_r)
-            CF_FORCE_LAUNCH(true, true, false);
+            CF_FORCE_FORMS(true, true);
         else
-            CF_FORCE_LAUNCH(true, false, false);
+            CF_FORCE_FORMS(true, false);
     } else if (c.grid.bin_shift) {
-        if (c.uniform_r)
-            CF_FORCE_LAUNCH(false, true, true);
-        else
-            CF_FORCE_LAUNCH(false, false, true);
+        if (apart) return cudaErrorInvalidValue;  // (no caller)
+        launch(c.uniform_r ? step_force_kernel<W, B, false, true, kBins> : step_force_kernel<W, B, false, false, kBins>);
     } else {
         if (c.uniform_r)
-            CF_FORCE_LAUNCH(false, true, false);
+            CF_FORCE_FORMS(false, true);
         else
-            CF_FORCE_LAUNCH(false, false, false);
+            CF_FORCE_FORMS(false, false);
     }
-#undef CF_FORCE_LAUNCH
+#undef CF_FORCE_FORMS
     note_launches(st);
     return cudaGetLastError();
 }
@@ -1086,14 +1098,13 @@ cudaError_t configure_step_force()
 
 cudaError_t launch_step_force(const StepConsts& c, const PairTables* tables, const float4* pos_sorted,
                               const uint32_t* vals_sorted, const uint32_t* cell_off, const Item* items,
-                              const int* n_items, int max_items, float4* pos, float4* vel, float4* acc, int* counts,
-                              cudaStream_t st)
+                              const int* n_items, int max_items, const StepState& state, cudaStream_t st)
 {
     if (c.n <= 0 || max_items <= 0) return cudaSuccess;
     if (c.split < 1 || c.split > 16 || (c.split & (c.split - 1)) != 0) return cudaErrorInvalidValue;
     cudaError_t e;
 #define CF_FORCE_VARIANT(W, B) \
-    launch_variant<W, B>(c, tables, pos_sorted, vals_sorted, cell_off, items, n_items, max_items, pos, vel, acc, counts, st)
+    launch_variant<W, B>(c, tables, pos_sorted, vals_sorted, cell_off, items, n_items, max_items, state, st)
     if (c.split <= 2)
         e = c.variant == 0 ? CF_FORCE_VARIANT(4, 6) : c.variant == 1 ? CF_FORCE_VARIANT(2, 10) : CF_FORCE_VARIANT(4, 4);
     else if (c.split == 4)
@@ -1102,7 +1113,7 @@ cudaError_t launch_step_force(const StepConsts& c, const PairTables* tables, con
         e = c.split == 8 ? CF_FORCE_VARIANT(8, 2) : CF_FORCE_VARIANT(16, 1);
 #undef CF_FORCE_VARIANT
     if (e != cudaSuccess || !c.integrate_apart) return e;
-    integrate_kernel<<<(c.n + 255) / 256, 256, 0, st>>>(c, pos, vel, acc, counts);
+    integrate_kernel<<<(c.n + 255) / 256, 256, 0, st>>>(c, state);
     note_launches(st);
     return cudaGetLastError();
 }
