@@ -113,26 +113,32 @@ __global__ void __launch_bounds__(kThreads)
     count[i] = (uint32_t)emit;
 }
 
-// The selections on the CSR cell list: half a warp per particle.  The list is sorted by type first
+// The selections on the CSR cell list: eight lanes per particle.  The list is sorted by type first
 // (Grid::by_type), so the particle's clipped stencil, at most nine rows of one contiguous range each,
 // holds particles of its own type only: with 8 types an eighth of the candidates.  The
-// ranges (one lane per row, concatenated by a prefix sum) are staged as a list of sorted
-// slots and the lanes test 16 candidates at a time.  A particle with more than 16 in range, or more
-// than the limit, is done again by the whole warp.  Bound by the dependent reads of one particle's work
-// (position, row offsets, candidates).  100,000 particles, half of them in clumps (proximity
+// ranges (one or two rows per lane, concatenated by a prefix sum) are staged as a list of
+// sorted slots and the lanes test eight candidates at a time.  A particle with more than 16 in range, or more
+// than the limit, is done again by the whole warp.  Bound by instruction issue: the work per warp
+// is much the same for one particle as for four.  100,000 particles, half of them in clumps (proximity
 // / mesh): 49 / 99 us with all types in one list (the mesh one thread per particle), 29 / 34 by
-// type with a warp per particle.
+// type with a warp per particle, 26 / 32 with half a warp, 19 / 24 with eight lanes; with four 19 / 30
+// and with one 20 / 45 (crowded particles then come 8 or 32 to a warp, one after the other).
 constexpr int kSelWarps = kThreads / 32;
-constexpr int kSelListCap = 256;  // candidates staged per warp at a time, 128 per half
+constexpr int kSelLanes = 8;                      // per particle
+constexpr int kSelGroups = 32 / kSelLanes;        // particles of a warp
+constexpr int kSelListCap = 256;                  // candidates staged per warp at a time
+constexpr int kSelFound = 16;                     // in range, without the whole warp
+
+constexpr int kSelRows = (9 + kSelLanes - 1) / kSelLanes;          // rows of a lane at most
+constexpr int kSelEntries = (kSelFound + kSelLanes - 1) / kSelLanes;  // found entries of a lane
 
 struct SelRange {
-    uint32_t beg;  // this lane's row: first sorted slot
-    int len, pre;  // entries, and those of the rows before
+    uint32_t beg[kSelRows];            // this lane's rows (lane, lane + kSelLanes, ...): first sorted slot
+    int len[kSelRows], pre[kSelRows];  // entries, and those of the rows before
     int total;
 };
 
-// Rows of the stencil of a particle at h, for the 16 lanes of half a warp (lane: 0 .. 15; whole = the
-// same in both halves).
+// Rows of the stencil of a particle at h, for its lanes (lane: 0 .. kSelLanes - 1).
 __device__ __forceinline__ SelRange stencil_rows(const float4& h, const uint32_t* __restrict__ cell_off, const Grid& g,
                                                  int n, int lane)
 {
@@ -148,29 +154,44 @@ __device__ __forceinline__ SelRange stencil_rows(const float4& h, const uint32_t
     const uint32_t type = __float_as_uint(h.w) & kTypeMask;
     const uint32_t base = (type < (uint32_t)g.worlds ? type : 0u) * (uint32_t)g.cells_w;
     SelRange r;
-    r.beg = 0u;
-    r.len = 0;
-    if (lane < nrows) {
-        // lane / ny for lane < 9 and ny in {1, 2, 3} without a division: (lane * 11) >> 5 = lane / 3
-        const int zq = ny == 3 ? (lane * 11) >> 5 : (ny == 2 ? lane >> 1 : lane);
-        const int y = ylo + (lane - zq * ny), z = zlo + zq;
-        const uint32_t row = base + (uint32_t)((z * my + y) * mx);
-        r.beg = cell_off[row + xlo];
-        r.len = (int)(cell_off[row + xhi + 1] - r.beg);
-        if (!CF_IN_BOUNDS(r.len, n + 1) || !CF_IN_BOUNDS(r.beg + r.len, n + 1)) r.len = 0;
-    }
-    int incl = r.len;
+    r.total = 0;
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o, 16);
-        if (lane >= o) incl += v;
+    for (int k = 0; k < kSelRows; k++) {
+        r.beg[k] = 0u;
+        r.len[k] = 0;
+        const int q = lane + kSelLanes * k;  // row
+        if (q < nrows) {
+            // q / ny for q < 9 and ny in {1, 2, 3} without a division: (q * 11) >> 5 = q / 3
+            const int zq = ny == 3 ? (q * 11) >> 5 : (ny == 2 ? q >> 1 : q);
+            const int y = ylo + (q - zq * ny), z = zlo + zq;
+            const uint32_t row = base + (uint32_t)((z * my + y) * mx);
+            r.beg[k] = cell_off[row + xlo];
+            r.len[k] = (int)(cell_off[row + xhi + 1] - r.beg[k]);
+            if (!CF_IN_BOUNDS(r.len[k], n + 1) || !CF_IN_BOUNDS(r.beg[k] + r.len[k], n + 1)) r.len[k] = 0;
+        }
     }
-    r.total = __shfl_sync(0xffffffffu, incl, 8, 16);
-    r.pre = incl - r.len;
+#pragma unroll
+    for (int k = 0; k < kSelRows; k++) {
+        int incl = r.len[k];
+#pragma unroll
+        for (int o = 1; o < kSelLanes; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o, kSelLanes);
+            if (lane >= o) incl += v;
+        }
+        r.pre[k] = r.total + incl - r.len[k];
+        r.total += __shfl_sync(0xffffffffu, incl, kSelLanes - 1, kSelLanes);
+    }
     return r;
 }
 
-// Calls fn(ok, j, d2) for the stencil's candidates, kLanes (16: each half its own particle's; 32)
+__device__ __forceinline__ void clear_rows(SelRange& r)
+{
+#pragma unroll
+    for (int k = 0; k < kSelRows; k++) r.len[k] = 0;
+    r.total = 0;
+}
+
+// Calls fn(ok, j, d2) for the stencil's candidates, kLanes (kSelLanes: each group its own particle's; 32)
 // at a time, the whole warp together: j is the candidate's particle index, ok: it is another
 // particle (with kAbove: of a larger index) within the distance.  list: the particle's staging
 // area, 8 kLanes entries; lane: 0 .. kLanes - 1.
@@ -180,11 +201,14 @@ __device__ __forceinline__ void sel_candidates(const SelRange& r, const float4* 
                                                int n, float dsq, uint32_t* list, int lane, Fn fn)
 {
     constexpr int kCap = 8 * kLanes;
-    const int most = kLanes == 32 ? r.total : max(r.total, __shfl_xor_sync(0xffffffffu, r.total, 16));
+    const int most = kLanes == 32 ? r.total : __reduce_max_sync(0xffffffffu, r.total);
     for (int base = 0; base < most; base += kCap) {
-        if (lane < 9) {
-            const int j0 = max(0, base - r.pre), j1 = min(r.len, base + kCap - r.pre);
-            for (int j = j0; j < j1; j++) list[r.pre + j - base] = r.beg + (uint32_t)j;
+#pragma unroll
+        for (int k = 0; k < kSelRows; k++) {
+            if (lane < min(kSelLanes, 9 - kSelLanes * k)) {
+                const int j0 = max(0, base - r.pre[k]), j1 = min(r.len[k], base + kCap - r.pre[k]);
+                for (int j = j0; j < j1; j++) list[r.pre[k] + j - base] = r.beg[k] + (uint32_t)j;
+            }
         }
         __syncwarp();
         const int lim = min(kCap, r.total - base), most_here = min(kCap, most - base);
@@ -207,23 +231,6 @@ __device__ __forceinline__ void sel_candidates(const SelRange& r, const float4* 
         }
         __syncwarp();
     }
-}
-
-// How many candidates of each half's particle qualify; the first 16, in any order, in `found`.
-template <bool kAbove>
-__device__ __forceinline__ int sel_found(const SelRange& r, const float4* __restrict__ pos_sorted,
-                                         const uint32_t* __restrict__ vals_sorted, const float4& h, uint32_t i, int n,
-                                         float dsq, uint32_t* list, float2* found, int half, int lane)
-{
-    int held = 0;
-    sel_candidates<16, kAbove>(r, pos_sorted, vals_sorted, h, i, n, dsq, list, lane, [&](bool ok, int j, float d2) {
-        const uint32_t qm = (__ballot_sync(0xffffffffu, ok) >> (16 * half)) & 0xffffu;
-        const int at = held + __popc(qm & ((1u << lane) - 1u));
-        if (ok && at < 16) found[at] = make_float2(__int_as_float(j), d2);
-        held += __popc(qm);
-    });
-    __syncwarp();
-    return held;
 }
 
 // The `cap` (at most 32) smallest qualifying indices of one particle as (j, d2) in lanes 0 ..
@@ -267,65 +274,94 @@ __device__ __forceinline__ float4 shfl4(const float4& v, int src)
                        __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
 }
 
-// Calls fn(lane, i, h, held, hj, hd, rank, begin, whole) for the two particles of a warp's halves: with
-// whole = false once for both, lane 0 .. 15 of each half, its particle's held entries (all that
-// qualify) in lanes 0 .. held-1 with their rank (kByDistance: by (distance, index), else by index)
-// and held < 0 where the particle is left to the second form; with whole = true for one such
-// particle at a time, lane 0 .. 31, its `cap` smallest indices.
+// Per particle fn(lane, lanes, i, h, held, above, entry): by its `lanes` lanes (kSelLanes, four particles at
+// once, or the whole warp), all together: held entries qualify (all of them, or the `cap` smallest
+// indices), `above` of them with an index above i; entry(e, j, rank) gives the lane's e-th entry
+// (false: none) with its index and rank (kByDistance: by (distance, index), else by index).
+// held < 0: not a particle of this call.
 template <bool kAbove, bool kByDistance, typename Fn>
-__device__ __forceinline__ void select_pair(const float4* __restrict__ pos_sorted,
-                                            const uint32_t* __restrict__ vals_sorted,
-                                            const uint32_t* __restrict__ cell_off, const Grid& g, int n, float dsq, int cap,
-                                            Fn fn)
+__device__ __forceinline__ void select_group(const float4* __restrict__ pos_sorted,
+                                             const uint32_t* __restrict__ vals_sorted,
+                                             const uint32_t* __restrict__ cell_off, const Grid& g, int n, float dsq, int cap,
+                                             Fn fn)
 {
     __shared__ uint32_t s_list[kSelWarps][kSelListCap];
-    __shared__ float2 s_found[kSelWarps][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4, l16 = lane & 15;
-    const int t = ((int)blockIdx.x * kSelWarps + warp) * 2 + half;
+    __shared__ float2 s_found[kSelWarps][kSelGroups][kSelFound];
+    const int wl = threadIdx.x & 31, warp = threadIdx.x >> 5, group = wl / kSelLanes, lane = wl % kSelLanes;
+    const int t = ((int)blockIdx.x * kSelWarps + warp) * kSelGroups + group;
     if (__all_sync(0xffffffffu, t >= n)) return;
     const bool mine = t < n;
     const float4 h = pos_sorted[mine ? t : n - 1];
     const uint32_t i = vals_sorted[mine ? t : n - 1];
-    SelRange r = stencil_rows(h, cell_off, g, n, l16);
-    if (!mine || !CF_IN_BOUNDS(i, n)) r.len = r.total = 0;  // (bounds-checked build)
-    int held = sel_found<kAbove>(r, pos_sorted, vals_sorted, h, i, n, dsq, s_list[warp] + half * (kSelListCap / 2),
-                                 s_found[warp] + half * 16, half, l16);
-    const bool over = held > min(cap, 16);
+    SelRange r = stencil_rows(h, cell_off, g, n, lane);
+    if (!mine || !CF_IN_BOUNDS(i, n)) clear_rows(r);  // (bounds-checked build)
+    float2* found = s_found[warp][group];
+    int held = 0;
+    sel_candidates<kSelLanes, kAbove>(r, pos_sorted, vals_sorted, h, i, n, dsq, s_list[warp] + group * (kSelListCap / kSelGroups),
+                                      lane, [&](bool ok, int j, float d2) {
+        const uint32_t qm = (__ballot_sync(0xffffffffu, ok) >> (kSelLanes * group)) & ((1u << kSelLanes) - 1u);
+        const int at = held + __popc(qm & ((1u << lane) - 1u));
+        if (ok && at < kSelFound) found[at] = make_float2(__int_as_float(j), d2);
+        held += __popc(qm);
+    });
+    __syncwarp();
+    const bool over = held > min(cap, kSelFound);
     const uint32_t again = __ballot_sync(0xffffffffu, over);
-    int hj = 0, rank = 0;
-    float hd = 0.0f;
     if (over || !mine) held = -1;
-    if (l16 < held) {
-        hj = __float_as_int(s_found[warp][half * 16 + l16].x);
-        hd = s_found[warp][half * 16 + l16].y;
+    // each lane's entries (in the order in which they were found) and their ranks
+    int hj[kSelEntries], rank[kSelEntries] = {}, above = 0;
+    float hd[kSelEntries];
+#pragma unroll
+    for (int e = 0; e < kSelEntries; e++) {
+        const float2 f = found[lane + kSelLanes * e];  // (past held: not used)
+        hj[e] = __float_as_int(f.x);
+        hd[e] = f.y;
     }
-    const int most = max(held, __shfl_xor_sync(0xffffffffu, held, 16));
-    for (int k = 0; k < most; k++) {
-        const float od = __shfl_sync(0xffffffffu, hd, k, 16);
-        const int oj = __shfl_sync(0xffffffffu, hj, k, 16);
-        if (k < held) rank += kByDistance ? (od < hd || (od == hd && oj < hj)) : oj < hj;
+    for (int k = 0; k < held; k++) {
+        const float2 o = found[k];
+        const int oj = __float_as_int(o.x);
+        above += oj > (int)i;
+#pragma unroll
+        for (int e = 0; e < kSelEntries; e++)
+            rank[e] += kByDistance ? (o.y < hd[e] || (o.y == hd[e] && oj < hj[e])) : oj < hj[e];
     }
-    fn(l16, i, h, held, hj, rank, false);
-    for (int q = 0; q < 2; q++) {
-        if (!((again >> (16 * q)) & 1u)) continue;
-        const float4 hq = shfl4(h, 16 * q);
-        const uint32_t iq = __shfl_sync(0xffffffffu, i, 16 * q);
+    __syncwarp();
+    fn(lane, kSelLanes, i, h, held, above, [&](int e, int& j, int& rk) {
+        j = hj[e];
+        rk = rank[e];
+        return lane + kSelLanes * e < held;
+    });
+    for (uint32_t rest = again; rest;) {
+        // one particle of them: its rows to the lanes that its own were
+        const int src = (__ffs(rest) - 1) & ~(kSelLanes - 1);
+        rest &= ~(((1u << kSelLanes) - 1u) << src);
+        const float4 hq = shfl4(h, src);
+        const uint32_t iq = __shfl_sync(0xffffffffu, i, src);
         SelRange rq;
-        rq.beg = __shfl_sync(0xffffffffu, r.beg, 16 * q + l16);
-        rq.len = __shfl_sync(0xffffffffu, r.len, 16 * q + l16);
-        rq.pre = __shfl_sync(0xffffffffu, r.pre, 16 * q + l16);
-        rq.total = __shfl_sync(0xffffffffu, r.total, 16 * q);
-        const int all = sel_smallest<kAbove>(rq, pos_sorted, vals_sorted, hq, iq, n, dsq, cap, s_list[warp], lane, hj, hd);
-        rank = lane;
+#pragma unroll
+        for (int k = 0; k < kSelRows; k++) {
+            rq.beg[k] = __shfl_sync(0xffffffffu, r.beg[k], src + lane);
+            rq.len[k] = __shfl_sync(0xffffffffu, r.len[k], src + lane);
+            rq.pre[k] = __shfl_sync(0xffffffffu, r.pre[k], src + lane);
+        }
+        rq.total = __shfl_sync(0xffffffffu, r.total, src);
+        int wj, wr = wl;
+        float wd;
+        const int all = sel_smallest<kAbove>(rq, pos_sorted, vals_sorted, hq, iq, n, dsq, cap, s_list[warp], wl, wj, wd);
         if (kByDistance) {
-            rank = 0;
+            wr = 0;
             for (int k = 0; k < all; k++) {
-                const float od = __shfl_sync(0xffffffffu, hd, k);
-                const int oj = __shfl_sync(0xffffffffu, hj, k);
-                rank += (od < hd || (od == hd && oj < hj)) ? 1 : 0;
+                const float od = __shfl_sync(0xffffffffu, wd, k);
+                const int oj = __shfl_sync(0xffffffffu, wj, k);
+                wr += (od < wd || (od == wd && oj < wj)) ? 1 : 0;
             }
         }
-        fn(lane, iq, hq, all, hj, rank, true);
+        const int up = __popc(__ballot_sync(0xffffffffu, wl < all && wj > (int)iq));
+        fn(wl, 32, iq, hq, all, up, [&](int e, int& j, int& rk) {
+            j = wj;
+            rk = wr;
+            return e == 0 && wl < all;
+        });
     }
 }
 
@@ -344,28 +380,34 @@ __global__ void __launch_bounds__(kThreads)
                                  const float4* __restrict__ pos, ColorTable colors, int n_colors,
                                  float* __restrict__ vertices, int cap_vertices)
 {
-    select_pair<true, true>(pos_sorted, vals_sorted, cell_off, g, n, dsq, 2 * max_conn,
-                            [&](int lane, uint32_t i, const float4& h, int held, int hj, int rank, bool whole) {
+    select_group<true, true>(pos_sorted, vals_sorted, cell_off, g, n, dsq, 2 * max_conn,
+                             [&](int lane, int lanes, uint32_t i, const float4& h, int held, int, auto entry) {
         const int emit = min(held, max_conn);
+        uint32_t base = 0u;
         if constexpr (kEmit) {
-            uint32_t base = 0u;
             if (lane == 0 && emit > 0) base = atomicAdd(count, (uint32_t)emit);
-            base = __shfl_sync(0xffffffffu, base, 0, whole ? 32 : 16);
-            if (lane < held && rank < emit && CF_IN_BOUNDS(hj, n)) {
+            base = __shfl_sync(0xffffffffu, base, 0, lanes);
+        } else {
+            if (lane == 0 && held >= 0 && CF_IN_BOUNDS(i, n)) count[i] = (uint32_t)emit;
+        }
+#pragma unroll
+        for (int e = 0; e < kSelEntries; e++) {
+            int j, rank;
+            if (!entry(e, j, rank) || rank >= emit || !CF_IN_BOUNDS(j, n)) continue;
+            if constexpr (kEmit) {
                 const size_t k = (size_t)base + (size_t)rank;
                 if (2 * k + 1 < (size_t)cap_vertices) {
                     // ParticleSimulation.cu:253-275: i then j, each x, y, z, r, g, b with i's colour
-                    const float4 q = pos[hj];
+                    const float4 q = pos[j];
                     const uint32_t c = (__float_as_uint(h.w) & kTypeMask) % (uint32_t)n_colors;
                     const float cr = colors.c[3 * c], cg = colors.c[3 * c + 1], cb = colors.c[3 * c + 2];
                     float* v = vertices + k * 12;
                     v[0] = h.x; v[1] = h.y; v[2] = h.z; v[3] = cr; v[4] = cg; v[5] = cb;
                     v[6] = q.x; v[7] = q.y; v[8] = q.z; v[9] = cr; v[10] = cg; v[11] = cb;
                 }
+            } else {
+                slots[(size_t)i * CF_MAX_PROX_CONN + rank] = j;
             }
-        } else {
-            if (lane < held && rank < emit) slots[(size_t)i * CF_MAX_PROX_CONN + rank] = hj;
-            if (lane == 0 && held >= 0 && CF_IN_BOUNDS(i, n)) count[i] = (uint32_t)emit;
         }
     });
 }
@@ -408,13 +450,14 @@ __global__ void __launch_bounds__(kThreads)
                        int32_t* __restrict__ slots, uint32_t* __restrict__ count)
 {
     // (distances as ParticleSimulation.cu:314-317, each operation rounded on its own in source order)
-    select_pair<false, false>(pos_sorted, vals_sorted, cell_off, g, n, dsq, min(max_conn, kMeshHeld),
-                              [&](int lane, uint32_t i, const float4&, int held, int hj, int rank, bool whole) {
-        const bool up = lane < held && hj > (int)i;
-        uint32_t ups = __ballot_sync(0xffffffffu, up);
-        if (!whole) ups = (ups >> (threadIdx.x & 16)) & 0xffffu;
-        const int above = __popc(ups), at = rank - (held - above);  // the entries above form the list's tail
-        if (up) slots[(size_t)i * kMeshHeld + at] = hj;
+    select_group<false, false>(pos_sorted, vals_sorted, cell_off, g, n, dsq, min(max_conn, kMeshHeld),
+                               [&](int lane, int, uint32_t i, const float4&, int held, int above, auto entry) {
+#pragma unroll
+        for (int e = 0; e < kSelEntries; e++) {
+            int j, rank;
+            // the entries above i form the list's tail
+            if (entry(e, j, rank) && j > (int)i) slots[(size_t)i * kMeshHeld + rank - (held - above)] = j;
+        }
         if (lane == 0 && held >= 0 && CF_IN_BOUNDS(i, n)) {
             if (above < kMeshHeld) slots[(size_t)i * kMeshHeld + kMeshHeld - 1] = -above;
             count[i] = (uint32_t)min(above * (above - 1) / 2, kMeshMaxTriangles);
@@ -423,12 +466,14 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // Triangles in particle order, each particle's in the reference's pair order, at offsets[i]; index
-// triples and / or vertices of 9 floats (position, flat normal, colour).  One warp
-// per 32 particles, whose triangles are consecutive: one triangle per lane, its
-// vertices through shared memory so that the warp writes one contiguous stretch (27 floats
-// a triangle).  Bound by that write: 100,000 particles with 195,000 triangles took 40 us
-// with a thread per particle writing its own, 30 with a warp per particle.
-constexpr int kEmitWarps = 4;
+// triples and / or vertices of 9 floats (position, flat normal, colour).  One block per
+// kEmitParticles particles, whose triangles are consecutive: its warps take them 32 at a time, one
+// per lane, vertices through shared memory so that a warp writes one contiguous stretch (27 floats
+// a triangle).  Bound by the chain of reads (offsets, list, positions) and, where particles have many triangles, by
+// the block with the most: 100,000 particles with 195,000 triangles took 40 us with a thread
+// per particle writing its own, 30 with a warp per particle, 19.7 with a warp per 32, 12.0 so.
+constexpr int kEmitWarps = 8;
+constexpr int kEmitParticles = 128;
 
 __global__ void __launch_bounds__(32 * kEmitWarps)
     mesh_emit_kernel(const int32_t* __restrict__ slots, const uint32_t* __restrict__ offsets, int n,
@@ -436,22 +481,23 @@ __global__ void __launch_bounds__(32 * kEmitWarps)
                      int32_t* __restrict__ tris, float* __restrict__ vertices, long long cap_tris)
 {
     __shared__ float s_vertices[kEmitWarps][32 * 27];
+    __shared__ uint32_t s_off[kEmitParticles + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int i0 = ((int)blockIdx.x * kEmitWarps + warp) * 32;
-    if (i0 >= n) return;
-    const uint32_t off = offsets[min(i0 + lane, n)];
-    const uint32_t begin = __shfl_sync(0xffffffffu, off, 0), end = offsets[min(i0 + 32, n)];
+    const int i0 = (int)blockIdx.x * kEmitParticles;
+    if (threadIdx.x <= kEmitParticles) s_off[threadIdx.x] = offsets[min(i0 + (int)threadIdx.x, n)];
+    __syncthreads();
+    const uint32_t begin = s_off[0], end = s_off[kEmitParticles];
     float* out = s_vertices[warp];
-    for (uint32_t t0 = begin; t0 < end; t0 += 32u) {
+    for (uint32_t t0 = begin + 32u * warp; t0 < end; t0 += 32u * kEmitWarps) {
         const uint32_t t = min(t0 + (uint32_t)lane, end - 1u);
         // the last particle whose triangles start at or before t
         int p = 0;
 #pragma unroll
-        for (int step = 16; step >= 1; step >>= 1)
-            if (__shfl_sync(0xffffffffu, off, p + step) <= t) p += step;
+        for (int step = kEmitParticles / 2; step >= 1; step >>= 1)
+            if (s_off[p + step] <= t) p += step;
         // (i0 + p < n: offsets[n] = end > t)
         const int i = i0 + p;
-        int rest = (int)(t - __shfl_sync(0xffffffffu, off, p));
+        int rest = (int)(t - s_off[p]);
         const int32_t* list = slots + (size_t)i * kMeshHeld;
         // pair `rest` of (a, b), a < b < m, in order of a then b
         const int last = list[kMeshHeld - 1], m = last < 0 ? -last : kMeshHeld;
@@ -512,7 +558,7 @@ cudaError_t launch_mesh_select(const float4* pos_sorted, const uint32_t* vals_so
                                cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    mesh_select_kernel<<<(n + 2 * kSelWarps - 1) / (2 * kSelWarps), kThreads, 0, st>>>(pos_sorted, vals_sorted, cell_off, g, n, dsq,
+    mesh_select_kernel<<<(n + kSelGroups * kSelWarps - 1) / (kSelGroups * kSelWarps), kThreads, 0, st>>>(pos_sorted, vals_sorted, cell_off, g, n, dsq,
                                                                             max_conn, slots, count);
     note_launches(st);
     return cudaGetLastError();
@@ -523,7 +569,7 @@ cudaError_t launch_mesh_emit(const int32_t* slots, const uint32_t* offsets, int 
                              cudaStream_t st)
 {
     if (n <= 0 || cap_tris <= 0) return cudaSuccess;
-    mesh_emit_kernel<<<(n + 32 * kEmitWarps - 1) / (32 * kEmitWarps), 32 * kEmitWarps, 0, st>>>(slots, offsets, n, pos, colors,
+    mesh_emit_kernel<<<(n + kEmitParticles - 1) / kEmitParticles, 32 * kEmitWarps, 0, st>>>(slots, offsets, n, pos, colors,
                                                                                    n_colors, tris, vertices, cap_tris);
     note_launches(st);
     return cudaGetLastError();
@@ -545,7 +591,7 @@ cudaError_t launch_proximity_select(const float4* pos_sorted, const uint32_t* va
                                     cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    proximity_select_warp_kernel<false><<<(n + 2 * kSelWarps - 1) / (2 * kSelWarps), kThreads, 0, st>>>(
+    proximity_select_warp_kernel<false><<<(n + kSelGroups * kSelWarps - 1) / (kSelGroups * kSelWarps), kThreads, 0, st>>>(
         pos_sorted, vals_sorted, cell_off, g, n, dsq, max_conn, slots, count, nullptr, ColorTable{}, 1, nullptr, 0);
     note_launches(st);
     return cudaGetLastError();
@@ -557,7 +603,7 @@ cudaError_t launch_proximity_select_vertices(const float4* pos_sorted, const uin
                                              float* vertices, int cap_vertices, uint32_t* total, cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    proximity_select_warp_kernel<true><<<(n + 2 * kSelWarps - 1) / (2 * kSelWarps), kThreads, 0, st>>>(
+    proximity_select_warp_kernel<true><<<(n + kSelGroups * kSelWarps - 1) / (kSelGroups * kSelWarps), kThreads, 0, st>>>(
         pos_sorted, vals_sorted, cell_off, g, n, dsq, max_conn, nullptr, total, pos, colors, n_colors, vertices,
         cap_vertices);
     note_launches(st);
