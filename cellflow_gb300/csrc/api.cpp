@@ -578,11 +578,11 @@ void apply_worlds(Grid& g, int worlds)
 // The step's two phases.  The cell list leaves the sorted keys and values in
 // buffer `which` of the scratch pair, a function of the grid alone
 // (cell_list_csr_buffer), which the force kernel reads.
-int enqueue_cell_list(cf_world* w, const StepConsts& c, const float4* pos, int* which)
+int enqueue_cell_list(cf_world* w, const StepConsts& c, const float4* pos, int* which, bool with_keys = false)
 {
     Scratch& s = w->s;
     CF_CUDA(launch_cell_list_csr(pos, w->n, c.grid, c.ext, w->num_types, s, s.cell_off, s.items, s.n_items, w->err,
-                                 which, w->stream));
+                                 which, w->stream, true, with_keys));
     return CF_OK;
 }
 
@@ -597,10 +597,10 @@ int enqueue_force(cf_world* w, const StepConsts& c, int which, const StepState& 
 // The world's own state, stepped in place.
 StepState in_place(cf_world* w) { return {w->pos, w->vel, w->counts, w->pos, w->vel, w->counts, w->acc}; }
 
-int enqueue_step(cf_world* w, const StepConsts& c, const StepState& state)
+int enqueue_step(cf_world* w, const StepConsts& c, const StepState& state, bool with_keys = false)
 {
     int which = 0;
-    int rc = enqueue_cell_list(w, c, state.pos, &which);
+    int rc = enqueue_cell_list(w, c, state.pos, &which, with_keys);
     if (rc) return rc;
     return enqueue_force(w, c, which, state);
 }
@@ -1753,7 +1753,7 @@ int cf_force_work(cf_world* w, const cf_step_params* p, uint64_t* staged, uint64
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
     if (rc) return rc;
     int which = 0;
-    rc = enqueue_cell_list(w, c, w->pos, &which);
+    rc = enqueue_cell_list(w, c, w->pos, &which, true);
     if (rc) return rc;
     Scratch& s = w->s;
     CF_CUDA(launch_force_work(c, s.keys[which], s.cell_off, s.items, s.n_items, max_step_items(w->n, c.grid),
@@ -1921,7 +1921,7 @@ int proximity_enqueue(cf_world* w, float distance, int max_conn)
         // cell_off[c] .. cell_off[c + 1]
         int which = 0;
         CF_CUDA(launch_cell_list_csr(w->pos, w->n, g, w->ext, w->num_types, s, s.cell_off, nullptr, nullptr, w->err,
-                                     &which, w->stream, false));
+                                     &which, w->stream, false, false));
         CF_CUDA(cudaMemsetAsync(s.prox_count + w->n, 0, sizeof(uint32_t), w->stream));
         CF_CUDA(launch_proximity_select(s.pos_sorted, s.vals[which], s.cell_off, g, w->n, dsq, max_conn, s.prox_slots,
                                         s.prox_count, w->stream));
@@ -1953,7 +1953,7 @@ int mesh_enqueue(cf_world* w, float distance, int max_conn)
     return run_selection(w, 1, g, dsq, max_conn, [&]() -> int {
         int which = 0;
         CF_CUDA(launch_cell_list_csr(w->pos, w->n, g, w->ext, w->num_types, s, s.cell_off, nullptr, nullptr, w->err,
-                                     &which, w->stream, false));
+                                     &which, w->stream, false, false));
         CF_CUDA(cudaMemsetAsync(s.mesh_count + w->n, 0, sizeof(uint32_t), w->stream));
         CF_CUDA(launch_mesh_select(s.pos_sorted, s.vals[which], s.cell_off, g, w->n, dsq,
                                    std::min(max_conn, CF_MESH_MAX_CONN), s.mesh_slots, s.mesh_count, w->stream));
@@ -2083,7 +2083,7 @@ int cf_proximity_vertices_device(cf_world* w, float distance, int max_conn, cons
         [&]() -> int {
             int which = 0;
             CF_CUDA(launch_cell_list_csr(w->pos, w->n, g, w->ext, w->num_types, s, s.cell_off, nullptr, nullptr,
-                                         w->err, &which, w->stream, false));
+                                         w->err, &which, w->stream, false, false));
             CF_CUDA(cudaMemsetAsync(total, 0, sizeof(uint32_t), w->stream));
             CF_CUDA(launch_proximity_select_vertices(s.pos_sorted, s.vals[which], s.cell_off, g, w->n, dsq,
                                                      max_conn, w->pos, ct, w->num_types, vertices, cap_vertices,
@@ -2503,7 +2503,7 @@ int replay_segment(cf_world* w, const StepConsts& c, int seg, const SegBuf& b, b
             const StepState state{from.pos, from.vel, from.cnt, to.pos, to.vel, to.cnt, r.acc_sink};
             if (lists) {
                 const ListInto into(w, b, t);
-                rc = enqueue_step(w, c, state);
+                rc = enqueue_step(w, c, state, true);
             } else {
                 rc = enqueue_step(w, c, state);
             }
@@ -2672,7 +2672,7 @@ int rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos_in,
             int e;
             if (keep && seg == last_seg) {
                 const ListInto into(w, b, s - seg * checkpoint_every);
-                e = enqueue_step(w, c, state);
+                e = enqueue_step(w, c, state, true);
             } else {
                 e = enqueue_step(w, c, state);
             }

@@ -445,7 +445,7 @@ int cell_list_launches(int n, int key_bits);
 // tiled path (4 kernels).
 cudaError_t launch_cell_list_csr(const float4* pos, int n, const Grid& g, const float* ext, int num_types,
                                  Scratch& s, uint32_t* cell_off, Item* items, int* n_items, int* err, int* which,
-                                 cudaStream_t st, bool stable = true);
+                                 cudaStream_t st, bool stable = true, bool with_keys = true);
 int cell_list_csr_buffer(int n, const Grid& g);
 int cell_list_csr_launches(int n, const Grid& g, bool with_plan);
 int cell_list_tiles(const Grid& g);  // 0 when the rows are longer than a tile
