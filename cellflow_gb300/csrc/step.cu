@@ -29,7 +29,7 @@
 //     points' own squared distance and B only has to cover the rounding of the
 //     positions.  The scalar form (four packed FP32 instructions per pair of
 //     candidates) cost 4 issue slots a candidate; this costs about 1.7.
-//   Drain: each lane walks its home's set bits (two pairs per trip; a
+//   Drain: each lane walks its home's set bits (three pairs per trip; a
 //     warp-uniform trip count, the largest hit count): the contracted distance
 //     of the 32-bit displacement; pairs below a second bound (<= the exact
 //     test for every pair) interact for certain, pairs above a third do not,
@@ -58,15 +58,16 @@
 // drain, latency and shared-memory bank conflicts at scattered slots.  Counted
 // at 100k evenly spread particles (3,340 items of 18 groups and 28 trips): about
 // 820 instructions for an item's start and end, 97 to stage and 67 to filter a
-// group of 32 candidates, 90 per trip of two pairs.  What brought the step there,
+// group of 32 candidates, 90 per trip of two pairs (three since: 532 to 521 us for
+// the step at 1M, 318 to 315 at 64 worlds of 20,000).  What brought the step there,
 // against one 32-bit lane per home filtering and draining stretches of the list
 // (force kernel, 100k and 1M in blobs): units dealt out entry by entry instead
 // of in stretches (28 trips per item instead of 37), band pairs put off to the end
 // of the unit instead of an exact test in the trip (61 instructions per trip),
 // predicated bit walking, all of a unit's positions in flight at once, the
 // tensor-core filter: 62 to 39 us and 737 to 469 us.  One list for an item that spans the box
-// in x, end cells twice, instead of a second pass for its last cells: 264 to 240 us for 64
-// worlds of 20,000 (14 cells a row, nearly every item), 469 to 459 at 1M.  An application
+// in x, end cells twice, instead of a second pass for its last cells (and the loop and
+// registers that took): 264 to 240 us for 64 worlds of 20,000, 469 to 459 at 1M.  An application
 // world of 10,000 particles with ~125 neighbours each (313 items): 276 to 32 us with
 // four warps per item, set by the SMs that get a third item.
 #include <cuda_fp16.h>
@@ -386,8 +387,8 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
                       float4* __restrict__ pos, float4* __restrict__ vel, float4* __restrict__ acc,
                       int* __restrict__ counts, const float4* __restrict__ vel_in, const int* __restrict__ counts_in)
 {
-    // pairs per drain trip: three where the registers allow (more independent work in each)
-    constexpr int kPer = kBlockWarps * kMinBlocks > 20 ? 2 : 3;
+    // pairs per drain trip (two: 459 for 446 us at 1M in blobs; four and more gain nothing with fewer warps)
+    constexpr int kPer = 3;
     extern __shared__ __align__(16) unsigned char s_dyn[];
     const int T = c.num_types, TT = T * T;
     const bool one_world = c.grid.worlds == 1;
@@ -1021,9 +1022,8 @@ bool integrate_apart(int n) { return n >= kIntegrateApart; }
 // fills the GPU, at most two per unit that an item of evenly spread particles
 // has (one below half a unit, where further warps only add their start: 10.9
 // against 13.6 us at 2,048 particles).  Occupancy: the most registers that hold
-// all warps at once, else (several waves) the most warps: six blocks of four, two pairs per
-// trip, against ten of two, three pairs, 459 / 475 us at 1M in blobs and 240 / 256 at 64
-// worlds of 20,000.
+// all warps at once, else (several waves) the most warps: six blocks of four against ten of
+// two 459 / 475 us at 1M in blobs and 240 / 256 at 64 worlds of 20,000.
 int default_force_variant(int n, const Grid& g)
 {
     const double cells = (double)g.cells, pop = (double)n / cells;

@@ -243,8 +243,7 @@ int cf_step(cf_world* w, const cf_step_params* p, int nsteps);
 int cf_step_host(cf_world* w, const cf_step_params* p, const cf_particle* in, cf_particle* out, int n);
 
 /* Force-kernel variants: v % 3 picks the registers and resident warps the
- * kernel is built for (0: 24 warps per SM, two pairs of a home at a time;
- * 1: 20 warps and 2: 16 warps, three pairs), v / 3 picks the warps per
+ * kernel is built for (0: 24 warps per SM, 1: 20, 2: 16), v / 3 picks the warps per
  * 32-particle item: 1, 2, 4, 8 or 16, which take the item's units of 256
  * candidates in turn (more warps for worlds too small to fill the GPU, or with
  * many neighbours; with 8 and 16 warps v % 3 makes no difference).  A world
