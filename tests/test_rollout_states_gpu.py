@@ -17,9 +17,10 @@ torch = pytest.importorskip("torch")
 # longer than the rollout
 @pytest.mark.parametrize("K,every", [(1, 1), (2, 1), (3, 1), (2, 2), (3, 2), (4, 2), (6, 2), (7, 3), (3, 8)])
 @pytest.mark.parametrize("own_stream", [False, True])
-def test_kept_and_replayed_segments_agree(cflib, K, every, own_stream):
-    n = 3000
-    sim, params, *_ = make_world(n, 4, 0.15, 21, 0.03)
+# (a radius of 0.55 gives a grid of 3 cells a row)
+@pytest.mark.parametrize("n,radius", [(3000, 0.15), (400, 0.55)])
+def test_kept_and_replayed_segments_agree(cflib, n, radius, K, every, own_stream):
+    sim, params, *_ = make_world(n, 4, radius, 21, 0.03)
     stream = torch.cuda.Stream()
     if own_stream:
         sim.set_stream(stream.cuda_stream)
@@ -57,3 +58,17 @@ def test_kept_and_replayed_segments_agree(cflib, K, every, own_stream):
     for other in got[1:]:
         for g, r in zip(other, got[0]):  # table gradients sum double atomics: order may differ
             np.testing.assert_allclose(g, r, rtol=1e-6, atol=1e-7 * np.abs(r).max())
+
+
+def test_states_with_the_integrator_apart(cflib):
+    """From 500,000 particles the integrator is a kernel of its own: it reads the state before the step too."""
+    n = 500_000
+    sim, params, *_ = make_world(n, 4, 0.02, 5, 0.03)
+    start = sim.get_state()
+    sim.rollout_forward(params, 3, 2)
+    end = sim.get_state()
+    sim.set_state(*start)
+    sim.simulate(params, 3)
+    for x, y in zip(sim.get_state(), end):
+        assert np.array_equal(x, y)
+    sim.close()
