@@ -222,8 +222,7 @@ void free_particles(cf_world* w)
     dev_free(s.tile_sums);
     dev_free(s.hist);
     dev_free(s.scan_tmp);
-    dev_free(s.cell_start);
-    dev_free(s.cell_end);
+    dev_free(s.cell_count);
     dev_free(s.prox_slots);
     dev_free(s.prox_count);
     dev_free(s.mesh_slots);
@@ -240,22 +239,6 @@ void free_particles(cf_world* w)
     w->counts = nullptr;
     w->aos = nullptr;
     s = Scratch();
-}
-
-int ensure_cells(cf_world* w, int cells)
-{
-    Scratch& s = w->s;
-    if ((size_t)cells <= s.cells_cap) return CF_OK;
-    CF_CUDA(cudaStreamSynchronize(w->stream));
-    drop_graphs(w);
-    dev_free(s.cell_start);
-    dev_free(s.cell_end);
-    s.cell_start = s.cell_end = nullptr;
-    s.cells_cap = 0;
-    CF_CUDA(dev_alloc(&s.cell_start, cells));
-    CF_CUDA(dev_alloc(&s.cell_end, cells));
-    s.cells_cap = (size_t)cells;
-    return CF_OK;
 }
 
 // CSR offsets (cells + 1 entries) and the scan partials they need.
@@ -278,9 +261,14 @@ int ensure_offsets(cf_world* w, int cells)
     }
     if ((size_t)cells + 1 > s.off_cap) {
         dev_free(s.cell_off);
-        s.cell_off = nullptr;
+        dev_free(s.cell_count);
+        s.cell_off = s.cell_count = nullptr;
         s.off_cap = 0;
+        s.count_clean = false;
         CF_CUDA(dev_alloc(&s.cell_off, (size_t)cells + 1));
+        CF_CUDA(dev_alloc(&s.cell_count, (size_t)cells + 1));
+        CF_CUDA(cudaMemsetAsync(s.cell_count, 0, sizeof(uint32_t) * ((size_t)cells + 1), w->stream));
+        s.count_clean = true;
         s.off_cap = (size_t)cells + 1;
     }
     if (need_tmp > s.scan_tmp_cap) {
@@ -612,7 +600,7 @@ int enqueue_step(cf_world* w, const StepConsts& c) { return enqueue_step(w, c, i
 // buffers change.
 int step_graph(cf_world* w, const StepConsts& c, int prof, cudaGraphExec_t* out)
 {
-    const void* bufs = w->s.cell_start;
+    const void* bufs = w->s.cell_count;
     if (w->graph[prof] && w->graph_bufs[prof] == bufs && std::memcmp(&w->graph_key[prof], &c, sizeof(c)) == 0) {
         *out = w->graph[prof];
         return CF_OK;
@@ -1382,8 +1370,6 @@ int cf_step(cf_world* w, const cf_step_params* p, int nsteps)
     StepConsts c;
     rc = prepare_step(w, p, &c, true);
     if (rc) return rc;
-    rc = ensure_cells(w, c.grid.cells);
-    if (rc) return rc;
     rc = ensure_plan(w, c.grid);
     if (rc) return rc;
     rc = ensure_offsets(w, c.grid.cells);
@@ -1509,11 +1495,10 @@ int cf_step_host(cf_world* w, const cf_step_params* p, const cf_particle* in, cf
     }
     StepConsts c;
     rc = prepare_step(w, p, &c, true);
-    if (!rc) rc = ensure_cells(w, c.grid.cells);
     if (!rc) rc = ensure_plan(w, c.grid);
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
     if (rc) return rc;
-    const void* bufs = w->s.cell_start;
+    const void* bufs = w->s.cell_count;
     if (!(w->host_graph && w->host_in == in && w->host_out == out && w->host_bufs == bufs &&
           std::memcmp(&w->host_key, &c, sizeof(c)) == 0)) {
         if (w->host_graph) cudaGraphExecDestroy(w->host_graph);
@@ -1713,8 +1698,6 @@ int cf_debug_cell_list(cf_world* w, const cf_step_params* p, uint32_t* cell_of, 
     rc = prepare_step(w, p, &c, false);
     if (rc) return rc;
     if (cells_cap < c.grid.cells) return fail(CF_ERR_CAPACITY, "cell arrays smaller than the grid");
-    rc = ensure_cells(w, c.grid.cells);
-    if (rc) return rc;
     rc = ensure_offsets(w, c.grid.cells);
     if (rc) return rc;
     // the step's own cell list: CSR offsets, stable radix order
@@ -1748,7 +1731,6 @@ int cf_force_work(cf_world* w, const cf_step_params* p, uint64_t* staged, uint64
     if (rc) return rc;
     StepConsts c;
     rc = prepare_step(w, p, &c, false);
-    if (!rc) rc = ensure_cells(w, c.grid.cells);
     if (!rc) rc = ensure_plan(w, c.grid);
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
     if (rc) return rc;
@@ -1807,7 +1789,6 @@ int cf_debug_force_bad_item(cf_world* w, const cf_step_params* p, int first)
     if (rc) return rc;
     StepConsts c;
     rc = prepare_step(w, p, &c, true);
-    if (!rc) rc = ensure_cells(w, c.grid.cells);
     if (!rc) rc = ensure_plan(w, c.grid);
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
     if (rc) return rc;
@@ -2275,8 +2256,7 @@ int cf_batch_capture(cf_batch* b, const cf_step_params* p, int nsteps)
     StepConsts c;
     rc = prepare_step(w, p, &c, true);
     if (rc) return rc;
-    rc = ensure_cells(w, c.grid.cells);
-    if (!rc) rc = ensure_plan(w, c.grid);
+    rc = ensure_plan(w, c.grid);
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
     if (rc) return rc;
     CF_CUDA(cudaStreamSynchronize(w->stream));
@@ -2632,7 +2612,6 @@ int rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos_in,
     if (checkpoint_every < 1) return fail(CF_ERR_INVALID, "checkpoint_every must be >= 1");
     StepConsts c;
     rc = prepare_step(w, p, &c, false);
-    if (!rc) rc = ensure_cells(w, c.grid.cells);
     if (!rc) rc = ensure_plan(w, c.grid);
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
     if (rc) return rc;
@@ -2684,7 +2663,7 @@ int rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos_in,
     };
     if (w->use_graphs && w->stream != nullptr) {
         // one graph for the whole loop, re-captured when its shape or buffers change
-        const void* bufs = w->s.cell_start;
+        const void* bufs = w->s.cell_count;
         if (!(r.fwd_graph && r.fwd_steps == nsteps && r.fwd_every == checkpoint_every && r.fwd_bufs == bufs &&
               r.fwd_ckpt == r.ckpt_pos && r.fwd_lists == (keep ? r.seg_off : nullptr) && std::memcmp(&r.fwd_key, &c, sizeof(c)) == 0)) {
             if (r.fwd_graph) cudaGraphExecDestroy(r.fwd_graph);
@@ -2739,7 +2718,6 @@ int rollout_backward(cf_world* w, const float* d_gpos, const float* d_gvel, int 
     int rc = CF_OK;
     StepConsts c;
     rc = prepare_step(w, &r.params, &c, false);
-    if (!rc) rc = ensure_cells(w, c.grid.cells);
     if (!rc) rc = ensure_plan(w, c.grid);
     if (!rc) rc = ensure_offsets(w, c.grid.cells);
     if (!rc) rc = ensure_rollout_lists(w, std::min(r.every, r.steps), c.grid.cells);
@@ -2758,7 +2736,7 @@ int rollout_backward(cf_world* w, const float* d_gpos, const float* d_gvel, int 
             CF_CUDA(cudaMemsetAsync(r.gv, 0, sizeof(float4) * n, w->stream));
     }
     if (w->use_graphs && w->stream != nullptr && !w->profiling) {
-        const void* bufs = w->s.cell_start;
+        const void* bufs = w->s.cell_count;
         const bool same = r.bwd_graph && r.bwd_steps == r.steps && r.bwd_every == r.every && r.bwd_bufs == bufs &&
                           r.bwd_lists == r.seg_off && r.bwd_kept == r.kept && std::memcmp(&r.bwd_key, &c, sizeof(c)) == 0;
         if (!same) {
@@ -2886,8 +2864,7 @@ int rdf_list(cf_world* w, const float* d_pos, int stride, int bins, float r_max,
     if (rc) return rc;
     *g = choose_step_grid(w->ext, rdf_cutoff(bins, r_max), kMaxCells);
     apply_worlds(*g, 1);
-    rc = ensure_cells(w, g->cells);
-    if (!rc) rc = ensure_offsets(w, g->cells);
+    rc = ensure_offsets(w, g->cells);
     if (rc) return rc;
     Rollout& r = w->ro;
     const float4* pos = w->pos;

@@ -8,7 +8,7 @@
 // Per-step scratch (cell list, sorted order):
 //   keys/vals  uint32 cell id and particle index, two buffers each (radix
 //              sort ping-pong); pos_sorted float4[n] snapshot in cell order;
-//   cell_start/cell_end uint32[cells]; radix histograms.
+//   cell_count/cell_off uint32[cells + 1]; radix histograms.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -217,6 +217,10 @@ struct Scratch {
     uint32_t* aux = nullptr;  // n
     uint2* tile_sums = nullptr;
     size_t tiles_cap = 0;
+    // populations of the tiled CSR build, as many as offsets: zero between calls (tile_apply leaves them
+    // so), unless a launch of the last call failed
+    uint32_t* cell_count = nullptr;
+    bool count_clean = false;
 };
 
 // Cells of one tile of the CSR build (whole rows; 16 KB of shared memory).

@@ -60,3 +60,40 @@ def test_binned_list_gives_the_same_step(cflib, radius, n):
     _, _, _, _, mag = oracle.step_f64(pos, vel, types, prev, table, radio, params)
     assert np.array_equal(got[0][1], co)
     check_step(got[0][0], po, vo, ao, mag, params.delta_t, 2.0, f"n={n}")
+
+
+def test_lists_of_different_grids_in_turn(cflib):
+    """Every build leaves the populations at zero for the next, whatever grid that has: steps on a grid by
+    cell, on one by bins and on a generic one, with the graph's and the mesh's lists by type between
+    them, give what fresh worlds give."""
+    n, T = 5000, 5
+    w = inputs.Workload("turns", n=n, num_types=T, radius=0.1, steps=1, seed=9)
+    pos, types, table = scattered(n, 0.02, 9), w.types(), w.table()
+
+    def world():
+        sim = ParticleSimulation(n, T, 2.0, 2.0, 2.0)
+        sim.setForceTable(table)
+        sim.setRadioByType(np.zeros(T, np.float32))
+        sim.set_particles(pos, types)
+        return sim
+
+    def step(sim, radius):
+        params = inputs.Workload("turns", n=n, num_types=T, radius=radius, steps=1, seed=9).params()
+        sim.set_particles(pos, types)
+        sim.simulate(params, 1)
+        return sim.getParticleData().tobytes(), sim.getNeighborCounts().tobytes()
+
+    one = world()
+    for radius in (0.1, 0.0125, 0.6, 0.05, 0.02, 0.1):
+        one.set_particles(pos, types)
+        edges = one.proximity_edges(0.03, 5)
+        got = step(one, radius)
+        one.set_particles(pos, types)
+        fresh = world()
+        assert np.array_equal(edges, fresh.proximity_edges(0.03, 5))
+        fresh.close()
+        fresh = world()
+        want = step(fresh, radius)
+        assert got[1] == want[1]
+        fresh.close()
+    one.close()
