@@ -448,6 +448,7 @@ __global__ void __launch_bounds__(32 * kRdfWarps)
         const float2 rest = queue[32 + lane];
         __syncwarp();
         queue[lane] = rest;
+        __syncwarp();  // (the next push stores over what other lanes have just stored)
         held = max(0, held - 32);
     };
     const int warps = (int)gridDim.x * kRdfWarps;
@@ -567,6 +568,7 @@ __global__ void __launch_bounds__(32 * kRdfWarps)
             const float4 rest = queue[32 + lane];
             __syncwarp();
             queue[lane] = rest;
+            __syncwarp();
             held = max(0, held - 32);
         };
         // a type outside [0, T) is reported by the cell list's hash; it contributes nothing here
