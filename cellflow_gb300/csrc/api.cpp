@@ -1849,6 +1849,10 @@ int run_selection(cf_world* w, int kind, const Grid& g, float dsq, int max_conn,
                   long long out_cap = -1, const ColorTable* colors = nullptr)
 {
     if (!w->use_graphs || w->stream == nullptr) return body();
+    // a caller's capture records the launches themselves (a graph cannot be launched into it)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CF_CUDA(cudaStreamIsCapturing(w->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return body();
     SelGraph& sg = w->sel_graph[kind];
     const ColorTable ct = colors ? *colors : ColorTable{};
     if (!(sg.exec && std::memcmp(&sg.g, &g, sizeof(g)) == 0 && sg.dsq == dsq && sg.max_conn == max_conn &&
