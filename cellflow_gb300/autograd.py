@@ -39,8 +39,12 @@ class _Ordered:
 
 
 def _rows(x: torch.Tensor, n: int, copy: bool = False) -> torch.Tensor:
-    """x as contiguous (n, 3) float32 on the GPU (its own memory with copy)."""
-    return x.detach().to("cuda", torch.float32, copy=copy).expand(n, 3).contiguous()
+    """x, broadcast as in an assignment (leading dimensions of one dropped), as contiguous (n, 3)
+    float32 on the GPU (its own memory with copy)."""
+    x = x.detach()
+    while x.dim() > 2 and x.shape[0] == 1:
+        x = x[0]
+    return x.to("cuda", torch.float32, copy=copy).expand(n, 3).contiguous()
 
 
 class Rollout(torch.autograd.Function):
