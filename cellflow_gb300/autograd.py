@@ -33,8 +33,10 @@ class _Ordered:
     def __enter__(self):
         check(load().cf_stream_wait(self.sim.handle, self.stream), "cf_stream_wait")
 
-    def __exit__(self, *exc):
-        check(load().cf_stream_signal(self.sim.handle, self.stream), "cf_stream_signal")
+    def __exit__(self, kind, *exc):
+        rc = load().cf_stream_signal(self.sim.handle, self.stream)
+        if kind is None:  # (else the block's own error is the one to raise)
+            check(rc, "cf_stream_signal")
         return False
 
 
