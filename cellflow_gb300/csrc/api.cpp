@@ -994,8 +994,6 @@ int cf_create(int n, int num_types, float w_, float h_, float d_, uint64_t seed,
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMemsetAsync"));
     e = dev_alloc(&w->tables, 1);
     if (e != cudaSuccess) return bail(cuda_fail(e, "cudaMalloc(tables)"));
-    e = configure_step_force();
-    if (e != cudaSuccess) return bail(cuda_fail(e, "cudaFuncSetAttribute(step_force_kernel)"));
     int rc = alloc_particles(w);
     if (rc) return bail(rc);
     // ParticleSimulation.cu:430-434: particles, force table (0.28, -0.20, 1.0), radius table

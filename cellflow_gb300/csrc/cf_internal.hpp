@@ -433,7 +433,6 @@ int default_force_variant(int n, const Grid& g);
 int max_step_items(int n, const Grid& g);
 int step_launches(int n);
 bool integrate_apart(int n);  // whether the integrator is a kernel of its own
-cudaError_t configure_step_force();
 cudaError_t launch_scan_exclusive(const uint32_t* in, uint32_t* out, int n, uint32_t* tmp, size_t tmp_cap,
                                   cudaStream_t st);
 size_t scan_tmp_entries(int n);

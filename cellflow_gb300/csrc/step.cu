@@ -74,7 +74,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <type_traits>
 
 #include "cf_internal.hpp"
 
@@ -921,35 +920,13 @@ __global__ void __launch_bounds__(1024)
     if (tid == 1023) *n_items = (int)s_chunk[1023];
 }
 
+constexpr size_t kSmemDefault = 48u << 10;  // of a block, without opting in
+
 // Shared memory of a block: staging per warp, the pair table without a uniform
 // radius, and the force table of one world or, in a batch, of each item of the block.
 size_t force_smem(int warps, int T, bool uniform, int force_tables)
 {
     return sizeof(WarpSmem) * warps + (size_t)T * T * ((uniform ? 0 : sizeof(float4)) + sizeof(float) * force_tables);
-}
-
-template <int W, int B, bool G, bool U, StepForm F>
-cudaError_t configure_one()
-{
-    return cudaFuncSetAttribute(step_force_kernel<W, B, G, U, F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)force_smem(W, CF_MAX_TYPES, U, W <= 4 ? W : 1));
-}
-
-template <int W, int B>
-cudaError_t configure_variant()
-{
-    cudaError_t e = cudaSuccess;
-    const auto forms = [&e](auto generic, auto uniform) {
-        constexpr bool G = decltype(generic)::value, U = decltype(uniform)::value;
-        if (e == cudaSuccess) e = configure_one<W, B, G, U, kInPlace>();
-        if (e == cudaSuccess) e = configure_one<W, B, G, U, kApart>();
-        if (e == cudaSuccess && !G) e = configure_one<W, B, false, U, kBins>();
-    };
-    forms(std::false_type(), std::false_type());
-    forms(std::false_type(), std::true_type());
-    forms(std::true_type(), std::false_type());
-    forms(std::true_type(), std::true_type());
-    return e;
 }
 
 // W = warps per block, B = resident blocks per SM the register budget is sized for.
@@ -961,7 +938,14 @@ cudaError_t launch_variant(const StepConsts& c, const PairTables* tables, const 
     const size_t smem = force_smem(W, c.num_types, c.uniform_r != 0, c.grid.worlds == 1 ? 1 : W / c.split);
     const int blocks = (int)(((long long)max_items * c.split + W - 1) / W);
     const bool apart = state.pos_out != state.pos;
+    cudaError_t e = cudaSuccess;
     const auto launch = [&](auto kernel) {
+        // opted in where a launch needs it (to the most that any does, the same from every thread): the attribute
+        // loads the kernel, and all 60 at a world's creation took a process's first one from 1.5 to 8 ms
+        if (smem > kSmemDefault)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)force_smem(W, CF_MAX_TYPES, false, W <= 4 ? W : 1));
+        if (e != cudaSuccess) return;
         kernel<<<blocks, 32 * W, smem, st>>>(c, tables, pos_sorted, vals_sorted, cell_off, items, n_items, max_items,
                                              state.pos_out, state.vel_out, state.acc, state.counts_out, state.vel,
                                              state.counts);
@@ -983,6 +967,7 @@ cudaError_t launch_variant(const StepConsts& c, const PairTables* tables, const 
             CF_FORCE_FORMS(false, false);
     }
 #undef CF_FORCE_FORMS
+    if (e != cudaSuccess) return e;
     note_launches(st);
     return cudaGetLastError();
 }
@@ -1048,19 +1033,6 @@ cudaError_t launch_step_plan(const uint32_t* cell_off, int n, const Grid& g, Ite
     plan_kernel<<<1, 1024, 0, st>>>(cell_off, g.m[0], g.m[1], g.m[2], g.worlds * g.m[1] * g.m[2], items, n_items);
     note_launches(st);
     return cudaGetLastError();
-}
-
-// Opt the force kernels into their dynamic shared memory (outside any
-// stream capture).
-cudaError_t configure_step_force()
-{
-    cudaError_t e = configure_variant<4, 6>();
-    if (e == cudaSuccess) e = configure_variant<4, 5>();
-    if (e == cudaSuccess) e = configure_variant<4, 4>();
-    if (e == cudaSuccess) e = configure_variant<2, 10>();
-    if (e == cudaSuccess) e = configure_variant<8, 2>();
-    if (e == cudaSuccess) e = configure_variant<16, 1>();
-    return e;
 }
 
 cudaError_t launch_step_force(const StepConsts& c, const PairTables* tables, const float4* pos_sorted,
