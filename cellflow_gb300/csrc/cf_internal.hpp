@@ -221,6 +221,7 @@ struct Scratch {
     // so), unless a launch of the last call failed
     uint32_t* cell_count = nullptr;
     bool count_clean = false;
+    int type_cells = 0;  // cells per type that memory left for the grids by type (0: no limit met)
 };
 
 // Cells of one tile of the CSR build (whole rows; 16 KB of shared memory).
@@ -522,7 +523,8 @@ cudaError_t launch_rdf_grad(const float* ext, const Grid& g, int n, int T, int b
 Grid choose_step_grid(const float* ext, float r_cut, int max_cells);
 int choose_bin_shift(const Grid& g, int n);
 Grid choose_prox_grid(const float* ext, float distance, int max_cells);
-Grid choose_type_grid(const float* ext, float distance, int types, int n);
+Grid choose_type_grid(const float* ext, float distance, int types, int per_type);
+int type_grid_cells(int types, int n);
 Grid canonical_grid(const float* ext, float r_max);
 float sqrt_threshold(float eff);
 float cutoff_distance(float threshold);
