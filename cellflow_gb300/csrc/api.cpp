@@ -204,6 +204,15 @@ void free_rollout(cf_world* w)
     r = Rollout();
 }
 
+// The offsets and the populations behind them.
+void free_offsets(Scratch& s)
+{
+    dev_free(s.cell_off);
+    s.cell_off = s.cell_count = nullptr;
+    s.off_cap = 0;
+    s.count_clean = false;
+}
+
 void free_particles(cf_world* w)
 {
     drop_graphs(w);
@@ -222,7 +231,6 @@ void free_particles(cf_world* w)
     dev_free(s.tile_sums);
     dev_free(s.hist);
     dev_free(s.scan_tmp);
-    dev_free(s.cell_count);
     dev_free(s.prox_slots);
     dev_free(s.prox_count);
     dev_free(s.mesh_slots);
@@ -233,7 +241,7 @@ void free_particles(cf_world* w)
     dev_free(s.row_count);
     dev_free(s.items);
     dev_free(s.n_items);
-    dev_free(s.cell_off);
+    free_offsets(s);
     dev_free(w->aos);
     w->pos = w->vel = w->acc = nullptr;
     w->counts = nullptr;
@@ -241,15 +249,17 @@ void free_particles(cf_world* w)
     s = Scratch();
 }
 
-// CSR offsets (cells + 1 entries) and the scan partials they need.
-int ensure_offsets(cf_world* w, int cells)
+// CSR offsets and populations (cells + 1 entries each, in one allocation) and what building them needs: the tile
+// sums, or where rows are longer than a tile the partials of a scan.
+int ensure_offsets(cf_world* w, const Grid& g)
 {
     Scratch& s = w->s;
-    const size_t need_tmp = scan_tmp_entries(cells + 1);
+    const size_t need_off = ((size_t)g.cells + 1 + 31) / 32 * 32;  // (the populations start on a line of their own)
+    const size_t need_tmp = cell_list_tiles(g) ? 0 : scan_tmp_entries(g.cells + 1);
     // tiles of the CSR build: at most 257 on grids spread thin, else every tile
     // holds more than kTileCellsMax / 2 cells
-    const size_t need_tiles = (size_t)cells / (kTileCellsMax / 2) + 2 + 257;
-    if ((size_t)cells + 1 <= s.off_cap && need_tmp <= s.scan_tmp_cap && need_tiles <= s.tiles_cap) return CF_OK;
+    const size_t need_tiles = (size_t)g.cells / (kTileCellsMax / 2) + 2 + 257;
+    if (need_off <= s.off_cap && need_tmp <= s.scan_tmp_cap && need_tiles <= s.tiles_cap) return CF_OK;
     CF_CUDA(cudaStreamSynchronize(w->stream));
     drop_graphs(w);
     if (need_tiles > s.tiles_cap) {
@@ -259,17 +269,13 @@ int ensure_offsets(cf_world* w, int cells)
         CF_CUDA(dev_alloc(&s.tile_sums, need_tiles));
         s.tiles_cap = need_tiles;
     }
-    if ((size_t)cells + 1 > s.off_cap) {
-        dev_free(s.cell_off);
-        dev_free(s.cell_count);
-        s.cell_off = s.cell_count = nullptr;
-        s.off_cap = 0;
-        s.count_clean = false;
-        CF_CUDA(dev_alloc(&s.cell_off, (size_t)cells + 1));
-        CF_CUDA(dev_alloc(&s.cell_count, (size_t)cells + 1));
-        CF_CUDA(cudaMemsetAsync(s.cell_count, 0, sizeof(uint32_t) * ((size_t)cells + 1), w->stream));
+    if (need_off > s.off_cap) {
+        free_offsets(s);
+        CF_CUDA(dev_alloc(&s.cell_off, 2 * need_off));
+        s.cell_count = s.cell_off + need_off;
+        s.off_cap = need_off;
+        CF_CUDA(cudaMemsetAsync(s.cell_count, 0, sizeof(uint32_t) * need_off, w->stream));
         s.count_clean = true;
-        s.off_cap = (size_t)cells + 1;
     }
     if (need_tmp > s.scan_tmp_cap) {
         dev_free(s.scan_tmp);
@@ -291,12 +297,8 @@ int ensure_before_list(cf_world* w, Ensure ensure)
     if (rc != CF_ERR_ALLOC || !s.off_cap) return rc;
     CF_CUDA(cudaStreamSynchronize(w->stream));
     drop_graphs(w);
-    dev_free(s.cell_off);
-    dev_free(s.cell_count);
-    s.cell_off = s.cell_count = nullptr;
     s.type_cells = std::max(1, (int)(s.off_cap / (size_t)w->num_types / 4));
-    s.off_cap = 0;
-    s.count_clean = false;
+    free_offsets(s);
     return ensure();
 }
 
@@ -397,7 +399,7 @@ int ensure_type_list(cf_world* w, float distance, Grid* g)
     int cells = s.type_cells ? std::min(s.type_cells, most) : most;
     for (;;) {
         *g = choose_type_grid(w->ext, distance, w->num_types, cells);
-        const int rc = ensure_offsets(w, g->cells);
+        const int rc = ensure_offsets(w, *g);
         if (rc != CF_ERR_ALLOC || g->cells_w == 1) return rc;
         cells = s.type_cells = std::max(1, std::min(cells, g->cells_w) / 4);
     }
@@ -1418,7 +1420,7 @@ int cf_step(cf_world* w, const cf_step_params* p, int nsteps)
     if (rc) return rc;
     rc = ensure_plan(w, c.grid);
     if (rc) return rc;
-    rc = ensure_offsets(w, c.grid.cells);
+    rc = ensure_offsets(w, c.grid);
     if (rc) return rc;
     const int prof = w->profiling ? 1 : 0;
     cudaGraphExec_t exec = nullptr;
@@ -1542,7 +1544,7 @@ int cf_step_host(cf_world* w, const cf_step_params* p, const cf_particle* in, cf
     StepConsts c;
     rc = prepare_step(w, p, &c, true);
     if (!rc) rc = ensure_plan(w, c.grid);
-    if (!rc) rc = ensure_offsets(w, c.grid.cells);
+    if (!rc) rc = ensure_offsets(w, c.grid);
     if (rc) return rc;
     const void* bufs = w->s.cell_count;
     if (!(w->host_graph && w->host_in == in && w->host_out == out && w->host_bufs == bufs &&
@@ -1744,7 +1746,7 @@ int cf_debug_cell_list(cf_world* w, const cf_step_params* p, uint32_t* cell_of, 
     rc = prepare_step(w, p, &c, false);
     if (rc) return rc;
     if (cells_cap < c.grid.cells) return fail(CF_ERR_CAPACITY, "cell arrays smaller than the grid");
-    rc = ensure_offsets(w, c.grid.cells);
+    rc = ensure_offsets(w, c.grid);
     if (rc) return rc;
     // the step's own cell list: CSR offsets, stable radix order
     int which = 0;
@@ -1778,7 +1780,7 @@ int cf_force_work(cf_world* w, const cf_step_params* p, uint64_t* staged, uint64
     StepConsts c;
     rc = prepare_step(w, p, &c, false);
     if (!rc) rc = ensure_plan(w, c.grid);
-    if (!rc) rc = ensure_offsets(w, c.grid.cells);
+    if (!rc) rc = ensure_offsets(w, c.grid);
     if (rc) return rc;
     int which = 0;
     rc = enqueue_cell_list(w, c, w->pos, &which, true);
@@ -1836,7 +1838,7 @@ int cf_debug_force_bad_item(cf_world* w, const cf_step_params* p, int first)
     StepConsts c;
     rc = prepare_step(w, p, &c, true);
     if (!rc) rc = ensure_plan(w, c.grid);
-    if (!rc) rc = ensure_offsets(w, c.grid.cells);
+    if (!rc) rc = ensure_offsets(w, c.grid);
     if (rc) return rc;
     int which = 0;
     rc = enqueue_cell_list(w, c, w->pos, &which);
@@ -1886,9 +1888,10 @@ namespace {
 // Proximity selection: cell list with the proximity grid, per-particle
 // edges, exclusive scan.  Enqueues only: offsets land in prox_count[0..n] and
 // the edge total in host_words[1] once the stream has reached this point.
-// Runs a selection pass through its cached graph (captured on first use and
-// whenever the grid, distance, limit, particle or type count changes; buffer
-// reallocations drop it), or directly when graphs are off.
+// Runs a selection pass through its cached graph (whose key is the grid, distance, limit, particle and type
+// count; buffer reallocations drop it), or directly when graphs are off and the first time with a key: a program that
+// makes a world and draws one frame does not pay for a graph (the first edge list of 100,000 particles in a fresh
+// world 386 us, 429 with the graph; the first mesh 323, 363).
 extern "C++" {
 template <typename Body>
 int run_selection(cf_world* w, int kind, const Grid& g, float dsq, int max_conn, Body body, const void* out = nullptr,
@@ -1901,11 +1904,22 @@ int run_selection(cf_world* w, int kind, const Grid& g, float dsq, int max_conn,
     if (capture != cudaStreamCaptureStatusNone) return body();
     SelGraph& sg = w->sel_graph[kind];
     const ColorTable ct = colors ? *colors : ColorTable{};
-    if (!(sg.exec && std::memcmp(&sg.g, &g, sizeof(g)) == 0 && sg.dsq == dsq && sg.max_conn == max_conn &&
-          sg.n == w->n && sg.types == w->num_types && sg.out == out && sg.out_cap == out_cap &&
+    if (!(std::memcmp(&sg.g, &g, sizeof(g)) == 0 && sg.dsq == dsq && sg.max_conn == max_conn && sg.n == w->n &&
+          sg.types == w->num_types && sg.out == out && sg.out_cap == out_cap &&
           std::memcmp(&sg.colors, &ct, sizeof(ct)) == 0)) {
         if (sg.exec) cudaGraphExecDestroy(sg.exec);
         sg = SelGraph();
+        sg.g = g;
+        sg.dsq = dsq;
+        sg.max_conn = max_conn;
+        sg.n = w->n;
+        sg.types = w->num_types;
+        sg.out = out;
+        sg.out_cap = out_cap;
+        sg.colors = ct;
+        return body();
+    }
+    if (!sg.exec) {
         cudaGraph_t graph = nullptr;
         CF_CUDA(cudaStreamBeginCapture(w->stream, cudaStreamCaptureModeThreadLocal));
         const int rc = body();
@@ -1919,14 +1933,6 @@ int run_selection(cf_world* w, int kind, const Grid& g, float dsq, int max_conn,
         if (e == cudaSuccess) e = cudaGraphInstantiate(&sg.exec, graph, 0);
         cudaGraphDestroy(graph);
         if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
-        sg.g = g;
-        sg.dsq = dsq;
-        sg.max_conn = max_conn;
-        sg.n = w->n;
-        sg.types = w->num_types;
-        sg.out = out;
-        sg.out_cap = out_cap;
-        sg.colors = ct;
     }
     CF_CUDA(cudaGraphLaunch(sg.exec, w->stream));
     note_launches(w->stream, sg.kernels);
@@ -2307,7 +2313,7 @@ int cf_batch_capture(cf_batch* b, const cf_step_params* p, int nsteps)
     rc = prepare_step(w, p, &c, true);
     if (rc) return rc;
     rc = ensure_plan(w, c.grid);
-    if (!rc) rc = ensure_offsets(w, c.grid.cells);
+    if (!rc) rc = ensure_offsets(w, c.grid);
     if (rc) return rc;
     CF_CUDA(cudaStreamSynchronize(w->stream));
     if (w->batch_graph) cudaGraphExecDestroy(w->batch_graph);
@@ -2663,7 +2669,7 @@ int rollout_forward(cf_world* w, const cf_step_params* p, const float* d_pos_in,
     StepConsts c;
     rc = prepare_step(w, p, &c, false);
     if (!rc) rc = ensure_plan(w, c.grid);
-    if (!rc) rc = ensure_offsets(w, c.grid.cells);
+    if (!rc) rc = ensure_offsets(w, c.grid);
     if (rc) return rc;
     const int ckpts = (nsteps + checkpoint_every - 1) / checkpoint_every;
     rc = ensure_rollout(w, ckpts, std::max(1, std::min(checkpoint_every, nsteps) - 1));
@@ -2769,7 +2775,7 @@ int rollout_backward(cf_world* w, const float* d_gpos, const float* d_gvel, int 
     StepConsts c;
     rc = prepare_step(w, &r.params, &c, false);
     if (!rc) rc = ensure_plan(w, c.grid);
-    if (!rc) rc = ensure_offsets(w, c.grid.cells);
+    if (!rc) rc = ensure_offsets(w, c.grid);
     if (!rc) rc = ensure_rollout_lists(w, std::min(r.every, r.steps), c.grid.cells);
     if (rc) return rc;
     const size_t n = (size_t)w->n;
@@ -2914,7 +2920,7 @@ int rdf_list(cf_world* w, const float* d_pos, int stride, int bins, float r_max,
     if (rc) return rc;
     *g = choose_step_grid(w->ext, rdf_cutoff(bins, r_max), kMaxCells);
     apply_worlds(*g, 1);
-    rc = ensure_offsets(w, g->cells);
+    rc = ensure_offsets(w, *g);
     if (rc) return rc;
     Rollout& r = w->ro;
     const float4* pos = w->pos;

@@ -217,8 +217,8 @@ struct Scratch {
     uint32_t* aux = nullptr;  // n
     uint2* tile_sums = nullptr;
     size_t tiles_cap = 0;
-    // populations of the tiled CSR build, as many as offsets: zero between calls (tile_apply leaves them
-    // so), unless a launch of the last call failed
+    // populations of the tiled CSR build, as many as offsets and behind them: zero between calls (tile_apply
+    // leaves them so), unless a launch of the last call failed
     uint32_t* cell_count = nullptr;
     bool count_clean = false;
     int type_cells = 0;  // cells per type that memory left for the grids by type (0: no limit met)
@@ -303,8 +303,8 @@ struct ColorTable {
 };
 
 struct SelGraph {
-    cudaGraphExec_t exec = nullptr;
-    long long kernels = 0;  // kernel nodes of exec
+    cudaGraphExec_t exec = nullptr;  // null: the key's first call ran directly
+    long long kernels = 0;           // kernel nodes of exec
     Grid g{};
     float dsq = 0.0f;
     int max_conn = -1, n = -1, types = -1;
