@@ -1,6 +1,6 @@
 """Builds the CUDA library libcellflow.so in-tree for sm_103a.
 
-Each translation unit of ``csrc/`` is compiled by nvcc in parallel into
+Each translation unit of ``csrc/`` (step.cu once more per form of the force kernel) is compiled by nvcc in parallel into
 ``cellflow_gb300/_build/`` and linked into ``cellflow_gb300/libcellflow.so``.
 Host code is compiled with ``-ffp-contract=off`` (the pair tables must round
 like the reference's float expressions); device code keeps nvcc's defaults
@@ -28,6 +28,8 @@ INCLUDE = PKG.parent / "include"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["api.cpp", "celllist.cu", "step.cu", "proximity.cu", "init.cu", "peak.cu", "noalloc.cu", "adjoint.cu",
            "preset.cpp"]
+# step.cu once more per form of the force kernel: (warps per block, blocks per SM), CF_FORCE_UNITS of cf_internal.hpp
+FORCE_UNITS = [(4, 6), (4, 5), (4, 4), (2, 10), (8, 2), (16, 1)]
 
 
 def nvcc() -> str:
@@ -44,9 +46,14 @@ def _flags(src: str, bounds: bool = False) -> list[str]:
     return common
 
 
-def _compile(src: str, bounds: bool = False) -> Path:
-    obj = (BUILD_BOUNDS if bounds else BUILD) / (src + ".o")
-    cmd = [nvcc(), *_flags(src, bounds), "-c", str(CSRC / src), "-o", str(obj)]
+def _compile(src: str, bounds: bool = False, force_unit: tuple[int, int] | None = None) -> Path:
+    name, defines = src, []
+    if force_unit:
+        warps, blocks = force_unit
+        name = f"{src}.{warps}_{blocks}"
+        defines = [f"-DCF_FORCE_WARPS={warps}", f"-DCF_FORCE_BLOCKS={blocks}"]
+    obj = (BUILD_BOUNDS if bounds else BUILD) / (name + ".o")
+    cmd = [nvcc(), *_flags(src, bounds), *defines, "-c", str(CSRC / src), "-o", str(obj)]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"nvcc failed for {src}:\n{' '.join(cmd)}\n{res.stdout}\n{res.stderr}")
@@ -67,8 +74,9 @@ def build(force: bool = False, bounds: bool = False) -> Path:
     if not force and not _stale(LIB_OUT):
         return LIB_OUT
     (BUILD_BOUNDS if bounds else BUILD).mkdir(exist_ok=True)
-    with concurrent.futures.ThreadPoolExecutor(max_workers=len(SOURCES)) as ex:
-        objs = list(ex.map(lambda src: _compile(src, bounds), SOURCES))
+    units = [(src, bounds, None) for src in SOURCES] + [("step.cu", bounds, unit) for unit in FORCE_UNITS]
+    with concurrent.futures.ThreadPoolExecutor(max_workers=len(units)) as ex:
+        objs = list(ex.map(lambda unit: _compile(*unit), units))
     tmp = LIB_OUT.with_suffix(".so.tmp")
     cmd = [nvcc(), "-shared", *ARCH, "-o", str(tmp), *map(str, objs)]
     res = subprocess.run(cmd, capture_output=True, text=True)

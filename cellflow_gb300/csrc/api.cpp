@@ -1809,8 +1809,11 @@ int cf_debug_bounds(int* checked, int* found, char* where, int where_cap, long l
     const struct {
         const char* file;
         cudaError_t (*take)(BoundsRecord*);
-    } units[] = {{"celllist.cu", bounds_take_celllist}, {"step.cu", bounds_take_step},
-                 {"proximity.cu", bounds_take_proximity}};
+    } units[] = {{"celllist.cu", bounds_take_celllist},
+#define CF_FORCE_UNIT(w, b) {"step.cu", bounds_take_step_##w##_##b},
+                 CF_FORCE_UNITS(CF_FORCE_UNIT)
+#undef CF_FORCE_UNIT
+                     {"proximity.cu", bounds_take_proximity}};
     bool first = true;
     for (const auto& u : units) {
         BoundsRecord r{};

@@ -83,7 +83,11 @@ __device__ __forceinline__ bool bounds_ok(long long idx, long long lim, int line
 #endif
 #endif
 cudaError_t bounds_take_celllist(BoundsRecord* out);
-cudaError_t bounds_take_step(BoundsRecord* out);
+// (the force kernel's units, one per warps and blocks: cellflow_gb300/build.py)
+#define CF_FORCE_UNITS(do) do(4, 6) do(4, 5) do(4, 4) do(2, 10) do(8, 2) do(16, 1)
+#define CF_FORCE_UNIT_READER(w, b) cudaError_t bounds_take_step_##w##_##b(BoundsRecord* out);
+CF_FORCE_UNITS(CF_FORCE_UNIT_READER)
+#undef CF_FORCE_UNIT_READER
 cudaError_t bounds_take_proximity(BoundsRecord* out);
 
 // Tables padded to the maximum type count so any 5-bit type index stays in

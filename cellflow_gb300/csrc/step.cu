@@ -831,6 +831,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
                   kForm == kApart ? counts_in : counts, pos, vel, acc, counts);
 }
 
+#ifndef CF_FORCE_WARPS
 __global__ void __launch_bounds__(256)
     integrate_kernel(StepConsts c, StepState state)
 {
@@ -920,6 +921,7 @@ __global__ void __launch_bounds__(1024)
     if (tid == 1023) *n_items = (int)s_chunk[1023];
 }
 
+#else
 constexpr size_t kSmemDefault = 48u << 10;  // of a block, without opting in
 
 // Shared memory of a block: staging per warp, the pair table without a uniform
@@ -929,7 +931,20 @@ size_t force_smem(int warps, int T, bool uniform, int force_tables)
     return sizeof(WarpSmem) * warps + (size_t)T * T * ((uniform ? 0 : sizeof(float4)) + sizeof(float) * force_tables);
 }
 
-// W = warps per block, B = resident blocks per SM the register budget is sized for.
+#endif
+
+}  // namespace
+
+// W = warps per block, B = resident blocks per SM the register budget is sized for.  Every (W, B) is a translation unit of
+// its own (this file with CF_FORCE_WARPS and CF_FORCE_BLOCKS), so that a process loads the forms of the one it
+// uses: in one unit the 60 forms took a process's first step 6.9 ms, now 0.8.
+template <int W, int B>
+cudaError_t launch_variant(const StepConsts& c, const PairTables* tables, const float4* pos_sorted,
+                           const uint32_t* vals_sorted, const uint32_t* cell_off, const Item* items,
+                           const int* n_items, int max_items, const StepState& state, cudaStream_t st);
+
+#ifdef CF_FORCE_WARPS
+
 template <int W, int B>
 cudaError_t launch_variant(const StepConsts& c, const PairTables* tables, const float4* pos_sorted,
                            const uint32_t* vals_sorted, const uint32_t* cell_off, const Item* items,
@@ -972,9 +987,16 @@ cudaError_t launch_variant(const StepConsts& c, const PairTables* tables, const 
     return cudaGetLastError();
 }
 
-}  // namespace
+template cudaError_t launch_variant<CF_FORCE_WARPS, CF_FORCE_BLOCKS>(
+    const StepConsts& c, const PairTables* tables, const float4* pos_sorted, const uint32_t* vals_sorted,
+    const uint32_t* cell_off, const Item* items, const int* n_items, int max_items, const StepState& state,
+    cudaStream_t st);
 
-CF_BOUNDS_READER(step)
+#define CF_FORCE_READER(w, b) CF_BOUNDS_READER(step_##w##_##b)
+#define CF_FORCE_READER_OF(w, b) CF_FORCE_READER(w, b)
+CF_FORCE_READER_OF(CF_FORCE_WARPS, CF_FORCE_BLOCKS)
+
+#else
 
 cudaError_t launch_force_work(const StepConsts& c, const uint32_t* keys_sorted, const uint32_t* cell_off,
                               const Item* items, const int* n_items, int max_items, unsigned long long* out,
@@ -1056,5 +1078,7 @@ cudaError_t launch_step_force(const StepConsts& c, const PairTables* tables, con
     note_launches(st);
     return cudaGetLastError();
 }
+
+#endif  // CF_FORCE_WARPS
 
 }  // namespace cf
