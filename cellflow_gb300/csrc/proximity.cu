@@ -15,6 +15,10 @@
 // per particle: arbitrary order, as the reference's append.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+
 #include "cf_internal.hpp"
 
 namespace cf {
@@ -113,35 +117,46 @@ __global__ void __launch_bounds__(kThreads)
     count[i] = (uint32_t)emit;
 }
 
-// The selections on the CSR cell list: eight lanes per particle.  The list is sorted by type first
+// The selections on the CSR cell list: 8, 16 or 32 lanes per particle (sel_lanes).  The list is sorted by type first
 // (Grid::by_type), so the particle's clipped stencil, at most nine rows of one contiguous range each,
 // holds particles of its own type only: with 8 types an eighth of the candidates.  The
 // ranges (one or two rows per lane, concatenated by a prefix sum) are staged as a list of
-// sorted slots and the lanes test eight candidates at a time.  A particle with more than 16 in range, or more
-// than the limit, is done again by the whole warp.  Bound by instruction issue: the work per warp
+// sorted slots and the lanes test as many candidates at a time.  Crowded particles, with more in range than their lanes
+// hold (16, or 32), are the whole warp's: those of one row of cells together, over the slots around them all (sel_crowd).
+// Bound by instruction issue: the work per warp
 // is much the same for one particle as for four.  100,000 particles, half of them in clumps (proximity
 // / mesh): 49 / 99 us with all types in one list (the mesh one thread per particle), 29 / 34 by
 // type with a warp per particle, 26 / 32 with half a warp, 19 / 24 with eight lanes; with four 19 / 30
-// and with one 20 / 45 (crowded particles then come 8 or 32 to a warp, one after the other).
+// and with one 20 / 45 (crowded particles then come 8 or 32 to a warp, one after the other).  Crowded, one type, 300,000
+// particles in a layer (the mesh call with 590 in range, limit 2): 7,715 us when each had a first pass over all candidates
+// and one of its own in which every candidate in range joined the set; 1,008 with a thread per particle on one
+// list; 561 so.
 constexpr int kSelWarps = kThreads / 32;
-constexpr int kSelLanes = 8;                      // per particle
-constexpr int kSelGroups = 32 / kSelLanes;        // particles of a warp
-constexpr int kSelListCap = 256;                  // candidates staged per warp at a time
-constexpr int kSelFound = 16;                     // in range, without the whole warp
 
-constexpr int kSelRows = (9 + kSelLanes - 1) / kSelLanes;          // rows of a lane at most
-constexpr int kSelEntries = (kSelFound + kSelLanes - 1) / kSelLanes;  // found entries of a lane
+// kLanes lanes per particle: 8, 16 or 32.
+template <int kLanes>
+struct Sel {
+    static constexpr int kGroups = 32 / kLanes;              // particles of a warp
+    static constexpr int kCap = 8 * kLanes;                  // candidates staged per particle at a time
+    static constexpr int kFound = kLanes == 8 ? 16 : 32;     // in range, without the whole warp
+    static constexpr int kRows = (9 + kLanes - 1) / kLanes;  // rows of a lane at most
+    static constexpr int kEntries = kFound / kLanes;         // found entries of a lane
+    static constexpr uint32_t kMask = kLanes == 32 ? 0xffffffffu : (1u << kLanes) - 1u;
+};
 
+template <int kLanes>
 struct SelRange {
-    uint32_t beg[kSelRows];            // this lane's rows (lane, lane + kSelLanes, ...): first sorted slot
-    int len[kSelRows], pre[kSelRows];  // entries, and those of the rows before
+    uint32_t beg[Sel<kLanes>::kRows];  // this lane's rows (lane, lane + kLanes, ...): first sorted slot
+    int len[Sel<kLanes>::kRows], pre[Sel<kLanes>::kRows];  // entries, and those of the rows before
     int total;
 };
 
-// Rows of the stencil of a particle at h, for its lanes (lane: 0 .. kSelLanes - 1).
-__device__ __forceinline__ SelRange stencil_rows(const float4& h, const uint32_t* __restrict__ cell_off, const Grid& g,
-                                                 int n, int lane)
+// Rows of the stencil of a particle at h, for its lanes (lane: 0 .. kLanes - 1).
+template <int kLanes>
+__device__ __forceinline__ SelRange<kLanes> stencil_rows(const float4& h, const uint32_t* __restrict__ cell_off,
+                                                         const Grid& g, int n, int lane)
 {
+    constexpr int kSelRows = Sel<kLanes>::kRows;
     const int mx = g.m[0], my = g.m[1], mz = g.m[2];
     const int cx = axis_cell(h.x, g.inv[0], mx);
     const int cy = axis_cell(h.y, g.inv[1], my);
@@ -153,13 +168,13 @@ __device__ __forceinline__ SelRange stencil_rows(const float4& h, const uint32_t
     // (a type outside [0, T) is reported by the hash, which counts it as type 0)
     const uint32_t type = __float_as_uint(h.w) & kTypeMask;
     const uint32_t base = (type < (uint32_t)g.worlds ? type : 0u) * (uint32_t)g.cells_w;
-    SelRange r;
+    SelRange<kLanes> r;
     r.total = 0;
 #pragma unroll
     for (int k = 0; k < kSelRows; k++) {
         r.beg[k] = 0u;
         r.len[k] = 0;
-        const int q = lane + kSelLanes * k;  // row
+        const int q = lane + kLanes * k;  // row
         if (q < nrows) {
             // q / ny for q < 9 and ny in {1, 2, 3} without a division: (q * 11) >> 5 = q / 3
             const int zq = ny == 3 ? (q * 11) >> 5 : (ny == 2 ? q >> 1 : q);
@@ -174,44 +189,53 @@ __device__ __forceinline__ SelRange stencil_rows(const float4& h, const uint32_t
     for (int k = 0; k < kSelRows; k++) {
         int incl = r.len[k];
 #pragma unroll
-        for (int o = 1; o < kSelLanes; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o, kSelLanes);
+        for (int o = 1; o < kLanes; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o, kLanes);
             if (lane >= o) incl += v;
         }
         r.pre[k] = r.total + incl - r.len[k];
-        r.total += __shfl_sync(0xffffffffu, incl, kSelLanes - 1, kSelLanes);
+        r.total += __shfl_sync(0xffffffffu, incl, kLanes - 1, kLanes);
     }
     return r;
 }
 
-__device__ __forceinline__ void clear_rows(SelRange& r)
+template <int kLanes>
+__device__ __forceinline__ void clear_rows(SelRange<kLanes>& r)
 {
 #pragma unroll
-    for (int k = 0; k < kSelRows; k++) r.len[k] = 0;
+    for (int k = 0; k < Sel<kLanes>::kRows; k++) r.len[k] = 0;
     r.total = 0;
 }
 
-// Calls fn(ok, j, d2) for the stencil's candidates, kLanes (kSelLanes: each group its own particle's; 32)
-// at a time, the whole warp together: j is the candidate's particle index, ok: it is another
-// particle (with kAbove: of a larger index) within the distance.  list: the particle's staging
-// area, 8 kLanes entries; lane: 0 .. kLanes - 1.
-template <int kLanes, bool kAbove, typename Fn>
-__device__ __forceinline__ void sel_candidates(const SelRange& r, const float4* __restrict__ pos_sorted,
-                                               const uint32_t* __restrict__ vals_sorted, const float4& h, uint32_t i,
-                                               int n, float dsq, uint32_t* list, int lane, Fn fn)
+// Squared distance, each operation rounded on its own (ParticleSimulation.cu:211-213, :314-317).
+__device__ __forceinline__ float sel_distance(const float4& q, const float4& h)
 {
-    constexpr int kCap = 8 * kLanes;
-    const int most = kLanes == 32 ? r.total : __reduce_max_sync(0xffffffffu, r.total);
+    const float dx = __fsub_rn(q.x, h.x), dy = __fsub_rn(q.y, h.y), dz = __fsub_rn(q.z, h.z);
+    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+}
+
+// Calls fn(ok, j, d2) for the stencil's candidates, kLanes at a time per particle, the whole warp together: j is the
+// candidate's particle index, ok: it is another particle (with kAbove: of a larger index) within the
+// distance.  Ends early where more() is false for every particle that has candidates left.  list: the
+// particle's staging area.
+template <int kLanes, bool kAbove, typename More, typename Fn>
+__device__ __forceinline__ void sel_candidates(const SelRange<kLanes>& r, const float4* __restrict__ pos_sorted,
+                                               const uint32_t* __restrict__ vals_sorted, const float4& h, uint32_t i,
+                                               int n, float dsq, bool skip, uint32_t* list, int lane, More more, Fn fn)
+{
+    constexpr int kCap = Sel<kLanes>::kCap, kSelRows = Sel<kLanes>::kRows;
+    const int total = skip ? 0 : r.total, most = __reduce_max_sync(0xffffffffu, total);
     for (int base = 0; base < most; base += kCap) {
+        if (base > 0 && !__any_sync(0xffffffffu, base < total && more())) break;
 #pragma unroll
         for (int k = 0; k < kSelRows; k++) {
-            if (lane < min(kSelLanes, 9 - kSelLanes * k)) {
-                const int j0 = max(0, base - r.pre[k]), j1 = min(r.len[k], base + kCap - r.pre[k]);
+            if (lane < min(kLanes, 9 - kLanes * k)) {
+                const int j0 = max(0, base - r.pre[k]), j1 = skip ? 0 : min(r.len[k], base + kCap - r.pre[k]);
                 for (int j = j0; j < j1; j++) list[r.pre[k] + j - base] = r.beg[k] + (uint32_t)j;
             }
         }
         __syncwarp();
-        const int lim = min(kCap, r.total - base), most_here = min(kCap, most - base);
+        const int lim = min(kCap, total - base), most_here = min(kCap, most - base);
         for (int g0 = 0; g0 < most_here; g0 += kLanes) {
             const int gg = g0 + lane;
             bool ok = false;
@@ -221,10 +245,7 @@ __device__ __forceinline__ void sel_candidates(const SelRange& r, const float4* 
                 const uint32_t u = list[gg];
                 const float4 q = pos_sorted[u];
                 j = (int)vals_sorted[u];
-                const float dx = __fsub_rn(q.x, h.x);
-                const float dy = __fsub_rn(q.y, h.y);
-                const float dz = __fsub_rn(q.z, h.z);
-                d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+                d2 = sel_distance(q, h);
                 ok = d2 < dsq && (kAbove ? j > (int)i : j != (int)i) && __float_as_uint(q.w) == __float_as_uint(h.w);
             }
             fn(ok, j, d2);
@@ -233,135 +254,227 @@ __device__ __forceinline__ void sel_candidates(const SelRange& r, const float4* 
     }
 }
 
-// The `cap` (at most 32) smallest qualifying indices of one particle as (j, d2) in lanes 0 ..
-// held-1, in index order: one at a time in ballot order, past the end of a full set dropped.
-template <bool kAbove>
-__device__ __forceinline__ int sel_smallest(const SelRange& r, const float4* __restrict__ pos_sorted,
-                                            const uint32_t* __restrict__ vals_sorted, const float4& h, uint32_t i, int n,
-                                            float dsq, int cap, uint32_t* list, int lane, int& hj, float& hd)
+// The crowded particles of a warp that lie in one row of cells (groups `members`, their homes in s_home, indices iq),
+// by the whole warp over the rows of cells around them all, 32 slots at a time: for each the `cap` (at most 32) smallest
+// qualifying indices as (j, d2) in lanes 0 .. held-1, in index order.  Once a set is full a candidate above its
+// largest index is dropped, for all of them before its position is read, as most are; a qualifying one joins at its
+// place, the largest falling out.
+template <int kGroups>
+struct Crowd {
+    int held[kGroups], hj[kGroups];
+    float hd[kGroups];
+};
+
+template <int kLanes, bool kAbove>
+__device__ __forceinline__ void sel_crowd(const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ vals_sorted,
+                                          const uint32_t* __restrict__ cell_off, const Grid& g, int n, float dsq, int cap,
+                                          uint32_t members, const float4* s_home, const int (&iq)[Sel<kLanes>::kGroups], int lane,
+                                          Crowd<Sel<kLanes>::kGroups>& c)
 {
-    int held = 0;
-    hj = 0;
-    hd = 0.0f;
-    sel_candidates<32, kAbove>(r, pos_sorted, vals_sorted, h, i, n, dsq, list, lane, [&](bool ok, int cj, float cd) {
-        uint32_t qm = __ballot_sync(0xffffffffu, ok);
-        while (qm) {
-            const int src = __ffs(qm) - 1;
-            qm &= qm - 1u;
-            const int j = __shfl_sync(0xffffffffu, cj, src);
-            const float d2 = __shfl_sync(0xffffffffu, cd, src);
-            const int pos = __popc(__ballot_sync(0xffffffffu, lane < held && hj < j));
-            if (pos >= cap) continue;
-            const int uj = __shfl_up_sync(0xffffffffu, hj, 1);
-            const float ud = __shfl_up_sync(0xffffffffu, hd, 1);
-            if (lane > pos && lane < cap) {
-                hj = uj;
-                hd = ud;
+    constexpr int kSelGroups = Sel<kLanes>::kGroups;
+    const float4 first = s_home[(__ffs(members) - 1) / kLanes], last = s_home[(31 - __clz(members)) / kLanes];
+    const int mx = g.m[0], my = g.m[1], mz = g.m[2];
+    const int xlo = max(axis_cell(first.x, g.inv[0], mx) - 1, 0), xhi = min(axis_cell(last.x, g.inv[0], mx) + 1, mx - 1);
+    const int cy = axis_cell(first.y, g.inv[1], my), cz = axis_cell(first.z, g.inv[2], mz);
+    const int ylo = max(cy - 1, 0), yhi = min(cy + 1, my - 1), zlo = max(cz - 1, 0), zhi = min(cz + 1, mz - 1);
+    const int ny = yhi - ylo + 1, nrows = ny * (zhi - zlo + 1);
+    const uint32_t type = __float_as_uint(first.w) & kTypeMask;
+    uint32_t beg = 0u;
+    int len = 0;
+    if (lane < nrows) {
+        const int zq = ny == 3 ? (lane * 11) >> 5 : (ny == 2 ? lane >> 1 : lane);
+        const uint32_t row = (type < (uint32_t)g.worlds ? type : 0u) * (uint32_t)g.cells_w +
+                             (uint32_t)(((zlo + zq) * my + ylo + (lane - zq * ny)) * mx);
+        beg = cell_off[row + xlo];
+        len = (int)(cell_off[row + xhi + 1] - beg);
+        if (!CF_IN_BOUNDS(len, n + 1) || !CF_IN_BOUNDS(beg + len, n + 1)) len = 0;
+    }
+    // chunks of 32 slots, those of each row apart
+    int before = (len + 31) >> 5;
+    const int own = before;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += v;
+    }
+    const int chunks = __shfl_sync(0xffffffffu, before, 15);
+    before -= own;
+    int worst[kSelGroups];  // above every index that the set can still take; of a full set its largest
+#pragma unroll
+    for (int q = 0; q < kSelGroups; q++) {
+        c.held[q] = c.hj[q] = 0;
+        c.hd[q] = 0.0f;
+        worst[q] = cap > 0 && (members >> (kLanes * q) & 1u) ? 0x7fffffff : -1;
+    }
+    // chunk k's slot of this lane and its index (none: the largest int)
+    const auto fetch = [&](int k, uint32_t& u) {
+        const int row = 31 - __clz(__ballot_sync(0xffffffffu, own > 0 && before <= k));
+        const int at = 32 * (k - __shfl_sync(0xffffffffu, before, row)) + lane;
+        u = __shfl_sync(0xffffffffu, beg, row) + (uint32_t)at;
+        return at < __shfl_sync(0xffffffffu, len, row) && CF_IN_BOUNDS(u, n) ? (int)vals_sorted[u] : 0x7fffffff;
+    };
+    uint32_t u_next = 0u;
+    int j_next = chunks > 0 ? fetch(0, u_next) : 0;
+    for (int k = 0; k < chunks; k++) {
+        const uint32_t u = u_next;
+        const int cj = j_next;
+        if (k + 1 < chunks) j_next = fetch(k + 1, u_next);
+        bool want = false;
+#pragma unroll
+        for (int q = 0; q < kSelGroups; q++) want |= cj < worst[q] && (kAbove ? cj > iq[q] : cj != iq[q]);
+        if (!__any_sync(0xffffffffu, want)) continue;
+        float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (want) p = pos_sorted[u];
+#pragma unroll
+        for (int q = 0; q < kSelGroups; q++) {
+            if (worst[q] < 0) continue;
+            const float4 h = s_home[q];
+            const float cd = sel_distance(p, h);
+            uint32_t qm = __ballot_sync(0xffffffffu, cj < worst[q] && (kAbove ? cj > iq[q] : cj != iq[q]) && cd < dsq &&
+                                                        __float_as_uint(p.w) == __float_as_uint(h.w));
+            if (!qm) continue;
+            while (qm) {
+                const int src = __ffs(qm) - 1;
+                qm &= qm - 1u;
+                const int j = __shfl_sync(0xffffffffu, cj, src);
+                const float d2 = __shfl_sync(0xffffffffu, cd, src);
+                const int pos = __popc(__ballot_sync(0xffffffffu, lane < c.held[q] && c.hj[q] < j));
+                if (pos >= cap) continue;
+                const int uj = __shfl_up_sync(0xffffffffu, c.hj[q], 1);
+                const float ud = __shfl_up_sync(0xffffffffu, c.hd[q], 1);
+                if (lane > pos && lane < cap) {
+                    c.hj[q] = uj;
+                    c.hd[q] = ud;
+                }
+                if (lane == pos) {
+                    c.hj[q] = j;
+                    c.hd[q] = d2;
+                }
+                c.held[q] = min(c.held[q] + 1, cap);
             }
-            if (lane == pos) {
-                hj = j;
-                hd = d2;
-            }
-            held = min(held + 1, cap);
+            if (c.held[q] == cap) worst[q] = __shfl_sync(0xffffffffu, c.hj[q], cap - 1);
         }
-    });
-    return held;
+    }
 }
 
-__device__ __forceinline__ float4 shfl4(const float4& v, int src)
-{
-    return make_float4(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
-                       __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
-}
-
-// Per particle fn(lane, lanes, i, h, held, above, entry): by its `lanes` lanes (kSelLanes, four particles at
+// Per particle fn(lane, lanes, i, h, held, above, entry): by its `lanes` lanes (kLanes, four particles at
 // once, or the whole warp), all together: held entries qualify (all of them, or the `cap` smallest
 // indices), `above` of them with an index above i; entry(e, j, rank) gives the lane's e-th entry
 // (false: none) with its index and rank (kByDistance: by (distance, index), else by index).
 // held < 0: not a particle of this call.
-template <bool kAbove, bool kByDistance, typename Fn>
+template <int kLanes, bool kAbove, bool kByDistance, typename Fn>
 __device__ __forceinline__ void select_group(const float4* __restrict__ pos_sorted,
                                              const uint32_t* __restrict__ vals_sorted,
                                              const uint32_t* __restrict__ cell_off, const Grid& g, int n, float dsq, int cap,
-                                             Fn fn)
+                                             int crowd, Fn fn)
 {
-    __shared__ uint32_t s_list[kSelWarps][kSelListCap];
+    constexpr int kSelGroups = Sel<kLanes>::kGroups, kSelFound = Sel<kLanes>::kFound, kSelEntries = Sel<kLanes>::kEntries;
+    constexpr uint32_t kGroupMask = Sel<kLanes>::kMask;
+    __shared__ uint32_t s_list[kSelWarps][kSelGroups][Sel<kLanes>::kCap];
     __shared__ float2 s_found[kSelWarps][kSelGroups][kSelFound];
-    const int wl = threadIdx.x & 31, warp = threadIdx.x >> 5, group = wl / kSelLanes, lane = wl % kSelLanes;
+    __shared__ float4 s_home[kSelWarps][kSelGroups];
+    const int wl = threadIdx.x & 31, warp = threadIdx.x >> 5, group = wl / kLanes, lane = wl % kLanes;
     const int t = ((int)blockIdx.x * kSelWarps + warp) * kSelGroups + group;
     if (__all_sync(0xffffffffu, t >= n)) return;
     const bool mine = t < n;
     const float4 h = pos_sorted[mine ? t : n - 1];
     const uint32_t i = vals_sorted[mine ? t : n - 1];
-    SelRange r = stencil_rows(h, cell_off, g, n, lane);
+    SelRange<kLanes> r = stencil_rows<kLanes>(h, cell_off, g, n, lane);
     if (!mine || !CF_IN_BOUNDS(i, n)) clear_rows(r);  // (bounds-checked build)
     float2* found = s_found[warp][group];
-    int held = 0;
-    sel_candidates<kSelLanes, kAbove>(r, pos_sorted, vals_sorted, h, i, n, dsq, s_list[warp] + group * (kSelListCap / kSelGroups),
-                                      lane, [&](bool ok, int j, float d2) {
-        const uint32_t qm = (__ballot_sync(0xffffffffu, ok) >> (kSelLanes * group)) & ((1u << kSelLanes) - 1u);
+    int held = r.total > crowd ? kSelFound + 1 : 0;
+    sel_candidates<kLanes, kAbove>(r, pos_sorted, vals_sorted, h, i, n, dsq, held > 0, s_list[warp][group], lane,
+                           [&] { return held <= kSelFound; }, [&](bool ok, int j, float d2) {
+        const uint32_t qm = (__ballot_sync(0xffffffffu, ok) >> (kLanes * group)) & kGroupMask;
         const int at = held + __popc(qm & ((1u << lane) - 1u));
         if (ok && at < kSelFound) found[at] = make_float2(__int_as_float(j), d2);
         held += __popc(qm);
     });
     __syncwarp();
-    const bool over = held > min(cap, kSelFound);
-    const uint32_t again = __ballot_sync(0xffffffffu, over);
-    if (over || !mine) held = -1;
+    const uint32_t again = __ballot_sync(0xffffffffu, mine && held > kSelFound);
+    if (held > kSelFound || !mine) held = 0;
     // each lane's entries (in the order in which they were found) and their ranks
-    int hj[kSelEntries], rank[kSelEntries] = {}, above = 0;
+    int hj[kSelEntries], rank[kSelEntries] = {};
     float hd[kSelEntries];
 #pragma unroll
     for (int e = 0; e < kSelEntries; e++) {
-        const float2 f = found[lane + kSelLanes * e];  // (past held: not used)
+        const float2 f = found[lane + kLanes * e];  // (past held: not used)
         hj[e] = __float_as_int(f.x);
         hd[e] = f.y;
     }
-    for (int k = 0; k < held; k++) {
-        const float2 o = found[k];
-        const int oj = __float_as_int(o.x);
-        above += oj > (int)i;
+    // those of the `cap` smallest indices, by the group's found entries: all, unless there are more
+    uint32_t kept = held < 32 ? (1u << held) - 1u : 0xffffffffu;
+    const bool many = __any_sync(0xffffffffu, held > cap);
+    if (!kByDistance || many) {
+        for (int k = 0; k < held; k++) {
+            const int oj = __float_as_int(found[k].x);
 #pragma unroll
-        for (int e = 0; e < kSelEntries; e++)
-            rank[e] += kByDistance ? (o.y < hd[e] || (o.y == hd[e] && oj < hj[e])) : oj < hj[e];
+            for (int e = 0; e < kSelEntries; e++) rank[e] += oj < hj[e];
+        }
+    }
+    if (many) {
+#pragma unroll
+        for (int e = 0; e < kSelEntries; e++) {
+            const uint32_t b = __ballot_sync(0xffffffffu, rank[e] < cap) >> (kLanes * group) & kGroupMask;
+            kept &= ~(kGroupMask << (kLanes * e)) | b << (kLanes * e);
+            if (kByDistance) rank[e] = 0;
+        }
+    }
+    int above = 0;
+#pragma unroll
+    for (int e = 0; e < kSelEntries; e++) {
+        const bool up = hj[e] > (int)i && (kept >> (lane + kLanes * e) & 1u);
+        above += __popc(__ballot_sync(0xffffffffu, up) >> (kLanes * group) & kGroupMask);
+    }
+    if (kByDistance) {
+        for (uint32_t rest = kept; rest; rest &= rest - 1u) {
+            const float2 o = found[__ffs(rest) - 1];
+            const int oj = __float_as_int(o.x);
+#pragma unroll
+            for (int e = 0; e < kSelEntries; e++) rank[e] += o.y < hd[e] || (o.y == hd[e] && oj < hj[e]);
+        }
     }
     __syncwarp();
-    fn(lane, kSelLanes, i, h, held, above, [&](int e, int& j, int& rk) {
+    fn(lane, kLanes, i, h, mine && !(again >> wl & 1u) ? __popc(kept) : -1, above, [&](int e, int& j, int& rk) {
         j = hj[e];
         rk = rank[e];
-        return lane + kSelLanes * e < held;
+        return (kept >> (lane + kLanes * e) & 1u) != 0u;
     });
-    for (uint32_t rest = again; rest;) {
-        // one particle of them: its rows to the lanes that its own were
-        const int src = (__ffs(rest) - 1) & ~(kSelLanes - 1);
-        rest &= ~(((1u << kSelLanes) - 1u) << src);
-        const float4 hq = shfl4(h, src);
-        const uint32_t iq = __shfl_sync(0xffffffffu, i, src);
-        SelRange rq;
+    if (!again) return;
+    // the crowded ones, those of a row of cells together
+    if (lane == 0) s_home[warp][group] = h;
+    __syncwarp();
+    const int row = (axis_cell(h.z, g.inv[2], g.m[2]) * g.m[1] + axis_cell(h.y, g.inv[1], g.m[1])) * (int)(kTypeMask + 1u) +
+                    (int)(__float_as_uint(h.w) & kTypeMask);
+    int iq[kSelGroups];
 #pragma unroll
-        for (int k = 0; k < kSelRows; k++) {
-            rq.beg[k] = __shfl_sync(0xffffffffu, r.beg[k], src + lane);
-            rq.len[k] = __shfl_sync(0xffffffffu, r.len[k], src + lane);
-            rq.pre[k] = __shfl_sync(0xffffffffu, r.pre[k], src + lane);
-        }
-        rq.total = __shfl_sync(0xffffffffu, r.total, src);
-        int wj, wr = wl;
-        float wd;
-        const int all = sel_smallest<kAbove>(rq, pos_sorted, vals_sorted, hq, iq, n, dsq, cap, s_list[warp], wl, wj, wd);
-        if (kByDistance) {
-            wr = 0;
-            for (int k = 0; k < all; k++) {
-                const float od = __shfl_sync(0xffffffffu, wd, k);
-                const int oj = __shfl_sync(0xffffffffu, wj, k);
-                wr += (od < wd || (od == wd && oj < wj)) ? 1 : 0;
+    for (int q = 0; q < kSelGroups; q++) iq[q] = (int)__shfl_sync(0xffffffffu, i, kLanes * q);
+    for (uint32_t rest = again; rest;) {
+        const uint32_t members = __ballot_sync(0xffffffffu, row == __shfl_sync(0xffffffffu, row, __ffs(rest) - 1)) & rest;
+        rest &= ~members;
+        Crowd<kSelGroups> c;
+        sel_crowd<kLanes, kAbove>(pos_sorted, vals_sorted, cell_off, g, n, dsq, cap, members, s_home[warp], iq, wl, c);
+#pragma unroll
+        for (int q = 0; q < kSelGroups; q++) {
+            if (!(members >> (kLanes * q) & 1u)) continue;
+            const int all = c.held[q], wj = c.hj[q];
+            const float wd = c.hd[q];
+            int wr = wl;
+            if (kByDistance) {
+                wr = 0;
+                for (int k = 0; k < all; k++) {
+                    const float od = __shfl_sync(0xffffffffu, wd, k);
+                    const int oj = __shfl_sync(0xffffffffu, wj, k);
+                    wr += (od < wd || (od == wd && oj < wj)) ? 1 : 0;
+                }
             }
+            const int up = __popc(__ballot_sync(0xffffffffu, wl < all && wj > iq[q]));
+            fn(wl, 32, (uint32_t)iq[q], s_home[warp][q], all, up, [&](int e, int& j, int& rk) {
+                j = wj;
+                rk = wr;
+                return e == 0 && wl < all;
+            });
         }
-        const int up = __popc(__ballot_sync(0xffffffffu, wl < all && wj > (int)iq));
-        fn(wl, 32, iq, hq, all, up, [&](int e, int& j, int& rk) {
-            j = wj;
-            rk = wr;
-            return e == 0 && wl < all;
-        });
     }
 }
 
@@ -372,15 +485,15 @@ __device__ __forceinline__ void select_group(const float4* __restrict__ pos_sort
 // reserves its edges' places with one atomic on *count (the running total) and
 // writes their line vertices itself (ParticleSimulation.cu:253-275: per edge the
 // vertex of i then of j, each x, y, z, r, g, b with the colour of i's type).
-template <bool kEmit>
+template <int kLanes, bool kEmit>
 __global__ void __launch_bounds__(kThreads)
     proximity_select_warp_kernel(const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ vals_sorted,
-                                 const uint32_t* __restrict__ cell_off, Grid g, int n, float dsq, int max_conn,
+                                 const uint32_t* __restrict__ cell_off, Grid g, int n, float dsq, int max_conn, int crowd,
                                  int32_t* __restrict__ slots, uint32_t* __restrict__ count,
                                  const float4* __restrict__ pos, ColorTable colors, int n_colors,
                                  float* __restrict__ vertices, int cap_vertices)
 {
-    select_group<true, true>(pos_sorted, vals_sorted, cell_off, g, n, dsq, 2 * max_conn,
+    select_group<kLanes, true, true>(pos_sorted, vals_sorted, cell_off, g, n, dsq, 2 * max_conn, crowd,
                              [&](int lane, int lanes, uint32_t i, const float4& h, int held, int, auto entry) {
         const int emit = min(held, max_conn);
         uint32_t base = 0u;
@@ -391,7 +504,7 @@ __global__ void __launch_bounds__(kThreads)
             if (lane == 0 && held >= 0 && CF_IN_BOUNDS(i, n)) count[i] = (uint32_t)emit;
         }
 #pragma unroll
-        for (int e = 0; e < kSelEntries; e++) {
+        for (int e = 0; e < Sel<kLanes>::kEntries; e++) {
             int j, rank;
             if (!entry(e, j, rank) || rank >= emit || !CF_IN_BOUNDS(j, n)) continue;
             if constexpr (kEmit) {
@@ -444,16 +557,17 @@ constexpr int kMeshMaxTriangles = 64;
 
 // slots: the particle's list entries above it, in index order; in the last slot, where fewer than
 // all slots are taken, their number, negated.
+template <int kLanes>
 __global__ void __launch_bounds__(kThreads)
     mesh_select_kernel(const float4* __restrict__ pos_sorted, const uint32_t* __restrict__ vals_sorted,
-                       const uint32_t* __restrict__ cell_off, Grid g, int n, float dsq, int max_conn,
+                       const uint32_t* __restrict__ cell_off, Grid g, int n, float dsq, int max_conn, int crowd,
                        int32_t* __restrict__ slots, uint32_t* __restrict__ count)
 {
     // (distances as ParticleSimulation.cu:314-317, each operation rounded on its own in source order)
-    select_group<false, false>(pos_sorted, vals_sorted, cell_off, g, n, dsq, min(max_conn, kMeshHeld),
+    select_group<kLanes, false, false>(pos_sorted, vals_sorted, cell_off, g, n, dsq, min(max_conn, kMeshHeld), crowd,
                                [&](int lane, int, uint32_t i, const float4&, int held, int above, auto entry) {
 #pragma unroll
-        for (int e = 0; e < kSelEntries; e++) {
+        for (int e = 0; e < Sel<kLanes>::kEntries; e++) {
             int j, rank;
             // the entries above i form the list's tail
             if (entry(e, j, rank) && j > (int)i) slots[(size_t)i * kMeshHeld + rank - (held - above)] = j;
@@ -549,6 +663,45 @@ __global__ void __launch_bounds__(32 * kEmitWarps)
     }
 }
 
+// Candidates from which on a particle is taken for crowded without looking, spread evenly over its 27 cells (above: only
+// those of larger index count): half as many again in range as its own lanes hold.
+template <int kLanes>
+int crowd_size(const Grid& g, float dsq, bool above)
+{
+    const double cells = 27.0 / ((double)g.inv[0] * g.inv[1] * g.inv[2]);  // their volume
+    const double reach = std::min(1.0, 4.19 * std::pow((double)dsq, 1.5) / cells) * (above ? 0.5 : 1.0);
+    const double size = 1.5 * Sel<kLanes>::kFound / std::max(reach, 1e-9);
+    return (int)std::min(size, 1e9);
+}
+
+// Blocks of a selection.
+template <int kLanes>
+int sel_blocks(int n)
+{
+    return (n + Sel<kLanes>::kGroups * kSelWarps - 1) / (Sel<kLanes>::kGroups * kSelWarps);
+}
+
+// Lanes per particle.  Few particles leave most of the GPU idle with eight, and the edge list of a single type, whose list
+// has the most candidates out of range, gains in clumps what evenly spread particles lose (device times, eight / sixteen
+// lanes: one type, 100,000 particles in blobs 91 / 85 us, evenly spread 26.3 / 27.2; 20,000 of 8 types evenly spread 16.3 / 19.2,
+// in blobs equal; with a warp per particle 4,000 in blobs 40.7, with sixteen lanes 43.3, with eight 47.3, host time included).
+int sel_lanes(int n, const Grid& g, bool edges)
+{
+    if (n <= 4096) return 32;
+    return n <= 10000 || (edges && g.worlds == 1) ? 16 : 8;
+}
+
+template <typename Launch>
+void with_lanes(int lanes, Launch launch)
+{
+    if (lanes == 32)
+        launch(std::integral_constant<int, 32>());
+    else if (lanes == 16)
+        launch(std::integral_constant<int, 16>());
+    else
+        launch(std::integral_constant<int, 8>());
+}
+
 }  // namespace
 
 CF_BOUNDS_READER(proximity)
@@ -558,8 +711,12 @@ cudaError_t launch_mesh_select(const float4* pos_sorted, const uint32_t* vals_so
                                cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    mesh_select_kernel<<<(n + kSelGroups * kSelWarps - 1) / (kSelGroups * kSelWarps), kThreads, 0, st>>>(pos_sorted, vals_sorted, cell_off, g, n, dsq,
-                                                                            max_conn, slots, count);
+    const auto launch = [&](auto lanes) {
+        constexpr int kLanes = decltype(lanes)::value;
+        mesh_select_kernel<kLanes><<<sel_blocks<kLanes>(n), kThreads, 0, st>>>(
+            pos_sorted, vals_sorted, cell_off, g, n, dsq, max_conn, crowd_size<kLanes>(g, dsq, false), slots, count);
+    };
+    with_lanes(sel_lanes(n, g, false), launch);
     note_launches(st);
     return cudaGetLastError();
 }
@@ -586,15 +743,32 @@ cudaError_t launch_proximity_select_cells(const float4* pos_sorted, const uint32
     return cudaGetLastError();
 }
 
+namespace {
+template <bool kEmit>
+cudaError_t launch_proximity_warps(const float4* pos_sorted, const uint32_t* vals_sorted, const uint32_t* cell_off,
+                                   const Grid& g, int n, float dsq, int max_conn, int32_t* slots, uint32_t* count,
+                                   const float4* pos, const ColorTable& colors, int n_colors, float* vertices,
+                                   int cap_vertices, cudaStream_t st)
+{
+    if (n <= 0) return cudaSuccess;
+    const auto launch = [&](auto lanes) {
+        constexpr int kLanes = decltype(lanes)::value;
+        proximity_select_warp_kernel<kLanes, kEmit><<<sel_blocks<kLanes>(n), kThreads, 0, st>>>(
+            pos_sorted, vals_sorted, cell_off, g, n, dsq, max_conn, crowd_size<kLanes>(g, dsq, true), slots, count, pos,
+            colors, n_colors, vertices, cap_vertices);
+    };
+    with_lanes(sel_lanes(n, g, true), launch);
+    note_launches(st);
+    return cudaGetLastError();
+}
+}  // namespace
+
 cudaError_t launch_proximity_select(const float4* pos_sorted, const uint32_t* vals_sorted, const uint32_t* cell_off,
                                     const Grid& g, int n, float dsq, int max_conn, int32_t* slots, uint32_t* count,
                                     cudaStream_t st)
 {
-    if (n <= 0) return cudaSuccess;
-    proximity_select_warp_kernel<false><<<(n + kSelGroups * kSelWarps - 1) / (kSelGroups * kSelWarps), kThreads, 0, st>>>(
-        pos_sorted, vals_sorted, cell_off, g, n, dsq, max_conn, slots, count, nullptr, ColorTable{}, 1, nullptr, 0);
-    note_launches(st);
-    return cudaGetLastError();
+    return launch_proximity_warps<false>(pos_sorted, vals_sorted, cell_off, g, n, dsq, max_conn, slots, count, nullptr,
+                                         ColorTable{}, 1, nullptr, 0, st);
 }
 
 cudaError_t launch_proximity_select_vertices(const float4* pos_sorted, const uint32_t* vals_sorted,
@@ -602,12 +776,8 @@ cudaError_t launch_proximity_select_vertices(const float4* pos_sorted, const uin
                                              const float4* pos, const ColorTable& colors, int n_colors,
                                              float* vertices, int cap_vertices, uint32_t* total, cudaStream_t st)
 {
-    if (n <= 0) return cudaSuccess;
-    proximity_select_warp_kernel<true><<<(n + kSelGroups * kSelWarps - 1) / (kSelGroups * kSelWarps), kThreads, 0, st>>>(
-        pos_sorted, vals_sorted, cell_off, g, n, dsq, max_conn, nullptr, total, pos, colors, n_colors, vertices,
-        cap_vertices);
-    note_launches(st);
-    return cudaGetLastError();
+    return launch_proximity_warps<true>(pos_sorted, vals_sorted, cell_off, g, n, dsq, max_conn, nullptr, total, pos, colors,
+                                        n_colors, vertices, cap_vertices, st);
 }
 
 cudaError_t launch_proximity_emit_edges(const int32_t* slots, const uint32_t* offsets, int n, int max_conn,
