@@ -16,8 +16,9 @@
 // for bit, and a world steps the same alone and in a batch.
 //
 // Coordinates are staged relative to an origin per item (the centre of the
-// stencil box where that keeps c - o exact, else 0), periodic shift folded in;
-// an unshifted displacement is then the reference's fl(c - h) bit for bit.
+// stencil box where that keeps c - o exact, else 0 or, in x, the box's right end), periodic shift folded in;
+// an unshifted displacement is then the reference's fl(c - h) bit for bit, and one across the box's face is rounded
+// at the scale of a few cells at most.
 //
 // Per unit, two phases:
 //   Filter: |c - h|^2 - B = |c|^2 + (|h|^2 - B) - 2 h.c for 32 homes x 8
@@ -46,8 +47,8 @@
 //   - a displacement is wrapped like the reference (subtract the extent where
 //     its test fires).  With at least 5 cells per axis that is exactly the
 //     stencil cells across the box edge: every staged range has one shift for every lane,
-//     added after the subtraction (exact path) as the reference does; an item that spans the
-//     box in x has its end cells' candidates twice, one period apart, and at most
+//     added after the subtraction (exact path) as the reference does; an item that reaches over the
+//     box in x has its last two cells' candidates twice, one period apart, and at most
 //     one of the two is within reach of a home.  With
 //     fewer cells both phases run the reference's tests per candidate;
 //   - force terms use rsqrt and exp approximations (a few ulp) and the
@@ -154,6 +155,27 @@ __device__ __forceinline__ void stencil_origin(int clo, int chi, float cs, float
         o = 0.0f;
         r = fmaxf(fabsf(lo), fabsf(hi)) + mg;
     }
+}
+
+// The origin in x and the radius of the box around it for an item of cells [x0, x1], and whether its list is folded.  A
+// candidate past the box's right end, staged as x plus the extent less the centre, would be rounded at the scale
+// of the item, the whole box in the end; items of a few cells leave it at that.  Others that lie in the right half take
+// the right end as their origin: what lies past it keeps its own x, and the rest is exact.  Else the item's homes of the last
+// cell are taken one period to the left, with the row's last two cells there too (both exact in the upper half of the
+// box) and the first cell as it is, all from the origin 0.  (Choosing between two homes per pair instead took
+// 64 worlds of 20,000 from 314 to 348 us and 1M in blobs from 520 to 549; this 318 and 519.)
+__device__ __forceinline__ bool stencil_origin_x(int x0, int x1, int mx, float cs, float ext, float& o, float& r)
+{
+    stencil_origin(x0 - 1, x1 + 1, cs, o, r);
+    if (x1 != mx - 1 || (o != 0.0f && x1 - x0 < 4)) return false;
+    if (o != 0.0f && 2 * (x0 - 1) > mx) {
+        o = ext;
+        r = cs * ((float)(mx - x0) + 1.05f);
+        return false;
+    }
+    o = 0.0f;
+    r = cs * ((float)mx + 0.05f);
+    return true;
 }
 
 constexpr int kSegs = 27;  // contiguous ranges of an item's candidates: 9 rows, up to three where a row wraps
@@ -280,8 +302,8 @@ __device__ __forceinline__ void copy_async_wait()
 // rounding of the threshold), on the unshifted coordinates h and o; p is the
 // staged candidate.
 template <bool kGeneric>
-__device__ __forceinline__ bool pair_exact(const StepConsts& c, const float4& h, const float* origin, const float4& p,
-                                           const float4& o, float thr)
+__device__ __forceinline__ bool pair_exact(const StepConsts& c, const float4& h, bool home_left, const float* origin,
+                                           const float4& p, const float4& o, float thr)
 {
     float ex = __fsub_rn(o.x, h.x), ey = __fsub_rn(o.y, h.y), ez = __fsub_rn(o.z, h.z);
     if (kGeneric) {
@@ -289,7 +311,7 @@ __device__ __forceinline__ bool pair_exact(const StepConsts& c, const float4& h,
         ey = wrap_ref(ey, c.ext[1], c.half[1]);
         ez = wrap_ref(ez, c.ext[2], c.half[2]);
     } else {
-        ex = __fadd_rn(ex, staged_shift(p.x + origin[0], o.x, c.ext[0]));
+        ex = __fadd_rn(ex, staged_shift(p.x + origin[0], o.x, c.ext[0]) + (home_left ? c.ext[0] : 0.0f));
         ey = __fadd_rn(ey, staged_shift(p.y + origin[1], o.y, c.ext[1]));
         ez = __fadd_rn(ez, staged_shift(p.z + origin[2], o.z, c.ext[2]));
     }
@@ -452,12 +474,15 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
     float sum_x = 0.0f, sum_y = 0.0f, sum_z = 0.0f;
     int sum_n = 0;
 
-    // the stencil's x cells: the item's and one each side.  On generic grids every cell once; else also
-    // those of an item that spans the box, whose end cells are then there twice, as they are and one
-    // period away: of a home and a candidate within reach of each other one copy is
+    // the stencil's x cells: the item's and one each side (on generic grids every cell once), or as stencil_origin_x
+    // folds them
     const bool ring = kGeneric && x1 - x0 + 3 >= mx;
     const int xlo = ring ? 0 : x0 - 1;
     const int xhi = ring ? mx - 1 : x1 + 1;  // inclusive
+    float ox = 0.0f, rx = 0.0f;
+    const bool folded = !kGeneric && stencil_origin_x(x0, x1, mx, c.cell[0], c.ext[0], ox, rx);
+    const bool home_left = folded && hx == mx - 1;  // (taken one period to the left)
+    const float home_x = home_left ? h.x - c.ext[0] : h.x;
 
     // segments: lane row + 9 part describes one contiguous range of the snapshot and
     // its periodic shift less the origin (zero on generic grids)
@@ -471,9 +496,18 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
         const int yy = yc + (row - dz * ny) - (ny > 1 ? 1 : 0), zz = zc + dz - (nz > 1 ? 1 : 0);
         const uint32_t cy = yy < 0 ? 1u : (yy >= my ? 2u : 0u);
         const uint32_t cz = zz < 0 ? 1u : (zz >= mz ? 2u : 0u);
-        // [xlo, xhi] in the box, left of it and right of it
-        const int xa = cx == 0u ? max(xlo, 0) : (cx == 1u ? xlo + mx : 0);
-        const int xb = cx == 0u ? min(xhi, mx - 1) : (cx == 1u ? (xlo < 0 ? mx - 1 : -1) : xhi - mx);
+        // [xlo, xhi] in the box, left of it and right of it; folded, the last two cells left of it, and the
+        // first one in the box if it is not there yet
+        int xa = cx == 0u ? max(xlo, 0) : (cx == 1u ? xlo + mx : 0);
+        int xb = cx == 0u ? min(xhi, mx - 1) : (cx == 1u ? (xlo < 0 ? mx - 1 : -1) : xhi - mx);
+        if (folded) {
+            if (cx == 1u) {
+                xa = mx - 2;
+                xb = mx - 1;
+            } else if (cx == 2u) {
+                xb = xlo > 0 ? 0 : -1;
+            }
+        }
         const uint32_t base = (uint32_t)it.world * (uint32_t)c.grid.cells_w +
                               (uint32_t)((wrap_index(zz, mz) * my + wrap_index(yy, my)) * mx);
         if (row < ny * nz && xb >= xa && CF_IN_BOUNDS(base + xb + 1, c.grid.cells + 1)) {
@@ -492,7 +526,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
             }
             if (!CF_IN_BOUNDS(seg_len, c.n + 1) || !CF_IN_BOUNDS(seg_beg + seg_len, c.n + 1)) seg_len = 0;
         }
-        shift = cx | cy << 2 | cz << 4;
+        shift = (folded && cx == 2u ? 0u : cx) | cy << 2 | cz << 4;
     }
 
     // Staging origin per axis (stencil_origin) for the stencil box (cells xlo..xhi,
@@ -504,11 +538,10 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
     // most the norm of (2^-10 r + 2^-22 box) over the axes.
     // The sums (products exact in 32 bits; |c|^2 and |h|^2 - B as two halves, 2^-22 each;
     // eight terms of at most 4 R^2 together) are off by less than 2^-16 R^2.
-    float ox = 0.0f, oy = 0.0f, oz = 0.0f, scale = 1.0f;
+    float oy = 0.0f, oz = 0.0f, scale = 1.0f;
     uint32_t a[4];
     if (!kGeneric) {
-        float rx, ry, rz;
-        stencil_origin(xlo, xhi, c.cell[0], ox, rx);
+        float ry, rz;
         stencil_origin(yc - 1, yc + 1, c.cell[1], oy, ry);
         stencil_origin(zc - 1, zc + 1, c.cell[2], oz, rz);
         const int e = (int)(__float_as_uint(fmaxf(rx, fmaxf(ry, rz))) >> 23);
@@ -522,7 +555,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
                     ez = fmaf(rz, 0x1p-10f, c.ext[2] * scale * 0x1p-22f);
         const float reach = sqrt_approx(fmaxf(thr_f, 0.0f)) * scale + sqrt_approx(fmaf(ez, ez, fmaf(ey, ey, ex * ex)));
         const float bnd = fmaf(reach * reach, 1.0f + 0x1p-16f, r2 * 0x1p-16f);
-        const uint32_t xy = half2_bits((h.x - ox) * scale, (h.y - oy) * scale);
+        const uint32_t xy = half2_bits((home_x - ox) * scale, (h.y - oy) * scale);
         const float qx = half_lo(xy), qy = half_hi(xy), qz = half_lo(half2_bits((h.z - oz) * scale, 0.0f));
         const float k = fmaf(qz, qz, fmaf(qy, qy, qx * qx)) - bnd;
         const float khi = half_lo(half2_bits(k, 0.0f));
@@ -547,8 +580,8 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
     }
     const int total = __shfl_sync(kAll, seg_pre, 31);
     seg_pre -= seg_len;
-    // the home's place in the list: its cell is in the centre row's in-box part
-    const int seg_c = (nz > 1 ? ny : 0) + (ny > 1 ? 1 : 0);
+    // the home's place in the list: its cell is in the centre row's in-box part, or left of it
+    const int seg_c = (nz > 1 ? ny : 0) + (ny > 1 ? 1 : 0) + (home_left ? 9 : 0);
     const int own = t - __shfl_sync(kAll, seg_beg - seg_pre, seg_c);
     // the list's segments without the empty ones
     const uint32_t full = __ballot_sync(kAll, seg_len > 0);
@@ -568,7 +601,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
     }
     __syncwarp();
     // the drain's coordinates: relative to the origin where some segment is shifted, raw elsewhere
-    const float hpx = shifted ? h.x - ox : h.x, hpy = shifted ? h.y - oy : h.y, hpz = shifted ? h.z - oz : h.z;
+    const float hpx = shifted ? home_x - ox : h.x, hpy = shifted ? h.y - oy : h.y, hpz = shifted ? h.z - oz : h.z;
 
     // units: the list's entries dealt out in turn (entry g to unit g mod units), so that every
     // unit holds an even share of every home's neighbours and its busiest lane stands out
@@ -790,7 +823,7 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
                         const float thr = kUniformR ? c.thr_uniform
                                                     : tables->threshold[type * kTableStride +
                                                                         (__float_as_uint(p.w) >> 2)];
-                        if (g < total && CF_IN_BOUNDS(j, c.n) && pair_exact<kGeneric>(c, h, origin, p, pos_sorted[j], thr)) {
+                        if (g < total && CF_IN_BOUNDS(j, c.n) && pair_exact<kGeneric>(c, h, home_left, origin, p, pos_sorted[j], thr)) {
                             count++;
                             fx = fmaf(k.dx, k.weight, fx);
                             fy = fmaf(k.dy, k.weight, fy);
@@ -865,14 +898,16 @@ __global__ void __launch_bounds__(256)
         const int ny = my > 1 ? 3 : 1, nz = mz > 1 ? 3 : 1;
         const bool ring = generic && x1 - x0 + 3 >= mx;
         const int xlo = ring ? 0 : x0 - 1, xhi = ring ? mx - 1 : x1 + 1;
+        float o, r;
+        const bool folded = !generic && stencil_origin_x(x0, x1, mx, c.cell[0], c.ext[0], o, r);
         for (int row = 0; row < ny * nz; row++) {
             const int dy_row = ny > 1 ? (row % ny) - 1 : 0, dz_row = nz > 1 ? (row / ny) - 1 : 0;
             const int yy = wrap_index(yc + dy_row, my), zz = wrap_index(zc + dz_row, mz);
             const uint32_t base = world_base + (uint32_t)((zz * my + yy) * mx);
             // in the box, left of it, right of it
             staged += cell_off[base + min(xhi, mx - 1) + 1] - cell_off[base + max(xlo, 0)];
-            if (xlo < 0) staged += cell_off[base + mx] - cell_off[base + xlo + mx];
-            if (xhi >= mx) staged += cell_off[base + xhi - mx + 1] - cell_off[base];
+            if (folded || xlo < 0) staged += cell_off[base + mx] - cell_off[base + (folded ? mx - 2 : xlo + mx)];
+            if (folded ? xlo > 0 : xhi >= mx) staged += cell_off[base + (folded ? 0 : xhi - mx) + 1] - cell_off[base];
         }
         tested = staged * (unsigned long long)it.count;
     }
