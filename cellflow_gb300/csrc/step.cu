@@ -207,17 +207,19 @@ __device__ __forceinline__ void item_barrier(int slot, int threads)
     }
 }
 
-// Two m16n8k8 products: 32 homes (fragments a[0..1] rows g and g + 8, a[2..3]
+// Two m16n8k8 products with 32-bit sums (with half-precision accumulators, 237 instead of 244 us a step for 64 worlds of
+// 20,000 and 491 instead of 510 for 1M, the instruction promises no more than half precision, 2^-11 of terms
+// several times the reach, and the bound below would not hold): 32 homes (fragments a[0..1] rows g and g + 8, a[2..3]
 // rows g + 16 and g + 24) against the 8 candidates of one fragment word b.
-// d[q]: row g + 8 q against columns 2 t (low half) and 2 t + 1 (high half).
-__device__ __forceinline__ void mma_32x8(const uint32_t (&a)[4], uint32_t b, uint32_t (&d)[4])
+// d[2 q + j]: row g + 8 q against column 2 t + j.
+__device__ __forceinline__ void mma_32x8(const uint32_t (&a)[4], uint32_t b, uint32_t (&d)[8])
 {
-    asm("mma.sync.aligned.m16n8k8.row.col.f16.f16.f16.f16 {%0, %1}, {%2, %3}, {%4}, {%5, %5};"
-        : "=r"(d[0]), "=r"(d[1])
-        : "r"(a[0]), "r"(a[1]), "r"(b), "r"(0u));
-    asm("mma.sync.aligned.m16n8k8.row.col.f16.f16.f16.f16 {%0, %1}, {%2, %3}, {%4}, {%5, %5};"
-        : "=r"(d[2]), "=r"(d[3])
-        : "r"(a[2]), "r"(a[3]), "r"(b), "r"(0u));
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(b), "f"(0.0f));
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%7, %7, %7, %7};"
+        : "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7])
+        : "r"(a[2]), "r"(a[3]), "r"(b), "f"(0.0f));
 }
 
 // Quotient and remainder of x by units, x at most kUnit * units (so that the
@@ -715,17 +717,23 @@ __global__ void __launch_bounds__(32 * kBlockWarps, kMinBlocks)
                     const uint4 b = *reinterpret_cast<const uint4*>(
                         w.row[1 + gi] + min(lane & 3, 2) * 32 + (lane >> 2) * 4);
                     const uint32_t bn[4] = {b.x, b.y, b.z, b.w};
-                    uint32_t d[4][4];
+                    // row q's eight sign bits: the top halves of its results two to a word, the top bytes of those
+                    // side by side in two words, the second shifted by four, so bit 3 of every nibble is a sign
+                    uint32_t r[4], lo[4];
 #pragma unroll
-                    for (int n = 0; n < 4; n++) mma_32x8(a, bn[n], d[n]);
-                    // row q's eight sign bits: the top bytes of its four words' halves side by side in
-                    // two words, the second shifted by four, so bit 3 of every nibble is a sign
-                    uint32_t r[4];
+                    for (int f = 0; f < 2; f++) {
+                        uint32_t d[2][8];
+                        mma_32x8(a, bn[2 * f], d[0]);
+                        mma_32x8(a, bn[2 * f + 1], d[1]);
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const uint32_t lo = __byte_perm(d[0][q], d[1][q], 0x7531),
-                                       hi = __byte_perm(d[2][q], d[3][q], 0x7531);
-                        r[q] = bit_select(lo, hi >> 4, 0x80808080u);
+                        for (int q = 0; q < 4; q++) {
+                            const uint32_t w = __byte_perm(__byte_perm(d[0][2 * q], d[0][2 * q + 1], 0x7632),
+                                                           __byte_perm(d[1][2 * q], d[1][2 * q + 1], 0x7632), 0x7531);
+                            if (f == 0)
+                                lo[q] = w;
+                            else
+                                r[q] = bit_select(lo[q], w >> 4, 0x80808080u);
+                        }
                     }
                     // the four rows' signs into one word, row q at bit 3 - q of every nibble; then a
                     // 4 x 4 transposition of the nibbles' bits over the quad leaves in lane 4 g + t the
