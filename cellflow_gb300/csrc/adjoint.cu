@@ -34,9 +34,6 @@
 #include "cf_internal.hpp"
 
 namespace cf {
-namespace {
-
-constexpr int kAdjThreads = 128;
 
 // Streaming multiprocessors of the current device (queried once; a query,
 // so also legal while a stream is being captured).
@@ -53,6 +50,10 @@ int num_sms()
     }
     return sms;
 }
+
+namespace {
+
+constexpr int kAdjThreads = 128;
 
 __device__ __forceinline__ float wrap_ref(float d, float ext, float half)
 {

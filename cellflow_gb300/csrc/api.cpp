@@ -238,7 +238,6 @@ void free_particles(cf_world* w)
     dev_free(s.out_idx);
     dev_free(s.counters);
     dev_free(s.cell_pop);
-    dev_free(s.row_count);
     dev_free(s.items);
     dev_free(s.n_items);
     free_offsets(s);
@@ -302,28 +301,22 @@ int ensure_before_list(cf_world* w, Ensure ensure)
     return ensure();
 }
 
-// Buffers of the force kernel's plan for this grid: per-row populations and
-// the item list (at most n/32 + rows items).
+// The force kernel's item list for this grid (at most n/32 + rows items).
 int ensure_plan(cf_world* w, const Grid& g)
 {
     Scratch& s = w->s;
-    const size_t rows = (size_t)g.m[1] * g.m[2];
     const size_t items = (size_t)max_step_items(w->n, g);
-    if (rows <= s.rows_cap && items <= s.items_cap && s.n_items) return CF_OK;
+    if (items <= s.items_cap && s.n_items) return CF_OK;
     return ensure_before_list(w, [&]() -> int {
         CF_CUDA(cudaStreamSynchronize(w->stream));
         drop_graphs(w);
-        dev_free(s.row_count);
         dev_free(s.items);
         dev_free(s.n_items);
-        s.row_count = nullptr;
         s.items = nullptr;
         s.n_items = nullptr;
-        s.rows_cap = s.items_cap = 0;
-        CF_CUDA(dev_alloc(&s.row_count, rows));
+        s.items_cap = 0;
         CF_CUDA(dev_alloc(&s.items, items));
         CF_CUDA(dev_alloc(&s.n_items, 1));
-        s.rows_cap = rows;
         s.items_cap = items;
         return CF_OK;
     });

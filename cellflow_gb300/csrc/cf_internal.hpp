@@ -118,7 +118,7 @@ struct Grid {
     int worlds;       // independent worlds sharing the grid (1 for a plain world; the types with by_type)
     int by_type;      // 1: the particles' types take the place of the worlds (one world's proximity selections)
     int cells_w;      // cells per world: m0 * m1 * m2
-    int bin_shift;    // offsets are kept per 2^bin_shift cells of a row (0: per cell; bin_rows)
+    int bin_shift;    // offsets are kept per 2^bin_shift cells of a row (0: per cell; row_bins)
 };
 
 // Bits of a particle index in a bin's entry (place_kernel); the bits above hold the cell's place in
@@ -190,7 +190,6 @@ struct Scratch {
     size_t hist_cap = 0;            // entries
     uint32_t* cell_start = nullptr;
     uint32_t* cell_end = nullptr;
-    size_t cells_cap = 0;
     float4* pos_sorted = nullptr;
     int n_cap = 0;
     // proximity
@@ -211,9 +210,6 @@ struct Scratch {
     // CSR cell offsets of the step (cells + 1 entries)
     uint32_t* cell_off = nullptr;
     size_t off_cap = 0;
-    // force-kernel plan: per-row populations and the row-aligned 32-particle items
-    uint32_t* row_count = nullptr;
-    size_t rows_cap = 0;
     Item* items = nullptr;       // row-aligned items of the force kernel
     size_t items_cap = 0;
     int* n_items = nullptr;
@@ -434,6 +430,7 @@ cudaError_t launch_force_work(const StepConsts& c, const uint32_t* keys_sorted, 
                               cudaStream_t st);
 cudaError_t launch_step_plan(const uint32_t* cell_off, int n, const Grid& g, Item* items, int* n_items,
                              cudaStream_t st);
+int num_sms();  // streaming multiprocessors of the current device
 int default_force_variant(int n, const Grid& g);
 int max_step_items(int n, const Grid& g);
 int step_launches(int n);

@@ -126,7 +126,6 @@ extern "C" int cf_proximity_edges_noalloc(const void* d_pos4, int n, float width
     s.scan_tmp_cap = kScanEntries;
     s.cell_start = reinterpret_cast<uint32_t*>(base + kOffStart);
     s.cell_end = reinterpret_cast<uint32_t*>(base + kOffEnd);
-    s.cells_cap = kNoAllocMaxCells;
     s.n_cap = kNoAllocMaxParticles;
     int* err = reinterpret_cast<int*>(base + kOffErr);
     if (radix_hist_entries(n) > s.hist_cap || scan_tmp_entries(n + 1) > s.scan_tmp_cap ||

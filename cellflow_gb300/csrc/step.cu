@@ -1058,7 +1058,6 @@ namespace {
 // 1.17M particles in 64 worlds: 304 against 321 us; 300k: equal; 100k: 45.9 against 44.3 (the
 // launch).
 constexpr int kIntegrateApart = 500000;
-constexpr int kSms = 152;
 }
 
 int max_step_items(int n, const Grid& g) { return (n + 31) / 32 + g.worlds * g.m[1] * g.m[2]; }
@@ -1080,12 +1079,12 @@ int default_force_variant(int n, const Grid& g)
     const double homes = std::min(32.0, std::max(pop * g.m[0], 1.0));
     const double candidates = 9.0 * pop * std::min((double)g.m[0], homes / pop + 3.0);
     const double items = n / 32.0 + 0.5 * std::min(cells / g.m[0], (double)n);
-    const double slots = 24.0 * kSms;
+    const double slots = 24.0 * num_sms();
     int split = 1;
     if (candidates >= 0.5 * kUnit)
         while (split < 8 && 2 * split * (n / 32.0) <= slots && split < 2.0 * std::ceil(candidates / kUnit)) split *= 2;
     const double warps = items * split;
-    const int occupancy = warps <= 16.0 * kSms ? 2 : warps <= 20.0 * kSms ? 1 : 0;
+    const int occupancy = warps <= 16.0 * num_sms() ? 2 : warps <= 20.0 * num_sms() ? 1 : 0;
     int log2 = 0;
     while ((1 << log2) < split) log2++;
     return occupancy + kForceOccupancies * log2;
