@@ -1054,10 +1054,12 @@ cudaError_t launch_force_work(const StepConsts& c, const uint32_t* keys_sorted, 
 
 namespace {
 // From this many particles the integrator is a kernel of its own, in particle order: the
-// force kernel's scattered access to a particle's state (six sectors) shrinks to one store.
-// 1.17M particles in 64 worlds: 304 against 321 us; 300k: equal; 100k: 45.9 against 44.3 (the
-// launch).
-constexpr int kIntegrateApart = 500000;
+// force kernel's scattered access to a particle's state (six sectors) shrinks to one store.  Apart / in the force kernel,
+// us a step (evenly spread with many and with few neighbours, in blobs, 64 worlds): 20,000 27.1 / 27.4, 27.0 / 27.5,
+// 29.3 / 31.2, 29.1 / 29.2; 70,000 41.4 / 43.5, 33.5 / 35.8, 64.0 / 62.0, 34.2 / 37.5; 100,000 59.9 / 59.8,
+// 41.6 / 44.8, 84.5 / 84.8, 39.5 / 43.3; 300,000 74 / 77, 68 / 72, 94 / 103, 76 / 93; 1M 253 / 261, 185 / 197, 320 / 340,
+// 225 / 255; below 10,000 up to 2.2 more for the launch.  From 100,000 it costs nothing anywhere.
+constexpr int kIntegrateApart = 100000;
 }
 
 int max_step_items(int n, const Grid& g) { return (n + 31) / 32 + g.worlds * g.m[1] * g.m[2]; }

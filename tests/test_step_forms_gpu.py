@@ -182,3 +182,26 @@ def test_records_of_different_grids_in_turn(cflib):
         assert step(fresh, radius) == got, radius
         fresh.close()
     one.close()
+
+
+@pytest.mark.parametrize("sizes", [[60000, 39999], [60000, 40000]])
+def test_integrator_apart_from_its_line_on(cflib, sizes):
+    """From 100,000 particles the integrator is a kernel of its own: a batch of as many gives the bits of its worlds
+    alone, which are below."""
+    parts = []
+    for k, n in enumerate(sizes):
+        params, types, table = parameters(n, 0.08, 0.0)
+        parts.append((inputs.uniform_positions(n, 5 + k), types, table))
+    batch = Batch(sizes, T, 2.0, 2.0, 2.0, seed=1)
+    batch.set_particles(np.concatenate([p[0] for p in parts]), np.concatenate([p[1] for p in parts]))
+    batch.set_force_tables(np.stack([p[2] for p in parts]))
+    batch.simulate(params, 2)
+    got, off = batch.get_state(), batch.offsets
+    batch.close()
+    for k, (pos, types, table) in enumerate(parts):
+        sim = make_world(sizes[k], table, np.zeros(T, np.float32))
+        sim.set_particles(pos, types)
+        sim.simulate(params, 2)
+        for x, y in zip(got, sim.get_state()):
+            assert np.array_equal(x[off[k]:off[k + 1]], y), k
+        sim.close()
