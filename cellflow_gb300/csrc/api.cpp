@@ -909,13 +909,12 @@ Grid choose_type_grid(const float* ext, float distance, int types, int per_type)
     return g;
 }
 
-// Its cells per type where memory allows: eight per particle over all types, twice that for a single one (whose list has the
-// most candidates: 100,000 particles in blobs, a distance of 1/200 of the box, 85 us with eight, 75 with sixteen; evenly
-// spread 26.9 and 27.3; with three types 70 and 61, but 25.4 and 25.8, 48.2 and 50.9 at 300,000), and half a million over
-// the types in small worlds.
+// Its cells per type where memory allows: eight per particle over all types; for a single type, whose list has the
+// most candidates, sixteen and at least half a million (100,000 particles in blobs, a distance of 1/200 of the box, 85 us
+// with eight, 75 with sixteen; evenly spread 26.9 and 27.3; with three types 70 and 61, but evenly spread 300,000 48 and 51).
 int type_grid_cells(int types, int n)
 {
-    const long long most = std::max((types == 1 ? 16ll : (types == 2 ? 12ll : 8ll)) * n, (1ll << 19) / types);
+    const long long most = types == 1 ? std::max(16ll * n, 1ll << 19) : std::max(8ll * n, 32768ll);
     return (int)std::max(1ll, std::min<long long>(kMaxCells, most) / types);
 }
 
