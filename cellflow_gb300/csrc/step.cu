@@ -1057,9 +1057,11 @@ namespace {
 // force kernel's scattered access to a particle's state (six sectors) shrinks to one store.  Apart / in the force kernel,
 // us a step (evenly spread with many and with few neighbours, in blobs, 64 worlds): 20,000 27.1 / 27.4, 27.0 / 27.5,
 // 29.3 / 31.2, 29.1 / 29.2; 70,000 41.4 / 43.5, 33.5 / 35.8, 64.0 / 62.0, 34.2 / 37.5; 100,000 59.9 / 59.8,
-// 41.6 / 44.8, 84.5 / 84.8, 39.5 / 43.3; 300,000 74 / 77, 68 / 72, 94 / 103, 76 / 93; 1M 253 / 261, 185 / 197, 320 / 340,
-// 225 / 255; below 10,000 up to 2.2 more for the launch.  From 100,000 it costs nothing anywhere.
-constexpr int kIntegrateApart = 100000;
+// 41.6 / 44.8, 84.5 / 84.8, 39.5 / 43.3; 150,000 90.6 / 89.6, 47.0 / 52.1, 136.5 / 137.3, 49.8 / 54.0; 300,000 74 / 77,
+// 68 / 72, 94 / 103, 76 / 93; 1M 253 / 261, 185 / 197, 320 / 340, 225 / 255; below 10,000 up to 2.2 more for the launch.  Worlds
+// whose particles have clustered over many steps gain less (100,000 after 25 to 100 steps, launches outside a graph:
+// 63.5 / 62.4 and 72.6 / 70.8).  From 150,000 it costs 1 % at most.
+constexpr int kIntegrateApart = 150000;
 }
 
 int max_step_items(int n, const Grid& g) { return (n + 31) / 32 + g.worlds * g.m[1] * g.m[2]; }

@@ -184,9 +184,9 @@ def test_records_of_different_grids_in_turn(cflib):
     one.close()
 
 
-@pytest.mark.parametrize("sizes", [[60000, 39999], [60000, 40000]])
+@pytest.mark.parametrize("sizes", [[90000, 59999], [90000, 60000]])
 def test_integrator_apart_from_its_line_on(cflib, sizes):
-    """From 100,000 particles the integrator is a kernel of its own: a batch of as many gives the bits of its worlds
+    """From 150,000 particles the integrator is a kernel of its own: a batch of as many gives the bits of its worlds
     alone, which are below."""
     parts = []
     for k, n in enumerate(sizes):
