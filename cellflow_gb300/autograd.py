@@ -20,6 +20,13 @@ from ._lib import GRAD_PARAMS, check, load
 from .world import ParticleSimulation, SimulationParams
 
 
+def _current_stream() -> int:
+    """The caller's current stream as a handle.  torch.cuda.current_stream() builds a Stream object in about 15 us;
+    where this torch has the call that gives the bare handle (which is not public), that one."""
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(torch.cuda.current_device()) if raw else torch.cuda.current_stream().cuda_stream
+
+
 class _Ordered:
     """Runs a block's library calls between the caller's current torch stream's earlier and
     later work: the world's stream waits for the caller's on entry and the caller's for the
@@ -27,8 +34,7 @@ class _Ordered:
 
     def __init__(self, sim: ParticleSimulation):
         self.sim = sim
-        # (the raw handle; torch.cuda.current_stream() builds a Stream object in about 15 us)
-        self.stream = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+        self.stream = _current_stream()
 
     def __enter__(self):
         check(load().cf_stream_wait(self.sim.handle, self.stream), "cf_stream_wait")

@@ -53,3 +53,9 @@ def test_a_failed_signal_is_raised_after_a_good_block(block):
         with o:
             pass
     assert lib.calls == ["wait", "signal"]
+
+
+def test_the_public_stream_call_is_enough(monkeypatch):
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: type("Stream", (), {"cuda_stream": 17})())
+    assert autograd._current_stream() == 17
