@@ -55,18 +55,19 @@
 //     contracted distance.
 //   The density factor, integrator and wrap are the reference's operations.
 //
-// What bounds it: instruction issue (55 to 70 % of the slots used) and, in the
-// drain, latency and shared-memory bank conflicts at scattered slots.  Counted
-// at 100k evenly spread particles (3,340 items of 18 groups and 28 trips): about
-// 820 instructions for an item's start and end, 97 to stage and 67 to filter a
-// group of 32 candidates, 90 per trip of two pairs (three since: 532 to 521 us for
-// the step at 1M, 318 to 315 at 64 worlds of 20,000).  What brought the step there,
+// What bounds it: instruction issue (42 to 62 % of the slots used) and, in the
+// drain, latency and shared-memory bank conflicts at scattered slots.  Counted with two pairs
+// a trip and half-precision sums in the filter, at 100k evenly spread particles (3,340 items of 18 groups and 28 trips):
+// about 820 instructions for an item's start and end, 97 to stage and 67 to filter a
+// group of 32 candidates, 90 per trip.  Three pairs a trip since (532 to 521 us for the step at 1M in
+// blobs, 318 to 315 at 64 worlds of 20,000), and the filter's sums in 32 bits (21.1 to 22.3 million warp instructions
+// at 100k, 63.4 to 64.2 us; 519 to 535 at 1M, 318 to 326 at the worlds).  What brought the step there,
 // against one 32-bit lane per home filtering and draining stretches of the list
 // (force kernel, 100k and 1M in blobs): units dealt out entry by entry instead
 // of in stretches (28 trips per item instead of 37), band pairs put off to the end
 // of the unit instead of an exact test in the trip (61 instructions per trip),
 // predicated bit walking, all of a unit's positions in flight at once, the
-// tensor-core filter: 62 to 39 us and 737 to 469 us.  One list for an item that spans the box
+// tensor-core filter: 62 to 39 us and 737 to 469 us.  One list for an item that reaches over the box
 // in x, end cells twice, instead of a second pass for its last cells (and the loop and
 // registers that took): 264 to 240 us for 64 worlds of 20,000, 469 to 459 at 1M.  An application
 // world of 10,000 particles with ~125 neighbours each (313 items): 276 to 32 us with
@@ -883,7 +884,7 @@ __global__ void __launch_bounds__(256)
               state.acc, state.counts_out);
 }
 
-// The filter's work of one step, from the cell list alone: per item and pass
+// The filter's work of one step, from the cell list alone: per item
 // the candidates staged (the union of its homes' stencils, as the force
 // kernel concatenates them) and the tests of them by the item's particles.
 // One thread per item; out[0] += staged, out[1] += staged * particles.
