@@ -115,7 +115,10 @@ long long cf_kernel_launches(void);
 /* Cap on the device memory the library itself holds (every buffer of every
  * world and batch), in bytes; 0 removes the cap.  An allocation that would
  * exceed it fails as cudaMalloc out of memory would: CF_ERR_ALLOC, with the
- * cap named in cf_last_error().  Lowering it frees nothing already held. */
+ * cap named in cf_last_error().  Lowering it frees nothing already held.
+ * Where memory is short, by this cap or the device's, the cell lists of the
+ * edge list and the mesh take coarser cells (the same results, slower) and
+ * give way to the buffers of other calls before a call fails. */
 int cf_set_device_memory_limit(size_t bytes);
 /* Device memory the library holds now, in bytes. */
 int cf_device_memory_in_use(size_t* bytes);
@@ -441,7 +444,9 @@ int cf_rollout_backward_xyz(cf_world* w, const float* d_gpos, const float* d_gve
  * world's current ones): bins of width D = r_max / bins, cubic B-spline
  * weights of support 2 bins each side of the centre (k + 1/2) D, each entry
  * normalised by N_a (N_b / V) 4 pi c_k^2 D.  d_hist receives T * T * bins
- * floats [a][b][k] (device).  T * T * bins <= 49152. */
+ * floats [a][b][k] (device).  T * T * bins <= 49152.  After a first call of
+ * the same sizes (which allocates) this and the gradient can be recorded by a
+ * stream capture of the caller's. */
 int cf_rdf(cf_world* w, const float* d_pos4, int bins, float r_max, float* d_hist);
 /* dL/dpos (device, n float4) of L(hist) given d_ghist = dL/dhist (device). */
 int cf_rdf_backward(cf_world* w, const float* d_pos4, int bins, float r_max, const float* d_ghist, float* d_gpos4);
